@@ -58,6 +58,7 @@ struct LLDispatchArgs {
   int* expert_counts;          // [L]
   int* expert_offsets;         // [L + 1]
   int* num_rows;               // [1] device copy of the row count
+  int* local_row;              // [T][K] output row of every slot whose expert lives on this rank, -1 otherwise (read by the combine)
   int* mailbox;                // mapped host memory (may be null): [0] rows, [3] epoch, [4..] counts
   long long capacity;          // rows available in recv_x
 };
@@ -69,6 +70,7 @@ struct LLCombineArgs {
   const __nv_bfloat16* x;      // [rows][H] expert outputs
   const int* recv_row_src;     // [rows]
   const int* num_rows;         // [1]
+  const int* local_row;        // [T][K] row in x of every slot whose expert lives on this rank (LLDispatchArgs::local_row)
   const long long* topk_idx;   // [T][K] of this rank's tokens
   const float* topk_w;         // [T][K] weights applied here, at the source
   int T, E;

@@ -11,6 +11,14 @@
 // a fixed (token, slot) slot at its source; the source waits per part and computes
 // sum_k w_k * row_k in slot order in fp32.
 //
+// What stays on the rank takes neither detour: its tokens are routed from the caller's table, its rows go
+// from the caller's tensor straight into the output rows (quantised on the way, cut into as many pieces as
+// there are warps), and the combine reads the rows of its own experts where they lie, through the row of
+// every (token, slot) that the dispatch leaves behind.  What bounds both kernels is the chain of dependent
+// steps, not bytes: on one GPU a captured round (hidden 7168, 256 experts, top-8, fp8) took 37.9 us for one
+// token while own rows went through flags and the staging area and one thread scanned the experts, 20.1 us
+// since; 93 bf16 tokens of 4096 (64 experts, top-6) 40.4 and 20.4 us.
+//
 // Re-entrancy: epochs live in device memory and select one of two banks, flags hold epochs and
 // are never cleared, a bank is reused only after the peers acknowledged the call before last.
 // Nothing depends on host state, so both kernels can be captured in a CUDA graph.
@@ -62,11 +70,6 @@ __device__ __forceinline__ int below8(const unsigned* m, int t) {
   for (int i = 0; i < w; ++i) n += __popc(m[i]);
   return n + __popc(m[w] & ((1u << (t & 31)) - 1u));
 }
-__device__ __forceinline__ int popc8(const unsigned* m) {
-  int n = 0;
-  for (int i = 0; i < kLLWords; ++i) n += __popc(m[i]);
-  return n;
-}
 __device__ __forceinline__ bool counts_ll(const int* row, int k, int E) {
   int e = row[k];
   if (e < 0 || e >= E) return false;
@@ -76,6 +79,39 @@ __device__ __forceinline__ bool counts_ll(const int* row, int k, int E) {
 }
 
 // ------------------------------------------------------------------------------------------ dispatch
+// One 16-byte piece (8 bf16 values) -> 8 e4m3 codes and the fp32 scale of its group of 128 values, which 16 consecutive
+// lanes hold together (a step of a warp covers two groups).  Lanes past the end pass zeros.
+__device__ __forceinline__ uint2 quant8(const int4& v, float& scale) {
+  float f[8];
+  const __nv_bfloat162* hh = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) { f[2 * q] = __low2float(hh[q]); f[2 * q + 1] = __high2float(hh[q]); }
+  float amax = 0.f;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) amax = fmaxf(amax, fabsf(f[q]));
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  amax = fmaxf(amax, 1e-4f);
+  const float inv = __frcp_rn(amax) * 448.0f;   // torch evaluates `448 / amax` (scalar / tensor) as reciprocal, then multiply
+  uint32_t q2[2] = {0u, 0u};
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    q2[q >> 2] |= (uint32_t)__nv_cvt_float_to_fp8(f[q] * inv, __NV_SATFINITE, __NV_E4M3) << (8 * (q & 3));
+  scale = amax / 448.0f;
+  return make_uint2(q2[0], q2[1]);
+}
+
+// Column range of piece `p` of `n` equal pieces of a row, in groups of 128 values (the last group may be short).
+__device__ __forceinline__ LLPart ll_piece(int H, int p, int n) {
+  const int nblk = (H + 127) / 128, bpp = (nblk + n - 1) / n;
+  LLPart r;
+  r.b0 = min(nblk, p * bpp); r.b1 = min(nblk, (p + 1) * bpp);
+  r.v0 = min(H, r.b0 * 128); r.v1 = min(H, r.b1 * 128);
+  return r;
+}
+
+constexpr int kOwnUnroll = 4;   // 16-byte pieces per lane of an own row that are read ahead of the layout
+
 template <bool kProfile>
 __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid_constant__ LLDispatchParams p) {
   const LLDispatchArgs& a = p.r[blockIdx.y];
@@ -90,15 +126,14 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
   const LLLayout ll = make_ll_layout(P, M, K, H);
   const long long bank_off = lay.ll + (long long)(epoch & 1) * ll.bank_bytes;
   const bool fp8 = a.mode != 0;
-  const int nsf = H / 128, row_bytes = fp8 ? H : H * 2;
+  const int nsf = H / 128, row_bytes = fp8 ? H : H * 2, src_bytes = a.mode == 1 ? H : H * 2;
 
   __shared__ unsigned s_emask[kMaxExperts][kLLWords];   // [(source, local expert)] -> tokens
   __shared__ unsigned s_hit[kMaxRanks][kLLWords];       // tokens of source r that reach this rank
   __shared__ unsigned s_own[kMaxRanks][kLLWords];       // my tokens that reach rank d
   __shared__ int s_off[kMaxExperts];                    // first output row of (source, local expert)
-  __shared__ int s_tot[kMaxExperts];
+  __shared__ int s_warp_rows[kLLThreads / 32];          // rows of the experts that each layout warp scans
   __shared__ int s_T[kMaxRanks];
-  __shared__ int s_rows;
   __shared__ int s_fail;                                // a wait of the layout warps ran out
 
   // profile instantiation only: phase stamps (nanoseconds since kernel start) of block 0 in Control::dbg[0..7]; the
@@ -114,15 +149,30 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
   auto layout_sync = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(LT) : "memory"); };
   if (threadIdx.x == 0) s_fail = 0;
 
-  // ---- bank reuse: the call before last must have been consumed everywhere
+  // ---- everything that needs no peer starts at once: this warp's first piece of an own row is read ahead, the masks are cleared
+  const int nblk = (H + 127) / 128;
+  const int pieces = max(1, min(nblk, total_warps / max(a.T, 1)));      // pieces of an own row
+  int4 ahead[kOwnUnroll];
+  LLPart own_pr = {0, 0, 0, 0};
+  if (gw < a.T * pieces) {
+    own_pr = ll_piece(H, gw % pieces, pieces);
+    const int lo = (a.mode == 1 ? own_pr.v0 : own_pr.v0 * 2) / 16, hi = (a.mode == 1 ? own_pr.v1 : own_pr.v1 * 2) / 16;
+    const int4* src = reinterpret_cast<const int4*>(reinterpret_cast<const uint8_t*>(a.x) + (size_t)(gw / pieces) * src_bytes);
+#pragma unroll
+    for (int i = 0; i < kOwnUnroll; ++i) {
+      const int u = lo + i * 32 + lane;
+      ahead[i] = u < hi ? __ldg(src + u) : make_int4(0, 0, 0, 0);
+    }
+  }
+  for (int i = threadIdx.x; i < E * kLLWords; i += kLLThreads) (&s_emask[0][0])[i] = 0u;
+  for (int i = threadIdx.x; i < kMaxRanks * kLLWords; i += kLLThreads) { (&s_own[0][0])[i] = 0u; (&s_hit[0][0])[i] = 0u; }
+  // ---- bank reuse: the call before last must have been consumed by the peers (this rank's own calls are ordered)
   int ok = 1;
-  if (threadIdx.x < P && epoch > 2)
+  if (threadIdx.x < P && threadIdx.x != me && epoch > 2)
     ok = wait_flag_ge(&ctl->ll_disp_ack[threadIdx.x], epoch - 2, ctx, kOpLLDispatch, 0, threadIdx.x);
   int alive = __syncthreads_and(ok);
 
-  // ---- my own routing: which destinations does each token reach
-  for (int i = threadIdx.x; i < kMaxRanks * kLLWords; i += kLLThreads) (&s_own[0][0])[i] = 0u;
-  __syncthreads();
+  // ---- my own routing: which ranks does each token reach, and which experts of this rank
   for (int t = threadIdx.x; t < a.T; t += kLLThreads) {   // one thread per token: K independent loads, dedup in registers
     int row[kMaxTopk];
 #pragma unroll
@@ -132,19 +182,23 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
     }
 #pragma unroll
     for (int k = 0; k < kMaxTopk; ++k)
-      if (k < K && counts_ll(row, k, E)) atomicOr(&s_own[row[k] / Lx][t >> 5], 1u << (t & 31));
+      if (k < K && counts_ll(row, k, E)) {
+        const int d = row[k] / Lx;
+        atomicOr(&s_own[d][t >> 5], 1u << (t & 31));
+        if (d == me) atomicOr(&s_emask[me * Lx + (row[k] - me * Lx)][t >> 5], 1u << (t & 31));
+      }
   }
   __syncthreads();
 
   stamp(0);
   if (alive) {
-    // ---- routing table: block b writes it to peer (me + b) % P (16-byte stores when the table allows), so all peers are
+    // ---- routing table: block b writes it to peer (me + 1 + b) % P (16-byte stores when the table allows), so all peers are
     // served at once and the table leaves in a couple of microseconds; rows to their destinations (all warps)
     {
       const int n = a.T * K;
       const bool vec = ((M * K) & 3) == 0 && (reinterpret_cast<uintptr_t>(a.topk_idx) & 15) == 0 &&
                        (!a.topk_w || (reinterpret_cast<uintptr_t>(a.topk_w) & 15) == 0);
-      for (int s = blockIdx.x; s < P; s += gridDim.x) {
+      for (int s = blockIdx.x + 1; s < P; s += gridDim.x) {
         const int d = (me + s) % P;
         uint8_t* base = ctx.ws[d] + bank_off;
         int* gi = reinterpret_cast<int*>(base + ll.gather_idx) + (size_t)me * M * K;
@@ -174,11 +228,11 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
     uint8_t* mine = ctx.ws[me] + bank_off;
     const int* gidx = reinterpret_cast<const int*>(mine + ll.gather_idx);
     if (warp < kLLSendWarps) {
-    // ================================================================ sending warps: every row part to its destination
+    // ================================================================ sending warps: every row part to its remote destinations
     PendingFlags pending;
-    for (int item = warp * gridDim.x + blockIdx.x; item < a.T * P * kLLParts; item += gridDim.x * kLLSendWarps) {
+    for (int item = warp * gridDim.x + blockIdx.x; item < a.T * (P - 1) * kLLParts; item += gridDim.x * kLLSendWarps) {
       const int part = item % kLLParts, td = item / kLLParts;
-      const int t = td / P, d = (me + td % P) % P;
+      const int t = td / (P - 1), d = (me + 1 + td % (P - 1)) % P;
       if (!((s_own[d][t >> 5] >> (t & 31)) & 1u)) continue;
       const LLPart pr = ll_part(H, part);
       if (pr.v0 >= pr.v1) continue;
@@ -186,7 +240,6 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
       uint8_t* base = ctx.ws[d] + bank_off;
       uint8_t* dst = base + ll.stage + ((size_t)me * M + j) * ll.msg_bytes;
       if (a.mode == 2) {  // bf16 -> e4m3 with one fp32 scale per 128 values, straight into the peer
-        // a lane owns 8 consecutive values (16 B); 16 lanes cover one 128-value group, a warp step covers two groups
         const int4* src = reinterpret_cast<const int4*>(reinterpret_cast<const uint8_t*>(a.x) + (size_t)t * H * 2);
         const int u_lo = pr.v0 / 8, u_hi = pr.v1 / 8, half = lane >> 4;
         constexpr int U = 8;
@@ -195,31 +248,17 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
 #pragma unroll
           for (int i = 0; i < U; ++i) {
             const int u = u0 + i * 32 + lane;
-            if (u < u_hi) v[i] = __ldg(src + u);
+            v[i] = u < u_hi ? __ldg(src + u) : make_int4(0, 0, 0, 0);
           }
 #pragma unroll
           for (int i = 0; i < U; ++i) {
             const int u = u0 + i * 32 + lane;
             if (u0 + i * 32 >= u_hi) break;           // warp-uniform
-            float f[8];
-            if (u >= u_hi) v[i] = make_int4(0, 0, 0, 0);   // groups are whole, so a step is all-or-nothing per half warp
-            const __nv_bfloat162* hh = reinterpret_cast<const __nv_bfloat162*>(&v[i]);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) { f[2 * q] = __low2float(hh[q]); f[2 * q + 1] = __high2float(hh[q]); }
-            float amax = 0.f;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) amax = fmaxf(amax, fabsf(f[q]));
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-            amax = fmaxf(amax, 1e-4f);
-            const float inv = __frcp_rn(amax) * 448.0f;   // torch evaluates `448 / amax` (scalar / tensor) as reciprocal, then multiply
-            uint32_t q2[2] = {0u, 0u};
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-              q2[q >> 2] |= (uint32_t)__nv_cvt_float_to_fp8(f[q] * inv, __NV_SATFINITE, __NV_E4M3) << (8 * (q & 3));
+            float scale;
+            const uint2 q = quant8(v[i], scale);      // groups are whole, so a step is all-or-nothing per half warp
             if (u < u_hi) {
-              *reinterpret_cast<uint2*>(dst + (size_t)u * 8) = make_uint2(q2[0], q2[1]);
-              if ((lane & 15) == 0) reinterpret_cast<float*>(dst + H)[(u0 + i * 32) / 16 + half] = amax / 448.0f;
+              *reinterpret_cast<uint2*>(dst + (size_t)u * 8) = q;
+              if ((lane & 15) == 0) reinterpret_cast<float*>(dst + H)[(u0 + i * 32) / 16 + half] = scale;
             }
           }
         }
@@ -237,29 +276,29 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
     pending.publish(epoch, lane);
     stamp(1);
     } else {
-    // ================================================================ layout warps: wait for all routing tables, derive the layout
+    // ================================================================ layout warps: wait for the peers' routing tables, derive the layout
     int ok = 1;
-    if (lt < P)
+    if (lt < P && lt != me)
       ok = wait_flag_ge(reinterpret_cast<unsigned long long*>(mine + ll.idx_flag) + lt, epoch, ctx, kOpLLDispatch, 1, lt);
     if (!ok) s_fail = 1;
+    if (lt < kMaxRanks)
+      s_T[lt] = lt == me ? a.T : (ok && lt < P) ? __ldcg(reinterpret_cast<const int*>(mine + ll.gather_hdr) + lt * 4) : 0;
     layout_sync();
     stamp(2, kLayoutFirst);
     if (!s_fail) {
-    if (lt < kMaxRanks)
-      s_T[lt] = lt < P ? __ldcg(reinterpret_cast<const int*>(mine + ll.gather_hdr) + lt * 4) : 0;
-    for (int i = lt; i < E * kLLWords; i += LT) (&s_emask[0][0])[i] = 0u;
-    for (int i = lt; i < kMaxRanks * kLLWords; i += LT) (&s_hit[0][0])[i] = 0u;
-    layout_sync();
     int maxT = 1;
     for (int r = 0; r < P; ++r) maxT = max(maxT, min(s_T[r], M));
-    // one thread per (source, token); the loads of four items are issued before the first of them is used
+    const int words = (maxT + 31) >> 5;               // mask words in use
+    if (P > 1) {
+    // one thread per (source, token) of the peers (this rank's masks are already set); the loads of four items are issued
+    // before the first of them is used
     constexpr int kBatch = 4;
     for (int i0 = lt; i0 < P * maxT; i0 += LT * kBatch) {
       int row[kBatch][kMaxTopk];
 #pragma unroll
       for (int b = 0; b < kBatch; ++b) {
         const int i = i0 + b * LT, r = i / maxT, t = i - r * maxT;
-        const bool live = i < P * maxT && t < s_T[r];
+        const bool live = i < P * maxT && t < s_T[r] && r != me;
 #pragma unroll
         for (int k = 0; k < kMaxTopk; ++k) row[b][k] = (live && k < K) ? __ldcg(gidx + ((size_t)r * M + t) * K + k) : -1;
       }
@@ -277,38 +316,53 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
       }
     }
     layout_sync();
-    for (int l = lt; l < Lx; l += LT) {
-      int tot = 0;
-      for (int r = 0; r < P; ++r) tot += popc8(s_emask[r * Lx + l]);
-      s_tot[l] = tot;
     }
-    layout_sync();
-    if (lt == 0) {
-      int run = 0;
-      for (int l = 0; l < Lx; ++l) { int v = s_tot[l]; s_tot[l] = run; run += v; }
-      s_rows = run;
+    // rows per local expert and their exclusive prefix: every thread owns `per` consecutive experts, a warp scan and the
+    // warps' totals give its first row (a serial scan by one thread took 6 us for 384 experts)
+    const int per = (Lx + LT - 1) / LT, l0 = min(Lx, lt * per), l1 = min(Lx, l0 + per);
+    auto rows_of = [&](int r, int l) {
+      int n = 0;
+      for (int w = 0; w < words; ++w) n += __popc(s_emask[r * Lx + l][w]);
+      return n;
+    };
+    int tot = 0;
+    for (int l = l0; l < l1; ++l)
+      for (int r = 0; r < P; ++r) { const int n = rows_of(r, l); s_off[r * Lx + l] = n; tot += n; }
+    int incl = tot;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += o;
     }
+    if (lane == 31) s_warp_rows[warp] = incl;
     layout_sync();
-    for (int l = lt; l < Lx; l += LT) {
-      int run = s_tot[l];
-      for (int r = 0; r < P; ++r) { s_off[r * Lx + l] = run; run += popc8(s_emask[r * Lx + l]); }
+    int run = incl - tot, all = 0;
+    for (int w = kLLSendWarps; w < nwarps; ++w) {
+      if (w < warp) run += s_warp_rows[w];
+      all += s_warp_rows[w];
+    }
+    for (int l = l0; l < l1; ++l) {
+      const int begin = run;
+      for (int r = 0; r < P; ++r) { const int n = s_off[r * Lx + l]; s_off[r * Lx + l] = run; run += n; }
       if (blockIdx.x == 0) {
-        a.expert_offsets[l] = s_tot[l];
-        a.expert_counts[l] = run - s_tot[l];
-        if (a.mailbox) a.mailbox[4 + l] = run - s_tot[l];
+        a.expert_offsets[l] = begin;
+        a.expert_counts[l] = run - begin;
+        if (a.mailbox) a.mailbox[4 + l] = run - begin;
       }
     }
-    layout_sync();
-    if (blockIdx.x == 0 && lt == 0) {
-      a.expert_offsets[Lx] = s_rows;
-      *a.num_rows = s_rows;
-      if (a.mailbox) {
-        a.mailbox[0] = s_rows;
-        __threadfence_system();
-        a.mailbox[3] = (int)(epoch & 0x7fffffff);
+    if (blockIdx.x == 0) {
+      if (a.mailbox) __threadfence_system();
+      layout_sync();
+      if (lt == 0) {
+        a.expert_offsets[Lx] = all;
+        *a.num_rows = all;
+        if (a.mailbox) {
+          a.mailbox[0] = all;
+          __threadfence_system();
+          a.mailbox[3] = (int)(epoch & 0x7fffffff);
+        }
       }
     }
-
     }
     stamp(3, kLayoutFirst);
     }
@@ -320,47 +374,129 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
     uint8_t* mine = ctx.ws[me] + bank_off;
     const int* gidx = reinterpret_cast<const int*>(mine + ll.gather_idx);
     const float* gw_ = reinterpret_cast<const float*>(mine + ll.gather_w);
-    int maxT = 1;
-    for (int r = 0; r < P; ++r) maxT = max(maxT, min(s_T[r], M));
-
-    // ---- poll row flags and write the output rows
-    const uint8_t* stage = mine + ll.stage;
     uint8_t* recv_x = reinterpret_cast<uint8_t*>(a.recv_x);
+    // lane k: the output row of slot k of token t of source r (-1: its expert lives elsewhere, or the slot is empty or repeated)
+    auto out_row_of = [&](int r, int t, int e) {
+      bool counts = e >= 0 && e < E && e / Lx == me;
+      for (int z = 0; z < K; ++z) {
+        const int ez = __shfl_sync(0xffffffffu, e, z);
+        if (z < lane && ez == e) counts = false;
+      }
+      if (!counts) return -1;
+      const int at = r * Lx + e - me * Lx, row = s_off[at] + below8(s_emask[at], t);
+      return row < a.capacity ? row : -1;
+    };
+
+    // ---- rows of this rank's own tokens: from the caller's tensor straight into every output row
+    for (int item = gw; item < a.T * pieces; item += total_warps) {
+      const int piece = item % pieces, t = item / pieces;
+      const LLPart pr = item == gw ? own_pr : ll_piece(H, piece, pieces);
+      int e = -1;
+      if (lane < K) {
+        const long long v = a.topk_idx[(size_t)t * K + lane];
+        e = (v < 0 || v >= E) ? -1 : (int)v;
+      }
+      const int row = out_row_of(me, t, e);
+      if (piece == 0 && lane < K) {
+        a.local_row[(size_t)t * K + lane] = row;
+        if (row >= 0) {
+          a.recv_row_src[row] = (me * M + t) * K + lane;
+          a.recv_w[row] = a.topk_w ? a.topk_w[(size_t)t * K + lane] : 0.f;
+        }
+      }
+      const unsigned live = __ballot_sync(0xffffffffu, row >= 0);
+      if (live == 0 || pr.v0 >= pr.v1) continue;
+      const int4* src = reinterpret_cast<const int4*>(reinterpret_cast<const uint8_t*>(a.x) + (size_t)t * src_bytes);
+      const int lo = (a.mode == 1 ? pr.v0 : pr.v0 * 2) / 16, hi = (a.mode == 1 ? pr.v1 : pr.v1 * 2) / 16;
+      for (int u0 = lo; u0 < hi; u0 += 32 * kOwnUnroll) {
+        int4 v[kOwnUnroll];
+#pragma unroll
+        for (int i = 0; i < kOwnUnroll; ++i) {
+          const int u = u0 + i * 32 + lane;
+          if (item == gw && u0 == lo) v[i] = ahead[i];
+          else v[i] = u < hi ? __ldg(src + u) : make_int4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int i = 0; i < kOwnUnroll; ++i) {
+          const int u = u0 + i * 32 + lane;
+          if (u0 + i * 32 >= hi) break;               // warp-uniform
+          if (a.mode == 2) {
+            float scale;
+            const uint2 q = quant8(v[i], scale);
+            for (unsigned m = live; m; m &= m - 1) {
+              const size_t o = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
+              if (u < hi) {
+                *reinterpret_cast<uint2*>(recv_x + o * H + (size_t)u * 8) = q;
+                if ((lane & 15) == 0) a.recv_sf[o * nsf + u / 16] = scale;
+              }
+            }
+          } else {
+            for (unsigned m = live; m; m &= m - 1) {
+              const size_t o = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
+              if (u < hi) reinterpret_cast<int4*>(recv_x + o * row_bytes)[u] = v[i];
+            }
+          }
+        }
+      }
+      if (a.mode == 1)
+        for (int b = pr.b0; b < pr.b1; b += 32) {
+          const float sf = b + lane < pr.b1 ? __ldg(a.x_sf + (size_t)t * nsf + b + lane) : 0.f;
+          for (unsigned m = live; m; m &= m - 1) {
+            const size_t o = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
+            if (b + lane < pr.b1) a.recv_sf[o * nsf + b + lane] = sf;
+          }
+        }
+    }
+
+    // ---- rows of the peers: poll the part flags and write the output rows
+    int maxT = 1;
+    for (int r = 0; r < P; ++r) if (r != me) maxT = max(maxT, min(s_T[r], M));
+    const uint8_t* stage = mine + ll.stage;
     // a staged row is materialised part by part, by whichever warp draws the part
-    for (int item = gw; item < P * maxT * kLLParts; item += total_warps) {
+    for (int item = gw; item < (P - 1) * maxT * kLLParts; item += total_warps) {
       const int part = item % kLLParts, it = item / kLLParts;
-      const int r = (me + it / maxT) % P, t = it % maxT;
+      const int r = (me + 1 + it / maxT) % P, t = it % maxT;
       if (t >= s_T[r] || !((s_hit[r][t >> 5] >> (t & 31)) & 1u)) continue;
       const LLPart pr = ll_part(H, part);
       if (pr.v0 >= pr.v1) continue;
       const int j = below8(s_hit[r], t);
-      int idx_row[kMaxTopk], rows[kMaxTopk], n = 0;
-      for (int k = 0; k < K; ++k) idx_row[k] = __ldcg(gidx + ((size_t)r * M + t) * K + k);   // issued before the flag wait
+      const int e = lane < K ? __ldcg(gidx + ((size_t)r * M + t) * K + lane) : -1;   // issued before the flag wait
       int got = 1;
       if (lane == 0)
         got = wait_flag_ge(reinterpret_cast<unsigned long long*>(mine + ll.row_flag) + ((size_t)r * M + j) * kLLParts + part, epoch,
                            ctx, kOpLLDispatch, 2, r);
       if (!__shfl_sync(0xffffffffu, got, 0)) break;
-      for (int k = 0; k < K; ++k) {
-        if (!counts_ll(idx_row, k, E) || idx_row[k] / Lx != me) continue;
-        const int el = idx_row[k] - me * Lx;
-        const int out_row = s_off[r * Lx + el] + below8(s_emask[r * Lx + el], t);
-        if (out_row >= a.capacity) continue;
-        rows[n++] = out_row;
-        if (lane == 0 && part == 0) {
-          a.recv_row_src[out_row] = (r * M + t) * K + k;
-          a.recv_w[out_row] = __ldcg(gw_ + ((size_t)r * M + t) * K + k);
+      const int row = out_row_of(r, t, e);
+      if (part == 0 && row >= 0) {
+        a.recv_row_src[row] = (r * M + t) * K + lane;
+        a.recv_w[row] = __ldcg(gw_ + ((size_t)r * M + t) * K + lane);
+      }
+      const unsigned live = __ballot_sync(0xffffffffu, row >= 0);
+      const uint8_t* src = stage + ((size_t)r * M + j) * ll.msg_bytes;
+      const int b_lo = fp8 ? pr.v0 : pr.v0 * 2, b_hi = fp8 ? pr.v1 : pr.v1 * 2, n = (b_hi - b_lo) / 16;
+      for (int u0 = 0; u0 < n; u0 += 32 * 8) {
+        int4 v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int u = u0 + i * 32 + lane;
+          if (u < n) v[i] = __ldcg(reinterpret_cast<const int4*>(src + b_lo) + u);
+        }
+        for (unsigned m = live; m; m &= m - 1) {
+          int4* d = reinterpret_cast<int4*>(recv_x + (size_t)__shfl_sync(0xffffffffu, row, __ffs(m) - 1) * row_bytes + b_lo);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int u = u0 + i * 32 + lane;
+            if (u < n) d[u] = v[i];
+          }
         }
       }
-      const uint8_t* src = stage + ((size_t)r * M + j) * ll.msg_bytes;
-      const int b_lo = fp8 ? pr.v0 : pr.v0 * 2, b_hi = fp8 ? pr.v1 : pr.v1 * 2;
-      int4* outs[kMaxTopk];
-      for (int i = 0; i < n; ++i) outs[i] = reinterpret_cast<int4*>(recv_x + (size_t)rows[i] * row_bytes + b_lo);
-      warp_copy_row<8>(outs, n, reinterpret_cast<const int4*>(src + b_lo), (b_hi - b_lo) / 16, lane);
       if (fp8)
-        for (int q = pr.b0 + lane; q < pr.b1; q += 32) {
-          const float v = __ldcg(reinterpret_cast<const float*>(src + H) + q);
-          for (int i = 0; i < n; ++i) a.recv_sf[(size_t)rows[i] * nsf + q] = v;
+        for (int b = pr.b0; b < pr.b1; b += 32) {
+          const float sf = b + lane < pr.b1 ? __ldcg(reinterpret_cast<const float*>(src + H) + b + lane) : 0.f;
+          for (unsigned m = live; m; m &= m - 1) {
+            const size_t o = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
+            if (b + lane < pr.b1) a.recv_sf[o * nsf + b + lane] = sf;
+          }
         }
     }
   }
@@ -405,22 +541,23 @@ __global__ void __launch_bounds__(kLLThreads) ep_combine_ll_kernel(const __grid_
   };
 
   int ok = 1;
-  if (threadIdx.x < P && epoch > 2)
+  if (threadIdx.x < P && threadIdx.x != me && epoch > 2)
     ok = wait_flag_ge(&ctl->ll_comb_ack[threadIdx.x], epoch - 2, ctx, kOpLLCombine, 0, threadIdx.x);
   const int alive = __syncthreads_and(ok);
   stamp(0);
 
   if (alive) {
-    // ---- return every expert row, part by part, to its (token, slot) slot at the source
-    const int R = *a.num_rows;
+    // ---- return every expert row of a peer's token, part by part, to its (token, slot) slot there
+    const int R = P > 1 ? *a.num_rows : 0;
     PendingFlags pending;
     for (int item = gw; item < R * kLLParts; item += total_warps) {
       const int r = item / kLLParts, part = item % kLLParts;
       const int code = a.recv_row_src[r];
       if (code < 0) continue;
+      const int src = code / (M * K), rem = code - src * M * K;
+      if (src == me) continue;
       const LLPart pr = ll_part(H, part);
       if (pr.v0 >= pr.v1) continue;
-      const int src = code / (M * K), rem = code - src * M * K;
       uint8_t* base = ctx.ws[src] + bank_off;
       int4* dst = reinterpret_cast<int4*>(base + ll.ret + (size_t)rem * row_bytes + (size_t)pr.v0 * 2);
       const int4* from = reinterpret_cast<const int4*>(reinterpret_cast<const uint8_t*>(a.x) + (size_t)r * row_bytes + (size_t)pr.v0 * 2);
@@ -429,19 +566,26 @@ __global__ void __launch_bounds__(kLLThreads) ep_combine_ll_kernel(const __grid_
     }
     pending.publish(epoch, lane);
     stamp(1);
-    // ---- weighted sum at the source, slot order, fp32: two warps per (token, part), each a half of the part's columns
+    // ---- weighted sum at the source, slot order, fp32: a warp takes `step` 16-byte columns of a part of a token.  Rows of
+    // this rank's own experts are read from x, the others from the return slots once their flags are set.
     uint8_t* mine = ctx.ws[me] + bank_off;
     const unsigned long long* flags = reinterpret_cast<const unsigned long long*>(mine + ll.ret_flag);
-    for (int item = gw; item < a.T * kLLParts * 2; item += total_warps) {
-      const int t = item / (kLLParts * 2), sub = item % (kLLParts * 2), part = sub >> 1, half = sub & 1;
+    const int part_units = ll_part(H, 0).v1 / 8;      // the first part is the widest
+    const int subs32 = (part_units + 31) / 32;
+    const int step = a.T * kLLParts * subs32 <= total_warps ? 32 : 64, subs = (part_units + step - 1) / step;
+    for (int item = gw; item < a.T * kLLParts * subs; item += total_warps) {
+      const int t = item / (kLLParts * subs), rest = item - t * (kLLParts * subs), part = rest / subs, sub = rest - part * subs;
       const LLPart pr = ll_part(H, part);
-      if (pr.v0 >= pr.v1) continue;
-      // lane k holds slot k: expert, weight, whether it counts (in range, first occurrence)
+      const int u_begin = pr.v0 / 8 + sub * step, u_end = min(pr.v1 / 8, u_begin + step);
+      if (u_begin >= u_end) continue;
+      // lane k holds slot k: expert, weight, whether it counts (in range, first occurrence), where its row is
       long long e = -1;
       float w = 0.f;
+      int local = -1;
       if (lane < K) {
         e = a.topk_idx[(size_t)t * K + lane];
         w = a.topk_w[(size_t)t * K + lane];
+        local = a.local_row[(size_t)t * K + lane];
       }
       bool counts = lane < K && e >= 0 && e < a.E;
       for (int z = 0; z < K; ++z) {
@@ -450,59 +594,57 @@ __global__ void __launch_bounds__(kLLThreads) ep_combine_ll_kernel(const __grid_
       }
       const unsigned valid = __ballot_sync(0xffffffffu, counts);
       int got = 1;
-      if (counts) got = wait_flag_ge(flags + ((size_t)t * K + lane) * kLLParts + part, epoch, ctx, kOpLLCombine, 1, me);
+      if (counts && local < 0) got = wait_flag_ge(flags + ((size_t)t * K + lane) * kLLParts + part, epoch, ctx, kOpLLCombine, 1, me);
       if (!__all_sync(0xffffffffu, got)) break;
-      const uint8_t* rows = mine + ll.ret + (size_t)t * K * row_bytes;
+      const unsigned long long my_row = reinterpret_cast<unsigned long long>(
+          local >= 0 ? reinterpret_cast<const uint8_t*>(a.x) + (size_t)local * row_bytes
+                     : mine + ll.ret + ((size_t)t * K + min(lane, K - 1)) * row_bytes);
       int4* out = reinterpret_cast<int4*>(reinterpret_cast<uint8_t*>(a.out) + (size_t)t * row_bytes);
-      const int u_lo = pr.v0 / 8, u_hi = pr.v1 / 8, hs = (u_hi - u_lo + 1) / 2;
-      const int u_begin = u_lo + half * hs, u_end = min(u_hi, u_begin + hs);
-      // two 16-byte columns per lane and step; the trip count is the same for every lane, which all take part in the shuffles
-      for (int ub = u_begin; ub < u_end; ub += 64) {
-        const int u0 = ub + lane;
-        const bool one = u0 < u_end, two = u0 + 32 < u_end;
-        float a0[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, a1[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int kb = 0; kb < K; kb += 8) {    // eight slots' loads in flight at a time
-          int4 v0[8], v1[8];
+      const int u0 = u_begin + lane;
+      const bool one = u0 < u_end, two = u0 + 32 < u_end;
+      float a0[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, a1[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      for (int kb = 0; kb < K; kb += 8) {    // eight slots' loads in flight at a time
+        int4 v0[8], v1[8];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            if (kb + k < K && ((valid >> (kb + k)) & 1u)) {
-              if (one) v0[k] = ld_cg_int4(rows + (size_t)(kb + k) * row_bytes + (size_t)u0 * 16);
-              if (two) v1[k] = ld_cg_int4(rows + (size_t)(kb + k) * row_bytes + (size_t)(u0 + 32) * 16);
-            }
+        for (int k = 0; k < 8; ++k) {
+          if (kb + k < K && ((valid >> (kb + k)) & 1u)) {
+            const int4* row = reinterpret_cast<const int4*>(__shfl_sync(0xffffffffu, my_row, kb + k));
+            if (one) v0[k] = __ldcg(row + u0);
+            if (two) v1[k] = __ldcg(row + u0 + 32);
           }
+        }
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            if (kb + k < K && ((valid >> (kb + k)) & 1u)) {      // warp-uniform
-              const float wk = __shfl_sync(0xffffffffu, w, kb + k);
-              const __nv_bfloat162* h0 = reinterpret_cast<const __nv_bfloat162*>(&v0[k]);
-              const __nv_bfloat162* h1 = reinterpret_cast<const __nv_bfloat162*>(&v1[k]);
+        for (int k = 0; k < 8; ++k) {
+          if (kb + k < K && ((valid >> (kb + k)) & 1u)) {      // warp-uniform
+            const float wk = __shfl_sync(0xffffffffu, w, kb + k);
+            const __nv_bfloat162* h0 = reinterpret_cast<const __nv_bfloat162*>(&v0[k]);
+            const __nv_bfloat162* h1 = reinterpret_cast<const __nv_bfloat162*>(&v1[k]);
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                // product and sum are rounded separately (no fused multiply-add), as the CPU oracle does
-                if (one) {
-                  a0[2 * i] = __fadd_rn(a0[2 * i], __fmul_rn(wk, __low2float(h0[i])));
-                  a0[2 * i + 1] = __fadd_rn(a0[2 * i + 1], __fmul_rn(wk, __high2float(h0[i])));
-                }
-                if (two) {
-                  a1[2 * i] = __fadd_rn(a1[2 * i], __fmul_rn(wk, __low2float(h1[i])));
-                  a1[2 * i + 1] = __fadd_rn(a1[2 * i + 1], __fmul_rn(wk, __high2float(h1[i])));
-                }
+            for (int i = 0; i < 4; ++i) {
+              // product and sum are rounded separately (no fused multiply-add), as the CPU oracle does
+              if (one) {
+                a0[2 * i] = __fadd_rn(a0[2 * i], __fmul_rn(wk, __low2float(h0[i])));
+                a0[2 * i + 1] = __fadd_rn(a0[2 * i + 1], __fmul_rn(wk, __high2float(h0[i])));
+              }
+              if (two) {
+                a1[2 * i] = __fadd_rn(a1[2 * i], __fmul_rn(wk, __low2float(h1[i])));
+                a1[2 * i + 1] = __fadd_rn(a1[2 * i + 1], __fmul_rn(wk, __high2float(h1[i])));
               }
             }
           }
         }
-        int4 o;
-        __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
-        if (one) {
+      }
+      int4 o;
+      __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+      if (one) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) oh[i] = __floats2bfloat162_rn(a0[2 * i], a0[2 * i + 1]);
-          out[u0] = o;
-        }
-        if (two) {
+        for (int i = 0; i < 4; ++i) oh[i] = __floats2bfloat162_rn(a0[2 * i], a0[2 * i + 1]);
+        out[u0] = o;
+      }
+      if (two) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) oh[i] = __floats2bfloat162_rn(a1[2 * i], a1[2 * i + 1]);
-          out[u0 + 32] = o;
-        }
+        for (int i = 0; i < 4; ++i) oh[i] = __floats2bfloat162_rn(a1[2 * i], a1[2 * i + 1]);
+        out[u0 + 32] = o;
       }
     }
   }

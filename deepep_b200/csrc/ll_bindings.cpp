@@ -48,9 +48,10 @@ void op_ll_dispatch(const WsLayout& lay, const std::vector<py::object>& sessions
     a.T = geti(d, "T"); a.E = geti(d, "E"); a.mode = geti(d, "mode");
     a.recv_x = ptr<void>(d, "recv_x"); a.recv_sf = ptr<float>(d, "recv_sf"); a.recv_w = ptr<float>(d, "recv_w");
     a.recv_row_src = ptr<int>(d, "recv_row_src"); a.expert_counts = ptr<int>(d, "expert_counts");
-    a.expert_offsets = ptr<int>(d, "expert_offsets"); a.num_rows = ptr<int>(d, "num_rows");
+    a.expert_offsets = ptr<int>(d, "expert_offsets"); a.num_rows = ptr<int>(d, "num_rows"); a.local_row = ptr<int>(d, "local_row");
     a.mailbox = geti(d, "use_mailbox", 0) ? s.mailbox_device() : nullptr;
     a.capacity = d["capacity"].cast<long long>();
+    if (!a.local_row && a.T > 0) throw std::invalid_argument("low-latency dispatch: local_row is missing");
     if (a.T < 0 || a.T > lay.max_tokens) throw std::invalid_argument("token count exceeds num_max_tokens_per_rank");
     if (a.E < a.ctx.world || a.E > kMaxExperts || a.E % a.ctx.world) throw std::invalid_argument("num_experts must be a multiple of the world size and at most 1024");
     if (a.mode != 0 && lay.hidden % 128) throw std::invalid_argument("fp8 dispatch needs hidden % 128 == 0");
@@ -73,7 +74,8 @@ void op_ll_combine(const WsLayout& lay, const std::vector<py::object>& sessions,
     a.x = ptr<const __nv_bfloat16>(d, "x"); a.recv_row_src = ptr<const int>(d, "recv_row_src");
     a.num_rows = ptr<const int>(d, "num_rows"); a.topk_idx = ptr<const long long>(d, "topk_idx");
     a.topk_w = ptr<const float>(d, "topk_w"); a.T = geti(d, "T"); a.E = geti(d, "E");
-    a.out = ptr<__nv_bfloat16>(d, "out");
+    a.out = ptr<__nv_bfloat16>(d, "out"); a.local_row = ptr<const int>(d, "local_row");
+    if (!a.local_row && a.T > 0) throw std::invalid_argument("low-latency combine: local_row is missing");
   }
   check(launch_ll_combine(p, n, blocks, reinterpret_cast<cudaStream_t>(stream)), "ep_combine_ll launch");
 }

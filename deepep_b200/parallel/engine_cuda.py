@@ -70,6 +70,7 @@ class RoutingPlan:
     has_weights: bool = False
     low_latency: bool = False
     num_rows_dev: Optional[torch.Tensor] = None
+    local_row: Optional[torch.Tensor] = None     # low latency: output row of every slot whose expert lives on this rank
     topk_w: Optional[torch.Tensor] = None
     rank_matrix: Optional[torch.Tensor] = None
     send_chunk_prefix: Optional[torch.Tensor] = None
@@ -420,12 +421,14 @@ class CudaEngine:
                                expert_counts=o["expert_counts"], expert_offsets=o["expert_offsets"],
                                recv_row_src=o["recv_row_src"], recv_w=o["recv_w"], recv_idx=None, has_weights=True)
             plan.num_rows_dev, plan.topk_w, plan.low_latency = o["num_rows"], topk_w[i], True
+            plan.local_row = torch.empty((max(T, 1), K), **i32)
             res.append((plan, o["recv_x"], o["recv_sf"]))
             args.append(dict(x=x.data_ptr(), x_sf=_ptr(sf), topk_idx=topk_idx[i].data_ptr(), topk_w=topk_w[i].data_ptr(), T=T,
                              E=num_experts, mode=mode, recv_x=o["recv_x"].data_ptr(), recv_sf=_ptr(o["recv_sf"]),
                              recv_w=o["recv_w"].data_ptr(), recv_row_src=o["recv_row_src"].data_ptr(),
                              expert_counts=o["expert_counts"].data_ptr(), expert_offsets=o["expert_offsets"].data_ptr(),
-                             num_rows=o["num_rows"].data_ptr(), use_mailbox=int(cpu_sync), capacity=cap))
+                             num_rows=o["num_rows"].data_ptr(),
+                             local_row=plan.local_row.data_ptr(), use_mailbox=int(cpu_sync), capacity=cap))
         self._timed("ll_dispatch", stream, lambda: self.C.ll_dispatch(lay, self.sessions, args, self.ll_blocks(), self._stream(stream),
                                                                              self._device_profile))
         if cpu_sync:
@@ -451,7 +454,7 @@ class CudaEngine:
         for i, plan in enumerate(plans):
             out = outs[i] if outs is not None else torch.empty((plan.num_tokens, lay.hidden), dtype=torch.bfloat16, device=dev)
             results.append(out)
-            args.append(dict(x=xs[i].data_ptr(), recv_row_src=plan.recv_row_src.data_ptr(), num_rows=plan.num_rows_dev.data_ptr(),
+            args.append(dict(x=xs[i].data_ptr(), recv_row_src=plan.recv_row_src.data_ptr(), num_rows=plan.num_rows_dev.data_ptr(), local_row=plan.local_row.data_ptr(),
                              topk_idx=plan.topk_idx.data_ptr(), topk_w=plan.topk_w.data_ptr(), T=plan.num_tokens,
                              E=plan.num_experts, out=out.data_ptr()))
         self._timed("ll_combine", stream, lambda: self.C.ll_combine(lay, self.sessions, args, self.ll_blocks(), self._stream(stream),
