@@ -2,6 +2,7 @@
 oracle (bit for bit: moved rows, and sums whose order and roundings the contract fixes)."""
 import pytest
 
+from test_ht_virtual_gpu import run_case
 from test_ll_gpu import _case as ll_case
 
 pytestmark = pytest.mark.gpu
@@ -18,3 +19,17 @@ pytestmark = pytest.mark.gpu
 ])
 def test_low_latency_splits(world, tokens, hidden, experts, topk, mode):
     ll_case(world, tokens, hidden, experts, topk, mode, routes="invalid", repeats=3)
+
+
+@pytest.mark.parametrize("world,tokens,hidden,experts,topk,kw", [
+    (1, [1], 7168, 256, 8, dict(dmode=2)),             # one token, many pieces
+    (1, [65], 8, 16, 9, {}),                           # rows of one 16-byte piece; two groups of operands per token
+    (1, [129], 520, 32, 16, dict(with_bias=True)),     # a short last span, sixteen operands
+    (1, [2300], 1032, 8, 2, {}),                       # more tokens than warps
+    (1, [640], 7168, 64, 6, dict(dmode=1, alignment=16)),
+    (2, [64, 63], 1544, 32, 16, dict(with_bias=True)), # partials and more than eight local rows
+    (4, [192, 1, 0, 65], 2048, 64, 12, dict(expand=False)),
+    (8, [40] * 8, 1024, 64, 16, dict(dmode=2, alignment=128)),
+])
+def test_high_throughput_splits(world, tokens, hidden, experts, topk, kw):
+    run_case(world, tokens, hidden, experts, topk, "invalid", repeats=2, **kw)
