@@ -1,4 +1,4 @@
-// Python bindings of the local expand / aggregate operators.
+// Python bindings of the local expand / aggregate operators and of the expert activation.
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
@@ -6,6 +6,7 @@
 #include <string>
 
 #include "kernels/expand_api.h"
+#include "kernels/swiglu_api.h"
 
 namespace py = pybind11;
 using namespace dep;
@@ -21,6 +22,17 @@ void check_launch(cudaError_t e, const char* what) {
 }  // namespace
 
 void bind_expand(py::module_& m) {
+  m.def("swiglu", [](const py::dict& d, bool backward, int blocks, uintptr_t stream) {
+    SwigluParams p{};
+    p.gu = eptr<const __nv_bfloat16>(d, "gu"); p.w = eptr<const float>(d, "w"); p.h = eptr<__nv_bfloat16>(d, "h");
+    p.dh = eptr<const __nv_bfloat16>(d, "dh"); p.dgu = eptr<__nv_bfloat16>(d, "dgu"); p.dw = eptr<float>(d, "dw");
+    p.rows = d["rows"].cast<long long>(); p.inter = d["inter"].cast<int>();
+    if (p.rows < 0 || p.inter < 8 || p.inter % 8) throw std::invalid_argument("swiglu: the width must be a positive multiple of 8");
+    if (p.rows > 0 && (!p.gu || (backward ? !p.dh || !p.dgu : !p.h))) throw std::invalid_argument("swiglu: a tensor is missing");
+    for (const void* q : {(const void*)p.gu, (const void*)p.h, (const void*)p.dh, (const void*)p.dgu})
+      if (reinterpret_cast<uintptr_t>(q) % 16) throw std::invalid_argument("swiglu: rows must start on a 16-byte boundary");
+    check_launch(launch_swiglu(p, backward, blocks, reinterpret_cast<cudaStream_t>(stream)), "swiglu");
+  });
   m.attr("expand_tile") = kExpandTile;
   m.def("expand", [](const py::dict& d, int blocks, uintptr_t stream) {
     ExpandParams p{};

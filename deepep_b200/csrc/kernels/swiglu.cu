@@ -1,0 +1,92 @@
+// silu(gate) * up * w over rows of [gate | up], and its backward pass (see swiglu_api.h).
+//
+// Bound by memory: forward reads 4 and writes 2 bytes per value, backward reads 6 and writes 4.  One warp per row, 16-byte
+// accesses, all arithmetic in fp32 with one rounding at the end; the row factor joins here, where a row is `inter` values
+// wide, so that neither the layer's output nor its gradient needs a pass of its own for it, and the factor's gradient is the
+// row sum of dh * silu(gate) * up, which backward has in registers.  As library passes over the two strided halves (silu,
+// product, factor, their gradients and a concatenation) the same work took 2.36 ms of a 7.6 ms training step (8192 tokens,
+// hidden 4096, 49152 rows, inter 1536); here forward takes 75 and backward 116 us (6.0 and 6.5 TB/s).
+#include "swiglu_api.h"
+
+namespace dep {
+
+constexpr int kSwigluThreads = 256;
+
+struct Vec8 { float v[8]; };
+__device__ __forceinline__ Vec8 unpack8(const int4& q) {
+  Vec8 r;
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { r.v[2 * i] = __low2float(h[i]); r.v[2 * i + 1] = __high2float(h[i]); }
+  return r;
+}
+__device__ __forceinline__ int4 pack8(const Vec8& r) {
+  int4 q;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(r.v[2 * i], r.v[2 * i + 1]);
+  return q;
+}
+
+template <bool kBackward>
+__global__ void __launch_bounds__(kSwigluThreads) swiglu_kernel(const __grid_constant__ SwigluParams p) {
+  const int lane = threadIdx.x & 31, units = p.inter / 8;
+  const long long warps = (long long)gridDim.x * (kSwigluThreads / 32);
+  for (long long row = (long long)blockIdx.x * (kSwigluThreads / 32) + (threadIdx.x >> 5); row < p.rows; row += warps) {
+    const int4* gate = reinterpret_cast<const int4*>(p.gu) + row * 2 * units;
+    const float w = p.w ? __ldg(p.w + row) : 1.f;
+    float dw = 0.f;
+    constexpr int U = 2;                       // 16-byte pieces of every operand in flight per lane
+    for (int u0 = lane; u0 < units; u0 += 32 * U) {
+      int4 g4[U], u4[U], d4[U];
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        const int u = u0 + i * 32;
+        if (u < units) {
+          g4[i] = __ldg(gate + u);
+          u4[i] = __ldg(gate + units + u);
+          if (kBackward) d4[i] = __ldg(reinterpret_cast<const int4*>(p.dh) + row * units + u);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        const int u = u0 + i * 32;
+        if (u >= units) break;
+        const Vec8 g = unpack8(g4[i]), up = unpack8(u4[i]);
+        if (!kBackward) {
+          Vec8 h;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) h.v[e] = __fdividef(g.v[e], 1.f + __expf(-g.v[e])) * up.v[e] * w;
+          reinterpret_cast<int4*>(p.h)[row * units + u] = pack8(h);
+        } else {
+          const Vec8 d = unpack8(d4[i]);
+          Vec8 dg, du;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float s = __fdividef(1.f, 1.f + __expf(-g.v[e])), silu = g.v[e] * s, dy = d.v[e] * w;
+            dw += d.v[e] * (silu * up.v[e]);
+            du.v[e] = dy * silu;
+            dg.v[e] = dy * up.v[e] * (s * (1.f + g.v[e] * (1.f - s)));
+          }
+          int4* out = reinterpret_cast<int4*>(p.dgu) + row * 2 * units;
+          out[u] = pack8(dg);
+          out[units + u] = pack8(du);
+        }
+      }
+    }
+    if (kBackward && p.dw) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) dw += __shfl_xor_sync(0xffffffffu, dw, o);
+      if (lane == 0) p.dw[row] = dw;
+    }
+  }
+}
+
+cudaError_t launch_swiglu(const SwigluParams& p, bool backward, int blocks, cudaStream_t stream) {
+  if (p.rows == 0) return cudaSuccess;
+  if (backward) swiglu_kernel<true><<<blocks, kSwigluThreads, 0, stream>>>(p);
+  else swiglu_kernel<false><<<blocks, kSwigluThreads, 0, stream>>>(p);
+  return cudaGetLastError();
+}
+
+}  // namespace dep
