@@ -87,8 +87,10 @@ void op_dispatch(const WsLayout& lay, const std::vector<py::object>& sessions, c
     a.slot_row = ptr<const int>(d, "slot_row"); a.topk_idx = ptr<const long long>(d, "topk_idx");
     a.rank_tokens = ptr<const int>(d, "rank_tokens"); a.rank_rows = ptr<const int>(d, "rank_rows");
     a.meta_stride = geti(d, "meta_stride");
-    a.recv_rows = geti(d, "recv_rows", 0);
     a.K = geti(d, "K"); a.E = geti(d, "E"); a.expand = geti(d, "expand", 1);
+    a.recv_rows = geti(d, "recv_rows", 0);
+    a.pad_counts = ptr<const int>(d, "pad_counts"); a.pad_offsets = ptr<const int>(d, "pad_offsets");
+    if (!a.pad_counts != !a.pad_offsets || (a.pad_offsets && a.E < a.ctx.world)) throw std::invalid_argument("dispatch: padding needs the expert counts, offsets and E");
     a.recv_x = ptr<void>(d, "recv_x"); a.recv_sf = ptr<float>(d, "recv_sf");
     a.prof = ptr<unsigned long long>(d, "prof");
     // (a rank without tokens, or without received rows, passes empty tensors whose address is null)

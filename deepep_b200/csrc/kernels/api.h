@@ -58,7 +58,9 @@ struct DispatchArgs {
   const int* stage_meta;
   const int* rank_tokens;
   const int* rank_rows;        // [P + 1] exclusive prefix of the staged rows per source (rank layout: first output row of a source)
-  int meta_stride, recv_rows;  // recv_rows: rows of recv_x (only read by the optional index checks; 0 = unknown)
+  int meta_stride, recv_rows;  // recv_rows: rows of recv_x (0 = unknown)
+  const int* pad_counts;       // [L] rows and [L + 1] first rows of the local experts when the rows that no token fills (between
+  const int* pad_offsets;      // an expert's rows and the next aligned block, and after the last block) are to be zeroed, or null
   int K, E, expand;
   void* recv_x;                // [R][H] 2-byte (mode 0) or e4m3 (modes 1, 2)
   float* recv_sf;              // [R][H/128] or null

@@ -336,10 +336,7 @@ class CudaEngine:
             else:
                 recv_x = torch.empty((rows, H), dtype=torch.float8_e4m3fn, device=dev)
                 recv_sf = torch.empty((rows, H // 128), dtype=torch.float32, device=dev)
-            if plan.expand and plan.alignment > 1:
-                recv_x.view(torch.uint8).zero_()
-                if recv_sf is not None:
-                    recv_sf.zero_()
+            padded = plan.expand and plan.alignment > 1      # the kernel zeroes the rows that no token fills
             outs.append((recv_x, recv_sf))
             args.append(dict(x=x.data_ptr(), x_sf=_ptr(sf), T=plan.num_tokens, mode=mode, send_slot=plan.send_slot.data_ptr(),
                              slot_row=plan.slot_row.data_ptr(), topk_idx=plan.topk_idx.data_ptr(),
@@ -347,6 +344,8 @@ class CudaEngine:
                              rank_tokens=plan.rank_tokens.data_ptr(), rank_rows=plan.rank_rows.data_ptr(),
                              meta_stride=plan.meta_stride, K=plan.num_topk, E=plan.num_experts, expand=int(plan.expand),
                              recv_x=recv_x.data_ptr(), recv_sf=_ptr(recv_sf), recv_rows=recv_x.shape[0],
+                             pad_counts=plan.expert_counts.data_ptr() if padded else None,
+                             pad_offsets=plan.expert_offsets.data_ptr() if padded else None,
                              prof=self._prof_buffer("dispatch", i)))
         send, recv = split if split is not None else self.split_blocks(blocks, self.dispatch_send_fraction, self.dispatch_blocks)
         self._timed("dispatch", stream, lambda: self.C.dispatch(lay, self.sessions, args, send, recv, self._stream(stream),

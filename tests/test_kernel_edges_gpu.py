@@ -3,6 +3,8 @@ oracle (bit for bit: moved rows, and sums whose order and roundings the contract
 import pytest
 import torch
 
+from deepep_b200.oracle import reference as R
+from helpers import bits_equal, make_routes, make_weights
 from test_ht_virtual_gpu import run_case
 from test_ll_gpu import _case as ll_case
 
@@ -60,3 +62,37 @@ def test_expert_activation(rows, inter, weighted):
     assert torch.all((x.grad.cpu().double() - g64.grad).abs() <= g64.grad.abs() * 2 ** -8 + 1e-5 * torch.cat([size, size], dim=1))
     if weighted:
         assert torch.all((f.grad.cpu().double() - f64.grad).abs() <= 1e-5 * (dh.double() * terms.detach()).abs().sum(1) + 1e-30)
+
+
+@pytest.mark.parametrize("payload", ["bf16", "fp8", "fp8_fused"])
+@pytest.mark.parametrize("alignment,experts", [(128, 24), (16, 700)])
+def test_padding_rows_are_zero(payload, alignment, experts):
+    """Rows that no token fills are zero whatever the memory held, rows of tokens are not touched, fresh and cached, with the
+    exact and with the worst-case row count."""
+    from deepep_b200 import ElasticBuffer
+    from deepep_b200.utils.math import per_token_cast_to_fp8
+
+    dev, T, H, K = torch.device("cuda"), 300, 896, 5
+    x = torch.randn((T, H), generator=torch.Generator().manual_seed(4)).bfloat16()
+    idx, w = make_routes("invalid", T, experts, K, 1, 6), make_weights(T, K, 2)
+    src = per_token_cast_to_fp8(x) if payload == "fp8" else x
+    ref, lays = R.dispatch([src], [idx], [w], experts, do_expand=True, expert_alignment=alignment, quantize_fp8=payload == "fp8_fused")
+    want = ref[0][0] if isinstance(ref[0][0], tuple) else (ref[0][0],)
+    used = torch.zeros((lays[0].num_rows,), dtype=torch.bool)
+    used[lays[0].row_index] = True
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K, use_fp8_dispatch=payload == "fp8_fused",
+                        explicitly_destroy=True)
+    on_gpu = tuple(t.to(dev) for t in src) if payload == "fp8" else src.to(dev)
+    handle = None
+    for exact in (True, True, False):
+        torch.full((64 << 20,), 0x55, dtype=torch.uint8, device=dev)        # what the outputs' memory holds before the call
+        fresh = dict(topk_idx=idx.to(dev), topk_weights=w.to(dev), num_experts=experts, expert_alignment=alignment, do_expand=True,
+                     do_cpu_sync=exact)
+        got, _, _, h, _ = buf.dispatch(on_gpu, **(fresh if handle is None or not exact else dict(handle=handle)))
+        handle = handle or h
+        got = got if isinstance(got, tuple) else (got,)
+        for g, e in zip(got, want):
+            rows = e.shape[0]
+            assert bits_equal(g[:rows][used.to(dev)], e[used]), "a token's row differs"
+            assert not bool(g.view(torch.uint8)[:rows][~used.to(dev)].any()) and not bool(g.view(torch.uint8)[rows:].any())
+    buf.destroy()
