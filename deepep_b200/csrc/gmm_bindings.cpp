@@ -20,7 +20,8 @@ template <class T> T* gptr(const py::dict& d, const char* key) {
 int gint(const py::dict& d, const char* key) { return d[key].cast<int>(); }
 
 // `gather` = true: a2av_gmm (A operand is the gathered buffer); false: gmm_a2av (A operand is x).
-void fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session, bool gather) {
+// Returns whether the single-rank kernel can serve the call.
+bool fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session, bool gather) {
   Session& s = session.cast<Session&>();
   a.ctx = s.ctx();
   const long long max_rows = d["max_rows"].cast<long long>(), max_k = d["max_k"].cast<long long>(), max_n = d["max_n"].cast<long long>();
@@ -44,14 +45,31 @@ void fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session
   if ((gather ? a.rows_in : a.out_rows_cap) > max_rows) throw std::invalid_argument("more rows than the group was sized for");
   if (!a.counts || (a.out_rows_cap > 0 && !a.out) || !a.tile_info || !a.num_tiles || (a.rows_in > 0 && !a.x) || (gather && (!a.gathered || !a.pulled)))
     throw std::invalid_argument("missing tensor");
+  // The single-rank kernel reads x and the weights while it writes the output and the gathered rows, so these must be
+  // disjoint from them; the general kernels write only after they have copied what an overlap would destroy.
+  const long long L = a.E / a.ctx.world;
+  const void* weight = gptr<const void>(d, "weight");
+  auto overlap = [](const void* p, long long n, const void* q, long long m) {
+    const uintptr_t u = (uintptr_t)p, v = (uintptr_t)q;
+    return p && q && n > 0 && m > 0 && u < v + (uintptr_t)m && v < u + (uintptr_t)n;
+  };
+  const bool keep = gather && d["gathered_wanted"].cast<bool>();
+  const long long x_bytes = (long long)a.rows_in * a.K * 2, out_bytes = (long long)a.out_rows_cap * a.N * 2,
+                  g_bytes = keep ? (long long)a.gathered_cap * a.K * 2 : 0, w_bytes = L * a.K * a.N * 2;
+  const bool local = a.ctx.world == 1 && !overlap(a.out, out_bytes, a.x, x_bytes) && !overlap(a.out, out_bytes, weight, w_bytes) &&
+                     !overlap(a.gathered, g_bytes, a.x, x_bytes) && !overlap(a.gathered, g_bytes, weight, w_bytes) &&
+                     !overlap(a.gathered, g_bytes, a.out, out_bytes) &&
+                     !overlap(a.counts, a.E * 4ll, a.out, out_bytes) && !overlap(a.counts, a.E * 4ll, a.gathered, g_bytes) &&
+                     ((uintptr_t)a.x | (uintptr_t)a.out | (keep ? (uintptr_t)a.gathered : 0)) % 16 == 0;
+  if (local && !keep) a.gathered = nullptr;
   const char* err = nullptr;
-  const void* a_base = gather ? (const void*)a.gathered : (const void*)a.x;
-  const long long a_rows = gather ? a.gathered_cap : a.rows_in;
+  const void* a_base = gather && !local ? (const void*)a.gathered : (const void*)a.x;
+  const long long a_rows = gather && !local ? a.gathered_cap : a.rows_in;
   // an empty operand still needs a valid map: point it at the weights
   if (!encode_bf16_map(&a.tmap_a, a_rows > 0 ? a_base : (const void*)d["weight"].cast<uintptr_t>(), a_rows > 0 ? a_rows : 1, a.K, kGmmBM, &err))
     throw std::runtime_error(err);
-  const long long L = a.E / a.ctx.world;
-  if (!encode_bf16_map(&a.tmap_b, gptr<const void>(d, "weight"), L * a.K, a.N, kGmmBK, &err)) throw std::runtime_error(err);
+  if (!encode_bf16_map(&a.tmap_b, weight, L * a.K, a.N, kGmmBK, &err)) throw std::runtime_error(err);
+  return local;
 }
 
 void op(const WsLayout& lay, const std::vector<py::object>& sessions, const std::vector<py::dict>& args, int blocks, uintptr_t stream,
@@ -60,8 +78,10 @@ void op(const WsLayout& lay, const std::vector<py::object>& sessions, const std:
   p.lay = lay;
   const int n = (int)args.size();
   if (n < 1 || n > kMaxRanks || (int)sessions.size() != n) throw std::invalid_argument("1..8 rank argument blocks expected");
-  for (int i = 0; i < n; ++i) fill(p.r[i], lay, args[i], sessions[i], gather);
-  const cudaError_t e = gather ? launch_a2av_gmm(p, n, blocks, reinterpret_cast<cudaStream_t>(stream))
+  bool local = n == 1;
+  for (int i = 0; i < n; ++i) local = fill(p.r[i], lay, args[i], sessions[i], gather) && local;
+  const cudaError_t e = local ? launch_gmm_local(p, blocks, reinterpret_cast<cudaStream_t>(stream))
+                        : gather ? launch_a2av_gmm(p, n, blocks, reinterpret_cast<cudaStream_t>(stream))
                                : launch_gmm_a2av(p, n, blocks, reinterpret_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) throw std::runtime_error(std::string(gather ? "a2av_gmm" : "gmm_a2av") + " launch: " + cudaGetErrorString(e));
 }

@@ -44,6 +44,7 @@ struct GmmArgs {
   const int* counts;               // [E] rows this rank sends to (a2av_gmm) / gets back from (gmm_a2av) every global expert
   __nv_bfloat16* out;              // a2av_gmm: [out_rows_cap, N] on the expert rank; gmm_a2av: [out_rows_cap, N] on the source rank
   __nv_bfloat16* gathered;         // a2av_gmm: [gathered_cap, K] the all-to-all-v result, A operand of the GEMM
+                                   // (single-rank form: a copy for the caller, or null)
   CUtensorMap tmap_a;              // A operand [rows, K] bf16: box 64 x 128, 128-byte swizzle
   CUtensorMap tmap_b;              // weights [L * K, N] bf16 (N contiguous): box 64 (N) x 64 (K), 128-byte swizzle
   int rows_in, E, K, N;
@@ -56,6 +57,8 @@ struct GmmArgs {
 struct GmmParams { WsLayout lay; GmmArgs r[kMaxRanks]; };
 cudaError_t launch_a2av_gmm(const GmmParams& p, int nranks, int blocks, cudaStream_t stream);
 cudaError_t launch_gmm_a2av(const GmmParams& p, int nranks, int blocks, cudaStream_t stream);
+// Either op on one rank (world 1) whose x, output, gathered rows and weights do not overlap: p.r[0] with tmap_a over x.
+cudaError_t launch_gmm_local(const GmmParams& p, int blocks, cudaStream_t stream);
 
 // 2-D bf16 tensor map, `cols` contiguous, 128-byte swizzle, box {64 columns, box_rows}.
 bool encode_bf16_map(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows, const char** error);

@@ -7,6 +7,8 @@
 //   gmm_a2av_kernel   grouped GEMM over the rows this rank holds; the epilogue stores each bf16 output row straight
 //                     into the workspace of the rank the row came from, at its place in that rank's expert-sorted
 //                     order; after a flag handshake every rank copies its returned rows into the output tensor.
+//   gmm_local_kernel  either op on a single rank, where the all-to-all-v is the identity: the GEMM reads x and writes
+//                     the output in place.
 //
 // GEMM: 256 x 256 tiles, K in steps of 64, A K-major and B (weights [K, N], N contiguous) MN-major, both moved by
 // TMA with the 128-byte swizzle; per stage two groups of four tcgen05.mma kind::f16 (M = 128, N = 256, K = 16), one
@@ -32,7 +34,6 @@ namespace dep {
 
 constexpr int kGmmGemmThreads = 320;                     // TMA warp, MMA warp, 8 epilogue warps
 constexpr int kGmmPullWarps = 2;
-constexpr int kGmmMaxStages = 4;
 constexpr int kGmmTileA = kGmmBM * kGmmBK * 2;           // 16 KB
 constexpr int kGmmBoxB = 64 * kGmmBK * 2;                // 8 KB: 64 K-rows of 64 N-values
 constexpr int kGmmTileB = (kGmmBN / 64) * kGmmBoxB;      // 32 KB
@@ -40,15 +41,12 @@ constexpr int kGmmPullChunk = 8;
 // Tiles are 256 rows x 256 columns: both 128-lane accumulators (all 512 tensor-memory columns) belong to one tile,
 // the two row halves share every B stage, and a stage moves 64 KB for twice the work (the kernel is bound by the
 // rate at which shared memory can be filled from L2, about 100 KB/us per SM, not by the tensor pipe).
-__host__ __device__ constexpr int gmm_tile_rows(bool) { return 2 * kGmmBM; }
-__host__ __device__ constexpr int gmm_stage_bytes(bool push) { return (gmm_tile_rows(push) / kGmmBM) * kGmmTileA + kGmmTileB; }
-__host__ __device__ constexpr int gmm_stages(bool push) { return 3; }
-__host__ __device__ constexpr size_t gmm_smem_bytes(bool push) {
-  return 1024 + (size_t)gmm_stages(push) * gmm_stage_bytes(push) + 256;
-}
+constexpr int kGmmHalves = 2, kGmmTileRows = kGmmHalves * kGmmBM;
+constexpr int kGmmStages = 3, kGmmStageBytes = kGmmHalves * kGmmTileA + kGmmTileB;
+constexpr size_t kGmmSmemBytes = 1024 + (size_t)kGmmStages * kGmmStageBytes + 256;
 
 struct GmmBarriers {
-  uint64_t full[kGmmMaxStages], empty[kGmmMaxStages], acc_full[2], acc_empty[2];
+  uint64_t full[kGmmStages], empty[kGmmStages], acc_full, acc_empty;
   uint32_t tmem_base;
   int failed;
 };
@@ -56,7 +54,7 @@ struct GmmBarriers {
 struct GmmShared {
   int seg_src[kMaxExperts];        // [l * P + s] first row of the segment on its owner (staged x / returned output)
   int seg_dst[kMaxExperts + 1];    // [l * P + s] first row of the segment on this rank (exclusive prefix)
-  int tile0[kMaxExperts + 1];      // [l] first tile of local expert l
+  int tile0[kMaxExperts + 1];      // [l] first tile of local expert l ([L]: number of tiles)
   int alive, total_rows, num_tiles;
 };
 
@@ -151,6 +149,46 @@ __device__ __forceinline__ void build_layout(const GmmArgs& a, GmmShared& sh, in
   }
 }
 
+// The layout of a single rank: segments are experts, and every block derives all of it from the counts (no table, no tile
+// list in memory, no grid barrier).  Run by all threads; `cap` = rows that x and the output both hold.
+__device__ __forceinline__ void build_layout_local(const GmmArgs& a, GmmShared& sh, int cap) {
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {
+    long long rows = 0, tiles = 0;
+    for (int e0 = 0; e0 < a.E; e0 += 32) {
+      const int e = e0 + lane, c = e < a.E ? max(a.counts[e], 0) : 0, t = c / kGmmTileRows + (c % kGmmTileRows != 0);
+      long long row_sum = c, tile_sum = t;
+      for (int d = 1; d < 32; d <<= 1) {
+        const long long r = __shfl_up_sync(0xffffffffu, row_sum, d), q = __shfl_up_sync(0xffffffffu, tile_sum, d);
+        if (lane >= d) { row_sum += r; tile_sum += q; }
+      }
+      if (e < a.E) { sh.seg_dst[e] = (int)(rows + row_sum - c); sh.tile0[e] = (int)(tiles + tile_sum - t); }
+      rows += __shfl_sync(0xffffffffu, row_sum, 31);
+      tiles += __shfl_sync(0xffffffffu, tile_sum, 31);
+    }
+    if (lane == 0) {
+      sh.alive = rows <= cap;                        // otherwise no tile is worked on, and the numbers above are not read
+      if (!sh.alive && a.error_flag) *a.error_flag = 2;
+      sh.seg_dst[a.E] = (int)rows;
+      sh.tile0[a.E] = (int)tiles;
+      sh.total_rows = sh.alive ? (int)rows : 0;
+      sh.num_tiles = sh.alive ? (int)tiles : 0;
+    }
+  }
+  __syncthreads();
+}
+
+// (expert, first row, rows) of row tile mt: the last expert whose first tile is not behind it (empty experts are skipped).
+__device__ __forceinline__ int4 local_tile(const GmmShared& sh, int experts, int mt) {
+  int lo = 0, hi = experts;      // invariant: tile0[lo] <= mt < tile0[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (sh.tile0[mid] <= mt) lo = mid; else hi = mid;
+  }
+  const int row = sh.seg_dst[lo] + (mt - sh.tile0[lo]) * kGmmTileRows;
+  return make_int4(lo, row, min(kGmmTileRows, sh.seg_dst[lo + 1] - row), 0);
+}
+
 // Segment that holds gathered row r: the last i with seg_dst[i] <= r (empty segments share a start and are skipped).
 __device__ __forceinline__ int find_segment(const GmmShared& sh, int n, int r) {
   int lo = 0, hi = n;            // invariant: seg_dst[lo] <= r < seg_dst[hi]
@@ -172,7 +210,7 @@ __device__ __forceinline__ void pull_phase(const GmmArgs& a, const GmmShared& sh
       const int r = row0 + lane, seg = find_segment(sh, a.E, r), l = seg / P;
       src_rank = seg - l * P;
       src_row = sh.seg_src[seg] + (r - sh.seg_dst[seg]);
-      tile = sh.tile0[l] + (r - sh.seg_dst[l * P]) / gmm_tile_rows(false);
+      tile = sh.tile0[l] + (r - sh.seg_dst[l * P]) / kGmmTileRows;
     }
 #pragma unroll 1
     for (int c = 0; c < kGmmPullChunk; ++c) {
@@ -192,15 +230,14 @@ __device__ __forceinline__ void pull_phase(const GmmArgs& a, const GmmShared& sh
 
 // ---------------------------------------------------------------- the grouped GEMM
 // kPush = false: rows of the tile go to a.out on this rank.  kPush = true: each row goes to the rank it came from.
-template <bool kPush>
+// kLocal: the tiles come from the block's own layout instead of the list in memory.
+// A tile of at most 128 rows loads and multiplies its first half only (16 experts of 313 rows: 48 halves instead of 64).
+template <bool kPush, bool kLocal>
 __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh, const int* a_ready, uint8_t* smem_raw,
                                           int cta, int num_ctas) {
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* tiles = smem_raw + (((raw + 1023u) & ~1023u) - raw);       // tiles need 1024-byte alignment
-  constexpr int kGmmStages = gmm_stages(kPush);
-  constexpr int kHalves = gmm_tile_rows(kPush) / kGmmBM;      // 128-row halves of a tile, one accumulator each
-  constexpr int kGmmStageBytes = gmm_stage_bytes(kPush);
-  constexpr int kOffB = kHalves * kGmmTileA;                  // B follows the A halves inside a stage
+  constexpr int kOffB = kGmmHalves * kGmmTileA;               // B follows the A halves inside a stage
   uint8_t* epi_smem = tiles + (size_t)kGmmStages * kGmmStageBytes;
   GmmBarriers* bars = reinterpret_cast<GmmBarriers*>(epi_smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -208,7 +245,8 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kGmmStages; ++s) { mbar_init(&bars->full[s], 1); mbar_init(&bars->empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&bars->acc_full[b], 1); mbar_init(&bars->acc_empty[b], 8); }
+    mbar_init(&bars->acc_full, 1);
+    mbar_init(&bars->acc_empty, 8);
     bars->failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     umma::prefetch_tensormap(&a.tmap_a);
@@ -225,7 +263,10 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
   volatile int* failed = &bars->failed;
   const int n_tiles = (a.N + kGmmBN - 1) / kGmmBN, k_steps = a.K / kGmmBK;
   const int total_tiles = sh.num_tiles * n_tiles;
-  const int4* tile_info = reinterpret_cast<const int4*>(a.tile_info);
+  auto tile_info = [&](int mt) {
+    if constexpr (kLocal) return local_tile(sh, a.E, mt);
+    else return __ldcg(reinterpret_cast<const int4*>(a.tile_info) + mt);
+  };
 
   if (warp == 0) {
     // ============================================================ TMA producer
@@ -233,7 +274,8 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
       uint32_t it = 0;
       for (int tile = cta; tile < total_tiles && !*failed; tile += num_ctas) {
         const int mt = tile / n_tiles, nb = tile - mt * n_tiles;
-        const int4 info = __ldcg(tile_info + mt);
+        const int4 info = tile_info(mt);
+        const int halves = info.z > kGmmBM ? 2 : 1;
         if (a_ready) {
           if (!wait_rows_ready(a_ready + mt, info.z, failed)) break;
           fence_proxy_async();            // rows written by this GPU's pull warps are about to be read by the copy engine
@@ -242,9 +284,8 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
           const int s = it % kGmmStages;
           if (!bounded_wait(&bars->empty[s], ((it / kGmmStages) & 1u) ^ 1u, failed)) break;
           uint8_t* dst = tiles + (size_t)s * kGmmStageBytes;
-          mbar_expect_tx(&bars->full[s], kGmmStageBytes);
-#pragma unroll
-          for (int m = 0; m < kHalves; ++m)       // rows past the end of the operand are filled with zeros
+          mbar_expect_tx(&bars->full[s], halves * kGmmTileA + kGmmTileB);
+          for (int m = 0; m < halves; ++m)        // rows past the end of the operand are filled with zeros
             umma::tma_load_2d(dst + m * kGmmTileA, &a.tmap_a, ks * kGmmBK, info.y + m * kGmmBM, &bars->full[s]);
 #pragma unroll
           for (int j = 0; j < kGmmBN / 64; ++j)   // a box past the last column is filled with zeros
@@ -258,10 +299,8 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
       const uint32_t idesc = instr_desc_bf16(kGmmBM, kGmmBN);
       uint32_t it = 0, local_tile = 0;
       for (int tile = cta; tile < total_tiles && !*failed; tile += num_ctas, ++local_tile) {
-        // one accumulator pair per tile (256-row tiles) or two alternating accumulators (128-row tiles)
-        const uint32_t b = kHalves == 2 ? 0u : (local_tile & 1u);
-        const uint32_t use = kHalves == 2 ? local_tile : (local_tile >> 1);
-        if (!bounded_wait(&bars->acc_empty[b], (use & 1u) ^ 1u, failed)) break;
+        const int halves = tile_info(tile / n_tiles).z > kGmmBM ? 2 : 1;
+        if (!bounded_wait(&bars->acc_empty, (local_tile & 1u) ^ 1u, failed)) break;
         umma::fence_after_sync();
         for (int ks = 0; ks < k_steps; ++ks, ++it) {
           const int s = it % kGmmStages;
@@ -269,16 +308,15 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
           umma::fence_after_sync();
           const uint32_t a_addr = smem_u32(tiles + (size_t)s * kGmmStageBytes);
           const uint64_t db = smem_desc_mn_sw128(a_addr + kOffB, kGmmBoxB);
-#pragma unroll
-          for (int m = 0; m < kHalves; ++m) {
+          for (int m = 0; m < halves; ++m) {
             const uint64_t da = umma::smem_desc_sw128(a_addr + m * kGmmTileA);
 #pragma unroll
             for (int k = 0; k < kGmmBK / 16; ++k)   // A: 16 values = 32 bytes inside the swizzle row; B: 16 K-rows = 2048 bytes
-              mma_f16(tmem + (kHalves == 2 ? m : b) * kGmmBN, da + 2 * k, db + (uint64_t)(16 * 128 / 16) * k, idesc, ks > 0 || k > 0);
+              mma_f16(tmem + m * kGmmBN, da + 2 * k, db + (uint64_t)(16 * 128 / 16) * k, idesc, ks > 0 || k > 0);
           }
           umma::commit(&bars->empty[s]);
         }
-        umma::commit(&bars->acc_full[b]);
+        umma::commit(&bars->acc_full);
       }
     }
   } else {
@@ -290,16 +328,13 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
     uint32_t local_tile = 0;
     for (int tile = cta; tile < total_tiles && !*failed; tile += num_ctas, ++local_tile) {
       const int mt = tile / n_tiles, nb = tile - mt * n_tiles;
-      const int4 info = __ldcg(tile_info + mt);
-      const uint32_t b = kHalves == 2 ? 0u : (local_tile & 1u);
-      const uint32_t use = kHalves == 2 ? local_tile : (local_tile >> 1);
+      const int4 info = tile_info(mt);
       // This warp drains its 32 lanes of both accumulators (rows m * 128 + quad * 32 + lane); each thread stores its
       // row's columns straight from registers, 64 contiguous bytes per 32 columns, to this rank's output (a2av_gmm) or
       // into the receive area of the rank the row came from (gmm_a2av).
-      if (!bounded_wait(&bars->acc_full[b], use & 1u, failed)) break;
+      if (!bounded_wait(&bars->acc_full, local_tile & 1u, failed)) break;
       umma::fence_after_sync();
-#pragma unroll
-      for (int m = 0; m < kHalves; ++m) {
+      for (int m = 0; m * kGmmBM < info.z; ++m) {
         const int r = m * kGmmBM + row_in_tile;
         uint8_t* dst_row = nullptr;
         if (r < info.z) {
@@ -336,7 +371,7 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
       }
       umma::fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->acc_empty[b]);
+      if (lane == 0) mbar_arrive(&bars->acc_empty);
     }
     if (kPush) __threadfence_system();   // rows pushed to peers are visible before this rank signals them
   }
@@ -392,12 +427,12 @@ __global__ void __launch_bounds__(kGmmGemmThreads + kGmmPullWarps * 32, 1) a2av_
   if (threadIdx.x < P) ok = wait_flag_ge(&ctl->gmm_flag[threadIdx.x][0], epoch, ctx, kOpA2avGmm, 1, threadIdx.x);
   alive = __syncthreads_and(ok) && alive;
 
-  build_layout(a, sh, alive, min(a.gathered_cap, a.out_rows_cap), gmm_tile_rows(false));
+  build_layout(a, sh, alive, min(a.gathered_cap, a.out_rows_cap), kGmmTileRows);
   __threadfence();
   grid.sync();
 
   if (warp < kGmmGemmThreads / 32) {
-    gmm_phase<false>(a, sh, a.pulled, smem_raw, blockIdx.x, gridDim.x);
+    gmm_phase<false, false>(a, sh, a.pulled, smem_raw, blockIdx.x, gridDim.x);
   } else {
     __syncthreads();                               // pairs with the set-up barrier inside gmm_phase
     pull_phase(a, sh, blockIdx.x * kGmmPullWarps + (warp - kGmmGemmThreads / 32), gridDim.x * kGmmPullWarps);
@@ -431,10 +466,10 @@ __global__ void __launch_bounds__(kGmmGemmThreads, 1) gmm_a2av_kernel(const __gr
   if (threadIdx.x < P) ok = wait_flag_ge(&ctl->gmm_flag[threadIdx.x][2], epoch, ctx, kOpGmmA2av, 0, threadIdx.x);
   int alive = __syncthreads_and(ok);
 
-  build_layout(a, sh, alive, a.rows_in, gmm_tile_rows(true));
+  build_layout(a, sh, alive, a.rows_in, kGmmTileRows);
   __threadfence();
   grid.sync();
-  gmm_phase<true>(a, sh, nullptr, smem_raw, blockIdx.x, gridDim.x);
+  gmm_phase<true, false>(a, sh, nullptr, smem_raw, blockIdx.x, gridDim.x);
   __threadfence_system();
   grid.sync();
 
@@ -449,6 +484,35 @@ __global__ void __launch_bounds__(kGmmGemmThreads, 1) gmm_a2av_kernel(const __gr
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->epoch[kOpGmmA2av] = epoch;
 }
 
+// ---------------------------------------------------------------- both ops on a single rank
+// Rows sorted by global expert are already grouped by local expert, and every result belongs to this rank.  The general
+// kernels copy x twice and pass four grid barriers (a2av_gmm), or write the output into the receive area and copy it from
+// there (gmm_a2av); here x is the A operand and the epilogue writes the output.  32768 rows of 7168 x 4096, 4 experts: 1811 -> 1551 us;
+// 5003 rows of 2048 x 7168, 16 experts: 257 -> 213 us (of which a part is the second halves of short tiles left out).
+__global__ void __launch_bounds__(kGmmGemmThreads + kGmmPullWarps * 32, 1) gmm_local_kernel(const __grid_constant__ GmmParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ GmmShared sh;
+  const GmmArgs& a = p.r[0];
+  build_layout_local(a, sh, min(min(a.rows_in, a.out_rows_cap), a.gathered_cap));
+  if (threadIdx.x < kGmmGemmThreads) {
+    gmm_phase<false, true>(a, sh, nullptr, smem_raw, blockIdx.x, gridDim.x);
+  } else {
+    __syncthreads();                               // pairs with the set-up barrier inside gmm_phase
+    if (a.gathered) {                              // the caller wants the all-to-all-v result as well
+      const size_t n = (size_t)sh.total_rows * a.K / 8, stride = (size_t)gridDim.x * kGmmPullWarps * 32;
+      const int4* from = reinterpret_cast<const int4*>(a.x);
+      for (size_t i = (size_t)blockIdx.x * kGmmPullWarps * 32 + threadIdx.x - kGmmGemmThreads; i < n; i += 4 * stride) {
+        int4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (i + j * stride < n) v[j] = __ldcs(from + i + j * stride);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (i + j * stride < n) reinterpret_cast<int4*>(a.gathered)[i + j * stride] = v[j];
+      }
+    }
+    __syncthreads();                               // pairs with the tear-down barrier inside gmm_phase
+  }
+}
+
 static cudaError_t launch(const void* fn, int threads, size_t smem, const GmmParams& p, int nranks, int blocks, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -457,10 +521,17 @@ static cudaError_t launch(const void* fn, int threads, size_t smem, const GmmPar
   return cudaLaunchCooperativeKernel(fn, grid, block, args, smem, stream);
 }
 cudaError_t launch_a2av_gmm(const GmmParams& p, int nranks, int blocks, cudaStream_t stream) {
-  return launch((const void*)a2av_gmm_kernel, kGmmGemmThreads + kGmmPullWarps * 32, gmm_smem_bytes(false), p, nranks, blocks, stream);
+  return launch((const void*)a2av_gmm_kernel, kGmmGemmThreads + kGmmPullWarps * 32, kGmmSmemBytes, p, nranks, blocks, stream);
 }
 cudaError_t launch_gmm_a2av(const GmmParams& p, int nranks, int blocks, cudaStream_t stream) {
-  return launch((const void*)gmm_a2av_kernel, kGmmGemmThreads, gmm_smem_bytes(true), p, nranks, blocks, stream);
+  return launch((const void*)gmm_a2av_kernel, kGmmGemmThreads, kGmmSmemBytes, p, nranks, blocks, stream);
+}
+
+cudaError_t launch_gmm_local(const GmmParams& p, int blocks, cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(gmm_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGmmSmemBytes);
+  if (e != cudaSuccess) return e;
+  gmm_local_kernel<<<blocks, kGmmGemmThreads + kGmmPullWarps * 32, kGmmSmemBytes, stream>>>(p);
+  return cudaGetLastError();
 }
 
 bool encode_bf16_map(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows, const char** error) {

@@ -145,7 +145,8 @@ class GmmEngine:
             g = gathered[i] if gathered is not None and gathered[i] is not None else self._gathered(i, outs[i].shape[0], xs[i].shape[1])
             used.append(g)
             d = self._common(i, xs[i], weights[i], counts[i], outs[i], num_experts)
-            d.update(gathered=g.data_ptr() if g.numel() else weights[i].data_ptr(), gathered_cap=g.shape[0])
+            d.update(gathered=g.data_ptr() if g.numel() else weights[i].data_ptr(), gathered_cap=g.shape[0],
+                     gathered_wanted=gathered is not None and gathered[i] is not None and g.numel() > 0)
             args.append(d)
         self.C.a2av_gmm(self.layout, self.sessions, args, self.blocks, stream.cuda_stream)
         return used

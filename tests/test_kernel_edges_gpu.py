@@ -96,3 +96,58 @@ def test_padding_rows_are_zero(payload, alignment, experts):
             assert bits_equal(g[:rows][used.to(dev)], e[used]), "a token's row differs"
             assert not bool(g.view(torch.uint8)[:rows][~used.to(dev)].any()) and not bool(g.view(torch.uint8)[rows:].any())
     buf.destroy()
+
+
+@pytest.mark.parametrize("counts,k,n", [
+    ([1], 64, 64),                                   # one row, one step, a quarter of a tile
+    ([128, 0, 129, 256, 257, 0, 127], 192, 320),     # both sides of a half tile and of a tile, empty experts, a short last tile
+    ([0, 0, 0], 128, 64),
+    ([3] * 300 + [700], 64, 576),                    # more experts than one scan step, many tiles per block
+])
+def test_grouped_gemm_on_one_rank(counts, k, n):
+    """Both operators on a single rank against float32 (bf16 results: 2^-8 relative, sums of k products: 1e-5 of their size), with
+    the gathered rows handed out; an output that overlaps x takes the general kernels and gives the same bits."""
+    from deepep_b200.ops import ep_gmm_fused as G
+    from deepep_b200.ops import load_native
+
+    C, dev, rows, E = load_native(), torch.device("cuda"), sum(counts), len(counts)
+    layout = C.make_mega_layout(1, 1, 128, 1, G.GmmEngine.region_bytes(C, max(rows, 1), max(k, n), max(k, n)))
+    s = C.Session(0, 1, layout.total, 20.0)
+    s.attach_peers([s.workspace])
+    try:
+        eng = G.GmmEngine([s], layout, dev, max(rows, 1), max(k, n), max(k, n))
+        gen = torch.Generator().manual_seed(rows + k)
+        x = torch.randn((rows, k), generator=gen).bfloat16()
+        w = torch.randn((E, k, n), generator=gen).bfloat16()
+        want, size, at = torch.zeros((rows, n)), torch.zeros((rows, n)), 0
+        for e, c in enumerate(counts):
+            want[at:at + c] = x[at:at + c].float() @ w[e].float()
+            size[at:at + c] = x[at:at + c].float().abs() @ w[e].float().abs()
+            at += c
+        dx, dw, dc = x.to(dev), w.to(dev), torch.tensor(counts, dtype=torch.int32, device=dev)
+        gathered, outs = torch.full_like(dx, 7.0), []
+        for _ in range(2):
+            out, back = (torch.full((rows, n), 5.0, dtype=torch.bfloat16, device=dev) for _ in range(2))
+            eng.a2av_gmm([dx], [dw], [dc], [out], [gathered], num_experts=E)
+            eng.gmm_a2av([dx], [dw], [dc], [back], num_experts=E)
+            outs += [out, back]
+        memory = torch.zeros((rows * max(k, n),), dtype=torch.bfloat16, device=dev)       # x and the output start at one address
+        shared_x, shared_out = memory[:rows * k].view(rows, k), memory[:rows * n].view(rows, n)
+        for op in (eng.a2av_gmm, eng.gmm_a2av):
+            shared_x.copy_(dx)
+            op([shared_x], [dw], [dc], [shared_out], num_experts=E)
+            outs.append(shared_out.clone())
+        eng.check()
+        assert bits_equal(gathered, x)
+        assert torch.all((outs[0].cpu().float() - want).abs() <= want.abs() * 2 ** -8 + 1e-5 * size)
+        for other in outs[1:]:
+            assert torch.equal(other, outs[0])
+        if rows:                                         # more rows than x holds: reported, and nothing is written
+            out = torch.full((rows, n), 5.0, dtype=torch.bfloat16, device=dev)
+            eng.gmm_a2av([dx], [dw], [dc + rows], [out], num_experts=E)
+            with pytest.raises(RuntimeError, match="row counts"):
+                eng.check()
+            assert bool((out == 5.0).all())
+    finally:
+        torch.cuda.synchronize()
+        s.close()
