@@ -245,32 +245,26 @@ __device__ __forceinline__ void finish_phase(const MegaFinishArgs& a, bool bump_
     const int* idx = reinterpret_cast<const int*>(ctx.ws[me] + a.in_off + in.idx);
     const float* w = reinterpret_cast<const float*>(ctx.ws[me] + a.in_off + in.w);
     const uint8_t* comb = ctx.ws[me] + a.comb_off;
-    // small batches: several warps share a token, each reduces a span of columns (a multiple of the 64-piece step)
-    const int units = H / 8;
-    const int parts = max(1, min(8, total_warps / max(a.T, 1)));
-    const int span = ((units + parts * 64 - 1) / (parts * 64)) * 64;
-    for (int item = gw; item < a.T * parts; item += total_warps) {
-      const int t = item / parts, part = item - t * parts;
-      if (part * span >= units) continue;
-      const int u_end = min(units, (part + 1) * span);
-      // lane k holds slot k: its weight and whether it counts (shared experts: every token, weight one)
-      float w_mine = 0.f;
-      bool counts = false;
-      if (lane < K) {
-        const int e = idx[(size_t)t * K + lane];
-        w_mine = w[(size_t)t * K + lane];
-        counts = e >= 0 && e < a.E;
-      } else if (lane < Kp) {
-        w_mine = 1.f;
-        counts = true;
-      }
+    // A work item is a span of 64 16-byte pieces of one token, dealt out statically: whole tokens were 2.3 waves of warps at
+    // 4096 tokens (layer 2013 us, in spans 1999).  Slot and weight of the next item are fetched while this one is summed.
+    const int units = H / 8, spans = (units + 63) / 64, items = a.T * spans;
+    // lane k holds slot k: its weight and whether it counts (shared experts: every token, weight one)
+    auto slot_of = [&](int item) { return lane < K && item < items ? __ldg(idx + (size_t)(item / spans) * K + lane) : -1; };
+    auto weight_of = [&](int item) { return lane < K && item < items ? __ldg(w + (size_t)(item / spans) * K + lane) : 1.f; };
+    int e_next = slot_of(gw);
+    float w_next = weight_of(gw);
+    for (int item = gw; item < items; item += total_warps) {
+      const int t = item / spans, ub = (item - t * spans) * 64, e = e_next;
+      const float w_mine = w_next;
+      e_next = slot_of(item + total_warps);
+      w_next = weight_of(item + total_warps);
+      const bool counts = lane < K ? (e >= 0 && e < a.E) : lane < Kp;
       const unsigned valid = __ballot_sync(0xffffffffu, counts);
       int4* out = reinterpret_cast<int4*>(reinterpret_cast<uint8_t*>(a.y) + (size_t)t * H * 2);
       const uint8_t* rows = comb + (size_t)t * Kp * H * 2;
-      // two 16-byte columns per lane and step; the trip count is the same for every lane, which all take part in the shuffles
-      for (int ub = part * span; ub < u_end; ub += 64) {
+      {                                        // two 16-byte columns per lane; every lane takes part in the shuffles
         const int u0 = ub + lane;
-        const bool one = u0 < u_end, two = u0 + 32 < u_end;
+        const bool one = u0 < units, two = u0 + 32 < units;
         float a0[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, a1[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int kb = 0; kb < Kp; kb += 8) {     // eight slots' loads in flight at a time
           int4 v0[8], v1[8];
