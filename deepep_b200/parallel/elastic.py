@@ -81,6 +81,11 @@ class EPHandle:
     def _tracked(self) -> List[torch.Tensor]:
         return [] if self._plan is None else list(self._plan.tensors())
 
+    def _kept(self) -> List[torch.Tensor]:
+        """The tensors an asynchronous call keeps alive until its event has been waited for."""
+        private = getattr(self._plan, "private_tensors", None)
+        return self._tracked() + (private() if private is not None else [])
+
     def _check_unchanged(self) -> None:
         now = tuple(self._stamp(t) for t in self._tracked())
         if now != self._snapshots:
@@ -443,7 +448,7 @@ class ElasticBuffer:
             recv_sf = _col_major(recv_sf)
         out_x = recv_x if recv_sf is None else (recv_x, recv_sf.view(torch.int32) if packed else recv_sf)
         event = self._leave(comm, async_with_compute_stream, [recv_x, recv_sf, recv_w, recv_idx, x_data, x_sf, topk_idx,
-                                                               topk_weights] + h._tracked(), allocate_on_comm_stream)
+                                                               topk_weights] + h._kept(), allocate_on_comm_stream)
         return out_x, recv_idx, recv_w, h, event
 
     def _note_failure(self, exc: Exception) -> None:
@@ -471,7 +476,7 @@ class ElasticBuffer:
                 recv_x, recv_sf = self.engine.dispatch([x_data if x_sf is None else (x_data, x_sf)], [handle._plan], mode,
                                                        blocks=num_sms or self.num_sms, stream=comm)[0]
         out_x = recv_x if recv_sf is None else (recv_x, recv_sf.view(torch.int32) if packed else recv_sf)
-        event = self._leave(comm, async_with_compute_stream, [recv_x, recv_sf, x_data, x_sf] + handle._tracked(),
+        event = self._leave(comm, async_with_compute_stream, [recv_x, recv_sf, x_data, x_sf] + handle._kept(),
                             allocate_on_comm_stream)
         return out_x, None, None, handle, event
 
@@ -485,7 +490,7 @@ class ElasticBuffer:
         recv_w = plan.recv_w[:rows]
         out_x = recv_x if recv_sf is None else (recv_x, recv_sf.view(torch.int32) if packed else recv_sf)
         event = self._leave(comm, async_with_compute_stream, [recv_x, recv_sf, recv_w, x_data, x_sf, topk_idx, topk_weights]
-                            + h._tracked(), allocated_on_comm)
+                            + h._kept(), allocated_on_comm)
         return out_x, None, recv_w, h, event
 
     def _make_handle(self, plan, expand, num_experts, alignment, num_sms, topk_idx, tokens, low_latency) -> EPHandle:
@@ -555,7 +560,7 @@ class ElasticBuffer:
                                                  blocks=num_sms or self.num_sms, stream=comm,
                                                  **({"split": split} if split is not None else {}))[0]
         event = self._leave(comm, async_with_compute_stream, [out, out_w, x, topk_weights] + [b for b in biases if b is not None]
-                            + handle._tracked(), allocate_on_comm_stream)
+                            + handle._kept(), allocate_on_comm_stream)
         return out, out_w, event
 
     # ------------------------------------------------------------------ validation helpers

@@ -78,7 +78,11 @@ class RoutingPlan:
     def tensors(self):
         return [t for t in (self.topk_idx, self.send_slot, self.slot_row, self.stage_meta, self.chunk_start, self.rank_tokens,
                             self.rank_rows, self.expert_counts, self.expert_offsets, self.recv_row_src, self.recv_w,
-                            self.recv_idx, self.num_rows_dev, self.local_row) if t is not None]
+                            self.recv_idx) if t is not None]
+
+    def private_tensors(self):
+        """What only the kernels write: kept alive with the others, but nothing a caller could change."""
+        return [] if self.local_row is None else [self.num_rows_dev, self.local_row]
 
 
 def _ptr(t: Optional[torch.Tensor]):
