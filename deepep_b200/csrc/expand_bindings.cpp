@@ -24,8 +24,8 @@ void check_launch(cudaError_t e, const char* what) {
 void bind_expand(py::module_& m) {
   m.def("swiglu", [](const py::dict& d, bool backward, int blocks, uintptr_t stream) {
     SwigluParams p{};
-    p.gu = eptr<const __nv_bfloat16>(d, "gu"); p.w = eptr<const float>(d, "w"); p.h = eptr<__nv_bfloat16>(d, "h");
-    p.dh = eptr<const __nv_bfloat16>(d, "dh"); p.dgu = eptr<__nv_bfloat16>(d, "dgu"); p.dw = eptr<float>(d, "dw");
+    p.gu = eptr<const __nv_bfloat16>(d, "gu"); p.h = eptr<__nv_bfloat16>(d, "h");
+    p.dh = eptr<const __nv_bfloat16>(d, "dh"); p.dgu = eptr<__nv_bfloat16>(d, "dgu");
     p.rows = d["rows"].cast<long long>(); p.inter = d["inter"].cast<int>();
     if (p.rows < 0 || p.inter < 8 || p.inter % 8) throw std::invalid_argument("swiglu: the width must be a positive multiple of 8");
     if (p.rows > 0 && (!p.gu || (backward ? !p.dh || !p.dgu : !p.h))) throw std::invalid_argument("swiglu: a tensor is missing");

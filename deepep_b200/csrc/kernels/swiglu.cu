@@ -1,11 +1,8 @@
-// silu(gate) * up * w over rows of [gate | up], and its backward pass (see swiglu_api.h).
+// silu(gate) * up over rows of [gate | up], and its backward pass (see swiglu_api.h).
 //
 // Bound by memory: forward reads 4 and writes 2 bytes per value, backward reads 6 and writes 4.  One warp per row, 16-byte
-// accesses, all arithmetic in fp32 with one rounding at the end; the row factor joins here, where a row is `inter` values
-// wide, so that neither the layer's output nor its gradient needs a pass of its own for it, and the factor's gradient is the
-// row sum of dh * silu(gate) * up, which backward has in registers.  As library passes over the two strided halves (silu,
-// product, factor, their gradients and a concatenation) the same work took 2.36 ms of a 7.6 ms training step (8192 tokens,
-// hidden 4096, 49152 rows, inter 1536); here forward takes 75 and backward 116 us (6.0 and 6.5 TB/s).
+// accesses, all arithmetic in fp32 with one rounding at the end.  As library passes over the two strided halves (silu,
+// product, their gradients and a concatenation) the same traffic is several passes.
 #include "swiglu_api.h"
 
 namespace dep {
@@ -34,8 +31,6 @@ __global__ void __launch_bounds__(kSwigluThreads) swiglu_kernel(const __grid_con
   const long long warps = (long long)gridDim.x * (kSwigluThreads / 32);
   for (long long row = (long long)blockIdx.x * (kSwigluThreads / 32) + (threadIdx.x >> 5); row < p.rows; row += warps) {
     const int4* gate = reinterpret_cast<const int4*>(p.gu) + row * 2 * units;
-    const float w = p.w ? __ldg(p.w + row) : 1.f;
-    float dw = 0.f;
     constexpr int U = 2;                       // 16-byte pieces of every operand in flight per lane
     for (int u0 = lane; u0 < units; u0 += 32 * U) {
       int4 g4[U], u4[U], d4[U];
@@ -56,28 +51,22 @@ __global__ void __launch_bounds__(kSwigluThreads) swiglu_kernel(const __grid_con
         if (!kBackward) {
           Vec8 h;
 #pragma unroll
-          for (int e = 0; e < 8; ++e) h.v[e] = __fdividef(g.v[e], 1.f + __expf(-g.v[e])) * up.v[e] * w;
+          for (int e = 0; e < 8; ++e) h.v[e] = __fdividef(g.v[e], 1.f + __expf(-g.v[e])) * up.v[e];
           reinterpret_cast<int4*>(p.h)[row * units + u] = pack8(h);
         } else {
           const Vec8 d = unpack8(d4[i]);
           Vec8 dg, du;
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            const float s = __fdividef(1.f, 1.f + __expf(-g.v[e])), silu = g.v[e] * s, dy = d.v[e] * w;
-            dw += d.v[e] * (silu * up.v[e]);
-            du.v[e] = dy * silu;
-            dg.v[e] = dy * up.v[e] * (s * (1.f + g.v[e] * (1.f - s)));
+            const float s = __fdividef(1.f, 1.f + __expf(-g.v[e])), silu = g.v[e] * s;
+            du.v[e] = d.v[e] * silu;
+            dg.v[e] = d.v[e] * up.v[e] * (s * (1.f + g.v[e] * (1.f - s)));
           }
           int4* out = reinterpret_cast<int4*>(p.dgu) + row * 2 * units;
           out[u] = pack8(dg);
           out[units + u] = pack8(du);
         }
       }
-    }
-    if (kBackward && p.dw) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) dw += __shfl_xor_sync(0xffffffffu, dw, o);
-      if (lane == 0) p.dw[row] = dw;
     }
   }
 }

@@ -1,4 +1,4 @@
-// SwiGLU with a per-row factor, forward and backward (the expert activation of the training layer).
+// SwiGLU forward and backward (the expert activation of the training layer).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -7,11 +7,9 @@ namespace dep {
 
 struct SwigluParams {
   const __nv_bfloat16* gu;     // [rows][2 * inter]: gate columns, then up columns
-  const float* w;              // [rows] factor of every row, or null (one)
-  __nv_bfloat16* h;            // forward: [rows][inter] = silu(gate) * up * w
+  __nv_bfloat16* h;            // forward: [rows][inter] = silu(gate) * up
   const __nv_bfloat16* dh;     // backward: [rows][inter] gradient of h
   __nv_bfloat16* dgu;          // backward: [rows][2 * inter]
-  float* dw;                   // backward: [rows] gradient of w, or null
   long long rows;
   int inter, pad;              // inter: a multiple of 8
 };

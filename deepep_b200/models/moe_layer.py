@@ -6,8 +6,6 @@ The reference documents the rule (``README.md:168-219``, ``docs/elastic.md:7-17`
 """
 from __future__ import annotations
 
-from typing import Optional
-
 import torch
 
 from ..parallel.elastic import ElasticBuffer
@@ -46,63 +44,55 @@ class _Combine(torch.autograd.Function):
 
 
 class _Swiglu(torch.autograd.Function):
-    """``silu(gate) * up * w`` of bf16 rows ``[gate | up]`` with an fp32 factor per row, one kernel each way."""
+    """``silu(gate) * up`` of bf16 rows ``[gate | up]``, one kernel each way."""
 
     @staticmethod
-    def forward(ctx, gate_up, row_weights):
-        from ..ops import require_native
-
+    def forward(ctx, gate_up):
         rows, width = gate_up.shape
         h = gate_up.new_empty((rows, width // 2))
-        ctx.save_for_backward(gate_up, row_weights)
-        require_native("the expert activation").swiglu(
-            dict(gu=gate_up.data_ptr(), w=None if row_weights is None else row_weights.data_ptr(), h=h.data_ptr(), rows=rows,
-                 inter=width // 2), False, _blocks(gate_up.device), torch.cuda.current_stream(gate_up.device).cuda_stream)
+        ctx.save_for_backward(gate_up)
+        _launch(gate_up, False, h=h)
         return h
 
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, grad):
-        from ..ops import require_native
-
-        gate_up, row_weights = ctx.saved_tensors
-        rows, width = gate_up.shape
+        gate_up, = ctx.saved_tensors
         grad = grad.contiguous()
         if grad.data_ptr() % 16:
             grad = grad.clone()
         out = torch.empty_like(gate_up)
-        out_w = torch.empty_like(row_weights) if row_weights is not None and ctx.needs_input_grad[1] else None
-        require_native("the expert activation").swiglu(
-            dict(gu=gate_up.data_ptr(), w=None if row_weights is None else row_weights.data_ptr(), dh=grad.data_ptr(),
-                 dgu=out.data_ptr(), dw=None if out_w is None else out_w.data_ptr(), rows=rows, inter=width // 2),
-            True, _blocks(gate_up.device), torch.cuda.current_stream(gate_up.device).cuda_stream)
-        return out, out_w
+        _launch(gate_up, True, dh=grad, dgu=out)
+        return out
 
 
-def _blocks(device) -> int:
-    return torch.cuda.get_device_properties(device).multi_processor_count * 8
+def _launch(gate_up: torch.Tensor, backward: bool, **tensors) -> None:
+    from ..ops import require_native
+
+    device = gate_up.device
+    rows, width = gate_up.shape
+    args = dict(gu=gate_up.data_ptr(), rows=rows, inter=width // 2, **{name: t.data_ptr() for name, t in tensors.items()})
+    with torch.cuda.device(device):
+        require_native("the expert activation").swiglu(args, backward, torch.cuda.get_device_properties(device).multi_processor_count * 8,
+                                                       torch.cuda.current_stream(device).cuda_stream)
 
 
-def _activate(gate_up: torch.Tensor, row_weights: Optional[torch.Tensor]) -> torch.Tensor:
-    """``silu(gate) * up`` times the rows' factors.  The kernel takes bf16 rows that are contiguous, 16-byte aligned and a
-    multiple of 8 values wide, with fp32 factors; anything else goes through torch."""
+def _activate(gate_up: torch.Tensor) -> torch.Tensor:
+    """``silu(gate) * up``.  The kernel takes bf16 rows that are contiguous, 16-byte aligned and a multiple of 8 values wide;
+    anything else goes through torch."""
     inter = gate_up.shape[1] // 2
     if (gate_up.is_cuda and gate_up.dtype == torch.bfloat16 and gate_up.is_contiguous() and inter % 8 == 0 and inter > 0
-            and gate_up.data_ptr() % 16 == 0
-            and (row_weights is None or (row_weights.dtype == torch.float32 and row_weights.is_contiguous()))):
-        return _Swiglu.apply(gate_up, row_weights)
+            and gate_up.data_ptr() % 16 == 0):
+        return _Swiglu.apply(gate_up)
     gate, up = gate_up.chunk(2, dim=-1)
-    h = torch.nn.functional.silu(gate) * up
-    return h if row_weights is None else h * row_weights.unsqueeze(1).to(h.dtype)
+    return torch.nn.functional.silu(gate) * up
 
 
 class ExpertParallelMoE(torch.nn.Module):
     """SwiGLU experts sharded over the ranks of ``buffer``; forward = dispatch -> local experts -> combine.
 
     ``w1 [L, 2I, H]`` holds gate rows then up rows, ``w2 [L, H, I]``; both bf16, Kaiming-uniform.
-    The routing weight multiplies each expert output row before combine (whose reduction is unweighted); with the grouped
-    GEMM it joins the activation instead, where a row is narrower and no pass of its own is needed:
-    ``(w * h) @ w2^T == w * (h @ w2^T)``.
+    The routing weight multiplies each expert output row before combine (whose reduction is unweighted).
     """
 
     def __init__(self, buffer: ElasticBuffer, num_experts: int, hidden: int, intermediate: int, device=None):
@@ -117,11 +107,10 @@ class ExpertParallelMoE(torch.nn.Module):
         self.w1, self.w2 = torch.nn.Parameter(w1), torch.nn.Parameter(w2)
         self.use_grouped_mm = None        # decided at the first GPU forward (set it to False to force the per-expert loop)
 
-    def experts(self, rows: torch.Tensor, psum: torch.Tensor, counts=None, row_weights: Optional[torch.Tensor] = None) -> torch.Tensor:
+    def experts(self, rows: torch.Tensor, psum: torch.Tensor, counts=None) -> torch.Tensor:
         """SwiGLU experts on expert-major rows.  On a GPU with a usable library grouped GEMM both projections are one
         ``torch._grouped_mm`` each (row ranges from the handle's cumulative counts, which stay on the device);
-        otherwise a loop over the experts with the host-side counts of the handle (no device synchronisation).
-        ``row_weights`` (fp32, optional) multiply the rows of the result."""
+        otherwise a loop over the experts with the host-side counts of the handle (no device synchronisation)."""
         if rows.is_cuda and self.use_grouped_mm is None:
             from ..utils.grouped_mm import grouped_mm_usable
 
@@ -129,7 +118,7 @@ class ExpertParallelMoE(torch.nn.Module):
         if rows.is_cuda and self.use_grouped_mm and rows.shape[0] > 0:
             offs = psum.to(torch.int32)
             gate_up = torch._grouped_mm(rows, self.w1.transpose(1, 2), offs=offs)
-            return torch._grouped_mm(_activate(gate_up, row_weights), self.w2.transpose(1, 2), offs=offs)
+            return torch._grouped_mm(_activate(gate_up), self.w2.transpose(1, 2), offs=offs)
         bounds = [0]
         for c in (counts if counts is not None else torch.diff(psum, prepend=psum.new_zeros(1)).tolist()):
             bounds.append(bounds[-1] + int(c))
@@ -138,17 +127,12 @@ class ExpertParallelMoE(torch.nn.Module):
             seg = rows[bounds[e]:bounds[e + 1]]
             gate, up = (seg @ self.w1[e].t()).chunk(2, dim=-1)
             outs.append((torch.nn.functional.silu(gate) * up) @ self.w2[e].t())
-        y = torch.cat(outs, dim=0) if outs else rows.new_zeros((0, self.w2.shape[1]))
-        return y if row_weights is None else y * row_weights.unsqueeze(1).to(y.dtype)
+        return torch.cat(outs, dim=0) if outs else rows.new_zeros((0, self.w2.shape[1]))
 
     def forward(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: torch.Tensor) -> torch.Tensor:
         holder = {}
         recv_x, recv_w, psum = _Dispatch.apply(self.buffer, x, topk_idx, topk_weights, self.num_experts, holder)
-        counts = holder["handle"].num_recv_tokens_per_expert_list
-        if type(self).experts is ExpertParallelMoE.experts:
-            y = self.experts(recv_x, psum, counts, recv_w)
-        else:                             # a subclass with experts of its own returns rows without weights
-            y = self.experts(recv_x, psum, counts) * recv_w.unsqueeze(1).to(recv_x.dtype)
+        y = self.experts(recv_x, psum, holder["handle"].num_recv_tokens_per_expert_list) * recv_w.unsqueeze(1).to(recv_x.dtype)
         return _Combine.apply(self.buffer, y.contiguous(), holder["handle"])
 
 

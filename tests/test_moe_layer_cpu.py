@@ -2,6 +2,7 @@
 import os
 import socket
 
+import pytest
 import torch
 import torch.distributed as dist
 import torch.multiprocessing as mp
@@ -84,3 +85,29 @@ def test_moe_layer_forward_backward():
         results = m.dict()
         mp.spawn(_worker, args=(world, port, results), nprocs=world, join=True)
         assert dict(results) == {0: True, 1: True}
+
+
+@pytest.mark.parametrize("where", ["instance", "class", "subclass"])
+def test_experts_can_be_replaced(monkeypatch, where):
+    """The layer calls ``experts(rows, psum, counts)``, wherever the method comes from, and applies the routing weight itself."""
+    from deepep_b200 import ElasticBuffer
+    from deepep_b200.models.moe_layer import ExpertParallelMoE
+
+    def doubled(rows, psum, counts):
+        assert len(counts) == E and int(psum[-1]) == rows.shape[0]
+        return rows * 2
+
+    kind = ExpertParallelMoE
+    if where == "class":
+        monkeypatch.setattr(ExpertParallelMoE, "experts", lambda self, rows, psum, counts: doubled(rows, psum, counts))
+    elif where == "subclass":
+        kind = type("Doubling", (ExpertParallelMoE,), {"experts": lambda self, rows, psum, counts: doubled(rows, psum, counts)})
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=512, hidden=H, num_topk=K, explicitly_destroy=True, device="cpu")
+    layer = kind(buf, E, H, I)
+    if where == "instance":
+        layer.experts = doubled
+    x, idx, w = _inputs(3)
+    y = layer(x, idx, w)
+    want = 2 * x.float() * w.bfloat16().float().sum(1, keepdim=True)
+    assert torch.allclose(y.float(), want, rtol=0.02, atol=0.02)
+    buf.destroy()
