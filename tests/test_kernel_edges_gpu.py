@@ -38,27 +38,50 @@ def test_high_throughput_splits(world, tokens, hidden, experts, topk, kw):
     run_case(world, tokens, hidden, experts, topk, "invalid", repeats=2, **kw)
 
 
+def _torch_activation(gate_up, grad):
+    x = gate_up.detach().requires_grad_()
+    gate, up = x.chunk(2, dim=-1)
+    h = torch.nn.functional.silu(gate) * up
+    h.backward(grad)
+    return h.detach(), x.grad
+
+
+def _same_values(a, b):
+    """Equal bit for bit, or both NaN."""
+    return bool(((a.view(torch.int16) == b.view(torch.int16)) | (a.isnan() & b.isnan())).all())
+
+
 @pytest.mark.parametrize("rows,inter", [(1, 8), (33, 264), (4, 1536), (2400, 520)])
 def test_expert_activation(rows, inter):
-    """silu(gate) * up and its gradient against float64.  The kernel works in fp32 and rounds once, so a bf16 result is within
-    half a step (2^-9 of its size) plus the fp32 error of its terms; 2^-8 and 1e-5 of the terms' sizes cover both, the exponential
-    (2^-21) included."""
+    """silu(gate) * up and its gradient are those of the separate bf16 operations, bit for bit."""
     from deepep_b200.models.moe_layer import _activate
 
     gen = torch.Generator().manual_seed(rows + inter)
-    gu = (3 * torch.randn((rows, 2 * inter), generator=gen)).bfloat16()
-    gu[0, 0], gu[0, inter - 1] = 120.0, -120.0                 # the exponential overflows, or vanishes
-    dh = torch.randn((rows, inter), generator=gen).bfloat16()
-    x = gu.cuda().requires_grad_()
+    gu = (3 * torch.randn((rows, 2 * inter), generator=gen)).bfloat16().cuda()
+    dh = torch.randn((rows, inter), generator=gen).bfloat16().cuda()
+    x = gu.clone().requires_grad_()
     h = _activate(x)
-    h.backward(dh.cuda())
-    g64 = gu.double().requires_grad_()
-    gate, up = g64.chunk(2, dim=1)
-    want = torch.nn.functional.silu(gate) * up
-    want.backward(dh.double())
-    assert torch.all((h.detach().cpu().double() - want.detach()).abs() <= want.detach().abs() * 2 ** -8 + 1e-30)
-    size = dh.double().abs() * (1 + gate.detach().abs()) * (1 + up.detach().abs())
-    assert torch.all((x.grad.cpu().double() - g64.grad).abs() <= g64.grad.abs() * 2 ** -8 + 1e-5 * torch.cat([size, size], dim=1))
+    h.backward(dh)
+    want, grad = _torch_activation(gu, dh)
+    assert _same_values(h.detach(), want) and _same_values(x.grad, grad)
+
+
+def test_expert_activation_of_every_gate_value():
+    """All 65536 bf16 gates (subnormals, infinities and NaN included) against ups and gradients of every size, special ones too."""
+    from deepep_b200.models.moe_layer import _activate
+
+    gen = torch.Generator().manual_seed(5)
+    gate = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    cols = 256
+    anything = lambda: torch.randint(-32768, 32768, (65536, cols), generator=gen, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    usual = lambda: torch.randn((65536, cols), generator=gen).bfloat16()
+    for up, dh in ((usual(), usual()), (anything(), usual()), (anything(), anything())):
+        gu = torch.cat([gate.unsqueeze(1).expand(-1, cols), up], dim=1).contiguous().cuda()
+        x = gu.clone().requires_grad_()
+        h = _activate(x)
+        h.backward(dh.cuda())
+        want, grad = _torch_activation(gu, dh.cuda())
+        assert _same_values(h.detach(), want) and _same_values(x.grad, grad)
 
 
 @pytest.mark.parametrize("payload", ["bf16", "fp8", "fp8_fused"])
