@@ -55,9 +55,13 @@ class _Swiglu(torch.autograd.Function):
         return h
 
     @staticmethod
-    @torch.autograd.function.once_differentiable
     def backward(ctx, grad):
         gate_up, = ctx.saved_tensors
+        again = torch.is_grad_enabled()                  # the gradient will be differentiated itself
+        if again or not _ordinary(gate_up, grad):
+            with torch.enable_grad():
+                h = _separate_operations(gate_up)
+            return torch.autograd.grad(h, gate_up, grad, create_graph=again)[0]
         grad = grad.contiguous()
         if grad.data_ptr() % 16:
             grad = grad.clone()
@@ -77,15 +81,29 @@ def _launch(gate_up: torch.Tensor, backward: bool, **tensors) -> None:
                                                        torch.cuda.current_stream(device).cuda_stream)
 
 
-def _activate(gate_up: torch.Tensor) -> torch.Tensor:
-    """``silu(gate) * up``.  The kernel takes bf16 rows that are contiguous, 16-byte aligned and a multiple of 8 values wide;
-    anything else goes through torch."""
-    inter = gate_up.shape[1] // 2
-    if (gate_up.is_cuda and gate_up.dtype == torch.bfloat16 and gate_up.is_contiguous() and inter % 8 == 0 and inter > 0
-            and gate_up.data_ptr() % 16 == 0):
-        return _Swiglu.apply(gate_up)
+def _ordinary(*tensors: torch.Tensor) -> bool:
+    """Tensors whose memory a kernel can read, in a call that nobody traces, batches or differentiates forward: a kernel behind
+    an address is invisible to all of these."""
+    return (all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors)
+            and torch._C._len_torch_dispatch_stack() == 0 and not torch._C._are_functorch_transforms_active()
+            and not any(torch._C._functorch.is_legacy_batchedtensor(t) for t in tensors)
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
+            and not any(torch.autograd.forward_ad.unpack_dual(t).tangent is not None for t in tensors))
+
+
+def _separate_operations(gate_up: torch.Tensor) -> torch.Tensor:
     gate, up = gate_up.chunk(2, dim=-1)
     return torch.nn.functional.silu(gate) * up
+
+
+def _activate(gate_up: torch.Tensor) -> torch.Tensor:
+    """``silu(gate) * up``.  The kernel takes bf16 rows that are contiguous, 16-byte aligned and a multiple of 8 values wide;
+    anything else goes through torch, with the same results."""
+    inter = gate_up.shape[1] // 2
+    if (_ordinary(gate_up) and gate_up.is_cuda and gate_up.dtype == torch.bfloat16 and gate_up.is_contiguous() and inter % 8 == 0
+            and inter > 0 and gate_up.data_ptr() % 16 == 0):
+        return _Swiglu.apply(gate_up)
+    return _separate_operations(gate_up)
 
 
 class ExpertParallelMoE(torch.nn.Module):

@@ -84,6 +84,31 @@ def test_expert_activation_of_every_gate_value():
         assert _same_values(h.detach(), want) and _same_values(x.grad, grad)
 
 
+def test_expert_activation_under_autograd_modes():
+    """Second derivatives, forward mode, batched gradients, vmap and tracing see the separate operations."""
+    from torch.autograd import forward_ad
+    from torch.fx.experimental.proxy_tensor import make_fx
+
+    from deepep_b200.models.moe_layer import _activate, _separate_operations
+
+    gen = torch.Generator().manual_seed(9)
+    gu, dh, v = (torch.randn(s, generator=gen).bfloat16().cuda() for s in ((17, 48), (17, 24), (17, 48)))
+    results = {}
+    for fn in (_activate, _separate_operations):
+        x, g = gu.clone().requires_grad_(), dh.clone().requires_grad_()
+        first, = torch.autograd.grad(fn(x), x, g, create_graph=True)
+        second = torch.autograd.grad(first, (x, g), v)
+        with forward_ad.dual_level():
+            tangent = forward_ad.unpack_dual(fn(forward_ad.make_dual(gu, v))).tangent.clone()
+        batched, = torch.autograd.grad(fn(x), x, torch.stack([dh, 2 * dh, -dh]), is_grads_batched=True)
+        mapped = torch.func.vmap(fn)(torch.stack([gu, v]))
+        results[fn] = [first.detach(), *second, tangent, batched, mapped]
+    for a, b in zip(*results.values()):
+        assert _same_values(a, b)
+    traced = make_fx(_activate)(gu)
+    assert any("silu" in str(n.target) for n in traced.graph.nodes) and _same_values(traced(v), _activate(v))
+
+
 @pytest.mark.parametrize("payload", ["bf16", "fp8", "fp8_fused"])
 @pytest.mark.parametrize("alignment,experts", [(128, 24), (16, 700)])
 def test_padding_rows_are_zero(payload, alignment, experts):
