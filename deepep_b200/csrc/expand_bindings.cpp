@@ -33,6 +33,17 @@ void bind_expand(py::module_& m) {
       if (reinterpret_cast<uintptr_t>(q) % 16) throw std::invalid_argument("swiglu: rows must start on a 16-byte boundary");
     check_launch(launch_swiglu(p, backward, blocks, reinterpret_cast<cudaStream_t>(stream)), "swiglu");
   });
+  m.def("row_scale", [](const py::dict& d, int blocks, uintptr_t stream) {
+    RowScaleParams p{};
+    p.a = eptr<const __nv_bfloat16>(d, "a"); p.w = eptr<const float>(d, "w"); p.out = eptr<__nv_bfloat16>(d, "out");
+    p.b = eptr<const __nv_bfloat16>(d, "b"); p.prod = eptr<__nv_bfloat16>(d, "prod");
+    p.rows = d["rows"].cast<long long>(); p.width = d["width"].cast<int>();
+    if (p.rows < 0 || p.width < 8 || p.width % 8) throw std::invalid_argument("row_scale: the width must be a positive multiple of 8");
+    if (p.rows > 0 && (!p.a || !p.w || (!p.out && !p.prod) || !p.b != !p.prod)) throw std::invalid_argument("row_scale: a tensor is missing");
+    for (const void* q : {(const void*)p.a, (const void*)p.out, (const void*)p.b, (const void*)p.prod})
+      if (reinterpret_cast<uintptr_t>(q) % 16) throw std::invalid_argument("row_scale: rows must start on a 16-byte boundary");
+    check_launch(launch_row_scale(p, blocks, reinterpret_cast<cudaStream_t>(stream)), "row_scale");
+  });
   m.attr("expand_tile") = kExpandTile;
   m.def("expand", [](const py::dict& d, int blocks, uintptr_t stream) {
     ExpandParams p{};

@@ -51,7 +51,7 @@ class _Swiglu(torch.autograd.Function):
         rows, width = gate_up.shape
         h = gate_up.new_empty((rows, width // 2))
         ctx.save_for_backward(gate_up)
-        _launch(gate_up, False, h=h)
+        _launch("swiglu", dict(gu=gate_up, h=h), dict(rows=rows, inter=width // 2), False)
         return h
 
     @staticmethod
@@ -62,23 +62,56 @@ class _Swiglu(torch.autograd.Function):
             with torch.enable_grad():
                 h = _separate_operations(gate_up)
             return torch.autograd.grad(h, gate_up, grad, create_graph=again)[0]
-        grad = grad.contiguous()
-        if grad.data_ptr() % 16:
-            grad = grad.clone()
+        rows, width = gate_up.shape
         out = torch.empty_like(gate_up)
-        _launch(gate_up, True, dh=grad, dgu=out)
+        _launch("swiglu", dict(gu=gate_up, dh=_readable(grad), dgu=out), dict(rows=rows, inter=width // 2), True)
         return out
 
 
-def _launch(gate_up: torch.Tensor, backward: bool, **tensors) -> None:
+class _WeighRows(torch.autograd.Function):
+    """bf16 rows times an fp32 weight each (rounded to bf16), one kernel each way; the weight's gradient is summed by torch."""
+
+    @staticmethod
+    def forward(ctx, rows, weights):
+        out = torch.empty_like(rows)
+        ctx.save_for_backward(rows, weights)
+        _launch("row_scale", dict(a=rows, w=weights, out=out), dict(rows=rows.shape[0], width=rows.shape[1]))
+        return out
+
+    @staticmethod
+    def backward(ctx, grad):
+        rows, weights = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        again = torch.is_grad_enabled()
+        if again or not _ordinary(rows, weights, grad):
+            with torch.enable_grad():
+                out = rows * weights.unsqueeze(1).to(rows.dtype)
+            grads = iter(torch.autograd.grad(out, [t for t, n in zip((rows, weights), need) if n], grad, create_graph=again))
+            return tuple(next(grads) if n else None for n in need)
+        tensors = dict(a=_readable(grad), w=weights)
+        if need[0]:
+            tensors["out"] = torch.empty_like(rows)
+        if need[1]:
+            tensors.update(b=rows, prod=torch.empty_like(rows))
+        _launch("row_scale", tensors, dict(rows=rows.shape[0], width=rows.shape[1]))
+        terms = tensors.get("prod")
+        return tensors.get("out"), None if terms is None else terms.sum(1, keepdim=True).to(weights.dtype).squeeze(1)
+
+
+def _launch(op: str, tensors: dict, sizes: dict, *flags) -> None:
     from ..ops import require_native
 
-    device = gate_up.device
-    rows, width = gate_up.shape
-    args = dict(gu=gate_up.data_ptr(), rows=rows, inter=width // 2, **{name: t.data_ptr() for name, t in tensors.items()})
+    device = next(iter(tensors.values())).device
     with torch.cuda.device(device):
-        require_native("the expert activation").swiglu(args, backward, torch.cuda.get_device_properties(device).multi_processor_count * 8,
-                                                       torch.cuda.current_stream(device).cuda_stream)
+        getattr(require_native("the training layer"), op)({**sizes, **{name: t.data_ptr() for name, t in tensors.items()}}, *flags,
+                                                          torch.cuda.get_device_properties(device).multi_processor_count * 8,
+                                                          torch.cuda.current_stream(device).cuda_stream)
+
+
+def _readable(grad: torch.Tensor) -> torch.Tensor:
+    """Contiguous and on a 16-byte boundary, as the kernels read it."""
+    grad = grad.contiguous()
+    return grad.clone() if grad.data_ptr() % 16 else grad
 
 
 def _ordinary(*tensors: torch.Tensor) -> bool:
@@ -104,6 +137,16 @@ def _activate(gate_up: torch.Tensor) -> torch.Tensor:
             and inter > 0 and gate_up.data_ptr() % 16 == 0):
         return _Swiglu.apply(gate_up)
     return _separate_operations(gate_up)
+
+
+def _weigh(rows: torch.Tensor, weights: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """``rows`` times their weights rounded to ``dtype``.  The kernel takes contiguous, 16-byte aligned bf16 rows of a multiple of
+    8 values and fp32 weights of the same number; anything else goes through torch, with the same results."""
+    if (_ordinary(rows, weights) and rows.is_cuda and rows.device == weights.device and rows.dtype == dtype == torch.bfloat16
+            and weights.dtype == torch.float32 and rows.dim() == 2 and weights.shape == rows.shape[:1] and rows.numel() > 0
+            and rows.shape[1] % 8 == 0 and rows.is_contiguous() and weights.is_contiguous() and rows.data_ptr() % 16 == 0):
+        return _WeighRows.apply(rows, weights)
+    return rows * weights.unsqueeze(1).to(dtype)
 
 
 class ExpertParallelMoE(torch.nn.Module):
@@ -150,7 +193,7 @@ class ExpertParallelMoE(torch.nn.Module):
     def forward(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: torch.Tensor) -> torch.Tensor:
         holder = {}
         recv_x, recv_w, psum = _Dispatch.apply(self.buffer, x, topk_idx, topk_weights, self.num_experts, holder)
-        y = self.experts(recv_x, psum, holder["handle"].num_recv_tokens_per_expert_list) * recv_w.unsqueeze(1).to(recv_x.dtype)
+        y = _weigh(self.experts(recv_x, psum, holder["handle"].num_recv_tokens_per_expert_list), recv_w, recv_x.dtype)
         return _Combine.apply(self.buffer, y.contiguous(), holder["handle"])
 
 

@@ -109,6 +109,32 @@ def test_expert_activation_under_autograd_modes():
     assert any("silu" in str(n.target) for n in traced.graph.nodes) and _same_values(traced(v), _activate(v))
 
 
+@pytest.mark.parametrize("rows,width", [(1, 8), (33, 1032), (1500, 4096), (7, 264)])
+def test_weighted_rows(rows, width):
+    """The product of rows with their weights and both gradients, against the separate operations bit for bit (values of every
+    size, infinities and NaN included), and their second derivatives."""
+    from deepep_b200.models.moe_layer import _weigh
+
+    gen = torch.Generator().manual_seed(rows)
+    anything = torch.randint(-32768, 32768, (rows, width), generator=gen, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    usual, dh = (torch.randn((rows, width), generator=gen).bfloat16() for _ in range(2))
+    w = torch.rand((rows,), generator=gen)
+    w[0] = float("inf") if rows > 1 else 1.5
+    for src, need in ((usual, (True, True)), (anything, (True, True)), (usual, (True, False)), (usual, (False, True))):
+        results = []
+        for fn in (lambda r, f: _weigh(r, f, torch.bfloat16), lambda r, f: r * f.unsqueeze(1).to(torch.bfloat16)):
+            r, f = src.cuda().requires_grad_(need[0]), w.cuda().requires_grad_(need[1])
+            out, wanted = fn(r, f), [t for t in (r, f) if t.requires_grad]
+            grads = torch.autograd.grad(out, wanted, dh.cuda(), retain_graph=True)
+            again = torch.autograd.grad(out, wanted, dh.cuda(), create_graph=True)
+            results.append([out.detach(), *grads, *[t.detach() for t in again]])
+        for a, b in zip(*results):
+            if a.dtype == torch.float32:               # the weights' gradients are bf16 sums handed back as fp32
+                assert bool(((a == b) | (a.isnan() & b.isnan())).all())
+            else:
+                assert _same_values(a, b)
+
+
 @pytest.mark.parametrize("payload", ["bf16", "fp8", "fp8_fused"])
 @pytest.mark.parametrize("alignment,experts", [(128, 24), (16, 700)])
 def test_padding_rows_are_zero(payload, alignment, experts):
