@@ -81,8 +81,8 @@ class RoutingPlan:
                             self.recv_idx) if t is not None]
 
     def private_tensors(self):
-        """What only the kernels write: kept alive with the others, but nothing a caller could change."""
-        return [] if self.local_row is None else [self.num_rows_dev, self.local_row]
+        """What the kernels of a low-latency handle use besides: kept alive with the others, but not watched for changes."""
+        return [t for t in (self.num_rows_dev, self.local_row, self.topk_w) if t is not None]
 
 
 def _ptr(t: Optional[torch.Tensor]):
