@@ -468,15 +468,16 @@ class ElasticBuffer:
         self._preflight("cached_dispatch", (x_data.shape[0] > 0, self.hidden, mode))
         comm = self._enter(previous_event, previous_event_before_epilogue)
         allocate_on_comm_stream = self._allocates_on_comm(allocate_on_comm_stream, previous_event, previous_event_before_epilogue)
+        kept: List[torch.Tensor] = []
         with self._on(comm if allocate_on_comm_stream else None):
             if handle.is_low_latency and hasattr(self.engine, "ll_dispatch"):
                 recv_x, recv_sf = self.engine.ll_dispatch_cached([x_data if x_sf is None else (x_data, x_sf)], [handle._plan],
-                                                                 mode, stream=comm)[0]
+                                                                 mode, stream=comm, kept=kept)[0]
             else:
                 recv_x, recv_sf = self.engine.dispatch([x_data if x_sf is None else (x_data, x_sf)], [handle._plan], mode,
                                                        blocks=num_sms or self.num_sms, stream=comm)[0]
         out_x = recv_x if recv_sf is None else (recv_x, recv_sf.view(torch.int32) if packed else recv_sf)
-        event = self._leave(comm, async_with_compute_stream, [recv_x, recv_sf, x_data, x_sf] + handle._kept(),
+        event = self._leave(comm, async_with_compute_stream, [recv_x, recv_sf, x_data, x_sf] + handle._kept() + kept,
                             allocate_on_comm_stream)
         return out_x, None, None, handle, event
 

@@ -445,10 +445,15 @@ class CudaEngine:
             return out
         return res
 
-    def ll_dispatch_cached(self, xs: Sequence, plans: Sequence[RoutingPlan], mode: int, stream=None):
-        """Re-run the self-contained low-latency dispatch with the routing saved in the plans (backward of combine)."""
+    def ll_dispatch_cached(self, xs: Sequence, plans: Sequence[RoutingPlan], mode: int, stream=None, kept: Optional[list] = None):
+        """Re-run the self-contained low-latency dispatch with the routing saved in the plans (backward of combine).  The kernel
+        writes a routing plan of its own, which nobody reads: its tensors are added to ``kept``, for a caller that does not make
+        the current stream wait for the call."""
         res = self.ll_dispatch(xs, [p.topk_idx for p in plans], [p.topk_w for p in plans], plans[0].num_experts, mode,
                                cpu_sync=False, stream=stream)
+        if kept is not None:
+            for plan, _, _ in res:
+                kept += plan.tensors() + plan.private_tensors()
         return [(rx[:p.num_rows], None if rsf is None else rsf[:p.num_rows]) for (_, rx, rsf), p in zip(res, plans)]
 
     def ll_combine(self, xs: Sequence[torch.Tensor], plans: Sequence[RoutingPlan], stream=None, outs: Optional[list] = None):

@@ -86,6 +86,10 @@ def test_low_latency_calls(buf):
                                            async_with_compute_stream=True)
     assert handle.is_low_latency
     _check(buf, event)
+    event = buf.dispatch(x, handle=handle, async_with_compute_stream=True)[4]
+    _check(buf, event)
+    event = buf.dispatch(x, handle=handle, async_with_compute_stream=True, allocate_on_comm_stream=True)[4]
+    _check(buf, event)
     out, _, event = buf.combine(rx, handle, async_with_compute_stream=True)
     _check(buf, event)
 

@@ -121,3 +121,29 @@ def test_ll_empty_batch_takes_the_same_path():
     torch.cuda.synchronize()
     assert out.shape == (0, H)
     buf.destroy()
+
+
+def test_ll_cached_dispatch_asynchronous():
+    """A cached low-latency dispatch that the caller waits for through its event gives the rows of the original, also when memory
+    is taken and given back on the current stream meanwhile."""
+    from deepep_b200 import ElasticBuffer
+
+    dev = torch.device("cuda")
+    T, H, E, K = 96, 2048, 32, 4
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=128, hidden=H, num_topk=K, explicitly_destroy=True)
+    x = torch.randn((T, H), generator=torch.Generator().manual_seed(3)).bfloat16().to(dev)
+    idx, w = make_routes("invalid", T, E, K, 1, 4).to(dev), make_weights(T, K, 5).to(dev)
+    rx, _, _, handle, _ = buf.dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E)
+    assert handle.is_low_latency
+    first, _, _ = buf.combine(rx, handle)
+    for _ in range(4):
+        again, _, _, _, event = buf.dispatch(x, handle=handle, async_with_compute_stream=True)
+        fills = [torch.full((n,), -1, dtype=torch.int32, device=dev) for n in (1, E, E + 1, 128 * K, T * K, rx.shape[0])]
+        with event:
+            pass
+        assert bits_equal(again, rx)
+        out, _, done = buf.combine(again, handle, async_with_compute_stream=True)
+        done.current_stream_wait()
+        assert bits_equal(out, first)
+        del fills
+    buf.destroy()
