@@ -70,7 +70,9 @@ class RoutingPlan:
     has_weights: bool = False
     low_latency: bool = False
     num_rows_dev: Optional[torch.Tensor] = None
-    local_row: Optional[torch.Tensor] = None     # low latency: output row of every slot whose expert lives on this rank
+    # low latency: int32 output row of every slot whose expert lives on this rank (the tensor, and the address in it)
+    local_row: Optional[torch.Tensor] = None
+    local_row_ptr: int = 0
     topk_w: Optional[torch.Tensor] = None
     rank_matrix: Optional[torch.Tensor] = None
     send_chunk_prefix: Optional[torch.Tensor] = None
@@ -82,7 +84,8 @@ class RoutingPlan:
 
     def private_tensors(self):
         """What the kernels of a low-latency handle use besides: kept alive with the others, but not watched for changes."""
-        return [t for t in (self.num_rows_dev, self.local_row, self.topk_w) if t is not None]
+        own = None if self.local_row is self.num_rows_dev else self.local_row
+        return [t for t in (self.num_rows_dev, own, self.topk_w) if t is not None]
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -417,21 +420,26 @@ class CudaEngine:
                          recv_sf=None if mode == 0 else torch.empty((cap, H // 128), dtype=torch.float32, device=dev),
                          recv_w=torch.empty((cap,), dtype=torch.float32, device=dev),
                          recv_row_src=torch.empty((cap,), **i32), expert_counts=torch.empty((local,), **i32),
-                         expert_offsets=torch.empty((local + 1,), **i32), num_rows=torch.empty((1,), **i32))
+                         expert_offsets=torch.empty((local + 1,), **i32), num_rows=torch.empty((1 + T * K,), **i32))
             plan = RoutingPlan(num_tokens=T, num_experts=num_experts, num_topk=K, expand=True, alignment=1, meta_stride=0,
                                num_rows=cap, num_staged_rows=0, expert_counts_list=None, topk_idx=topk_idx[i], send_slot=None,
                                slot_row=None, stage_meta=None, chunk_start=None, rank_tokens=None, rank_rows=None,
                                expert_counts=o["expert_counts"], expert_offsets=o["expert_offsets"],
                                recv_row_src=o["recv_row_src"], recv_w=o["recv_w"], recv_idx=None, has_weights=True)
             plan.num_rows_dev, plan.topk_w, plan.low_latency = o["num_rows"], topk_w[i], True
-            plan.local_row = torch.empty((max(T, 1), K), **i32)
+            if outputs is None:      # behind the row count: a small eager call is bound by the host, and an allocation of its own costs it 2 us
+                plan.local_row = o["num_rows"]
+                plan.local_row_ptr = o["num_rows"].data_ptr() + 4
+            else:
+                plan.local_row = torch.empty((max(T, 1) * K,), **i32)
+                plan.local_row_ptr = plan.local_row.data_ptr()
             res.append((plan, o["recv_x"], o["recv_sf"]))
             args.append(dict(x=x.data_ptr(), x_sf=_ptr(sf), topk_idx=topk_idx[i].data_ptr(), topk_w=topk_w[i].data_ptr(), T=T,
                              E=num_experts, mode=mode, recv_x=o["recv_x"].data_ptr(), recv_sf=_ptr(o["recv_sf"]),
                              recv_w=o["recv_w"].data_ptr(), recv_row_src=o["recv_row_src"].data_ptr(),
                              expert_counts=o["expert_counts"].data_ptr(), expert_offsets=o["expert_offsets"].data_ptr(),
                              num_rows=o["num_rows"].data_ptr(),
-                             local_row=plan.local_row.data_ptr(), use_mailbox=int(cpu_sync), capacity=cap))
+                             local_row=plan.local_row_ptr, use_mailbox=int(cpu_sync), capacity=cap))
         self._timed("ll_dispatch", stream, lambda: self.C.ll_dispatch(lay, self.sessions, args, self.ll_blocks(), self._stream(stream),
                                                                              self._device_profile))
         if cpu_sync:
@@ -462,9 +470,9 @@ class CudaEngine:
         for i, plan in enumerate(plans):
             out = outs[i] if outs is not None else torch.empty((plan.num_tokens, lay.hidden), dtype=torch.bfloat16, device=dev)
             results.append(out)
-            args.append(dict(x=xs[i].data_ptr(), recv_row_src=plan.recv_row_src.data_ptr(), num_rows=plan.num_rows_dev.data_ptr(), local_row=plan.local_row.data_ptr(),
-                             topk_idx=plan.topk_idx.data_ptr(), topk_w=plan.topk_w.data_ptr(), T=plan.num_tokens,
-                             E=plan.num_experts, out=out.data_ptr()))
+            args.append(dict(x=xs[i].data_ptr(), recv_row_src=plan.recv_row_src.data_ptr(), num_rows=plan.num_rows_dev.data_ptr(),
+                             local_row=plan.local_row_ptr, topk_idx=plan.topk_idx.data_ptr(), topk_w=plan.topk_w.data_ptr(),
+                             T=plan.num_tokens, E=plan.num_experts, out=out.data_ptr()))
         self._timed("ll_combine", stream, lambda: self.C.ll_combine(lay, self.sessions, args, self.ll_blocks(), self._stream(stream),
                                                                            self._device_profile))
         return results

@@ -147,3 +147,24 @@ def test_ll_cached_dispatch_asynchronous():
         assert bits_equal(out, first)
         del fills
     buf.destroy()
+
+
+@pytest.mark.parametrize("mode,tensors", [(0, 6), (2, 7)])
+def test_ll_dispatch_allocates_its_outputs_only(mode, tensors):
+    """An eager dispatch is bound by the host: rows, scales, weights, sources, counts, offsets and the row count are all the
+    tensors it makes (the rows of the rank's own slots lie behind the row count)."""
+    from deepep_b200.ops import load_native
+    from deepep_b200.parallel.virtual import VirtualWorld
+
+    T, H, E, K = 20, 256, 16, 4
+    with VirtualWorld(1, T, H, K, timeout=10.0, ll_bytes=load_native().ll_region_bytes(1, T, K, H)) as vw:
+        x = torch.randn((T, H), generator=torch.Generator().manual_seed(1)).bfloat16().cuda()
+        idx, w = make_routes("random", T, E, K, 1, 2).cuda(), make_weights(T, K, 3).cuda()
+        counted = lambda: torch.cuda.memory_stats()["allocation.all.allocated"]
+        before = counted()
+        (plan, rx, _), = vw.engine.ll_dispatch([x], [idx], [w], E, mode, cpu_sync=False)
+        assert counted() - before == tensors
+        torch.cuda.synchronize()
+        assert int(plan.num_rows_dev[0]) == T * K and sorted(plan.num_rows_dev[1:].tolist()) == list(range(T * K))
+        if mode == 0:
+            assert bits_equal(rx[plan.num_rows_dev[1:].long()], x.repeat_interleave(K, 0))
