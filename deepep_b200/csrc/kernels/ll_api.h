@@ -73,7 +73,7 @@ struct LLCombineArgs {
   const int* local_row;        // [T][K] row in x of every slot whose expert lives on this rank (LLDispatchArgs::local_row)
   const long long* topk_idx;   // [T][K] of this rank's tokens
   const float* topk_w;         // [T][K] weights applied here, at the source
-  int T, E;
+  int T, E, x_rows, pad;       // x_rows: rows of x, which bound what num_rows, recv_row_src and local_row may name
   __nv_bfloat16* out;          // [T][H]
 };
 struct LLCombineParams { WsLayout lay; int profile, pad; LLCombineArgs r[kMaxRanks]; };     // profile: the same into Control::dbg[8..15]

@@ -370,6 +370,10 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
     __syncthreads();
     alive = !s_fail;
   }
+  if (!alive) {     // a wait ran out: the handle names no rows (a combine may be queued behind this launch already)
+    for (int i = blockIdx.x * kLLThreads + threadIdx.x; i < a.T * K; i += gridDim.x * kLLThreads) a.local_row[i] = -1;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.num_rows = 0;
+  }
   if (alive) {
     uint8_t* mine = ctx.ws[me] + bank_off;
     const int* gidx = reinterpret_cast<const int*>(mine + ll.gather_idx);
@@ -529,6 +533,7 @@ __global__ void __launch_bounds__(kLLThreads) ep_combine_ll_kernel(const __grid_
   const int gw = warp * gridDim.x + blockIdx.x, total_warps = gridDim.x * nwarps;
   Control* ctl = control_of(ctx.ws[me]);
   const unsigned long long epoch = ctl->epoch[kOpLLCombine] + 1;
+  const int aborted = ld_volatile_int(&ctl->abort);    // set: an earlier call gave up, the handle's tensors may never have been written
   const LLLayout ll = make_ll_layout(P, M, K, H);
   const long long bank_off = lay.ll + (long long)(epoch & 1) * ll.bank_bytes;
   const int row_bytes = H * 2;
@@ -548,14 +553,15 @@ __global__ void __launch_bounds__(kLLThreads) ep_combine_ll_kernel(const __grid_
 
   if (alive) {
     // ---- return every expert row of a peer's token, part by part, to its (token, slot) slot there
-    const int R = P > 1 ? *a.num_rows : 0;
+    int R = P > 1 ? min(*a.num_rows, a.x_rows) : 0;
+    if (aborted) R = 0;
     PendingFlags pending;
     for (int item = gw; item < R * kLLParts; item += total_warps) {
       const int r = item / kLLParts, part = item % kLLParts;
       const int code = a.recv_row_src[r];
       if (code < 0) continue;
       const int src = code / (M * K), rem = code - src * M * K;
-      if (src == me) continue;
+      if (src == me || src >= P) continue;
       const LLPart pr = ll_part(H, part);
       if (pr.v0 >= pr.v1) continue;
       uint8_t* base = ctx.ws[src] + bank_off;
@@ -593,8 +599,12 @@ __global__ void __launch_bounds__(kLLThreads) ep_combine_ll_kernel(const __grid_
         if (z < lane && ez == e) counts = false;
       }
       const unsigned valid = __ballot_sync(0xffffffffu, counts);
-      int got = 1;
-      if (counts && local < 0) got = wait_flag_ge(flags + ((size_t)t * K + lane) * kLLParts + part, epoch, ctx, kOpLLCombine, 1, me);
+      int got = !aborted;
+      if (got && counts && local >= a.x_rows) {        // the handle and x do not belong together
+        report_failure(ctx, kStatusBadArgument, kOpLLCombine, 2, me, a.x_rows, local);
+        got = 0;
+      }
+      if (got && counts && local < 0) got = wait_flag_ge(flags + ((size_t)t * K + lane) * kLLParts + part, epoch, ctx, kOpLLCombine, 1, me);
       if (!__all_sync(0xffffffffu, got)) break;
       const unsigned long long my_row = reinterpret_cast<unsigned long long>(
           local >= 0 ? reinterpret_cast<const uint8_t*>(a.x) + (size_t)local * row_bytes

@@ -73,7 +73,7 @@ void op_ll_combine(const WsLayout& lay, const std::vector<py::object>& sessions,
     a.ctx = sessions[i].cast<Session&>().ctx();
     a.x = ptr<const __nv_bfloat16>(d, "x"); a.recv_row_src = ptr<const int>(d, "recv_row_src");
     a.num_rows = ptr<const int>(d, "num_rows"); a.topk_idx = ptr<const long long>(d, "topk_idx");
-    a.topk_w = ptr<const float>(d, "topk_w"); a.T = geti(d, "T"); a.E = geti(d, "E");
+    a.topk_w = ptr<const float>(d, "topk_w"); a.T = geti(d, "T"); a.E = geti(d, "E"); a.x_rows = geti(d, "x_rows");
     a.out = ptr<__nv_bfloat16>(d, "out"); a.local_row = ptr<const int>(d, "local_row");
     if (!a.local_row && a.T > 0) throw std::invalid_argument("low-latency combine: local_row is missing");
   }

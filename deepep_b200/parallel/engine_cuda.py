@@ -33,6 +33,7 @@ WAIT_SITES = {
     (3, 0): "the peer to finish the previous combine", (3, 1): "the partial sums of an expert rank",
     (4, 0): "the peer to release the bank used two calls ago", (4, 1): "the peer's routing table", (4, 2): "a part of a row from a source rank",
     (5, 0): "the peer to release the bank used two calls ago", (5, 1): "a part of an expert's row",
+    (5, 2): "rows that the expert outputs do not have",
     (6, 0): "the peer's inputs and routing table", (6, 1): "the peer's combine rows",
     (7, 0): "the peer to finish the previous call", (7, 1): "the peer's staged rows and row table",
     (8, 0): "the peer's row table", (8, 1): "the rows returned by the peer",
@@ -472,7 +473,7 @@ class CudaEngine:
             results.append(out)
             args.append(dict(x=xs[i].data_ptr(), recv_row_src=plan.recv_row_src.data_ptr(), num_rows=plan.num_rows_dev.data_ptr(),
                              local_row=plan.local_row_ptr, topk_idx=plan.topk_idx.data_ptr(), topk_w=plan.topk_w.data_ptr(),
-                             T=plan.num_tokens, E=plan.num_experts, out=out.data_ptr()))
+                             T=plan.num_tokens, E=plan.num_experts, out=out.data_ptr(), x_rows=xs[i].shape[0]))
         self._timed("ll_combine", stream, lambda: self.C.ll_combine(lay, self.sessions, args, self.ll_blocks(), self._stream(stream),
                                                                            self._device_profile))
         return results

@@ -168,3 +168,77 @@ def test_ll_dispatch_allocates_its_outputs_only(mode, tensors):
         assert int(plan.num_rows_dev[0]) == T * K and sorted(plan.num_rows_dev[1:].tolist()) == list(range(T * K))
         if mode == 0:
             assert bits_equal(rx[plan.num_rows_dev[1:].long()], x.repeat_interleave(K, 0))
+
+
+def _one_rank(T, H, E, K):
+    from deepep_b200.ops import load_native
+    from deepep_b200.parallel.virtual import VirtualWorld
+
+    x = torch.randn((T, H), generator=torch.Generator().manual_seed(1)).bfloat16()
+    idx, w = make_routes("random", T, E, K, 1, 2), make_weights(T, K, 3)
+    return VirtualWorld(1, T, H, K, timeout=0.05, ll_bytes=load_native().ll_region_bytes(1, T, K, H)), x, idx, w
+
+
+def test_ll_combine_after_an_abort_touches_nothing():
+    """Once a wait of the rank ran out, a queued combine neither reads the handle's tables nor writes the output; with the status
+    cleared the same handle works again."""
+    world, x, idx, w = _one_rank(24, 512, 16, 4)
+    with world as vw:
+        (plan, rx, _), = vw.engine.ll_dispatch([x.cuda()], [idx.cuda()], [w.cuda()], 16, 0)
+        vw.sessions[0].wait_probe(torch.cuda.current_stream().cuda_stream)
+        out = torch.full((24, 512), 7.0, dtype=torch.bfloat16, device="cuda")
+        vw.engine.ll_combine([rx], [plan], outs=[out])
+        torch.cuda.synchronize()
+        assert vw.sessions[0].status()["where"] == 99 and bool((out == 7.0).all())
+        vw.sessions[0].clear_status()
+        vw.engine.ll_combine([rx], [plan], outs=[out])
+        torch.cuda.synchronize()
+        vw.engine.check_status()
+        ref, lays = R.dispatch([x], [idx], [w], 16, do_expand=True)
+        assert bits_equal(out, R.low_latency_combine([ref[0][0]], lays, [w], [24])[0])
+
+
+def test_ll_combine_reports_rows_that_x_does_not_have():
+    """A table that names rows behind the expert outputs is reported and the rows are not used (the memory behind is there)."""
+    from deepep_b200.parallel.engine_cuda import CommunicationError
+
+    world, x, idx, w = _one_rank(24, 512, 16, 4)
+    with world as vw:
+        (plan, rx, _), = vw.engine.ll_dispatch([x.cuda()], [idx.cuda()], [w.cuda()], 16, 0)
+        rows = rx.shape[0]
+        both = torch.cat([rx, rx])
+        plan.num_rows_dev[1:] += rows
+        out = torch.full((24, 512), 7.0, dtype=torch.bfloat16, device="cuda")
+        vw.engine.ll_combine([both[:rows]], [plan], outs=[out])
+        torch.cuda.synchronize()
+        assert bool((out == 7.0).all())
+        with pytest.raises(CommunicationError, match="bad argument .*rows that the expert outputs do not have"):
+            vw.engine.check_status()
+
+
+def test_ll_dispatch_that_gives_up_leaves_no_rows_behind():
+    """One of two ranks runs alone: its wait for the peer's routing table runs out, the handle's tables say 'no rows', and a
+    combine that was queued behind the dispatch without a look at the host writes nothing."""
+    from deepep_b200.ops import load_native
+    from deepep_b200.parallel.engine_cuda import CudaEngine
+
+    C, T, H, E, K = load_native(), 24, 512, 16, 4
+    layout = C.make_layout(2, T, H, K, C.ll_region_bytes(2, T, K, H), 0, 0)
+    ranks = [C.Session(r, 2, layout.total, 0.05) for r in range(2)]
+    try:
+        for s in ranks:
+            s.attach_peers([r.workspace for r in ranks])
+        eng = CudaEngine(ranks[:1], layout, torch.device("cuda", torch.cuda.current_device()))
+        x = torch.randn((T, H), generator=torch.Generator().manual_seed(1)).bfloat16().cuda()
+        idx, w = make_routes("random", T, E, K, 2, 2).cuda(), make_weights(T, K, 3).cuda()
+        (plan, rx, _), = eng.ll_dispatch([x], [idx], [w], E, 0, cpu_sync=False)
+        out = torch.full((T, H), 7.0, dtype=torch.bfloat16, device="cuda")
+        eng.ll_combine([rx], [plan], outs=[out])
+        torch.cuda.synchronize()
+        st = ranks[0].status()
+        assert st["code"] == 1 and st["op"] == 4 and st["where"] == 1 and st["peer"] == 1
+        assert int(plan.num_rows_dev[0]) == 0 and bool((plan.num_rows_dev[1:] == -1).all()) and bool((out == 7.0).all())
+    finally:
+        torch.cuda.synchronize()
+        for s in ranks:
+            s.close()
