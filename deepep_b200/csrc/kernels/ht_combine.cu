@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(kCombineThreads, 1) ep_combine_ht_kernel(const
   const int row_bytes = H * 2, units = H / 8;  // 16-byte units per row
   Control* ctl = control_of(ctx.ws[me]);
   const unsigned long long epoch = ctl->epoch[kOpCombine] + 1;
+  const bool aborted = ld_volatile_int(&ctl->abort) != 0;   // an earlier call gave up, the plan's tensors may never have been written
   const uint8_t* x = reinterpret_cast<const uint8_t*>(a.x);
   const bool expert_side = (int)blockIdx.x < p.send_blocks;
   PhaseClock<kProfile> clk;
@@ -161,10 +162,10 @@ __global__ void __launch_bounds__(kCombineThreads, 1) ep_combine_ht_kernel(const
     // ================================================================ expert side: reduce + return
     int ok = 1;
     if (lane < P) ok = wait_flag_ge(&ctl->comb_ack[lane], epoch - 1, ctx, kOpCombine, 0, lane);
-    const bool alive = __all_sync(0xffffffffu, ok);
+    const bool alive = __all_sync(0xffffffffu, ok) && !aborted;
     clk.mark(kProfWait);
     // the sources whose rows are returned through a partial: all ranks, or all but this one
-    const int S = p.local_direct ? P - 1 : P, first = p.local_direct ? 1 : 0;
+    const int S = aborted ? 0 : p.local_direct ? P - 1 : P, first = p.local_direct ? 1 : 0;
     int max_nb = 0;
     for (int s = 0; s < S; ++s) {
       const int r = (me + first + s) % P;
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(kCombineThreads, 1) ep_combine_ht_kernel(const
     const uint8_t* partial = ctx.ws[me] + lay.partial;
     const float* wret = reinterpret_cast<const float*>(ctx.ws[me] + lay.wret);
     const unsigned long long* flags = reinterpret_cast<const unsigned long long*>(ctx.ws[me] + lay.comb_flag);
-    const int t_stop = min(a.T, p.t_end);
+    const int t_stop = aborted ? 0 : min(a.T, p.t_end);
     for (int t = p.t_begin + next_ticket(&ctl->ticket[kOpCombine][1], lane); t < t_stop;
          t = p.t_begin + next_ticket(&ctl->ticket[kOpCombine][1], lane)) {
       const int ss = lane < P ? a.send_slot[(size_t)t * P + lane] : -1;

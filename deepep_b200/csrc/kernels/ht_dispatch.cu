@@ -168,6 +168,7 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) ep_dispatch_ht_kernel(con
   const int q = lane >> 3, c = lane & 7;      // metadata of a group is fetched by lane = (token of the group) * 8 + field
   Control* ctl = control_of(ctx.ws[me]);
   const unsigned long long epoch = ctl->epoch[kOpDispatch] + 1;
+  const bool aborted = ld_volatile_int(&ctl->abort) != 0;   // an earlier call gave up, the plan's tensors may never have been written
 
   const bool fp8 = a.mode != kDispatchBf16;
   const int nsf = fp8 ? H / 128 : 0;
@@ -177,14 +178,14 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) ep_dispatch_ht_kernel(con
   PhaseClock<kProfile> clk;
   clk.start();
 
-  if (a.pad_offsets)
+  if (a.pad_offsets && !aborted)
     zero_padding(a, a.E / P, row_bytes, nsf, (int)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, gridDim.x * (kDispatchThreads / 32), lane);
 
   if (sender) {
     // ================================================================ sender
     int ok = 1;
     if (lane < P) ok = wait_flag_ge(&ctl->disp_ack[lane], epoch - 1, ctx, kOpDispatch, 0, lane);
-    bool alive = __all_sync(0xffffffffu, ok);
+    bool alive = __all_sync(0xffffffffu, ok) && !aborted;
     clk.mark(kProfWait);
     // a work item is a group of tokens, or a column piece of one token when no peer waits for flags
     const int Lx = a.E / P, per_item = p.pieces > 0 ? 1 : kGroupTokens, pieces = max(1, p.pieces);
@@ -268,7 +269,7 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) ep_dispatch_ht_kernel(con
     const uint8_t* stage = ctx.ws[me] + lay.stage;
     const unsigned long long* flags = reinterpret_cast<const unsigned long long*>(ctx.ws[me] + lay.disp_flag);
     // the sources whose rows pass through the staging area: all ranks, or all but this one
-    const int S = p.local_direct ? P - 1 : P, first = p.local_direct ? 1 : 0;
+    const int S = aborted ? 0 : p.local_direct ? P - 1 : P, first = p.local_direct ? 1 : 0;
     int max_nb = 0;
     for (int s = 0; s < S; ++s) {
       const int r = (me + first + s) % P;

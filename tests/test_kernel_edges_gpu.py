@@ -222,3 +222,72 @@ def test_grouped_gemm_on_one_rank(counts, k, n):
     finally:
         torch.cuda.synchronize()
         s.close()
+
+
+@pytest.fixture
+def filled_outputs(monkeypatch):
+    """Whatever the engine allocates holds 0x55 in every byte before a kernel sees it."""
+    empty = torch.empty
+
+    def filled(*args, **kwargs):
+        t = empty(*args, **kwargs)
+        if t.is_cuda:
+            t.view(torch.uint8).fill_(0x55)
+        return t
+
+    monkeypatch.setattr(torch, "empty", filled)
+
+
+def _untouched(t):
+    return bool((t.view(torch.uint8) == 0x55).all())
+
+
+@pytest.mark.parametrize("alignment", [1, 16])
+def test_high_throughput_calls_after_an_abort_touch_nothing(filled_outputs, alignment):
+    """Once a wait of the rank ran out, calls queued behind it neither read the plan nor write their outputs."""
+    from deepep_b200.parallel.virtual import VirtualWorld
+
+    dev, T, H, E, K = torch.device("cuda"), 70, 256, 8, 3
+    x = torch.randn((T, H), generator=torch.Generator().manual_seed(4)).bfloat16().to(dev)
+    idx, w = make_routes("invalid", T, E, K, 1, 6).to(dev), make_weights(T, K, 2).to(dev)
+    with VirtualWorld(1, T, H, K, timeout=0.05) as vw:
+        eng = vw.engine
+        eng.local_direct = False                           # through the staging area and the partials, as with peers
+        plans = eng.notify([idx], [w], E, alignment=alignment)
+        (rows, _), = eng.dispatch([x], plans, 0)
+        vw.sessions[0].wait_probe(torch.cuda.current_stream().cuda_stream)
+        (later, _), = eng.dispatch([x], plans, 0)
+        (out, out_w), = eng.combine([rows], plans, [plans[0].recv_w[:plans[0].num_rows].contiguous()])
+        torch.cuda.synchronize()
+        assert vw.sessions[0].status()["where"] == 99
+        assert not _untouched(rows) and _untouched(later) and _untouched(out) and _untouched(out_w)
+
+
+def test_routing_pass_that_gives_up_leaves_an_empty_plan(filled_outputs):
+    """One of two ranks runs alone: its wait for the peer's table runs out, the plan says 'no rows', and the calls queued behind
+    it without a look at the host touch nothing."""
+    from deepep_b200.ops import load_native
+    from deepep_b200.parallel.engine_cuda import CudaEngine
+
+    C, dev, T, H, E, K = load_native(), torch.device("cuda", torch.cuda.current_device()), 300, 256, 8, 3
+    layout = C.make_layout(2, T, H, K)
+    ranks = [C.Session(r, 2, layout.total, 0.05) for r in range(2)]
+    try:
+        for s in ranks:
+            s.attach_peers([r.workspace for r in ranks])
+        eng = CudaEngine(ranks[:1], layout, dev)
+        x = torch.randn((T, H), generator=torch.Generator().manual_seed(4)).bfloat16().to(dev)
+        idx, w = make_routes("invalid", T, E, K, 2, 6).to(dev), make_weights(T, K, 2).to(dev)
+        plans = eng.notify([idx], [w], E, alignment=16, cpu_sync=False)
+        (rows, _), = eng.dispatch([x], plans, 0)
+        (out, _), = eng.combine([rows], plans, [None])
+        torch.cuda.synchronize()
+        st = ranks[0].status()
+        assert st["code"] == 1 and st["op"] == 1 and st["where"] == 1 and st["peer"] == 1
+        plan = plans[0]
+        assert not bool(plan.rank_rows.any()) and not bool(plan.expert_counts.any()) and not bool(plan.expert_offsets.any())
+        assert _untouched(rows) and _untouched(out) and all(r.guard_intact() for r in ranks)
+    finally:
+        torch.cuda.synchronize()
+        for s in ranks:
+            s.close()
