@@ -168,6 +168,12 @@ __global__ void __launch_bounds__(kNotifyThreads) ep_notify_kernel(const __grid_
     __syncthreads();
   }
   grid.sync();
+  // a block whose wait ran out has counted nothing: all blocks give up together and leave an empty plan
+  if (P > 1 && __syncthreads_or(threadIdx.x == 0 && ld_volatile_int(&ctl->abort))) {
+    alive = 0;
+    if (threadIdx.x < kMaxRanks) s_T[threadIdx.x] = 0;
+    __syncthreads();
+  }
 
   stamp(2);
   // ---- D1: exclusive scans over tiles
