@@ -84,9 +84,9 @@ class RoutingPlan:
                             self.recv_idx) if t is not None]
 
     def private_tensors(self):
-        """What the kernels of a low-latency handle use besides: kept alive with the others, but not watched for changes."""
+        """What the kernels use besides: kept alive with the others, but not watched for changes."""
         own = None if self.local_row is self.num_rows_dev else self.local_row
-        return [t for t in (self.num_rows_dev, own, self.topk_w) if t is not None]
+        return [t for t in (self.num_rows_dev, own, self.topk_w, self.rank_matrix) if t is not None]
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -297,7 +297,10 @@ class CudaEngine:
                         if topk_w[i] is not None else None),
                 recv_idx=None if expand else torch.empty((rcap, K), dtype=torch.int64, device=dev),
                 has_weights=topk_w[i] is not None)
-            plan.rank_matrix = torch.zeros((P, P), **i32) if rank_matrix else None
+            if rank_matrix:              # cleared where it is written: the launch stream may not wait for the current one any more
+                plan.rank_matrix = torch.empty((P, P), **i32)
+                with torch.cuda.stream(stream) if stream is not None else contextlib.nullcontext():
+                    plan.rank_matrix.zero_()
             plans.append(plan)
             sc = self._scratch[i]
             args.append(dict(topk_idx=idx.data_ptr(), topk_w=_ptr(topk_w[i]), T=T, E=num_experts, K=K, expand=int(expand),

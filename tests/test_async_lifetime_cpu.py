@@ -105,3 +105,31 @@ def test_high_throughput_calls(buf, expand, alignment):
     _check(buf, event)
     event = buf.combine(rx, handle, topk_weights=rw, bias=(x, x.clone()), async_with_compute_stream=True)[2]
     _check(buf, event)
+
+
+def test_v1_rank_matrix(buf, monkeypatch):
+    """The per-rank counts of the V1 handle are added up on the communication stream: cleared there too, and kept alive."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    inside, cleared = [], []
+
+    @contextlib.contextmanager
+    def on(stream):
+        inside.append(stream)
+        yield
+        inside.pop()
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            if "zero" in str(func):
+                cleared.append(bool(inside))
+            return func(*args, **(kwargs or {}))
+
+    monkeypatch.setattr(torch.cuda, "stream", on)
+    x, idx, w = _inputs()
+    with Watch():
+        event = buf.dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E, do_expand=False, do_cpu_sync=False,
+                             num_max_tokens_per_rank=512, async_with_compute_stream=True, _rank_matrix=True)[4]
+    assert cleared == [True]
+    assert any(key == "rank_matrix" for _, key, _ in buf.engine.C.addresses)
+    _check(buf, event)
