@@ -20,7 +20,7 @@ template <class T> T* gptr(const py::dict& d, const char* key) {
 int gint(const py::dict& d, const char* key) { return d[key].cast<int>(); }
 
 // `gather` = true: a2av_gmm (A operand is the gathered buffer); false: gmm_a2av (A operand is x).
-// Returns whether the single-rank kernel can serve the call.
+// Returns whether the single-rank kernel can serve the call, which needs no gathered buffer.
 bool fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session, bool gather) {
   Session& s = session.cast<Session&>();
   a.ctx = s.ctx();
@@ -43,7 +43,7 @@ bool fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session
   if (a.K > max_k || a.N > max_n) throw std::invalid_argument("k or n exceeds what the group was sized for");
   if (a.rows_in < 0 || a.out_rows_cap < 0) throw std::invalid_argument("negative row count");
   if ((gather ? a.rows_in : a.out_rows_cap) > max_rows) throw std::invalid_argument("more rows than the group was sized for");
-  if (!a.counts || (a.out_rows_cap > 0 && !a.out) || !a.tile_info || !a.num_tiles || (a.rows_in > 0 && !a.x) || (gather && (!a.gathered || !a.pulled)))
+  if (!a.counts || (a.out_rows_cap > 0 && !a.out) || !a.tile_info || !a.num_tiles || (a.rows_in > 0 && !a.x) || (gather && !a.pulled))
     throw std::invalid_argument("missing tensor");
   // The single-rank kernel reads x and the weights while it writes the output and the gathered rows, so these must be
   // disjoint from them; the general kernels write only after they have copied what an overlap would destroy.
@@ -53,7 +53,7 @@ bool fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session
     const uintptr_t u = (uintptr_t)p, v = (uintptr_t)q;
     return p && q && n > 0 && m > 0 && u < v + (uintptr_t)m && v < u + (uintptr_t)n;
   };
-  const bool keep = gather && d["gathered_wanted"].cast<bool>();
+  const bool keep = gather && a.gathered;
   const long long x_bytes = (long long)a.rows_in * a.K * 2, out_bytes = (long long)a.out_rows_cap * a.N * 2,
                   g_bytes = keep ? (long long)a.gathered_cap * a.K * 2 : 0, w_bytes = L * a.K * a.N * 2;
   const bool local = a.ctx.world == 1 && !overlap(a.out, out_bytes, a.x, x_bytes) && !overlap(a.out, out_bytes, weight, w_bytes) &&
@@ -61,10 +61,9 @@ bool fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session
                      !overlap(a.gathered, g_bytes, a.out, out_bytes) &&
                      !overlap(a.counts, a.E * 4ll, a.out, out_bytes) && !overlap(a.counts, a.E * 4ll, a.gathered, g_bytes) &&
                      ((uintptr_t)a.x | (uintptr_t)a.out | (keep ? (uintptr_t)a.gathered : 0)) % 16 == 0;
-  if (local && !keep) a.gathered = nullptr;
   const char* err = nullptr;
   const void* a_base = gather && !local ? (const void*)a.gathered : (const void*)a.x;
-  const long long a_rows = gather && !local ? a.gathered_cap : a.rows_in;
+  const long long a_rows = gather && !local ? (a.gathered ? a.gathered_cap : 0) : a.rows_in;
   // an empty operand still needs a valid map: point it at the weights
   if (!encode_bf16_map(&a.tmap_a, a_rows > 0 ? a_base : (const void*)d["weight"].cast<uintptr_t>(), a_rows > 0 ? a_rows : 1, a.K, kGmmBM, &err))
     throw std::runtime_error(err);
@@ -72,7 +71,8 @@ bool fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session
   return local;
 }
 
-void op(const WsLayout& lay, const std::vector<py::object>& sessions, const std::vector<py::dict>& args, int blocks, uintptr_t stream,
+// False: nothing was launched, because the general kernel has to serve the call and a gathered buffer is missing.
+bool op(const WsLayout& lay, const std::vector<py::object>& sessions, const std::vector<py::dict>& args, int blocks, uintptr_t stream,
         bool gather) {
   GmmParams p{};
   p.lay = lay;
@@ -80,10 +80,13 @@ void op(const WsLayout& lay, const std::vector<py::object>& sessions, const std:
   if (n < 1 || n > kMaxRanks || (int)sessions.size() != n) throw std::invalid_argument("1..8 rank argument blocks expected");
   bool local = n == 1;
   for (int i = 0; i < n; ++i) local = fill(p.r[i], lay, args[i], sessions[i], gather) && local;
+  for (int i = 0; i < n && gather && !local; ++i)
+    if (!p.r[i].gathered) return false;
   const cudaError_t e = local ? launch_gmm_local(p, blocks, reinterpret_cast<cudaStream_t>(stream))
                         : gather ? launch_a2av_gmm(p, n, blocks, reinterpret_cast<cudaStream_t>(stream))
                                : launch_gmm_a2av(p, n, blocks, reinterpret_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) throw std::runtime_error(std::string(gather ? "a2av_gmm" : "gmm_a2av") + " launch: " + cudaGetErrorString(e));
+  return true;
 }
 }  // namespace
 
@@ -94,7 +97,7 @@ void bind_gmm(py::module_& m) {
   });
   m.def("gmm_region_bytes", [](long long max_rows, long long max_k, long long max_n) { return gmm_region(max_rows, max_k, max_n).total; });
   m.def("a2av_gmm", [](const WsLayout& lay, const std::vector<py::object>& sessions, const std::vector<py::dict>& args, int blocks,
-                       uintptr_t stream) { op(lay, sessions, args, blocks, stream, true); });
+                       uintptr_t stream) { return op(lay, sessions, args, blocks, stream, true); });
   m.def("gmm_a2av", [](const WsLayout& lay, const std::vector<py::object>& sessions, const std::vector<py::dict>& args, int blocks,
                        uintptr_t stream) { op(lay, sessions, args, blocks, stream, false); });
 }

@@ -138,16 +138,19 @@ class GmmEngine:
                     pulled=sc["pulled"].data_ptr(), err=sc["err"].data_ptr())
 
     def a2av_gmm(self, xs, weights, counts, outs, gathered=None, num_experts: int = 0, stream=None) -> List[torch.Tensor]:
-        """``gathered[i]`` (optional) receives the all-to-all-v result; returns the gathered buffers that were used."""
+        """``gathered[i]`` (optional) receives the all-to-all-v result.  Returns every rank's gathered rows: in the tensor that was
+        given, in a buffer of the engine (until its next call), or, where a single rank multiplies its rows in place, ``x``."""
         stream = torch.cuda.current_stream(self.device) if stream is None else stream
-        args, used = [], []
-        for i in range(self.n):
-            g = gathered[i] if gathered is not None and gathered[i] is not None else self._gathered(i, outs[i].shape[0], xs[i].shape[1])
-            used.append(g)
-            d = self._common(i, xs[i], weights[i], counts[i], outs[i], num_experts)
-            d.update(gathered=g.data_ptr() if g.numel() else weights[i].data_ptr(), gathered_cap=g.shape[0],
-                     gathered_wanted=gathered is not None and gathered[i] is not None and g.numel() > 0)
-            args.append(d)
+        used = [None if gathered is None or gathered[i] is None or not gathered[i].numel() else gathered[i] for i in range(self.n)]
+        args = [self._common(i, xs[i], weights[i], counts[i], outs[i], num_experts) for i in range(self.n)]
+        for i, g in enumerate(used):
+            args[i].update(gathered=None if g is None else g.data_ptr(), gathered_cap=outs[i].shape[0] if g is None else g.shape[0])
+        if self.world == 1 and self.C.a2av_gmm(self.layout, self.sessions, args, self.blocks, stream.cuda_stream):
+            return [xs[i] if g is None else g for i, g in enumerate(used)]
+        for i, g in enumerate(used):
+            if g is None:
+                used[i] = g = self._gathered(i, outs[i].shape[0], xs[i].shape[1])
+                args[i].update(gathered=g.data_ptr() if g.numel() else weights[i].data_ptr(), gathered_cap=g.shape[0])
         self.C.a2av_gmm(self.layout, self.sessions, args, self.blocks, stream.cuda_stream)
         return used
 

@@ -202,11 +202,16 @@ def test_grouped_gemm_on_one_rank(counts, k, n):
             eng.a2av_gmm([dx], [dw], [dc], [out], [gathered], num_experts=E)
             eng.gmm_a2av([dx], [dw], [dc], [back], num_experts=E)
             outs += [out, back]
+        out = torch.full((rows, n), 5.0, dtype=torch.bfloat16, device=dev)
+        assert bits_equal(eng.a2av_gmm([dx], [dw], [dc], [out], num_experts=E)[0], x)      # the gathered rows, without a buffer
+        outs.append(out)
+        assert eng.scratch[0]["gathered"] is None
         memory = torch.zeros((rows * max(k, n),), dtype=torch.bfloat16, device=dev)       # x and the output start at one address
         shared_x, shared_out = memory[:rows * k].view(rows, k), memory[:rows * n].view(rows, n)
         for op in (eng.a2av_gmm, eng.gmm_a2av):
             shared_x.copy_(dx)
-            op([shared_x], [dw], [dc], [shared_out], num_experts=E)
+            used = op([shared_x], [dw], [dc], [shared_out], num_experts=E)
+            assert used is None or bits_equal(used[0], x)
             outs.append(shared_out.clone())
         eng.check()
         assert bits_equal(gathered, x)
