@@ -157,7 +157,10 @@ __device__ __forceinline__ void zero_padding(const DispatchArgs& a, int local_ex
   for (int row = a.pad_offsets[local_experts] + gw; row < a.recv_rows; row += warps) zero_row(row);
 }
 
-template <bool kProfile>
+// kPieces: one rank that keeps all its rows, the work items are column pieces of tokens.  Several ranks run without: their items
+// are groups of tokens with a flag each, and none of the arithmetic of pieces (8 ranks x 512 tokens of 4096 emulated in one launch
+// on one GPU: 129 us, 134 with the number of pieces as a variable and a ticket taken ahead).
+template <bool kProfile, bool kPieces>
 __global__ void __launch_bounds__(kDispatchThreads, 1) ep_dispatch_ht_kernel(const __grid_constant__ DispatchParams p) {
   const DispatchArgs& a = p.r[blockIdx.y];
   const WsLayout& lay = p.lay;
@@ -178,8 +181,16 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) ep_dispatch_ht_kernel(con
   PhaseClock<kProfile> clk;
   clk.start();
 
-  if (a.pad_offsets && !aborted)
-    zero_padding(a, a.E / P, row_bytes, nsf, (int)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, gridDim.x * (kDispatchThreads / 32), lane);
+  auto pad = [&]() {
+    if (a.pad_offsets && !aborted)
+      zero_padding(a, a.E / P, row_bytes, nsf, (int)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, gridDim.x * (kDispatchThreads / 32), lane);
+    clk.mark(kProfData);
+  };
+  // One rank starts with the padding, a fixed share per warp, and the tickets even it out (4096 tokens quantised to fp8, top-8 of
+  // 256 experts in blocks of 128 rows, with the launch: 104 us, 110 with the padding last).  With peers the senders serve them
+  // first, and receivers, whose rows are not here yet, start with it (2 ranks x 1024 tokens of 7168 over 64 experts, emulated in
+  // one launch: 74 us, 98 with the padding first everywhere).
+  if constexpr (kPieces) pad();
 
   if (sender) {
     // ================================================================ sender
@@ -188,9 +199,9 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) ep_dispatch_ht_kernel(con
     bool alive = __all_sync(0xffffffffu, ok) && !aborted;
     clk.mark(kProfWait);
     // a work item is a group of tokens, or a column piece of one token when no peer waits for flags
-    const int Lx = a.E / P, per_item = p.pieces > 0 ? 1 : kGroupTokens, pieces = max(1, p.pieces);
+    const int Lx = a.E / P, per_item = kPieces ? 1 : kGroupTokens, pieces = kPieces ? p.pieces : 1;
     const int ngroups = (a.T + per_item - 1) / per_item * pieces;
-    const int per_piece = p.pieces > 0 ? ((units + pieces - 1) / pieces + 31) / 32 * 32 : units;   // 16-byte pieces of an output row
+    const int per_piece = kPieces ? ((units + pieces - 1) / pieces + 31) / 32 * 32 : units;   // 16-byte pieces of an output row
     const uint8_t* x = reinterpret_cast<const uint8_t*>(a.x);
     const int src_row_bytes = a.mode == kDispatchFp8Given ? H : H * 2;
     uint8_t* recv_x = reinterpret_cast<uint8_t*>(a.recv_x);
@@ -199,8 +210,9 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) ep_dispatch_ht_kernel(con
     int ticket = next_ticket(&ctl->ticket[kOpDispatch][0], lane);
     while (ticket < ngroups && alive) {
       const int gi = ticket, t0 = gi / pieces * per_item, count = min(a.T - t0, per_item);
-      const int u_begin = min(units, gi % pieces * per_piece), u_count = min(units - u_begin, per_piece);
-      ticket = next_ticket(&ctl->ticket[kOpDispatch][0], lane);      // its round trip overlaps this item
+      const int u_begin = kPieces ? min(units, gi % pieces * per_piece) : 0, u_count = kPieces ? min(units - u_begin, per_piece) : units;
+      // its round trip overlaps this item; with peers a warp takes no group while it still sends one
+      if constexpr (kPieces) ticket = next_ticket(&ctl->ticket[kOpDispatch][0], lane);
       // routing of the whole group in one round of loads: lane (q, c) holds send_slot[t0 + q][c] and the local output rows
       // of slots c and c + 8 of token t0 + q (-1: the slot's expert lives elsewhere)
       int ss = -1, sr0 = -1, sr1 = -1;
@@ -258,11 +270,13 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) ep_dispatch_ht_kernel(con
       clk.mark(kProfData);
       // publish the group: every lane's stores are ordered before the flag by the warp barrier + release
       __syncwarp();
-      if (p.pieces == 0 && lane < P && !(p.local_direct && lane == me))
+      if (!kPieces && lane < P && !(p.local_direct && lane == me))
         st_release_sys(reinterpret_cast<unsigned long long*>(ctx.ws[lane] + lay.disp_flag) + (size_t)me * NG + gi, epoch);
       clk.mark(kProfPublish);
+      if constexpr (!kPieces) ticket = next_ticket(&ctl->ticket[kOpDispatch][0], lane);
     }
   }
+  if constexpr (!kPieces) pad();
   {
     // ================================================================ receiver (sender warps join once all groups are sent)
     uint8_t* recv_x = reinterpret_cast<uint8_t*>(a.recv_x);
@@ -357,7 +371,8 @@ cudaError_t launch_dispatch(const DispatchParams& params, int nranks, cudaStream
   }
   dim3 grid(p.send_blocks + p.recv_blocks, nranks), block(kDispatchThreads);
   void* args[] = {const_cast<DispatchParams*>(&p)};
-  const void* fn = p.profile ? (const void*)ep_dispatch_ht_kernel<true> : (const void*)ep_dispatch_ht_kernel<false>;
+  const void* fn = p.pieces > 0 ? (p.profile ? (const void*)ep_dispatch_ht_kernel<true, true> : (const void*)ep_dispatch_ht_kernel<false, true>)
+                                : (p.profile ? (const void*)ep_dispatch_ht_kernel<true, false> : (const void*)ep_dispatch_ht_kernel<false, false>);
   return cudaLaunchCooperativeKernel(fn, grid, block, args, 0, stream);
 }
 
