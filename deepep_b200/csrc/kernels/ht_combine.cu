@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(kCombineThreads, 1) ep_combine_local_kernel(co
       out[u] = pack_bf16x8(acc);
     }
     if (a.out_w && u0 == 0) return_values(a, t, 1, 0, K, true, entry, n, rec3, row0, nullptr, lane);
-    clk.add_rows(n);
+    if (u0 == 0) clk.add_rows(n);                            // a row counts once, with its first span
     clk.mark(kProfData);
     f = f1;
   }

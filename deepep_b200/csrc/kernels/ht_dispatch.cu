@@ -182,9 +182,10 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) ep_dispatch_ht_kernel(con
   clk.start();
 
   auto pad = [&]() {
-    if (a.pad_offsets && !aborted)
+    if (a.pad_offsets && !aborted) {
       zero_padding(a, a.E / P, row_bytes, nsf, (int)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, gridDim.x * (kDispatchThreads / 32), lane);
-    clk.mark(kProfData);
+      clk.mark(kProfData);
+    }
   };
   // One rank starts with the padding, a fixed share per warp, and the tickets even it out (4096 tokens quantised to fp8, top-8 of
   // 256 experts in blocks of 128 rows, with the launch: 104 us, 110 with the padding last).  With peers the senders serve them
@@ -265,7 +266,7 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) ep_dispatch_ht_kernel(con
           warp_fanout<false>(reinterpret_cast<const int4*>(src) + u_begin, u_count, dst + (size_t)u_begin * 16, mask, lane);
           if (fp8 && u_begin == 0) warp_fanout_f32<false>(a.x_sf + (size_t)t * nsf, nsf, dst_sf, mask, lane);
         }
-        clk.add_rows(__popc(mask));
+        if (u_begin == 0) clk.add_rows(__popc(mask));      // a row counts once, with its first piece
       }
       clk.mark(kProfData);
       // publish the group: every lane's stores are ordered before the flag by the warp barrier + release

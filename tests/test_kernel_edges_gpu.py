@@ -169,6 +169,28 @@ def test_padding_rows_are_zero(payload, alignment, experts):
     buf.destroy()
 
 
+@pytest.mark.parametrize("hidden,expand,alignment", [(7168, True, 1), (7168, True, 128), (4096, False, 1), (64, True, 16)])
+def test_device_profile_counts_every_row_once(hidden, expand, alignment):
+    """On one rank, however many pieces and spans a row is cut into: the dispatch's records add up to the rows written, those of
+    the combine to the rows read."""
+    from deepep_b200.parallel.virtual import VirtualWorld
+
+    T, E, K = 333, 16, 4
+    x = torch.randn((T, hidden), generator=torch.Generator().manual_seed(1)).bfloat16()
+    idx, w = make_routes("invalid", T, E, K, 1, 2), make_weights(T, K, 3)
+    _, lays = R.dispatch([x], [idx], [w], E, do_expand=expand, expert_alignment=alignment)
+    with VirtualWorld(1, T, hidden, K, timeout=10.0) as vw:
+        eng = vw.engine
+        plans = eng.notify([idx.cuda()], [w.cuda()], E, expand=expand, alignment=alignment)
+        eng.enable_device_profile(True)
+        (rows, _), = eng.dispatch([x.cuda()], plans, 0)
+        eng.combine([rows], plans, [None])
+        prof = eng.pop_device_profile()
+        eng.check_status()
+    for op in ("dispatch", "combine"):
+        assert sum(b["rows"] for b in prof[op, 0]) == lays[0].row_index.numel(), op
+
+
 @pytest.mark.parametrize("counts,k,n", [
     ([1], 64, 64),                                   # one row, one step, a quarter of a tile
     ([128, 0, 129, 256, 257, 0, 127], 192, 320),     # both sides of a half tile and of a tile, empty experts, a short last tile
