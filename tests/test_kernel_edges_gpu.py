@@ -135,11 +135,30 @@ def test_weighted_rows(rows, width):
                 assert _same_values(a, b)
 
 
+@pytest.fixture
+def filled_outputs(monkeypatch):
+    """Whatever the engine allocates holds 0x55 in every byte before a kernel sees it."""
+    empty = torch.empty
+
+    def filled(*args, **kwargs):
+        t = empty(*args, **kwargs)
+        if t.is_cuda:
+            t.view(torch.uint8).fill_(0x55)
+            torch.cuda.synchronize()              # the kernels may run on another stream
+        return t
+
+    monkeypatch.setattr(torch, "empty", filled)
+
+
+def _untouched(t):
+    return bool((t.view(torch.uint8) == 0x55).all())
+
+
 @pytest.mark.parametrize("payload", ["bf16", "fp8", "fp8_fused"])
 @pytest.mark.parametrize("alignment,experts", [(128, 24), (16, 700)])
-def test_padding_rows_are_zero(payload, alignment, experts):
-    """Rows that no token fills are zero whatever the memory held, rows of tokens are not touched, fresh and cached, with the
-    exact and with the worst-case row count."""
+def test_padding_rows_are_zero(filled_outputs, payload, alignment, experts):
+    """Rows that no token fills, and their scales, are zero whatever the memory held, rows of tokens are not touched, fresh and
+    cached, with the exact and with the worst-case row count."""
     from deepep_b200 import ElasticBuffer
     from deepep_b200.utils.math import per_token_cast_to_fp8
 
@@ -156,7 +175,6 @@ def test_padding_rows_are_zero(payload, alignment, experts):
     on_gpu = tuple(t.to(dev) for t in src) if payload == "fp8" else src.to(dev)
     handle = None
     for exact in (True, True, False):
-        torch.full((64 << 20,), 0x55, dtype=torch.uint8, device=dev)        # what the outputs' memory holds before the call
         fresh = dict(topk_idx=idx.to(dev), topk_weights=w.to(dev), num_experts=experts, expert_alignment=alignment, do_expand=True,
                      do_cpu_sync=exact)
         got, _, _, h, _ = buf.dispatch(on_gpu, **(fresh if handle is None or not exact else dict(handle=handle)))
@@ -249,24 +267,6 @@ def test_grouped_gemm_on_one_rank(counts, k, n):
     finally:
         torch.cuda.synchronize()
         s.close()
-
-
-@pytest.fixture
-def filled_outputs(monkeypatch):
-    """Whatever the engine allocates holds 0x55 in every byte before a kernel sees it."""
-    empty = torch.empty
-
-    def filled(*args, **kwargs):
-        t = empty(*args, **kwargs)
-        if t.is_cuda:
-            t.view(torch.uint8).fill_(0x55)
-        return t
-
-    monkeypatch.setattr(torch, "empty", filled)
-
-
-def _untouched(t):
-    return bool((t.view(torch.uint8) == 0x55).all())
 
 
 @pytest.mark.parametrize("alignment", [1, 16])
