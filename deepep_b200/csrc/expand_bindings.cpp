@@ -22,26 +22,29 @@ void check_launch(cudaError_t e, const char* what) {
 }  // namespace
 
 void bind_expand(py::module_& m) {
-  m.def("swiglu", [](const py::dict& d, bool backward, int blocks, uintptr_t stream) {
+  // `dh` null: h from gu; otherwise the gradient of gu.
+  m.def("swiglu", [](uintptr_t gu, uintptr_t dh, uintptr_t out, long long rows, int inter, int blocks, uintptr_t stream) {
     SwigluParams p{};
-    p.gu = eptr<const __nv_bfloat16>(d, "gu"); p.h = eptr<__nv_bfloat16>(d, "h");
-    p.dh = eptr<const __nv_bfloat16>(d, "dh"); p.dgu = eptr<__nv_bfloat16>(d, "dgu");
-    p.rows = d["rows"].cast<long long>(); p.inter = d["inter"].cast<int>();
-    if (p.rows < 0 || p.inter < 8 || p.inter % 8) throw std::invalid_argument("swiglu: the width must be a positive multiple of 8");
-    if (p.rows > 0 && (!p.gu || (backward ? !p.dh || !p.dgu : !p.h))) throw std::invalid_argument("swiglu: a tensor is missing");
-    for (const void* q : {(const void*)p.gu, (const void*)p.h, (const void*)p.dh, (const void*)p.dgu})
-      if (reinterpret_cast<uintptr_t>(q) % 16) throw std::invalid_argument("swiglu: rows must start on a 16-byte boundary");
-    check_launch(launch_swiglu(p, backward, blocks, reinterpret_cast<cudaStream_t>(stream)), "swiglu");
+    p.gu = reinterpret_cast<const __nv_bfloat16*>(gu);
+    p.dh = reinterpret_cast<const __nv_bfloat16*>(dh);
+    (dh ? p.dgu : p.h) = reinterpret_cast<__nv_bfloat16*>(out);
+    p.rows = rows; p.inter = inter;
+    if (rows < 0 || inter < 8 || inter % 8) throw std::invalid_argument("swiglu: the width must be a positive multiple of 8");
+    if (rows > 0 && (!gu || !out)) throw std::invalid_argument("swiglu: a tensor is missing");
+    if ((gu | dh | out) % 16) throw std::invalid_argument("swiglu: rows must start on a 16-byte boundary");
+    check_launch(launch_swiglu(p, dh != 0, blocks, reinterpret_cast<cudaStream_t>(stream)), "swiglu");
   });
-  m.def("row_scale", [](const py::dict& d, int blocks, uintptr_t stream) {
+  // `out` and the pair `b`, `prod` may be null, not both.
+  m.def("row_scale", [](uintptr_t a, uintptr_t w, uintptr_t out, uintptr_t b, uintptr_t prod, long long rows, int width, int blocks,
+                        uintptr_t stream) {
     RowScaleParams p{};
-    p.a = eptr<const __nv_bfloat16>(d, "a"); p.w = eptr<const float>(d, "w"); p.out = eptr<__nv_bfloat16>(d, "out");
-    p.b = eptr<const __nv_bfloat16>(d, "b"); p.prod = eptr<__nv_bfloat16>(d, "prod");
-    p.rows = d["rows"].cast<long long>(); p.width = d["width"].cast<int>();
-    if (p.rows < 0 || p.width < 8 || p.width % 8) throw std::invalid_argument("row_scale: the width must be a positive multiple of 8");
-    if (p.rows > 0 && (!p.a || !p.w || (!p.out && !p.prod) || !p.b != !p.prod)) throw std::invalid_argument("row_scale: a tensor is missing");
-    for (const void* q : {(const void*)p.a, (const void*)p.out, (const void*)p.b, (const void*)p.prod})
-      if (reinterpret_cast<uintptr_t>(q) % 16) throw std::invalid_argument("row_scale: rows must start on a 16-byte boundary");
+    p.a = reinterpret_cast<const __nv_bfloat16*>(a); p.w = reinterpret_cast<const float*>(w);
+    p.out = reinterpret_cast<__nv_bfloat16*>(out);
+    p.b = reinterpret_cast<const __nv_bfloat16*>(b); p.prod = reinterpret_cast<__nv_bfloat16*>(prod);
+    p.rows = rows; p.width = width;
+    if (rows < 0 || width < 8 || width % 8) throw std::invalid_argument("row_scale: the width must be a positive multiple of 8");
+    if (rows > 0 && (!a || !w || (!out && !prod) || !b != !prod)) throw std::invalid_argument("row_scale: a tensor is missing");
+    if ((a | out | b | prod) % 16) throw std::invalid_argument("row_scale: rows must start on a 16-byte boundary");
     check_launch(launch_row_scale(p, blocks, reinterpret_cast<cudaStream_t>(stream)), "row_scale");
   });
   m.attr("expand_tile") = kExpandTile;

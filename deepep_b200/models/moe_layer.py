@@ -6,8 +6,13 @@ The reference documents the rule (``README.md:168-219``, ``docs/elastic.md:7-17`
 """
 from __future__ import annotations
 
-import torch
+from contextlib import nullcontext
+from functools import lru_cache
 
+import torch
+from torch.autograd import forward_ad
+
+from ..ops import require_native
 from ..parallel.elastic import ElasticBuffer
 
 
@@ -51,7 +56,7 @@ class _Swiglu(torch.autograd.Function):
         rows, width = gate_up.shape
         h = gate_up.new_empty((rows, width // 2))
         ctx.save_for_backward(gate_up)
-        _launch("swiglu", dict(gu=gate_up, h=h), dict(rows=rows, inter=width // 2), False)
+        _launch("swiglu", gate_up, gate_up.data_ptr(), 0, h.data_ptr(), rows, width // 2)
         return h
 
     @staticmethod
@@ -62,9 +67,8 @@ class _Swiglu(torch.autograd.Function):
             with torch.enable_grad():
                 h = _separate_operations(gate_up)
             return torch.autograd.grad(h, gate_up, grad, create_graph=again)[0]
-        rows, width = gate_up.shape
-        out = torch.empty_like(gate_up)
-        _launch("swiglu", dict(gu=gate_up, dh=_readable(grad), dgu=out), dict(rows=rows, inter=width // 2), True)
+        grad, out = _readable(grad), torch.empty_like(gate_up)
+        _launch("swiglu", gate_up, gate_up.data_ptr(), grad.data_ptr(), out.data_ptr(), gate_up.shape[0], gate_up.shape[1] // 2)
         return out
 
 
@@ -75,7 +79,7 @@ class _WeighRows(torch.autograd.Function):
     def forward(ctx, rows, weights):
         out = torch.empty_like(rows)
         ctx.save_for_backward(rows, weights)
-        _launch("row_scale", dict(a=rows, w=weights, out=out), dict(rows=rows.shape[0], width=rows.shape[1]))
+        _launch("row_scale", rows, rows.data_ptr(), weights.data_ptr(), out.data_ptr(), 0, 0, *rows.shape)
         return out
 
     @staticmethod
@@ -88,24 +92,24 @@ class _WeighRows(torch.autograd.Function):
                 out = rows * weights.unsqueeze(1).to(rows.dtype)
             grads = iter(torch.autograd.grad(out, [t for t, n in zip((rows, weights), need) if n], grad, create_graph=again))
             return tuple(next(grads) if n else None for n in need)
-        tensors = dict(a=_readable(grad), w=weights)
-        if need[0]:
-            tensors["out"] = torch.empty_like(rows)
-        if need[1]:
-            tensors.update(b=rows, prod=torch.empty_like(rows))
-        _launch("row_scale", tensors, dict(rows=rows.shape[0], width=rows.shape[1]))
-        terms = tensors.get("prod")
-        return tensors.get("out"), None if terms is None else terms.sum(1, keepdim=True).to(weights.dtype).squeeze(1)
+        grad = _readable(grad)
+        out = torch.empty_like(rows) if need[0] else None
+        terms = torch.empty_like(rows) if need[1] else None
+        _launch("row_scale", rows, grad.data_ptr(), weights.data_ptr(), 0 if out is None else out.data_ptr(),
+                0 if terms is None else rows.data_ptr(), 0 if terms is None else terms.data_ptr(), *rows.shape)
+        return out, None if terms is None else terms.sum(1, keepdim=True).to(weights.dtype).squeeze(1)
 
 
-def _launch(op: str, tensors: dict, sizes: dict, *flags) -> None:
-    from ..ops import require_native
+def _launch(op: str, like: torch.Tensor, *args) -> None:
+    """Launches a kernel on the current stream of the device of ``like``."""
+    kernel, index = getattr(require_native("the training layer"), op), like.get_device()
+    with torch.cuda.device(index) if index != torch.cuda.current_device() else nullcontext():
+        kernel(*args, _blocks(index), torch.cuda.current_stream(index).cuda_stream)
 
-    device = next(iter(tensors.values())).device
-    with torch.cuda.device(device):
-        getattr(require_native("the training layer"), op)({**sizes, **{name: t.data_ptr() for name, t in tensors.items()}}, *flags,
-                                                          torch.cuda.get_device_properties(device).multi_processor_count * 8,
-                                                          torch.cuda.current_stream(device).cuda_stream)
+
+@lru_cache(maxsize=None)
+def _blocks(index: int) -> int:
+    return torch.cuda.get_device_properties(index).multi_processor_count * 8
 
 
 def _readable(grad: torch.Tensor) -> torch.Tensor:
@@ -117,11 +121,11 @@ def _readable(grad: torch.Tensor) -> torch.Tensor:
 def _ordinary(*tensors: torch.Tensor) -> bool:
     """Tensors whose memory a kernel can read, in a call that nobody traces, batches or differentiates forward: a kernel behind
     an address is invisible to all of these."""
-    return (all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors)
-            and torch._C._len_torch_dispatch_stack() == 0 and not torch._C._are_functorch_transforms_active()
-            and not any(torch._C._functorch.is_legacy_batchedtensor(t) for t in tensors)
-            and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
-            and not any(torch.autograd.forward_ad.unpack_dual(t).tangent is not None for t in tensors))
+    if (torch._C._len_torch_dispatch_stack() or torch._C._are_functorch_transforms_active() or torch.jit.is_tracing()
+            or torch.compiler.is_compiling()):
+        return False
+    return all(type(t) in (torch.Tensor, torch.nn.Parameter) and not torch._C._functorch.is_legacy_batchedtensor(t)
+               and forward_ad.unpack_dual(t).tangent is None for t in tensors)
 
 
 def _separate_operations(gate_up: torch.Tensor) -> torch.Tensor:
