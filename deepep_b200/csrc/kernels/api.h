@@ -36,7 +36,7 @@ struct NotifyArgs {
   int* recv_row_src;           // [rcap] (source * Tmax + token) * K + slot of every output row, -1 for padding
   float* recv_w;               // [rcap] (expanded) or [rcap][K] (rank layout); may be null
   long long* recv_idx;         // [rcap][K] destination-local expert ids (rank layout) or null
-  int* rank_matrix;            // optional [P][P], zeroed by the caller: tokens that source i sends to rank j (every rank computes all of it)
+  int* rank_matrix;            // optional [P][P], cleared by the launcher: tokens that source i sends to rank j (every rank computes all of it)
   int* mailbox;                // mapped host memory: [0] rows, [1] staged rows, [2] max tokens, [3] epoch, [4..] counts
   long long rcap;
 };

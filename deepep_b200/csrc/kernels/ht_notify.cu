@@ -364,6 +364,12 @@ __global__ void __launch_bounds__(kNotifyThreads) ep_notify_kernel(const __grid_
 }
 
 cudaError_t launch_notify(const NotifyParams& p, int nranks, int blocks, cudaStream_t stream) {
+  for (int i = 0; i < nranks; ++i) {
+    const NotifyArgs& a = p.r[i];
+    if (!a.rank_matrix) continue;
+    const cudaError_t e = cudaMemsetAsync(a.rank_matrix, 0, sizeof(int) * a.ctx.world * a.ctx.world, stream);
+    if (e != cudaSuccess) return e;
+  }
   dim3 grid(blocks, nranks), block(kNotifyThreads);
   void* args[] = {const_cast<NotifyParams*>(&p)};
   const void* fn = p.profile ? (const void*)ep_notify_kernel<true> : (const void*)ep_notify_kernel<false>;

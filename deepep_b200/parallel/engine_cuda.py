@@ -297,10 +297,7 @@ class CudaEngine:
                         if topk_w[i] is not None else None),
                 recv_idx=None if expand else torch.empty((rcap, K), dtype=torch.int64, device=dev),
                 has_weights=topk_w[i] is not None)
-            if rank_matrix:              # cleared where it is written: the launch stream may not wait for the current one any more
-                plan.rank_matrix = torch.empty((P, P), **i32)
-                with torch.cuda.stream(stream) if stream is not None else contextlib.nullcontext():
-                    plan.rank_matrix.zero_()
+            plan.rank_matrix = torch.empty((P, P), **i32) if rank_matrix else None      # cleared by the launcher, on its stream
             plans.append(plan)
             sc = self._scratch[i]
             args.append(dict(topk_idx=idx.data_ptr(), topk_w=_ptr(topk_w[i]), T=T, E=num_experts, K=K, expand=int(expand),
