@@ -15,9 +15,9 @@
 // from the caller's tensor straight into the output rows (quantised on the way, cut into as many pieces as
 // there are warps), and the combine reads the rows of its own experts where they lie, through the row of
 // every (token, slot) that the dispatch leaves behind.  What bounds both kernels is the chain of dependent
-// steps, not bytes: on one GPU a captured round (hidden 7168, 256 experts, top-8, fp8) took 37.9 us for one
-// token while own rows went through flags and the staging area and one thread scanned the experts, 20.1 us
-// since; 93 bf16 tokens of 4096 (64 experts, top-6) 40.4 and 20.4 us.
+// steps, not bytes: on one GPU a captured round (hidden 7168, 256 experts, top-8, fp8) took 34.8 us for one
+// token while own rows went through flags and the staging area and one thread scanned the experts, 18.4 us
+// since; 93 bf16 tokens of 4096 (64 experts, top-6) 41.3 and 20.5 us.
 //
 // Re-entrancy: epochs live in device memory and select one of two banks, flags hold epochs and
 // are never cleared, a bank is reused only after the peers acknowledged the call before last.

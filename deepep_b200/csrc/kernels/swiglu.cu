@@ -76,8 +76,8 @@ __global__ void __launch_bounds__(kSwigluThreads) swiglu_kernel(const __grid_con
   }
 }
 
-// Bound by memory.  49152 rows of 4096: 129 us one product, 257 us both (6.2 TB/s); as a library product with a broadcast factor 449 us each way, and 173 us for the
-// terms of the weight's gradient.
+// Bound by memory.  49152 rows of 4096: 129 us one product, 257 us both (6.2 TB/s); as a library product with a broadcast factor
+// 449 us each way, and 173 us for the terms of the weight's gradient.
 __global__ void __launch_bounds__(kSwigluThreads) row_scale_kernel(const __grid_constant__ RowScaleParams p) {
   const int lane = threadIdx.x & 31, units = p.width / 8;
   const long long warps = (long long)gridDim.x * (kSwigluThreads / 32);
