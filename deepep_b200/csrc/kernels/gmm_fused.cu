@@ -108,7 +108,7 @@ __device__ __forceinline__ void publish_table(const GmmArgs& a, int* table, int 
 
 // Segments (local expert, source rank) of this rank's gathered order, from every rank's table.  Run by all threads
 // of every block (each block keeps its own copy in shared memory); block 0 also writes the tile list.
-__device__ __forceinline__ void build_layout(const GmmArgs& a, GmmShared& sh, int alive, int gathered_cap, int tile_rows) {
+__device__ __forceinline__ void build_layout(const GmmArgs& a, GmmShared& sh, int alive, int gathered_cap) {
   const RankCtx& ctx = a.ctx;
   const int P = ctx.world, me = ctx.rank, L = a.E / P;
   int bad = 0;
@@ -129,7 +129,7 @@ __device__ __forceinline__ void build_layout(const GmmArgs& a, GmmShared& sh, in
       const int begin = run;
       for (int s = 0; s < P; ++s) { run += sh.seg_dst[l * P + s + 1]; sh.seg_dst[l * P + s + 1] = run; }
       sh.tile0[l] = tiles;
-      tiles += (run - begin + tile_rows - 1) / tile_rows;
+      tiles += (run - begin + kGmmTileRows - 1) / kGmmTileRows;
     }
     sh.tile0[L] = tiles;
     const bool fits = !bad && run <= gathered_cap && tiles <= a.max_tiles;
@@ -142,8 +142,8 @@ __device__ __forceinline__ void build_layout(const GmmArgs& a, GmmShared& sh, in
   if (blockIdx.x == 0) {
     for (int l = threadIdx.x; l < L; l += (int)blockDim.x) {
       const int begin = sh.seg_dst[l * P], rows = sh.seg_dst[(l + 1) * P] - begin;
-      for (int t = 0; sh.alive && t * tile_rows < rows; ++t)
-        reinterpret_cast<int4*>(a.tile_info)[sh.tile0[l] + t] = make_int4(l, begin + t * tile_rows, min(tile_rows, rows - t * tile_rows), 0);
+      for (int t = 0; sh.alive && t * kGmmTileRows < rows; ++t)
+        reinterpret_cast<int4*>(a.tile_info)[sh.tile0[l] + t] = make_int4(l, begin + t * kGmmTileRows, min(kGmmTileRows, rows - t * kGmmTileRows), 0);
     }
     if (threadIdx.x == 0) { a.num_tiles[0] = sh.num_tiles; a.num_tiles[1] = sh.total_rows; }
   }
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(kGmmGemmThreads + kGmmPullWarps * 32, 1) a2av_
   if (threadIdx.x < P) ok = wait_flag_ge(&ctl->gmm_flag[threadIdx.x][0], epoch, ctx, kOpA2avGmm, 1, threadIdx.x);
   alive = __syncthreads_and(ok) && alive;
 
-  build_layout(a, sh, alive, min(a.gathered_cap, a.out_rows_cap), kGmmTileRows);
+  build_layout(a, sh, alive, min(a.gathered_cap, a.out_rows_cap));
   __threadfence();
   grid.sync();
 
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kGmmGemmThreads, 1) gmm_a2av_kernel(const __gr
   if (threadIdx.x < P) ok = wait_flag_ge(&ctl->gmm_flag[threadIdx.x][2], epoch, ctx, kOpGmmA2av, 0, threadIdx.x);
   int alive = __syncthreads_and(ok);
 
-  build_layout(a, sh, alive, a.rows_in, kGmmTileRows);
+  build_layout(a, sh, alive, a.rows_in);
   __threadfence();
   grid.sync();
   gmm_phase<true, false>(a, sh, nullptr, smem_raw, blockIdx.x, gridDim.x);
