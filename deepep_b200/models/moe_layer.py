@@ -121,8 +121,9 @@ def _readable(grad: torch.Tensor) -> torch.Tensor:
 def _ordinary(*tensors: torch.Tensor) -> bool:
     """Tensors whose memory a kernel can read, in a call that nobody traces, batches or differentiates forward: a kernel behind
     an address is invisible to all of these."""
-    if (torch._C._len_torch_dispatch_stack() or torch._C._are_functorch_transforms_active() or torch.jit.is_tracing()
-            or torch.compiler.is_compiling()):
+    if torch.compiler.is_compiling():                    # first: a compiler follows the rest of this function no further
+        return False
+    if torch._C._len_torch_dispatch_stack() or torch._C._are_functorch_transforms_active() or torch.jit.is_tracing():
         return False
     return all(type(t) in (torch.Tensor, torch.nn.Parameter) and not torch._C._functorch.is_legacy_batchedtensor(t)
                and forward_ad.unpack_dual(t).tangent is None for t in tensors)

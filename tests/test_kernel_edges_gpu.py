@@ -105,6 +105,7 @@ def test_expert_activation_under_autograd_modes():
         results[fn] = [first.detach(), *second, tangent, batched, mapped]
     for a, b in zip(*results.values()):
         assert _same_values(a, b)
+    assert _same_values(torch.compile(_activate, backend="eager", fullgraph=True)(gu), _activate(gu))
     traced = make_fx(_activate)(gu)
     assert any("silu" in str(n.target) for n in traced.graph.nodes) and _same_values(traced(v), _activate(v))
 

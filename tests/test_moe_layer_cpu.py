@@ -111,3 +111,13 @@ def test_experts_can_be_replaced(monkeypatch, where):
     want = 2 * x.float() * w.bfloat16().float().sum(1, keepdim=True)
     assert torch.allclose(y.float(), want, rtol=0.02, atol=0.02)
     buf.destroy()
+
+
+def test_activation_and_weighting_compile_as_a_whole():
+    """The choice between kernel and separate operations does not break a compiler's graph."""
+    from deepep_b200.models import moe_layer as M
+
+    rows, weights = torch.randn((4, 32)).bfloat16(), torch.rand((4,))
+    for fn, args in ((M._activate, (rows,)), (lambda r, w: M._weigh(r, w, torch.bfloat16), (rows, weights))):
+        whole = torch.compile(fn, backend="eager", fullgraph=True)
+        assert torch.equal(whole(*args), fn(*args))
