@@ -6,7 +6,6 @@ The reference documents the rule (``README.md:168-219``, ``docs/elastic.md:7-17`
 """
 from __future__ import annotations
 
-from contextlib import nullcontext
 from functools import lru_cache
 
 import torch
@@ -103,8 +102,12 @@ class _WeighRows(torch.autograd.Function):
 def _launch(op: str, like: torch.Tensor, *args) -> None:
     """Launches a kernel on the current stream of the device of ``like``."""
     kernel, index = getattr(require_native("the training layer"), op), like.get_device()
-    with torch.cuda.device(index) if index != torch.cuda.current_device() else nullcontext():
-        kernel(*args, _blocks(index), torch.cuda.current_stream(index).cuda_stream)
+    args += _blocks(index), torch._C._cuda_getCurrentRawStream(index)
+    if index == torch.cuda.current_device():
+        kernel(*args)
+    else:
+        with torch.cuda.device(index):
+            kernel(*args)
 
 
 @lru_cache(maxsize=None)
@@ -125,8 +128,12 @@ def _ordinary(*tensors: torch.Tensor) -> bool:
         return False
     if torch._C._len_torch_dispatch_stack() or torch._C._are_functorch_transforms_active() or torch.jit.is_tracing():
         return False
-    return all(type(t) in (torch.Tensor, torch.nn.Parameter) and not torch._C._functorch.is_legacy_batchedtensor(t)
-               and forward_ad.unpack_dual(t).tangent is None for t in tensors)
+    for t in tensors:
+        if type(t) not in (torch.Tensor, torch.nn.Parameter) or torch._C._functorch.is_legacy_batchedtensor(t):
+            return False
+        if forward_ad._current_level >= 0 and forward_ad.unpack_dual(t).tangent is not None:
+            return False
+    return True
 
 
 def _separate_operations(gate_up: torch.Tensor) -> torch.Tensor:
