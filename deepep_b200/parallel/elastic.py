@@ -320,16 +320,18 @@ class ElasticBuffer:
         kernels, which only wait for the event, would overwrite it under them."""
         return bool(allocate_on_comm_stream) or any(_as_event(e) is not None for e in events)
 
-    def _leave(self, comm, async_with_compute_stream: bool, resources: Sequence[Any],
+    def _leave(self, comm, async_with_compute_stream: bool, resources: Sequence[Any], handle: EPHandle,
                allocated_on_comm: bool = False) -> EventOverlap:
-        """Sync mode: the current stream waits for the call.  Async mode: the caller waits on the returned event."""
+        """Sync mode: the current stream waits for the call.  Async mode: the caller waits on the returned event, which holds
+        ``resources`` and the tensors of ``handle``."""
         if comm is None:
             return EventOverlap()
         cur = torch.cuda.current_stream(self.device)
         if async_with_compute_stream:
-            return EventOverlap._from_resources(EventHandle(comm), tuple(resources))
+            return EventOverlap._from_resources(EventHandle(comm), (*resources, *handle._kept()))
         cur.wait_stream(comm)
         if allocated_on_comm:
+            resources = (*resources, *handle._kept())
             # The outputs belong to the communication stream's memory pool but will be used on the current stream: tell
             # the allocator, or it could hand a dropped block to the next communication kernel while compute still reads it.
             for t in resources:
@@ -448,7 +450,7 @@ class ElasticBuffer:
             recv_sf = _col_major(recv_sf)
         out_x = recv_x if recv_sf is None else (recv_x, recv_sf.view(torch.int32) if packed else recv_sf)
         event = self._leave(comm, async_with_compute_stream, [recv_x, recv_sf, recv_w, recv_idx, x_data, x_sf, topk_idx,
-                                                               topk_weights] + h._kept(), allocate_on_comm_stream)
+                                                               topk_weights], h, allocate_on_comm_stream)
         return out_x, recv_idx, recv_w, h, event
 
     def _note_failure(self, exc: Exception) -> None:
@@ -477,7 +479,7 @@ class ElasticBuffer:
                 recv_x, recv_sf = self.engine.dispatch([x_data if x_sf is None else (x_data, x_sf)], [handle._plan], mode,
                                                        blocks=num_sms or self.num_sms, stream=comm)[0]
         out_x = recv_x if recv_sf is None else (recv_x, recv_sf.view(torch.int32) if packed else recv_sf)
-        event = self._leave(comm, async_with_compute_stream, [recv_x, recv_sf, x_data, x_sf] + handle._kept() + kept,
+        event = self._leave(comm, async_with_compute_stream, [recv_x, recv_sf, x_data, x_sf] + kept, handle,
                             allocate_on_comm_stream)
         return out_x, None, None, handle, event
 
@@ -490,8 +492,8 @@ class ElasticBuffer:
         h._saved_weights = topk_weights
         recv_w = plan.recv_w[:rows]
         out_x = recv_x if recv_sf is None else (recv_x, recv_sf.view(torch.int32) if packed else recv_sf)
-        event = self._leave(comm, async_with_compute_stream, [recv_x, recv_sf, recv_w, x_data, x_sf, topk_idx, topk_weights]
-                            + h._kept(), allocated_on_comm)
+        event = self._leave(comm, async_with_compute_stream, [recv_x, recv_sf, recv_w, x_data, x_sf, topk_idx, topk_weights],
+                            h, allocated_on_comm)
         return out_x, None, recv_w, h, event
 
     def _make_handle(self, plan, expand, num_experts, alignment, num_sms, topk_idx, tokens, low_latency) -> EPHandle:
@@ -560,8 +562,8 @@ class ElasticBuffer:
                 out, out_w = self.engine.combine([x], [plan], [topk_weights], bias=None if bias is None else [tuple(biases)],
                                                  blocks=num_sms or self.num_sms, stream=comm,
                                                  **({"split": split} if split is not None else {}))[0]
-        event = self._leave(comm, async_with_compute_stream, [out, out_w, x, topk_weights] + [b for b in biases if b is not None]
-                            + handle._kept(), allocate_on_comm_stream)
+        event = self._leave(comm, async_with_compute_stream, [out, out_w, x, topk_weights] + [b for b in biases if b is not None],
+                            handle, allocate_on_comm_stream)
         return out, out_w, event
 
     # ------------------------------------------------------------------ validation helpers
