@@ -217,7 +217,7 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
 
   if (warp == 0) {
     // ============================================================ TMA producer
-    if (lane == 0) {
+    if (umma::elect_one()) {
       uint32_t it = 0;
       // The ticket of the NEXT tile is taken while the current tile is being loaded, so the round trip of the atomic is
       // off the path between two tiles.  A CTA still works through its tickets in increasing order, which is all the
@@ -290,7 +290,8 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
     }
   } else if (warp == 1) {
     // ============================================================ MMA issuer
-    if (lane == 0 && crank == 0) {
+    if (crank == 0) {
+     if (umma::elect_one()) {
       // A is e4m3 (format 0); B is e2m1 (5) or e4m3 (0), per GEMM.  A pair issues M = 256: 128 rows in each CTA.
       constexpr int kInstrM = kPair ? 2 * kGemmBM : kGemmBM;
       const uint32_t idesc1 = umma::instr_desc_mxf8f6f4(kInstrM, kGemmBN, 0, g1.b_fp8 ? 0 : 5);
@@ -351,6 +352,7 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
       }
       if (mma_stats)
         *mma_stats = ((unsigned long long)(waited >> 4) << 32) | (unsigned long long)(((clock64() - loop_start) >> 4) & 0xffffffffll);
+     }
     } else if (kPair && lane == 0) {
       // ---- odd CTA of a pair: no MMAs to issue; forward "accumulator drained" to the even CTA, once per tile
       const uint32_t acc_fwd = umma::map_to_cta(smem_u32(&bars->peer_acc_empty), 0);
