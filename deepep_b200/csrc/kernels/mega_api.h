@@ -14,6 +14,7 @@ constexpr int kGemmBM = 128;   // token rows per tile (TMEM lanes)
 constexpr int kGemmBN = 256;   // output columns per tile
 constexpr int kGemmBK = 128;   // K elements per pipeline stage (one 128-byte swizzle row of fp8)
 constexpr int kSfChunk = 512;  // bytes of block scales of 128 rows x 128 K-elements (ue8m0 per 32)
+constexpr int kSfGroup = 4;    // chunks of consecutive K steps that one copy brings
 
 // Scale factors of a [rows, K] operand are stored as 512-byte chunks, one per (128-row block, 128-K block):
 // byte (r % 32) * 16 + (r % 128) / 32 * 4 + (k / 32) % 4 of chunk (r / 128) * (K / 128) + k / 128.
@@ -32,11 +33,9 @@ enum GemmEpilogue : int {
 
 struct MegaGemmParams {
   CUtensorMap tmap_a;        // activations [rows_pad, K] e4m3, box 128 x 128, 128-byte swizzle
-  CUtensorMap tmap_b;        // weights, tiled as [(rows / 128) * (K / 128) * 128, 128 values]: e2m1 pairs that the copy engine widens
-                             // to one byte per value, or e4m3 bytes (b_fp8)
-  CUtensorMap tmap_sfa, tmap_sfb;   // the chunked scales as [chunks][512 B] (CTA pairs load them through the copy engine's tile path)
-  const uint8_t* sfa;        // chunked scales of A
-  const uint8_t* sfb;        // chunked scales of B
+  CUtensorMap tmap_b;        // weights, tiled as [rows / 128][(K / 128) * 128][128 values]: e2m1 pairs that the copy engine widens
+                             // to one byte per value, or e4m3 bytes (b_fp8); a box holds the 128 rows of a CTA of a pair, or 256
+  CUtensorMap tmap_sfa, tmap_sfb;   // the chunked scales as [chunks][512 B], kSfGroup chunks a box
   const int* mtile_expert;   // [max_mtiles] local expert of each 128-row tile
   const int* a_ready;        // optional: rows of each tile of A in place so far; a tile's loads start at 128
   const int* num_mtiles;     // device scalar: tiles in use
@@ -62,10 +61,13 @@ struct MegaGemmParams {
 };
 cudaError_t launch_mega_gemm(const MegaGemmParams& p, int blocks, cudaStream_t stream);
 
-// Encodes a 2-D tensor map with a {128 (K), 128 (rows)} box and the 128-byte swizzle.
+// Encodes e4m3 activations [rows, k] as a 2-D tensor map with a {128 (K), 128 (rows)} box and the 128-byte swizzle.
+bool encode_operand_map(CUtensorMap* map, const void* base, long long rows, long long k, const char** error);
+// Encodes tiled weights [row_blocks][k_steps * 128][128 values] as a 3-D map with a {128, 128, box_blocks} box, 128-byte swizzle.
 // fp4 = true: elements are packed e2m1 pairs that the copy engine widens to one byte each in shared memory.
-bool encode_operand_map(CUtensorMap* map, const void* base, long long rows, long long k, bool fp4, const char** error);
-// Encodes an array of 512-byte scale chunks as a 2-D map {128 x uint32, chunks} with a one-chunk box, no swizzle.
+bool encode_weights_map(CUtensorMap* map, const void* base, long long row_blocks, long long k_steps, int box_blocks, bool fp4,
+                        const char** error);
+// Encodes an array of 512-byte scale chunks as a 2-D map {128 x uint32, chunks} with a box of kSfGroup chunks, no swizzle.
 bool encode_sf_map(CUtensorMap* map, const void* base, long long chunks, const char** error);
 
 // Phase stamps of the fused kernel, one record per CTA (globaltimer nanoseconds): kernel start, inputs quantised and

@@ -20,6 +20,7 @@
 namespace dep {
 
 constexpr int kPullWarps = 2;                                    // warps beside the GEMM roles that pull tokens from peers
+constexpr int kStages = 4, kPairStages = 5;                      // operand pipeline (a CTA of a pair holds half of the weights tile)
 constexpr int kFusedThreads = kGemmThreads + kPullWarps * 32;
 
 template <bool kPair>
@@ -40,8 +41,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) mega_moe_kernel(const __grid
   const int warp = threadIdx.x >> 5;
   if (warp < kGemmThreads / 32) {
     unsigned long long* stats = a.route.timer ? a.route.timer + (size_t)blockIdx.x * kMegaTimerWords + kTimMmaThread : nullptr;
-    if constexpr (kPair) gemm_phase<true>(a.g1, &a.g2, a.ready, smem_raw, 4, blockIdx.x / 2, gridDim.x / 2, a.tile_counter, a.interleave, 1, stats);
-    else gemm_phase<false>(a.g1, &a.g2, a.ready, smem_raw, 3, blockIdx.x, gridDim.x, a.tile_counter, a.interleave, 1, stats);
+    if constexpr (kPair) gemm_phase<true>(a.g1, &a.g2, a.ready, smem_raw, kPairStages, blockIdx.x / 2, gridDim.x / 2, a.tile_counter, a.interleave, 1, stats);
+    else gemm_phase<false>(a.g1, &a.g2, a.ready, smem_raw, kStages, blockIdx.x, gridDim.x, a.tile_counter, a.interleave, 1, stats);
   } else {
     // the pull warps take part in the block (and, for CTA pairs, cluster) barriers of gemm_phase's set-up and tear-down
     if constexpr (kPair) { __syncthreads(); umma::cluster_sync_all(); }
@@ -57,8 +58,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) mega_moe_kernel(const __grid
 }
 
 cudaError_t launch_mega_fused(const MegaFusedParams& p, int nranks, int blocks, cudaStream_t stream) {
-  const size_t smem = gemm_smem_bytes(3, true);
   bool pair = p.r[0].pair != 0;
+  const size_t smem = gemm_smem_bytes(pair ? kPairStages : kStages, pair);
   for (int i = 0; i < nranks; ++i)
     if ((p.r[i].pair != 0) != pair || (p.r[i].route.tile_pairs != 0) != pair) return cudaErrorInvalidValue;
   const void* fn = pair ? (const void*)mega_moe_kernel<true> : (const void*)mega_moe_kernel<false>;

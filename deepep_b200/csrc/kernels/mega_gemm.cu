@@ -5,7 +5,7 @@ namespace dep {
 
 __global__ void __launch_bounds__(kGemmThreads, 1) mega_gemm_kernel(const __grid_constant__ MegaGemmParams p) {
   extern __shared__ uint8_t smem_raw[];
-  gemm_phase<false>(p, nullptr, nullptr, smem_raw, p.stages ? p.stages : (p.epi == kEpiCombine ? 3 : 4), blockIdx.x, gridDim.x, nullptr, 0,
+  gemm_phase<false>(p, nullptr, nullptr, smem_raw, p.stages ? p.stages : 4, blockIdx.x, gridDim.x, nullptr, 0,
                     p.commit_every ? p.commit_every : 1);
 }
 // The same as CTA pairs: launched as clusters of two CTAs.
@@ -16,12 +16,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) mega_gemm_pair_kernel(const _
 }
 
 cudaError_t launch_mega_gemm(const MegaGemmParams& p, int blocks, cudaStream_t stream) {
-  // shared memory: the operand pipeline (a CTA of a pair holds half of the weights tile), the scale chunks, the epilogue's
-  // staging area for the combine epilogue, barriers
-  const bool staging = p.epi == kEpiCombine;
-  const int stages = p.stages ? p.stages : (p.pair ? 4 : (staging ? 3 : 4));
-  const size_t stage_bytes = (size_t)kTileABytes + (p.pair ? 128 : kGemmBN) * kGemmBK + kSfStageBytes;
-  const size_t smem = 1024 + stages * stage_bytes + (staging ? kEpiStageBytes : 0) + 256;
+  const int stages = p.stages ? p.stages : 4;
+  const size_t smem = gemm_smem_bytes(stages, p.pair);
   if (smem > 227 * 1024) return cudaErrorInvalidValue;
   const void* fn = p.pair ? (const void*)mega_gemm_pair_kernel : (const void*)mega_gemm_kernel;
   // the attribute belongs to the current device, so it is set on every launch (a process may drive several GPUs)
@@ -64,7 +60,7 @@ bool encode_sf_map(CUtensorMap* map, const void* base, long long chunks, const c
   if (!encode) return false;
   cuuint64_t dims[2] = {kSfChunk / 4, (cuuint64_t)(chunks > 0 ? chunks : 1)};
   cuuint64_t strides[1] = {kSfChunk};
-  cuuint32_t box[2] = {kSfChunk / 4, 1};
+  cuuint32_t box[2] = {kSfChunk / 4, kSfGroup};
   cuuint32_t elem[2] = {1, 1};
   CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box, elem,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
@@ -76,14 +72,12 @@ bool encode_sf_map(CUtensorMap* map, const void* base, long long chunks, const c
   return true;
 }
 
-bool encode_operand_map(CUtensorMap* map, const void* base, long long rows, long long k, bool fp4, const char** error) {
+static bool encode_values(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
+                          const cuuint32_t* box, bool fp4, const char** error) {
   EncodeFn encode = tensor_map_encoder(error);
   if (!encode) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)(fp4 ? k / 2 : k)};
-  cuuint32_t box[2] = {kGemmBK, 128};
-  cuuint32_t elem[2] = {1, 1};
-  CUresult r = encode(map, fp4 ? CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base),
+  cuuint32_t elem[3] = {1, 1, 1};
+  CUresult r = encode(map, fp4 ? CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B : CU_TENSOR_MAP_DATA_TYPE_UINT8, rank, const_cast<void*>(base),
                       dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
@@ -91,6 +85,21 @@ bool encode_operand_map(CUtensorMap* map, const void* base, long long rows, long
     return false;
   }
   return true;
+}
+
+bool encode_operand_map(CUtensorMap* map, const void* base, long long rows, long long k, const char** error) {
+  const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)k};
+  const cuuint32_t box[2] = {kGemmBK, 128};
+  return encode_values(map, base, 2, dims, strides, box, false, error);
+}
+
+bool encode_weights_map(CUtensorMap* map, const void* base, long long row_blocks, long long k_steps, int box_blocks, bool fp4,
+                        const char** error) {
+  const cuuint64_t row = fp4 ? kGemmBK / 2 : kGemmBK;
+  const cuuint64_t dims[3] = {(cuuint64_t)kGemmBK, (cuuint64_t)k_steps * 128, (cuuint64_t)row_blocks};
+  const cuuint64_t strides[2] = {row, row * (cuuint64_t)k_steps * 128};
+  const cuuint32_t box[3] = {kGemmBK, 128, (cuuint32_t)box_blocks};
+  return encode_values(map, base, 3, dims, strides, box, fp4, error);
 }
 
 }  // namespace dep

@@ -19,14 +19,14 @@
 // id to the MMA and epilogue warps through a ring of mbarriers), which balances the long GEMM1 tiles
 // and the short GEMM2 tiles over the SMs; the stand-alone launch keeps the static round-robin.
 //
-// Tile shape: issuing one tcgen05 instruction costs the MMA thread about 50 cycles (measured), so a
-// stage of four N=128 MMAs (256 tensor cycles) was issue-bound; N=256 doubles the work per instruction.
-// A 128 x 256 fp32 accumulator takes 256 of the 512 TMEM columns and the scales need more, so there is
-// one accumulator: the next tile's loads are prefetched during the epilogue, its MMAs start once the
-// epilogue warps have drained the accumulator.  Both fused epilogues therefore park the bf16-rounded
-// accumulator in shared memory first, hand tensor memory back, and only then do their arithmetic and
-// their stores.  The stage time (about 0.6 us for 48 KB) is set by the rate at which shared memory
-// is filled from L2, not by the tensor pipe (0.27 us).
+// Tile shape: 128 x 256 is the widest MMA of one CTA.  A K step (128 x 256 x 128) takes the tensor pipe 512 cycles; its
+// operands are 48 KB written to and read from shared memory, 768 cycles at 128 bytes a cycle, so shared memory, and at large
+// sizes the power limit behind it, bound the loop (CTA pairs read and write a third less; see `kPair` below).  A 128 x 256 fp32
+// accumulator takes 256 of the 512 TMEM columns and the scales need more, so there is one accumulator; the epilogue warps drain
+// it into registers as bf16, 64 a thread, before anything else, and the next tile's MMAs overlap the arithmetic and the stores.
+// Scales travel in groups of four K steps (kSfGroup), both 128-row blocks of weights in one box, and the rows of the combine
+// epilogue are turned in registers, which leaves shared memory for four stages instead of three.  32 experts, hidden 7168,
+// intermediate 2048, GEMM phases of the fused layer: 1264 -> 1158 us at 4096 tokens, 192 -> 169 us at 64.
 // All waits are bounded; a wait that runs out sets an error flag, the CTA stops issuing work,
 // frees its tensor memory and returns.
 //
@@ -45,15 +45,19 @@ constexpr int kGemmMaxStages = kGemmMaxStagesHost;
 constexpr int kTileABytes = kGemmBM * kGemmBK;       // 16 KB
 constexpr int kTileBBytes = kGemmBN * kGemmBK;       // 32 KB in shared memory (one byte per value)
 constexpr int kStageBytes = kTileABytes + kTileBBytes;
-constexpr int kSfStageBytes = (1 + kGemmBN / 128) * kSfChunk;   // A scales + B scales of one stage
+// Scales travel in groups of kSfGroup K steps, whose chunks of one row block are contiguous: three copies of 2 KB per group.  As
+// three copies of 512 bytes per K step they alone held a step at 0.42 us where the tensor pipe needs 0.28.
+constexpr int kSfSlots = 2;                                     // groups in shared memory
+constexpr int kSfPart = kSfGroup * kSfChunk;                    // one row block's scales of a group
+constexpr int kSfSlotBytes = (1 + kGemmBN / 128) * kSfPart;     // A scales + B scales of a group
 constexpr int kEpiWarpCols = kGemmBN / 2;            // columns handled by one epilogue warp
-constexpr int kEpiStageBytes = kEpiWarps * 32 * kEpiWarpCols * 2;   // bf16 staging: each warp parks its 32 x 128 block
 constexpr int kTmemCols = 512;
 constexpr int kSfColBase = kGemmBN;                  // scale columns start after the accumulator
 constexpr int kSfColsPerStage = 4 + 4 * (kGemmBN / 128);
 
-__host__ __device__ constexpr size_t gemm_smem_bytes(int stages, bool staging) {
-  return 1024 + (size_t)stages * (kStageBytes + kSfStageBytes) + (staging ? kEpiStageBytes : 0) + 256;
+// A CTA of a pair holds half of the weights tile.
+__host__ __device__ constexpr size_t gemm_smem_bytes(int stages, bool pair) {
+  return 1024 + (size_t)stages * (kStageBytes - (pair ? kTileBBytes / 2 : 0)) + kSfSlots * kSfSlotBytes + 512;
 }
 
 // The MMA thread releases pipeline stages in groups of `commit_every` (one tcgen05.commit per group); a stage is
@@ -120,6 +124,25 @@ __device__ __forceinline__ bool wait_rows_ready(const int* counter, int need, vo
   *failed = site;
   return false;
 }
+// Eight 16-byte pieces per lane, transposed among groups of eight lanes: lane q of a group gets piece q of the group's lane i in
+// place of piece i.
+__device__ __forceinline__ void transpose_pieces(uint32_t (&w)[32], int lane) {
+#pragma unroll
+  for (int m = 1; m < 8; m <<= 1) {
+    const bool upper = (lane & m) != 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (i & m) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t& lo = w[4 * i + j];
+        uint32_t& hi = w[4 * (i | m) + j];
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? lo : hi, m);
+        if (upper) lo = got; else hi = got;
+      }
+    }
+  }
+}
 __device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
 // Position in the fused schedule -> tile id (ids below num_mtiles * n1 are GEMM1 tiles, the rest GEMM2 tiles).
@@ -157,14 +180,14 @@ __device__ __forceinline__ int fetch_tile(GemmBarriers* bars, uint32_t local_til
 // `tile_counter` (may be null): tiles are handed out in list order by an atomic counter, whichever CTA is free takes
 // the next one (it must be zero when the first CTA arrives); null: CTA c takes tiles c, c + num_ctas, ...
 // Either way a tile is only ever taken after all tiles before it, so a GEMM2 tile's wait for its GEMM1 tiles ends.
-// `smem_raw` must provide gemm_smem_bytes(stages, staging) bytes.
+// `smem_raw` must provide gemm_smem_bytes(stages, kPair) bytes.
 //
 // kPair: the CTAs of a cluster of two work on one 256-row tile pair (row blocks 2j and 2j + 1, which the routing layout
 // gives to the same expert).  Each CTA loads its own 128 rows of A and HALF of the 256 weight rows of B; the even CTA
 // issues tcgen05.mma.cta_group::2 (M = 256), which reads both halves of B from the two CTAs' shared memory, so a stage
 // fills 32 KB per CTA instead of 48 KB for the same tensor work.  Both CTAs' loads count their bytes on the even CTA's
 // "stage full" barrier; the odd CTA's MMA warp forwards its "accumulator drained" barrier; the even CTA's commits arrive
-// on both CTAs' barriers.  `cta` / `num_ctas` count pairs then, `stages` may be 4, and all threads of both CTAs must
+// on both CTAs' barriers.  `cta` / `num_ctas` count pairs then, and all threads of both CTAs must
 // make this call (cluster barriers).
 template <bool kPair>
 __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaGemmParams* g2, int* ready, uint8_t* smem_raw,
@@ -177,9 +200,7 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
   constexpr int kStage = kTileABytes + kBBoxes * 128 * kGemmBK;       // bytes of A and B per stage in this CTA
   const uint32_t crank = kPair ? umma::cluster_ctarank() : 0u;        // 0: issues the MMAs
   uint8_t* sf_smem = tiles + (size_t)stages * kStage;
-  uint8_t* epi_smem = sf_smem + (size_t)stages * kSfStageBytes;
-  const bool staging = g1.epi == kEpiCombine || (g2 && g2->epi == kEpiCombine);
-  GemmBarriers* bars = reinterpret_cast<GemmBarriers*>(epi_smem + (staging ? kEpiStageBytes : 0));
+  GemmBarriers* bars = reinterpret_cast<GemmBarriers*>(sf_smem + kSfSlots * kSfSlotBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -218,7 +239,11 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
   if (warp == 0) {
     // ============================================================ TMA producer
     if (umma::elect_one()) {
-      uint32_t it = 0;
+      uint32_t it = 0, sf_group = 0, sf_end0 = 0, sf_end1 = 0;   // sf_endN: the step behind the group that slot N holds
+      auto wait_released = [&](uint32_t step) {                  // the MMAs of a step (and all before it) have completed
+        const uint32_t grp = step / (uint32_t)commit_every;
+        return bounded_wait(&bars->released[grp % kGroupRing], (grp / kGroupRing) & 1u, failed, kWaitGroupReleased);
+      };
       // The ticket of the NEXT tile is taken while the current tile is being loaded, so the round trip of the atomic is
       // off the path between two tiles.  A CTA still works through its tickets in increasing order, which is all the
       // argument for the end of every GEMM2 wait needs.
@@ -257,32 +282,45 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
         }
         for (int ks = 0; ks < p.k_steps; ++ks, ++it) {
           const int s = it % stages;
-          if (it >= (uint32_t)stages) {     // the stage's previous contents have been consumed: their group was released
-            const uint32_t grp = (it - (uint32_t)stages) / (uint32_t)commit_every;
-            if (!bounded_wait(&bars->released[grp % kGroupRing], (grp / kGroupRing) & 1u, failed, kWaitGroupReleased)) break;
-          }
+          // the stage's previous contents have been consumed: their group was released
+          if (it >= (uint32_t)stages && !wait_released(it - (uint32_t)stages)) break;
+          const bool group_start = ks % kSfGroup == 0;
           uint8_t* a_dst = tiles + (size_t)s * kStage;
-          uint8_t* sf_dst = sf_smem + (size_t)s * kSfStageBytes;
+          uint8_t* sf_dst = sf_smem + (sf_group & 1u) * kSfSlotBytes;
+          if (group_start) {
+            // The slot's previous group ended at step sf_end - 1.  With whole groups and up to five stages the wait above covers
+            // it; after tiles whose last group is short it is a younger step (two steps back at least, so already loaded).
+            const uint32_t sf_end = sf_group & 1u ? sf_end1 : sf_end0;
+            if (sf_end > 0 && sf_end + (uint32_t)stages > it + 1 && !wait_released(sf_end - 1)) break;
+            const uint32_t end = it + (uint32_t)min(kSfGroup, p.k_steps - ks);
+            if (sf_group & 1u) sf_end1 = end; else sf_end0 = end;
+            ++sf_group;
+          }
+          // a group past the end of its row block brings chunks that are not used (zeros behind the last row block)
+          const int sf_bytes = group_start ? kSfSlotBytes : 0;
           if constexpr (kPair) {
             // both CTAs' bytes are counted on the even CTA's barrier, which the MMA thread waits on
             const uint32_t bar = umma::map_to_cta(smem_u32(&bars->full[s]), 0);
-            if (crank == 0) mbar_expect_tx(&bars->full[s], 2 * (kTileABytes + p.b_tx_bytes + kSfStageBytes));
+            if (crank == 0) mbar_expect_tx(&bars->full[s], 2 * (kTileABytes + p.b_tx_bytes + sf_bytes));
             umma::tma_load_2d_pair(a_dst, &p.tmap_a, ks * kGemmBK, mt * kGemmBM, bar);
-            umma::tma_load_2d_pair(sf_dst, &p.tmap_sfa, 0, mt * p.k_steps + ks, bar);
             // this CTA's half of the 256 weight rows, and the scales of all of them (each CTA of a pair needs them all)
-            umma::tma_load_2d_pair(a_dst + kTileABytes, &p.tmap_b, 0, ((brow / 128 + (int)crank) * p.k_steps + ks) * 128, bar);
+            umma::tma_load_3d_pair(a_dst + kTileABytes, &p.tmap_b, 0, ks * 128, brow / 128 + (int)crank, bar);
+            if (group_start) {
+              umma::tma_load_2d_pair(sf_dst, &p.tmap_sfa, 0, mt * p.k_steps + ks, bar);
 #pragma unroll
-            for (int h = 0; h < kGemmBN / 128; ++h)
-              umma::tma_load_2d_pair(sf_dst + (1 + h) * kSfChunk, &p.tmap_sfb, 0, (brow / 128 + h) * p.k_steps + ks, bar);
+              for (int h = 0; h < kGemmBN / 128; ++h)
+                umma::tma_load_2d_pair(sf_dst + (1 + h) * kSfPart, &p.tmap_sfb, 0, (brow / 128 + h) * p.k_steps + ks, bar);
+            }
           } else {
-            mbar_expect_tx(&bars->full[s], kTileABytes + kBBoxes * p.b_tx_bytes + kSfStageBytes);
+            mbar_expect_tx(&bars->full[s], kTileABytes + kBBoxes * p.b_tx_bytes + sf_bytes);
             umma::tma_load_2d(a_dst, &p.tmap_a, ks * kGemmBK, mt * kGemmBM, &bars->full[s]);
-            bulk_g2s(sf_dst, p.sfa + ((size_t)mt * p.k_steps + ks) * kSfChunk, kSfChunk, &bars->full[s]);
+            // both 128-row blocks of weights in one box; the second continues the swizzled tile of the first
+            umma::tma_load_3d(a_dst + kTileABytes, &p.tmap_b, 0, ks * 128, brow / 128, &bars->full[s]);
+            if (group_start) {
+              umma::tma_load_2d(sf_dst, &p.tmap_sfa, 0, mt * p.k_steps + ks, &bars->full[s]);
 #pragma unroll
-            for (int h = 0; h < kGemmBN / 128; ++h) {     // 128 weight rows per box; consecutive boxes continue the same swizzled tile
-              umma::tma_load_2d(a_dst + kTileABytes + h * 128 * kGemmBK, &p.tmap_b, 0, ((brow / 128 + h) * p.k_steps + ks) * 128,
-                                &bars->full[s]);
-              bulk_g2s(sf_dst + (1 + h) * kSfChunk, p.sfb + ((size_t)(brow / 128 + h) * p.k_steps + ks) * kSfChunk, kSfChunk, &bars->full[s]);
+              for (int h = 0; h < kGemmBN / 128; ++h)
+                umma::tma_load_2d(sf_dst + (1 + h) * kSfPart, &p.tmap_sfb, 0, (brow / 128 + h) * p.k_steps + ks, &bars->full[s]);
             }
           }
         }
@@ -305,7 +343,7 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
           umma::commit(bar);
         }
       };
-      uint32_t it = 0;
+      uint32_t it = 0, sf_group = 0;
       long long waited = 0;                      // cycles spent waiting for operands (only counted when asked for)
       const long long loop_start = mma_stats ? clock64() : 0;
       for (uint32_t local_tile = 0;; ++local_tile) {
@@ -324,18 +362,19 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
           if (mma_stats) waited += clock64() - w0;
           umma::fence_after_sync();
           const uint32_t a_addr = smem_u32(tiles + (size_t)s * kStage);
-          const uint32_t sf_addr = smem_u32(sf_smem + (size_t)s * kSfStageBytes);
+          if (ks % kSfGroup == 0) ++sf_group;
+          const uint32_t sf_addr = smem_u32(sf_smem + ((sf_group - 1) & 1u) * kSfSlotBytes + (ks % kSfGroup) * kSfChunk);
           const uint32_t tsfa = tmem + kSfColBase + s * kSfColsPerStage, tsfb = tsfa + 4;
           if constexpr (kPair) {
             umma::copy_sf_to_tmem_pair(tsfa, umma::smem_desc_sf(sf_addr));
 #pragma unroll
             for (int h = 0; h < kGemmBN / 128; ++h)
-              umma::copy_sf_to_tmem_pair(tsfb + 4 * h, umma::smem_desc_sf(sf_addr + (1 + h) * kSfChunk));
+              umma::copy_sf_to_tmem_pair(tsfb + 4 * h, umma::smem_desc_sf(sf_addr + (1 + h) * kSfPart));
           } else {
             umma::copy_sf_to_tmem(tsfa, umma::smem_desc_sf(sf_addr));
 #pragma unroll
             for (int h = 0; h < kGemmBN / 128; ++h)
-              umma::copy_sf_to_tmem(tsfb + 4 * h, umma::smem_desc_sf(sf_addr + (1 + h) * kSfChunk));
+              umma::copy_sf_to_tmem(tsfb + 4 * h, umma::smem_desc_sf(sf_addr + (1 + h) * kSfPart));
           }
           const uint64_t da = umma::smem_desc_sw128(a_addr), db = umma::smem_desc_sw128(a_addr + kTileABytes);
 #pragma unroll
@@ -368,7 +407,6 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
     const int quad = warp & 3;                       // TMEM lanes [32 * quad, 32 * quad + 32)
     const int part = (warp - 2) >> 2;                // which half of the tile's columns this warp handles
     const int row_in_tile = quad * 32 + lane;
-    uint8_t* stage = epi_smem + (size_t)(warp - 2) * 32 * kEpiWarpCols * 2;
     uint32_t first_done = 0;
     for (uint32_t local_tile = 0;; ++local_tile) {
       const int tile = fetch_tile(bars, local_tile, failed, kPair && crank != 0);
@@ -381,46 +419,86 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
       umma::fence_after_sync();
       const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
       const long long row = (long long)mt * kGemmBM + row_in_tile;
-      uint32_t v[32], u[32];
-      if (p.epi == kEpiCombine) {
-        // bf16 rows go to the source rank's combine slots.
-        // 1) drain this warp's 32 x 128 block into shared memory as bf16 and hand the accumulator back at once
-        const int code = p.row_src[row];
-        uint8_t* dst_row = nullptr;
-        if (code >= 0) {
-          const int src = code / (p.max_tokens * p.topk), rem = code - src * p.max_tokens * p.topk;
-          dst_row = p.ws[src] + p.comb_off + ((size_t)rem * p.hidden + (size_t)nb * kGemmBN) * 2;
-        }
-        uint4* mine = reinterpret_cast<uint4*>(stage + (size_t)lane * kEpiWarpCols * 2);   // 256 B per row = 16 pieces
-        __syncwarp();                                     // the previous tile's block has been written out
-        for (int c = 0; c < kEpiWarpCols; c += 32) {
-          umma::tmem_ld32(taddr + part * kEpiWarpCols + c, v);
+      if (p.epi != kEpiStoreF32) {
+        // Both epilogues round the accumulator to bf16 first, so this warp's 32 x 128 block fits into 64 registers a thread: it
+        // is drained at once and tensor memory handed back, and the next tile's MMAs overlap everything that follows.
+        uint32_t held[2][32];      // SwiGLU: [32-column group][16 words of gate, 16 of up]; combine: [64-column half][words]
+        const bool swiglu = p.epi == kEpiSwigluQuant;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t v[32];
+          // SwiGLU: columns [0, 128) of a tile are gate rows of W1, [128, 256) the matching up rows
+          const int col = swiglu ? (i & 1) * (kGemmBN / 2) + (part * 2 + (i >> 1)) * 32 : part * kEpiWarpCols + i * 32;
+          umma::tmem_ld32(taddr + col, v);
           umma::tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint32_t w0[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              __nv_bfloat162 b0 = __floats2bfloat162_rn(__uint_as_float(v[8 * i + 2 * j]), __uint_as_float(v[8 * i + 2 * j + 1]));
-              w0[j] = *reinterpret_cast<uint32_t*>(&b0);
-            }
-            mine[(c / 8 + i) ^ (lane & 15)] = make_uint4(w0[0], w0[1], w0[2], w0[3]);   // XOR swizzle against bank conflicts
+          for (int j = 0; j < 16; ++j) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+            held[i >> 1][(i & 1) * 16 + j] = *reinterpret_cast<const uint32_t*>(&b);
           }
         }
         umma::fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->acc_empty);
-        // 2) write the block out: 16 lanes x 16 B cover one row's 256-byte segment, 2 rows per instruction
-#pragma unroll 4
-        for (int r0 = 0; r0 < 32; r0 += 2) {
-          const int rr = r0 + (lane >> 4), piece = lane & 15;
-          uint8_t* drow = reinterpret_cast<uint8_t*>(__shfl_sync(0xffffffffu, (unsigned long long)dst_row, rr));
-          const uint4 val = reinterpret_cast<const uint4*>(stage + (size_t)rr * kEpiWarpCols * 2)[piece ^ (rr & 15)];
-          if (drow) reinterpret_cast<uint4*>(drow + (size_t)part * kEpiWarpCols * 2)[piece] = val;
+        if (!swiglu) {
+          // bf16 rows go to the source rank's combine slots.  Eight lanes exchange their rows' 16-byte pieces (a transpose in
+          // registers; staged in shared memory the rows took the space of the fourth pipeline stage), so that the eight cover
+          // one row's 128-byte segment, four rows per store instruction.
+          const int code = p.row_src[row];
+          uint8_t* dst_row = nullptr;
+          if (code >= 0) {
+            const int src = code / (p.max_tokens * p.topk), rem = code - src * p.max_tokens * p.topk;
+            dst_row = p.ws[src] + p.comb_off + ((size_t)rem * p.hidden + (size_t)nb * kGemmBN + part * kEpiWarpCols) * 2;
+          }
+#pragma unroll
+          for (int half = 0; half < 2; ++half) transpose_pieces(held[half], lane);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            uint8_t* drow = reinterpret_cast<uint8_t*>(__shfl_sync(0xffffffffu, (unsigned long long)dst_row, (lane & 24) + i));
+            if (drow) {
+#pragma unroll
+              for (int half = 0; half < 2; ++half)
+                *reinterpret_cast<uint4*>(drow + half * 128 + (lane & 7) * 16) =
+                    make_uint4(held[half][4 * i], held[half][4 * i + 1], held[half][4 * i + 2], held[half][4 * i + 3]);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            const int half = part * 2 + hh;
+            float h[32], amax = 0.f;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const __nv_bfloat162 bg = *reinterpret_cast<const __nv_bfloat162*>(&held[hh][i / 2]);
+              const __nv_bfloat162 bu = *reinterpret_cast<const __nv_bfloat162*>(&held[hh][16 + i / 2]);
+              const float g = i & 1 ? __high2float(bg) : __low2float(bg), up = i & 1 ? __high2float(bu) : __low2float(bu);
+              // div.approx: the IEEE division has a slow path for huge / non-finite operands, which padding rows (whatever
+              // the row buffer held) do contain; it made this epilogue, and with it the whole tile, measurably slower
+              const float act = __fdividef(g, 1.0f + __expf(fminf(fmaxf(-g, -80.f), 80.f))) * up;
+              h[i] = bf16_round(act);
+              amax = fmaxf(amax, fabsf(h[i]));
+            }
+            // MX scale: 2^(floor(log2(amax)) - 8), at least 2^-127; values saturate at 448
+            int e = (int)((__float_as_uint(fmaxf(amax, 1.1754944e-38f)) >> 23) & 0xff) - 127 - 8;
+            e = max(e, -127);
+            const float inv = __uint_as_float((uint32_t)(127 - e) << 23);   // 2^-e, exact (e in [-127, 120])
+            uint32_t q[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              q[i] = (uint32_t)__nv_cvt_float_to_fp8(h[4 * i] * inv, __NV_SATFINITE, __NV_E4M3) |
+                     ((uint32_t)__nv_cvt_float_to_fp8(h[4 * i + 1] * inv, __NV_SATFINITE, __NV_E4M3) << 8) |
+                     ((uint32_t)__nv_cvt_float_to_fp8(h[4 * i + 2] * inv, __NV_SATFINITE, __NV_E4M3) << 16) |
+                     ((uint32_t)__nv_cvt_float_to_fp8(h[4 * i + 3] * inv, __NV_SATFINITE, __NV_E4M3) << 24);
+            }
+            const long long col = (long long)nb * (kGemmBN / 2) + half * 32;
+            uint4* dst = reinterpret_cast<uint4*>(p.a2 + row * p.inter + col);
+            dst[0] = make_uint4(q[0], q[1], q[2], q[3]);
+            dst[1] = make_uint4(q[4], q[5], q[6], q[7]);
+            p.a2_sf[sf_offset(row, col, p.inter)] = (uint8_t)(e + 127);
+          }
         }
-        continue;   // the accumulator was already released
-      }
-      if (p.epi == kEpiStoreF32) {
+      } else {
+        uint32_t v[32];
         for (int c = part * (kGemmBN / 2); c < (part + 1) * (kGemmBN / 2); c += 32) {
           umma::tmem_ld32(taddr + c, v);
           umma::tmem_ld_wait();
@@ -429,89 +507,6 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
           for (int i = 0; i < 8; ++i) dst[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
                                                              __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
         }
-      } else {
-        // SwiGLU + requantisation: columns [0, 128) are gate rows of W1, [128, 256) the matching up rows.
-        // With a staging area the bf16-rounded accumulator (the first step of the math anyway) is parked in shared
-        // memory and tensor memory is handed back before the arithmetic, so the next tile's MMAs overlap it.
-        uint4* mine = reinterpret_cast<uint4*>(stage + (size_t)lane * kEpiWarpCols * 2);   // 256 B per row = 16 pieces
-        if (staging) {
-          __syncwarp();
-#pragma unroll
-          for (int hh = 0; hh < kGemmBN / 128; ++hh) {
-            const int half = part * (kGemmBN / 128) + hh;
-            umma::tmem_ld32(taddr + half * 32, v);
-            umma::tmem_ld32(taddr + kGemmBN / 2 + half * 32, u);
-            umma::tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint32_t wg[4], wu[4];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                __nv_bfloat162 bg = __floats2bfloat162_rn(__uint_as_float(v[8 * i + 2 * j]), __uint_as_float(v[8 * i + 2 * j + 1]));
-                __nv_bfloat162 bu = __floats2bfloat162_rn(__uint_as_float(u[8 * i + 2 * j]), __uint_as_float(u[8 * i + 2 * j + 1]));
-                wg[j] = *reinterpret_cast<uint32_t*>(&bg);
-                wu[j] = *reinterpret_cast<uint32_t*>(&bu);
-              }
-              mine[(hh * 8 + i) ^ (lane & 15)] = make_uint4(wg[0], wg[1], wg[2], wg[3]);
-              mine[(hh * 8 + 4 + i) ^ (lane & 15)] = make_uint4(wu[0], wu[1], wu[2], wu[3]);
-            }
-          }
-          umma::fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars->acc_empty);
-        }
-        for (int half = part * (kGemmBN / 128); half < (part + 1) * (kGemmBN / 128); ++half) {
-          float gv[32], uv[32];
-          if (staging) {
-            const int hh = half - part * (kGemmBN / 128);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const uint4 pg = mine[(hh * 8 + i) ^ (lane & 15)], pu = mine[(hh * 8 + 4 + i) ^ (lane & 15)];
-              const __nv_bfloat162* bg = reinterpret_cast<const __nv_bfloat162*>(&pg);
-              const __nv_bfloat162* bu = reinterpret_cast<const __nv_bfloat162*>(&pu);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                gv[8 * i + 2 * j] = __low2float(bg[j]); gv[8 * i + 2 * j + 1] = __high2float(bg[j]);
-                uv[8 * i + 2 * j] = __low2float(bu[j]); uv[8 * i + 2 * j + 1] = __high2float(bu[j]);
-              }
-            }
-          } else {
-            umma::tmem_ld32(taddr + half * 32, v);
-            umma::tmem_ld32(taddr + kGemmBN / 2 + half * 32, u);
-            umma::tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) { gv[i] = bf16_round(__uint_as_float(v[i])); uv[i] = bf16_round(__uint_as_float(u[i])); }
-          }
-          float h[32], amax = 0.f;
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float g = gv[i], up = uv[i];
-            // div.approx: the IEEE division has a slow path for huge / non-finite operands, which padding rows (whatever
-            // the row buffer held) do contain; it made this epilogue, and with it the whole tile, measurably slower
-            const float act = __fdividef(g, 1.0f + __expf(fminf(fmaxf(-g, -80.f), 80.f))) * up;
-            h[i] = bf16_round(act);
-            amax = fmaxf(amax, fabsf(h[i]));
-          }
-          // MX scale: 2^(floor(log2(amax)) - 8), at least 2^-127; values saturate at 448
-          int e = (int)((__float_as_uint(fmaxf(amax, 1.1754944e-38f)) >> 23) & 0xff) - 127 - 8;
-          e = max(e, -127);
-          const float inv = __uint_as_float((uint32_t)(127 - e) << 23);   // 2^-e, exact (e in [-127, 120])
-          uint32_t q[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            q[i] = (uint32_t)__nv_cvt_float_to_fp8(h[4 * i] * inv, __NV_SATFINITE, __NV_E4M3) |
-                   ((uint32_t)__nv_cvt_float_to_fp8(h[4 * i + 1] * inv, __NV_SATFINITE, __NV_E4M3) << 8) |
-                   ((uint32_t)__nv_cvt_float_to_fp8(h[4 * i + 2] * inv, __NV_SATFINITE, __NV_E4M3) << 16) |
-                   ((uint32_t)__nv_cvt_float_to_fp8(h[4 * i + 3] * inv, __NV_SATFINITE, __NV_E4M3) << 24);
-          }
-          const long long col = (long long)nb * (kGemmBN / 2) + half * 32;
-          uint4* dst = reinterpret_cast<uint4*>(p.a2 + row * p.inter + col);
-          dst[0] = make_uint4(q[0], q[1], q[2], q[3]);
-          dst[1] = make_uint4(q[4], q[5], q[6], q[7]);
-          p.a2_sf[sf_offset(row, col, p.inter)] = (uint8_t)(e + 127);
-        }
-      }
-      if (!(p.epi == kEpiSwigluQuant && staging)) {      // (that path released the accumulator before its arithmetic)
         umma::fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->acc_empty);

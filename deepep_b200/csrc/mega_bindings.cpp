@@ -32,20 +32,20 @@ void fill_gemm(MegaGemmParams& p, const py::dict& d, py::object session) {
   const long long rows_pad = getl(d, "rows_pad"), k = getl(d, "k"), b_rows = getl(d, "b_rows");
   if (rows_pad % kGemmBM || k % kGemmBK || b_rows % kGemmBN) throw std::invalid_argument("rows and K must be multiples of 128, weight rows of 256");
   const char* err = nullptr;
-  if (!encode_operand_map(&p.tmap_a, ptr<const void>(d, "a"), rows_pad, k, false, &err)) throw std::runtime_error(err);
+  if (!encode_operand_map(&p.tmap_a, ptr<const void>(d, "a"), rows_pad, k, &err)) throw std::runtime_error(err);
   // weights are stored tiled: every (128-row, 128-K) block is one contiguous run of 128 rows x 64 (e2m1) or 128 (e4m3) bytes
   p.b_fp8 = geti(d, "b_fp8", 0) ? 1 : 0;
-  if (!encode_operand_map(&p.tmap_b, ptr<const void>(d, "b"), b_rows * (k / kGemmBK), kGemmBK, !p.b_fp8, &err)) throw std::runtime_error(err);
-  p.sfa = ptr<const uint8_t>(d, "sfa"); p.sfb = ptr<const uint8_t>(d, "sfb");
-  if (!encode_sf_map(&p.tmap_sfa, p.sfa, (rows_pad / kGemmBM) * (k / kGemmBK), &err)) throw std::runtime_error(err);
-  if (!encode_sf_map(&p.tmap_sfb, p.sfb, (b_rows / 128) * (k / kGemmBK), &err)) throw std::runtime_error(err);
+  p.pair = geti(d, "pair", 0) ? 1 : 0;
+  if (!encode_weights_map(&p.tmap_b, ptr<const void>(d, "b"), b_rows / 128, k / kGemmBK, p.pair ? 1 : kGemmBN / 128, !p.b_fp8, &err))
+    throw std::runtime_error(err);
+  if (!encode_sf_map(&p.tmap_sfa, ptr<const void>(d, "sfa"), (rows_pad / kGemmBM) * (k / kGemmBK), &err)) throw std::runtime_error(err);
+  if (!encode_sf_map(&p.tmap_sfb, ptr<const void>(d, "sfb"), (b_rows / 128) * (k / kGemmBK), &err)) throw std::runtime_error(err);
   p.mtile_expert = ptr<const int>(d, "mtile_expert"); p.num_mtiles = ptr<const int>(d, "num_mtiles");
   p.a_ready = ptr<const int>(d, "a_ready");
   p.max_mtiles = (int)(rows_pad / kGemmBM);
   p.n_total = geti(d, "n_total"); p.n_tiles = p.n_total / kGemmBN; p.k_steps = (int)(k / kGemmBK);
   if (p.n_total % kGemmBN) throw std::invalid_argument("output width must be a multiple of 256");
   p.epi = geti(d, "epi");
-  p.pair = geti(d, "pair", 0) ? 1 : 0;
   p.stages = geti(d, "stages", 0); p.commit_every = geti(d, "commit_every", 0);
   if (p.stages < 0 || p.stages > kGemmMaxStagesHost || p.stages == 1 || p.commit_every < 0 || p.commit_every > 2)
     throw std::invalid_argument("stages must be 0 or 2..6, commit_every 0, 1 or 2");
@@ -112,6 +112,7 @@ void op_mega_fused(const WsLayout& lay, const std::vector<py::object>& sessions,
     p.r[i].tile_counter = ptr<int>(d, "tile_counter");
     p.r[i].interleave = geti(d, "interleave", 1);
     p.r[i].pair = geti(d, "pair", 0) ? 1 : 0;
+    if (p.r[i].pair != p.r[i].g1.pair || p.r[i].pair != p.r[i].g2.pair) throw std::invalid_argument("the GEMMs' boxes disagree about CTA pairs");
     if (p.r[i].pair && n > 1) throw std::invalid_argument("CTA pairs are for one rank per GPU (virtual ranks share the SMs)");
     if (!p.r[i].ready || !p.r[i].route.pulled) throw std::invalid_argument("the fused kernel needs the ready and pulled counter arrays");
   }

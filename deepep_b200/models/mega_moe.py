@@ -193,6 +193,7 @@ class MegaEngine:
                 route_args[i]["pulled"] = sc["pulled"].data_ptr()
                 route_args[i]["tile_pairs"] = int(pair)
                 gemm1_args[i]["a_ready"] = sc["pulled"].data_ptr()
+                gemm1_args[i]["pair"] = gemm2_args[i]["pair"] = int(pair)
             blocks = max(1, min(self.gemm_blocks, self.sm_count // self.n))
             C.mega_fused(lay, self.sessions, [dict(route=route_args[i], finish=finish_args[i], gemm1=gemm1_args[i],
                                                   gemm2=gemm2_args[i], ready=self.scratch[i]["ready"].data_ptr(),

@@ -7,7 +7,7 @@ from deepep_b200.oracle import megamoe as O
 pytestmark = pytest.mark.gpu
 
 
-def _run(rows_per_expert, n_total, k, seed=0, b_tx=None, pair=False, stages=0, commit_every=0):
+def _run(rows_per_expert, n_total, k, seed=0, b_tx=None, pair=False, stages=0, commit_every=0, blocks=148):
     from deepep_b200.ops import load_native
 
     C = load_native()
@@ -39,7 +39,7 @@ def _run(rows_per_expert, n_total, k, seed=0, b_tx=None, pair=False, stages=0, c
         args["stages"] = stages
     if commit_every:
         args["commit_every"] = commit_every
-    C.mega_gemm(args, None, 148, torch.cuda.current_stream().cuda_stream)
+    C.mega_gemm(args, None, blocks, torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
     assert d["err"].item() == 0, "a pipeline wait ran out inside the GEMM kernel"
     out = d["c"].cpu()
@@ -77,3 +77,11 @@ def test_pipeline_depth_and_commit_grouping():
     _run([128, 256], 256, 2048, seed=5, stages=4, commit_every=2)
     _run([256, 512], 512, 2048, seed=6, pair=True, stages=6, commit_every=2)
     _run([256], 256, 2048, seed=7, pair=True, stages=3)
+
+
+@pytest.mark.parametrize("k", [128, 256, 640, 896, 1152])
+@pytest.mark.parametrize("pair, stages", [(False, 2), (False, 4), (True, 4), (True, 6)])
+def test_short_scale_groups(k, pair, stages):
+    """Tiles whose last group of scales holds one to four of its K steps, several tiles per CTA in a row: the two slots of the
+    scales are filled again while younger steps than the oldest stage are still being multiplied."""
+    _run([256, 100, 130], 512, k, seed=k + stages, pair=pair, stages=stages, blocks=2)
