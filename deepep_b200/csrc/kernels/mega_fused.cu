@@ -35,8 +35,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) mega_moe_kernel(const __grid
     if (threadIdx.x == 0 && a.tile_counter) *a.tile_counter = 0;
   }
   route_layout_phase(a.route, grid, sh);          // handshake, counts, tile layout (grid barriers inside)
-  __threadfence();
-  grid.sync();
   // The token pull overlaps the GEMMs: rows are pulled tile by tile, a GEMM1 tile starts once its rows have arrived.
   const int warp = threadIdx.x >> 5;
   if (warp < kGemmThreads / 32) {
@@ -52,7 +50,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) mega_moe_kernel(const __grid
     if constexpr (kPair) umma::cluster_sync_all();
   }
   mega_stamp(a.route.timer, kTimGemm);             // this CTA ran out of tiles (or of rows to pull)
-  __threadfence_system();
+  fence_for_peers(a.route.ctx.world);
   grid.sync();
   finish_phase(a.finish, true);
 }

@@ -524,7 +524,7 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
         ++first_done;
       }
     }
-    __threadfence_system();       // rows pushed to peers are visible before the kernel (or its next phase) signals them
+    if (!g2) __threadfence_system();   // rows pushed to peers are visible before the next kernel signals them (the fused layer fences itself)
   }
 
   umma::fence_before_sync();

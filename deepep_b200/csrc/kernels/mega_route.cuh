@@ -45,10 +45,17 @@ struct RouteShared {
   int alive, total_rows;
 };
 
-constexpr int kPullChunk = 8;   // consecutive rows one warp pulls before it moves on
+constexpr int kPullChunk = 8;                            // rows one warp pulls before it moves on
+constexpr int kPullStride = kGemmBM / kPullChunk;        // distance of a chunk's rows, and chunks per tile
 
 __device__ __forceinline__ void mega_stamp(unsigned long long* timer, int slot) {
   if (timer != nullptr && threadIdx.x == 0) timer[(size_t)blockIdx.x * kMegaTimerWords + slot] = global_timer_ns();
+}
+
+// What this thread wrote is visible to the peers, or, on a single rank, to the rest of the GPU.
+__device__ __forceinline__ void fence_for_peers(int world) {
+  if (world > 1) __threadfence_system();
+  else __threadfence();
 }
 
 // bf16 [T, H] -> e4m3 codes and one ue8m0 exponent per 32 values, written into this rank's symmetric input block.
@@ -111,24 +118,22 @@ __device__ __forceinline__ void route_layout_phase(const MegaRouteArgs& a, cg::g
   mega_stamp(a.timer, kTimStart);
   if (a.x_bf16 != nullptr)   // the caller passed bf16 activations: quantise them into the symmetric input block first
     quantize_inputs_phase(a, ctx.ws[me] + a.in_off + in.x, ctx.ws[me] + a.in_off + in.x_sf);
-  // ---- handshake: my inputs are in place (stream order, or just written above), tell everybody, wait for everybody
-  __threadfence_system();
-  if (blockIdx.x == 0 && threadIdx.x < P) {
+  // ---- handshake: my inputs are in place (stream order, or just written above), tell everybody, wait for everybody.  What this
+  // rank's own blocks wrote is ordered by the grid barrier, so it needs neither a system fence nor the rank's own flag.
+  if (blockIdx.x == 0) {
     if (threadIdx.x == 0) reinterpret_cast<int*>(ctx.ws[me] + a.in_off + in.hdr)[0] = a.T;
-    __threadfence_system();
+    for (int l = threadIdx.x; l < Lx + S; l += (int)blockDim.x) a.expert_rows[l] = 0;    // counted up behind the barrier
   }
+  fence_for_peers(P);
   grid.sync();
   if (blockIdx.x == 0 && threadIdx.x < P) st_release_sys(&control_of(ctx.ws[threadIdx.x])->mega_flag[me][0], epoch);
   int ok = 1;
-  if (threadIdx.x < P) ok = wait_flag_ge(&ctl->mega_flag[threadIdx.x][0], epoch, ctx, kOpMega, 0, threadIdx.x);
+  if (threadIdx.x < P && threadIdx.x != me) ok = wait_flag_ge(&ctl->mega_flag[threadIdx.x][0], epoch, ctx, kOpMega, 0, threadIdx.x);
   const int alive = __syncthreads_and(ok);
   if (threadIdx.x < kMaxRanks)
     sh.T[threadIdx.x] = (alive && threadIdx.x < P) ? __ldcg(reinterpret_cast<const int*>(ctx.ws[threadIdx.x] + a.in_off + in.hdr)) : 0;
   if (threadIdx.x == 0) sh.alive = alive;
-  // zero the per-expert counters
-  if (blockIdx.x == 0) for (int l = threadIdx.x; l < Lx + S; l += (int)blockDim.x) a.expert_rows[l] = 0;
   __syncthreads();
-  grid.sync();
   mega_stamp(a.timer, kTimHandshake);
 
   // ---- pass 1: the routed slots of every local expert (own rank first, then the peers in ring order)
@@ -152,30 +157,45 @@ __device__ __forceinline__ void route_layout_phase(const MegaRouteArgs& a, cg::g
   __threadfence();
   grid.sync();
 
-  // ---- tile layout: every expert starts at a multiple of 128 rows (256 with CTA pairs)
-  for (int l = threadIdx.x; l < Lx + S; l += (int)blockDim.x) sh.rows[l] = min(__ldcg(a.expert_rows + l), cap);   // parallel loads
+  // ---- tile layout: every expert starts at a multiple of 128 rows (256 with CTA pairs).  Every block derives all of it and
+  // writes the same tile list, so no block waits for another one's (the writes race with equal values).
+  for (int l = threadIdx.x; l < Lx + S; l += (int)blockDim.x) sh.rows[l] = min(__ldcg(a.expert_rows + l), cap);
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x, unit = a.tile_pairs ? 2 * kGemmBM : kGemmBM;      // with CTA pairs an expert owns whole pairs of tiles
     int run = 0;
-    for (int l = 0; l < Lx + S; ++l) {
-      const int c = sh.rows[l];
-      sh.base[l] = run;
-      const int unit = a.tile_pairs ? 2 * kGemmBM : kGemmBM;      // with CTA pairs an expert owns whole pairs of tiles
-      const int tiles = (c + unit - 1) / unit * (unit / kGemmBM);
-      if (blockIdx.x == 0)
-        for (int t = 0; t < tiles && run / kGemmBM + t < a.max_mtiles; ++t) a.mtile_expert[run / kGemmBM + t] = l;
-      run += tiles * kGemmBM;
+    for (int l0 = 0; l0 < Lx + S; l0 += 32) {
+      const int l = l0 + lane, rows = l < Lx + S ? (sh.rows[l] + unit - 1) / unit * unit : 0;
+      int sum = rows;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, sum, d);
+        if (lane >= d) sum += o;
+      }
+      if (l < Lx + S) sh.base[l] = run + sum - rows;
+      run += __shfl_sync(0xffffffffu, sum, 31);
     }
-    sh.total_rows = min(run, a.max_mtiles * kGemmBM);
-    if (blockIdx.x == 0) *a.num_mtiles = sh.total_rows / kGemmBM;
+    if (lane == 0) {
+      sh.total_rows = min(run, a.max_mtiles * kGemmBM);
+      *a.num_mtiles = sh.total_rows / kGemmBM;
+    }
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < sh.total_rows / kGemmBM; t += (int)blockDim.x) {
+    int lo = 0, hi = Lx + S;       // the last expert that starts at this tile or before it (empty ones share a start and are skipped)
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (sh.base[mid] <= t * kGemmBM) lo = mid; else hi = mid;
+    }
+    a.mtile_expert[t] = lo;
   }
   __syncthreads();
   mega_stamp(a.timer, kTimLayout);
 }
 
-// Pulls the routed tokens from their owners in row order (tile by tile, so that the first tiles are complete first);
-// warp `gw` of `total_warps` warps.  Padding rows get row_src = -1; their payload is never read back (tile rows are
-// independent in the GEMMs).
+// Pulls the routed tokens from their owners (tile by tile, so that the first tiles are complete first); warp `gw` of
+// `total_warps` warps.  A chunk is every kPullStride-th row of a tile: an expert's few rows of a decode batch, which are the first
+// rows of its tile, are then shared out over the tile's chunks (16 rows in one chunk or two keep as many warps busy for eight rows
+// in a row).  Padding rows get row_src = -1; their payload is never read back (tile rows are independent in the GEMMs).
 __device__ __forceinline__ void route_pull_phase(const MegaRouteArgs& a, const RouteShared& sh, int gw, int total_warps) {
   const RankCtx& ctx = a.ctx;
   const int P = ctx.world, K = a.K, H = a.H, M = a.max_tokens;
@@ -183,11 +203,12 @@ __device__ __forceinline__ void route_pull_phase(const MegaRouteArgs& a, const R
   const MegaInput in = mega_input_layout(M, H, K);
   const int cap = P * M, Kp = K + a.S;
   if (!sh.alive) return;
-  for (int row0 = gw * kPullChunk; row0 < sh.total_rows; row0 += total_warps * kPullChunk) {
-    // lane j < kPullChunk looks up row row0 + j
+  for (int chunk = gw; chunk < sh.total_rows / kPullChunk; chunk += total_warps) {
+    const int tile = chunk / kPullStride, row0 = tile * kGemmBM + chunk % kPullStride;
+    // lane j < kPullChunk looks up row row0 + j * kPullStride
     int entry = -1;
-    if (lane < kPullChunk && row0 + lane < sh.total_rows) {
-      const int row = row0 + lane, l = __ldcg(a.mtile_expert + row / kGemmBM), j = row - sh.base[l];
+    if (lane < kPullChunk) {
+      const int row = row0 + lane * kPullStride, l = __ldcg(a.mtile_expert + tile), j = row - sh.base[l];
       if (j < sh.rows[l]) entry = __ldcg(a.expert_list + (size_t)l * cap + j);
       a.row_src[row] = entry;
     }
@@ -195,7 +216,7 @@ __device__ __forceinline__ void route_pull_phase(const MegaRouteArgs& a, const R
     for (int c = 0; c < kPullChunk; ++c) {
       const int en = __shfl_sync(0xffffffffu, entry, c);
       if (en < 0) continue;
-      const long long row = row0 + c;
+      const long long row = row0 + c * kPullStride;
       const int r = en / (M * Kp), t = (en - r * M * Kp) / Kp;
       const uint8_t* peer = ctx.ws[r] + a.in_off;
       const int4* from = reinterpret_cast<const int4*>(peer + in.x + (size_t)t * H);
@@ -208,7 +229,7 @@ __device__ __forceinline__ void route_pull_phase(const MegaRouteArgs& a, const R
     if (a.pulled) {            // tell the GEMM that these rows of the tile (payload or padding mark) are in place
       __threadfence();
       __syncwarp();
-      if (lane == 0) atomicAdd(a.pulled + row0 / kGemmBM, min(kPullChunk, sh.total_rows - row0));
+      if (lane == 0) atomicAdd(a.pulled + tile, kPullChunk);
     }
   }
   if (a.timer != nullptr && lane == 0)     // the CTA's pull warps all write this word; the last one to finish wins
@@ -234,11 +255,11 @@ __device__ __forceinline__ void finish_phase(const MegaFinishArgs& a, bool bump_
 
   // my GEMM2 finished before this kernel started (stream order, its remote writes were fenced)
   if (blockIdx.x == 0 && threadIdx.x < P) {
-    __threadfence_system();
+    fence_for_peers(P);
     st_release_sys(&control_of(ctx.ws[threadIdx.x])->mega_flag[me][1], epoch);
   }
   int ok = 1;
-  if (threadIdx.x < P) ok = wait_flag_ge(&ctl->mega_flag[threadIdx.x][1], epoch, ctx, kOpMega, 1, threadIdx.x);
+  if (threadIdx.x < P && threadIdx.x != me) ok = wait_flag_ge(&ctl->mega_flag[threadIdx.x][1], epoch, ctx, kOpMega, 1, threadIdx.x);
   const int alive = __syncthreads_and(ok);
   mega_stamp(a.timer, kTimFinishSync);
   if (alive) {
