@@ -270,7 +270,7 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
 
   if (warp == 0) {
     // ============================================================ TMA producer
-    if (lane == 0) {
+    if (umma::elect_one()) {
       uint32_t it = 0;
       for (int tile = cta; tile < total_tiles && !*failed; tile += num_ctas) {
         const int mt = tile / n_tiles, nb = tile - mt * n_tiles;
@@ -295,7 +295,7 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
     }
   } else if (warp == 1) {
     // ============================================================ MMA issuer
-    if (lane == 0) {
+    if (umma::elect_one()) {
       const uint32_t idesc = instr_desc_bf16(kGmmBM, kGmmBN);
       uint32_t it = 0, local_tile = 0;
       for (int tile = cta; tile < total_tiles && !*failed; tile += num_ctas, ++local_tile) {
@@ -323,55 +323,66 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
     // ============================================================ epilogue (warps 2..9)
     const int quad = warp & 3;                       // TMEM lanes [32 * quad, 32 * quad + 32)
     const int part = (warp - 2) >> 2;                // which half of the tile's columns this warp handles
-    const int row_in_tile = quad * 32 + lane;
     constexpr int kCols = kGmmBN / 2;
     uint32_t local_tile = 0;
     for (int tile = cta; tile < total_tiles && !*failed; tile += num_ctas, ++local_tile) {
       const int mt = tile / n_tiles, nb = tile - mt * n_tiles;
       const int4 info = tile_info(mt);
-      // This warp drains its 32 lanes of both accumulators (rows m * 128 + quad * 32 + lane); each thread stores its
-      // row's columns straight from registers, 64 contiguous bytes per 32 columns, to this rank's output (a2av_gmm) or
-      // into the receive area of the rank the row came from (gmm_a2av).
+      // This warp drains its 32 lanes of an accumulator into registers as bf16, and hands tensor memory back before it stores
+      // the last half, so that the next tile's MMAs overlap the stores.  Stored straight from each thread's row, 64 bytes
+      // at a time, with the accumulators held until then: 5003 rows of 2048 x 7168, 16 experts 167 us instead of 151, 32768 rows of
+      // 7168 x 4096, 4 experts 1330 instead of 1291.  Eight lanes exchange their rows' 16-byte pieces first:
+      // together they cover one row's 128-byte segment of this rank's output (a2av_gmm) or of the receive area of the rank
+      // the row came from (gmm_a2av).
       if (!bounded_wait(&bars->acc_full, local_tile & 1u, failed)) break;
       umma::fence_after_sync();
-      for (int m = 0; m * kGmmBM < info.z; ++m) {
-        const int r = m * kGmmBM + row_in_tile;
+      const int halves = info.z > kGmmBM ? 2 : 1;
+      for (int m = 0; m < halves; ++m) {
+        const int r = m * kGmmBM + quad * 32 + lane;
+        const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + m * kGmmBN + part * kCols;
+        uint32_t held[2][32];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t v[32];
+          umma::tmem_ld32(taddr + i * 32, v);
+          umma::tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+            held[i >> 1][(i & 1) * 16 + j] = *reinterpret_cast<const uint32_t*>(&b);
+          }
+        }
+        if (m + 1 == halves) {
+          umma::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->acc_empty);
+        }
         uint8_t* dst_row = nullptr;
         if (r < info.z) {
           const int g = info.y + r;
           if (!kPush) {
-            dst_row = reinterpret_cast<uint8_t*>(a.out) + ((size_t)g * a.N + (size_t)nb * kGmmBN) * 2;
+            dst_row = reinterpret_cast<uint8_t*>(a.out) + ((size_t)g * a.N + (size_t)nb * kGmmBN + part * kCols) * 2;
           } else {
             int seg = info.x * P;
             while (seg + 1 < (info.x + 1) * P && sh.seg_dst[seg + 1] <= g) ++seg;
             const long long back = sh.seg_src[seg] + (g - sh.seg_dst[seg]);
-            dst_row = a.ctx.ws[seg - info.x * P] + a.data_off + ((size_t)back * a.N + (size_t)nb * kGmmBN) * 2;
+            dst_row = a.ctx.ws[seg - info.x * P] + a.data_off + ((size_t)back * a.N + (size_t)nb * kGmmBN + part * kCols) * 2;
           }
         }
-        const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + m * kGmmBN + part * kCols;
-        uint32_t v[32];
-        for (int c = 0; c < kCols; c += 32) {
-          umma::tmem_ld32(taddr + c, v);
-          umma::tmem_ld_wait();
-          const int col = nb * kGmmBN + part * kCols + c;
-          if (dst_row && col < a.N) {
-            uint4* dst = reinterpret_cast<uint4*>(dst_row + (size_t)(part * kCols + c) * 2);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint32_t w0[4];
+        for (int half = 0; half < 2; ++half) transpose_pieces(held[half], lane);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                __nv_bfloat162 b0 = __floats2bfloat162_rn(__uint_as_float(v[8 * i + 2 * j]), __uint_as_float(v[8 * i + 2 * j + 1]));
-                w0[j] = *reinterpret_cast<uint32_t*>(&b0);
-              }
-              dst[i] = make_uint4(w0[0], w0[1], w0[2], w0[3]);
-            }
+        for (int i = 0; i < 8; ++i) {
+          uint8_t* drow = reinterpret_cast<uint8_t*>(__shfl_sync(0xffffffffu, (unsigned long long)dst_row, (lane & 24) + i));
+          if (drow) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half)
+              if (nb * kGmmBN + part * kCols + half * 64 < a.N)       // N is a multiple of 64
+                *reinterpret_cast<uint4*>(drow + half * 128 + (lane & 7) * 16) =
+                    make_uint4(held[half][4 * i], held[half][4 * i + 1], held[half][4 * i + 2], held[half][4 * i + 3]);
           }
         }
       }
-      umma::fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->acc_empty);
     }
     if (kPush) __threadfence_system();   // rows pushed to peers are visible before this rank signals them
   }

@@ -84,6 +84,43 @@ def test_single_rank_grouped_gemm():
     _world(1, 4, 256, 256, 600)
 
 
+@pytest.mark.parametrize("counts, K, N", [
+    ([1], 64, 64), ([1, 383], 128, 192), ([256, 257, 0, 128, 511, 512, 513, 129], 320, 320), ([4097, 3], 576, 448),
+    ([700], 1024, 7168), ([0, 2000, 1, 130, 0, 260], 192, 7168)])
+def test_tile_edges_on_a_single_rank(counts, K, N):
+    """Edges of the 256-row tiles (one half, both, a row more), empty experts, column blocks past the last one, K loops shorter
+    and longer than the pipeline, fewer tiles than blocks and many more."""
+    from deepep_b200.ops import load_native
+
+    C, dev, E, rows = load_native(), torch.device("cuda"), len(counts), sum(counts)
+    gen = torch.Generator().manual_seed(rows + K)
+    x = torch.randn((rows, K), generator=gen).to(torch.bfloat16)
+    w = (torch.randn((E, K, N), generator=gen) / K ** 0.5).to(torch.bfloat16)
+    ref = torch.cat([a.float() @ b.float() for a, b in zip(x.split(counts), w)])
+    layout = C.make_mega_layout(1, 1, 128, 1, G.GmmEngine.region_bytes(C, rows, K, N))
+    session = C.Session(0, 1, layout.total, 20.0)
+    session.attach_peers([session.workspace])
+    try:
+        eng = G.GmmEngine([session], layout, dev, rows, K, N)
+        c = torch.tensor(counts, dtype=torch.int32, device=dev)
+        d_x, d_w = x.to(dev), w.to(dev)
+        for out_rows in (rows, rows + 3):
+            out = torch.full((out_rows, N), float("nan"), dtype=torch.bfloat16, device=dev)
+            gathered = torch.full((rows, K), float("nan"), dtype=torch.bfloat16, device=dev)
+            eng.a2av_gmm([d_x], [d_w], [c], [out], [gathered], num_experts=E)
+            back = torch.full((rows, N), float("nan"), dtype=torch.bfloat16, device=dev)
+            eng.gmm_a2av([d_x], [d_w], [c], [back], num_experts=E)
+            torch.cuda.synchronize()
+            eng.check()
+            assert torch.equal(gathered.cpu(), x)
+            # one rounding to bf16 (2^-9 of the value) behind fp32 sums of K products
+            assert torch.allclose(out[:rows].float().cpu(), ref, rtol=2.0 ** -8, atol=1e-4) and bool(out[rows:].isnan().all())
+            assert torch.equal(out[:rows], back)
+    finally:
+        torch.cuda.synchronize()
+        session.close()
+
+
 def test_two_ranks_odd_sizes():
     _world(2, 6, 192, 320, 500, seed=3, empty_expert=2)
 
