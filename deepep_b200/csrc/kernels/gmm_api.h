@@ -14,6 +14,7 @@ namespace dep {
 
 constexpr int kGmmBM = 128;   // rows per accumulator (TMEM lanes); a2av_gmm tiles hold two of them
 constexpr int kGmmBN = 256;   // output columns per tile
+constexpr int kGmmNarrowBN = 128;   // the same where tiles of 256 columns leave SMs without work
 constexpr int kGmmBK = 64;    // K elements per pipeline stage (one 128-byte swizzle row of bf16)
 constexpr int kGmmTableInts = 4 + kMaxExperts + 1;   // header (rows, -, -, -) + exclusive prefix of the per-expert row counts
 
@@ -57,6 +58,15 @@ struct GmmArgs {
 struct GmmParams { WsLayout lay; GmmArgs r[kMaxRanks]; };
 cudaError_t launch_a2av_gmm(const GmmParams& p, int nranks, int blocks, cudaStream_t stream);
 cudaError_t launch_gmm_a2av(const GmmParams& p, int nranks, int blocks, cudaStream_t stream);
+// Tiles of 128 columns where those of 256 would leave half of the blocks without one.  An SM fills its shared memory with about
+// 100 KB/us whatever its neighbours do, and a K step of a narrow tile is 48 KB instead of 64.  Narrow / wide, us: 300 rows of
+// 7168 x 4096 (one expert, 32 wide tiles) 57 / 81, 1500 rows of 2048 x 1024 over 8 experts (38) 28 / 38, 3000 rows of 2048 x 1024
+// over 8 experts (62) 30 / 38; beyond the line, 3000 rows of 2048 x 1024 over 16 experts (78) 46 / 42, 3000 rows of 2048 x 2048 over
+// 8 experts (124) 46 / 42.  The counts are on the device: an expert is taken to have a tile, and half a tile more than its rows fill.
+inline bool gmm_use_narrow_tiles(long long rows, long long experts, long long n, long long blocks) {
+  const long long filled = rows / kGmmBM + experts, least = 2 * (rows < experts ? rows : experts);     // twice the row tiles
+  return (filled > least ? filled : least) * ((n + kGmmBN - 1) / kGmmBN) <= blocks;
+}
 // Either op on one rank (world 1) whose x, output, gathered rows and weights do not overlap: p.r[0] with tmap_a over x.
 cudaError_t launch_gmm_local(const GmmParams& p, int blocks, cudaStream_t stream);
 

@@ -13,6 +13,7 @@
 // GEMM: 256 x 256 tiles, K in steps of 64, A K-major and B (weights [K, N], N contiguous) MN-major, both moved by
 // TMA with the 128-byte swizzle; per stage two groups of four tcgen05.mma kind::f16 (M = 128, N = 256, K = 16), one
 // group per 128-row half of the tile, each half with its own fp32 accumulator in tensor memory (2 x 256 columns).
+// One rank with few tiles works on tiles of 128 columns and four stages (`gmm_use_narrow_tiles`).
 // The two halves share every B stage: the kernel is bound by the rate at which one SM's shared memory is filled
 // from L2 (measured about 100 KB/us), and the shared B cuts the bytes per FLOP by a third against 128-row tiles.
 // Expert row blocks are not padded: a tile that reaches past its expert's rows computes rows that the epilogue drops.
@@ -36,17 +37,18 @@ constexpr int kGmmGemmThreads = 320;                     // TMA warp, MMA warp, 
 constexpr int kGmmPullWarps = 2;
 constexpr int kGmmTileA = kGmmBM * kGmmBK * 2;           // 16 KB
 constexpr int kGmmBoxB = 64 * kGmmBK * 2;                // 8 KB: 64 K-rows of 64 N-values
-constexpr int kGmmTileB = (kGmmBN / 64) * kGmmBoxB;      // 32 KB
 constexpr int kGmmPullChunk = 8;
 // Tiles are 256 rows x 256 columns: both 128-lane accumulators (all 512 tensor-memory columns) belong to one tile,
 // the two row halves share every B stage, and a stage moves 64 KB for twice the work (the kernel is bound by the
 // rate at which shared memory can be filled from L2, about 100 KB/us per SM, not by the tensor pipe).
 constexpr int kGmmHalves = 2, kGmmTileRows = kGmmHalves * kGmmBM;
-constexpr int kGmmStages = 3, kGmmStageBytes = kGmmHalves * kGmmTileA + kGmmTileB;
-constexpr size_t kGmmSmemBytes = 1024 + (size_t)kGmmStages * kGmmStageBytes + 256;
+constexpr int gmm_stage_bytes(int bn) { return kGmmHalves * kGmmTileA + bn / 64 * kGmmBoxB; }
+constexpr int gmm_stages(int bn) { return bn == kGmmBN ? 3 : 4; }      // the same 192 KB for tiles of 256 and of 128 columns
+constexpr size_t kGmmSmemBytes = 1024 + (size_t)gmm_stages(kGmmBN) * gmm_stage_bytes(kGmmBN) + 256;
+static_assert(gmm_stages(kGmmNarrowBN) * gmm_stage_bytes(kGmmNarrowBN) == gmm_stages(kGmmBN) * gmm_stage_bytes(kGmmBN), "one size of shared memory");
 
 struct GmmBarriers {
-  uint64_t full[kGmmStages], empty[kGmmStages], acc_full, acc_empty;
+  uint64_t full[4], empty[4], acc_full, acc_empty;
   uint32_t tmem_base;
   int failed;
 };
@@ -232,19 +234,21 @@ __device__ __forceinline__ void pull_phase(const GmmArgs& a, const GmmShared& sh
 // kPush = false: rows of the tile go to a.out on this rank.  kPush = true: each row goes to the rank it came from.
 // kLocal: the tiles come from the block's own layout instead of the list in memory.
 // A tile of at most 128 rows loads and multiplies its first half only (16 experts of 313 rows: 48 halves instead of 64).
-template <bool kPush, bool kLocal>
+// kBN: columns of a tile.
+template <bool kPush, bool kLocal, int kBN = kGmmBN>
 __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh, const int* a_ready, uint8_t* smem_raw,
                                           int cta, int num_ctas) {
+  constexpr int kStages = gmm_stages(kBN), kStageBytes = gmm_stage_bytes(kBN), kLoadB = kBN / 64 * kGmmBoxB;
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* tiles = smem_raw + (((raw + 1023u) & ~1023u) - raw);       // tiles need 1024-byte alignment
   constexpr int kOffB = kGmmHalves * kGmmTileA;               // B follows the A halves inside a stage
-  uint8_t* epi_smem = tiles + (size_t)kGmmStages * kGmmStageBytes;
+  uint8_t* epi_smem = tiles + (size_t)kStages * kStageBytes;
   GmmBarriers* bars = reinterpret_cast<GmmBarriers*>(epi_smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int P = a.ctx.world;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kGmmStages; ++s) { mbar_init(&bars->full[s], 1); mbar_init(&bars->empty[s], 1); }
+    for (int s = 0; s < kStages; ++s) { mbar_init(&bars->full[s], 1); mbar_init(&bars->empty[s], 1); }
     mbar_init(&bars->acc_full, 1);
     mbar_init(&bars->acc_empty, 8);
     bars->failed = 0;
@@ -261,7 +265,7 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
   umma::fence_after_sync();
   const uint32_t tmem = bars->tmem_base;
   volatile int* failed = &bars->failed;
-  const int n_tiles = (a.N + kGmmBN - 1) / kGmmBN, k_steps = a.K / kGmmBK;
+  const int n_tiles = (a.N + kBN - 1) / kBN, k_steps = a.K / kGmmBK;
   const int total_tiles = sh.num_tiles * n_tiles;
   auto tile_info = [&](int mt) {
     if constexpr (kLocal) return local_tile(sh, a.E, mt);
@@ -281,32 +285,32 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
           fence_proxy_async();            // rows written by this GPU's pull warps are about to be read by the copy engine
         }
         for (int ks = 0; ks < k_steps; ++ks, ++it) {
-          const int s = it % kGmmStages;
-          if (!bounded_wait(&bars->empty[s], ((it / kGmmStages) & 1u) ^ 1u, failed)) break;
-          uint8_t* dst = tiles + (size_t)s * kGmmStageBytes;
-          mbar_expect_tx(&bars->full[s], halves * kGmmTileA + kGmmTileB);
+          const int s = it % kStages;
+          if (!bounded_wait(&bars->empty[s], ((it / kStages) & 1u) ^ 1u, failed)) break;
+          uint8_t* dst = tiles + (size_t)s * kStageBytes;
+          mbar_expect_tx(&bars->full[s], halves * kGmmTileA + kLoadB);
           for (int m = 0; m < halves; ++m)        // rows past the end of the operand are filled with zeros
             umma::tma_load_2d(dst + m * kGmmTileA, &a.tmap_a, ks * kGmmBK, info.y + m * kGmmBM, &bars->full[s]);
 #pragma unroll
-          for (int j = 0; j < kGmmBN / 64; ++j)   // a box past the last column is filled with zeros
-            umma::tma_load_2d(dst + kOffB + j * kGmmBoxB, &a.tmap_b, nb * kGmmBN + j * 64, info.x * a.K + ks * kGmmBK, &bars->full[s]);
+          for (int j = 0; j < kBN / 64; ++j)   // a box past the last column is filled with zeros
+            umma::tma_load_2d(dst + kOffB + j * kGmmBoxB, &a.tmap_b, nb * kBN + j * 64, info.x * a.K + ks * kGmmBK, &bars->full[s]);
         }
       }
     }
   } else if (warp == 1) {
     // ============================================================ MMA issuer
     if (umma::elect_one()) {
-      const uint32_t idesc = instr_desc_bf16(kGmmBM, kGmmBN);
+      const uint32_t idesc = instr_desc_bf16(kGmmBM, kBN);
       uint32_t it = 0, local_tile = 0;
       for (int tile = cta; tile < total_tiles && !*failed; tile += num_ctas, ++local_tile) {
         const int halves = tile_info(tile / n_tiles).z > kGmmBM ? 2 : 1;
         if (!bounded_wait(&bars->acc_empty, (local_tile & 1u) ^ 1u, failed)) break;
         umma::fence_after_sync();
         for (int ks = 0; ks < k_steps; ++ks, ++it) {
-          const int s = it % kGmmStages;
-          if (!bounded_wait(&bars->full[s], (it / kGmmStages) & 1u, failed)) break;
+          const int s = it % kStages;
+          if (!bounded_wait(&bars->full[s], (it / kStages) & 1u, failed)) break;
           umma::fence_after_sync();
-          const uint32_t a_addr = smem_u32(tiles + (size_t)s * kGmmStageBytes);
+          const uint32_t a_addr = smem_u32(tiles + (size_t)s * kStageBytes);
           const uint64_t db = smem_desc_mn_sw128(a_addr + kOffB, kGmmBoxB);
           for (int m = 0; m < halves; ++m) {
             const uint64_t da = umma::smem_desc_sw128(a_addr + m * kGmmTileA);
@@ -323,7 +327,7 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
     // ============================================================ epilogue (warps 2..9)
     const int quad = warp & 3;                       // TMEM lanes [32 * quad, 32 * quad + 32)
     const int part = (warp - 2) >> 2;                // which half of the tile's columns this warp handles
-    constexpr int kCols = kGmmBN / 2;
+    constexpr int kCols = kBN / 2;
     uint32_t local_tile = 0;
     for (int tile = cta; tile < total_tiles && !*failed; tile += num_ctas, ++local_tile) {
       const int mt = tile / n_tiles, nb = tile - mt * n_tiles;
@@ -340,9 +344,9 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
       for (int m = 0; m < halves; ++m) {
         const int r = m * kGmmBM + quad * 32 + lane;
         const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + m * kGmmBN + part * kCols;
-        uint32_t held[2][32];
+        uint32_t held[kCols / 64][32];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < kCols / 32; ++i) {
           uint32_t v[32];
           umma::tmem_ld32(taddr + i * 32, v);
           umma::tmem_ld_wait();
@@ -361,23 +365,23 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
         if (r < info.z) {
           const int g = info.y + r;
           if (!kPush) {
-            dst_row = reinterpret_cast<uint8_t*>(a.out) + ((size_t)g * a.N + (size_t)nb * kGmmBN + part * kCols) * 2;
+            dst_row = reinterpret_cast<uint8_t*>(a.out) + ((size_t)g * a.N + (size_t)nb * kBN + part * kCols) * 2;
           } else {
             int seg = info.x * P;
             while (seg + 1 < (info.x + 1) * P && sh.seg_dst[seg + 1] <= g) ++seg;
             const long long back = sh.seg_src[seg] + (g - sh.seg_dst[seg]);
-            dst_row = a.ctx.ws[seg - info.x * P] + a.data_off + ((size_t)back * a.N + (size_t)nb * kGmmBN + part * kCols) * 2;
+            dst_row = a.ctx.ws[seg - info.x * P] + a.data_off + ((size_t)back * a.N + (size_t)nb * kBN + part * kCols) * 2;
           }
         }
 #pragma unroll
-        for (int half = 0; half < 2; ++half) transpose_pieces(held[half], lane);
+        for (int half = 0; half < kCols / 64; ++half) transpose_pieces(held[half], lane);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           uint8_t* drow = reinterpret_cast<uint8_t*>(__shfl_sync(0xffffffffu, (unsigned long long)dst_row, (lane & 24) + i));
           if (drow) {
 #pragma unroll
-            for (int half = 0; half < 2; ++half)
-              if (nb * kGmmBN + part * kCols + half * 64 < a.N)       // N is a multiple of 64
+            for (int half = 0; half < kCols / 64; ++half)
+              if (nb * kBN + part * kCols + half * 64 < a.N)       // N is a multiple of 64
                 *reinterpret_cast<uint4*>(drow + half * 128 + (lane & 7) * 16) =
                     make_uint4(held[half][4 * i], held[half][4 * i + 1], held[half][4 * i + 2], held[half][4 * i + 3]);
           }
@@ -500,13 +504,14 @@ __global__ void __launch_bounds__(kGmmGemmThreads, 1) gmm_a2av_kernel(const __gr
 // kernels copy x twice and pass four grid barriers (a2av_gmm), or write the output into the receive area and copy it from
 // there (gmm_a2av); here x is the A operand and the epilogue writes the output.  32768 rows of 7168 x 4096, 4 experts: 1811 -> 1551 us;
 // 5003 rows of 2048 x 7168, 16 experts: 257 -> 213 us (of which a part is the second halves of short tiles left out).
+template <int kBN>
 __global__ void __launch_bounds__(kGmmGemmThreads + kGmmPullWarps * 32, 1) gmm_local_kernel(const __grid_constant__ GmmParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ GmmShared sh;
   const GmmArgs& a = p.r[0];
   build_layout_local(a, sh, min(min(a.rows_in, a.out_rows_cap), a.gathered_cap));
   if (threadIdx.x < kGmmGemmThreads) {
-    gmm_phase<false, true>(a, sh, nullptr, smem_raw, blockIdx.x, gridDim.x);
+    gmm_phase<false, true, kBN>(a, sh, nullptr, smem_raw, blockIdx.x, gridDim.x);
   } else {
     __syncthreads();                               // pairs with the set-up barrier inside gmm_phase
     if (a.gathered) {                              // the caller wants the all-to-all-v result as well
@@ -539,10 +544,13 @@ cudaError_t launch_gmm_a2av(const GmmParams& p, int nranks, int blocks, cudaStre
 }
 
 cudaError_t launch_gmm_local(const GmmParams& p, int blocks, cudaStream_t stream) {
-  cudaError_t e = cudaFuncSetAttribute(gmm_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGmmSmemBytes);
+  const GmmArgs& a = p.r[0];
+  const void* fn = gmm_use_narrow_tiles(a.rows_in, a.E, a.N, blocks) ? (const void*)gmm_local_kernel<kGmmNarrowBN>
+                                                                     : (const void*)gmm_local_kernel<kGmmBN>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGmmSmemBytes);
   if (e != cudaSuccess) return e;
-  gmm_local_kernel<<<blocks, kGmmGemmThreads + kGmmPullWarps * 32, kGmmSmemBytes, stream>>>(p);
-  return cudaGetLastError();
+  void* args[] = {const_cast<GmmParams*>(&p)};
+  return cudaLaunchKernel(fn, dim3(blocks), dim3(kGmmGemmThreads + kGmmPullWarps * 32), args, kGmmSmemBytes, stream);
 }
 
 bool encode_bf16_map(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows, const char** error) {

@@ -86,10 +86,10 @@ def test_single_rank_grouped_gemm():
 
 @pytest.mark.parametrize("counts, K, N", [
     ([1], 64, 64), ([1, 383], 128, 192), ([256, 257, 0, 128, 511, 512, 513, 129], 320, 320), ([4097, 3], 576, 448),
-    ([700], 1024, 7168), ([0, 2000, 1, 130, 0, 260], 192, 7168)])
+    ([700], 1024, 7168), ([0, 2000, 1, 130, 0, 260], 192, 7168), ([256, 257, 0, 128, 511, 512, 513, 129], 320, 1984), ([300], 640, 1024)])
 def test_tile_edges_on_a_single_rank(counts, K, N):
     """Edges of the 256-row tiles (one half, both, a row more), empty experts, column blocks past the last one, K loops shorter
-    and longer than the pipeline, fewer tiles than blocks and many more."""
+    and longer than the pipeline, fewer tiles than blocks (narrow tiles) and many more."""
     from deepep_b200.ops import load_native
 
     C, dev, E, rows = load_native(), torch.device("cuda"), len(counts), sum(counts)
