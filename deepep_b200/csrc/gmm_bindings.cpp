@@ -65,9 +65,10 @@ bool fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session
   const void* a_base = gather && !local ? (const void*)a.gathered : (const void*)a.x;
   const long long a_rows = gather && !local ? (a.gathered ? a.gathered_cap : 0) : a.rows_in;
   // an empty operand still needs a valid map: point it at the weights
-  if (!encode_bf16_map(&a.tmap_a, a_rows > 0 ? a_base : (const void*)d["weight"].cast<uintptr_t>(), a_rows > 0 ? a_rows : 1, a.K, kGmmBM, &err))
+  if (!encode_bf16_map(&a.tmap_a, a_rows > 0 ? a_base : (const void*)d["weight"].cast<uintptr_t>(), a_rows > 0 ? a_rows : 1, a.K, kGmmBM,
+                       true, &err))
     throw std::runtime_error(err);
-  if (!encode_bf16_map(&a.tmap_b, weight, L * a.K, a.N, kGmmBK, &err)) throw std::runtime_error(err);
+  if (!encode_bf16_map(&a.tmap_b, weight, L * a.K, a.N, kGmmBK, false, &err)) throw std::runtime_error(err);
   return local;
 }
 
@@ -96,6 +97,7 @@ void bind_gmm(py::module_& m) {
     return std::vector<long long>{g.table_a, g.table_b, g.stage, g.recv, g.total};
   });
   m.def("gmm_region_bytes", [](long long max_rows, long long max_k, long long max_n) { return gmm_region(max_rows, max_k, max_n).total; });
+  m.def("gmm_narrow_tiles", &gmm_narrow_tiles, "whether one rank works on tiles of 128 columns");
   m.def("a2av_gmm", [](const WsLayout& lay, const std::vector<py::object>& sessions, const std::vector<py::dict>& args, int blocks,
                        uintptr_t stream) { return op(lay, sessions, args, blocks, stream, true); });
   m.def("gmm_a2av", [](const WsLayout& lay, const std::vector<py::object>& sessions, const std::vector<py::dict>& args, int blocks,

@@ -46,7 +46,7 @@ struct GmmArgs {
   __nv_bfloat16* out;              // a2av_gmm: [out_rows_cap, N] on the expert rank; gmm_a2av: [out_rows_cap, N] on the source rank
   __nv_bfloat16* gathered;         // a2av_gmm: [gathered_cap, K] the all-to-all-v result, A operand of the GEMM
                                    // (single-rank form: a copy for the caller, or null)
-  CUtensorMap tmap_a;              // A operand [rows, K] bf16: box 64 x 128, 128-byte swizzle
+  CUtensorMap tmap_a;              // A operand [rows, K] bf16, 3-D with z = 0: box 64 x 128, 128-byte swizzle
   CUtensorMap tmap_b;              // weights [L * K, N] bf16 (N contiguous): box 64 (N) x 64 (K), 128-byte swizzle
   int rows_in, E, K, N;
   int out_rows_cap, gathered_cap, max_tiles, pad;
@@ -58,19 +58,33 @@ struct GmmArgs {
 struct GmmParams { WsLayout lay; GmmArgs r[kMaxRanks]; };
 cudaError_t launch_a2av_gmm(const GmmParams& p, int nranks, int blocks, cudaStream_t stream);
 cudaError_t launch_gmm_a2av(const GmmParams& p, int nranks, int blocks, cudaStream_t stream);
-// Tiles of 128 columns where those of 256 would leave half of the blocks without one.  An SM fills its shared memory with about
-// 100 KB/us whatever its neighbours do, and a K step of a narrow tile is 48 KB instead of 64.  Narrow / wide, us: 300 rows of
-// 7168 x 4096 (one expert, 32 wide tiles) 57 / 81, 1500 rows of 2048 x 1024 over 8 experts (38) 28 / 38, 3000 rows of 2048 x 1024
-// over 8 experts (62) 30 / 38; beyond the line, 3000 rows of 2048 x 1024 over 16 experts (78) 46 / 42, 3000 rows of 2048 x 2048 over
-// 8 experts (124) 46 / 42.  The counts are on the device: an expert is taken to have a tile, and half a tile more than its rows fill.
-inline bool gmm_use_narrow_tiles(long long rows, long long experts, long long n, long long blocks) {
-  const long long filled = rows / kGmmBM + experts, least = 2 * (rows < experts ? rows : experts);     // twice the row tiles
-  return (filled > least ? filled : least) * ((n + kGmmBN - 1) / kGmmBN) <= blocks;
+// Whether one rank works on tiles of 128 columns instead of 256: `rows` in `row_tiles` tiles of up to 256 rows, the last of `last_rows`.
+// Every block decides this from the counts that it lays its tiles out from.  Both widths were timed for 7425 combinations of rows,
+// experts, k and n with the weights not in L2; us of a launch in a captured graph, narrow / wide:
+//  * Narrow tiles that all start at once (5512 points, 0.60 to 0.91 of the wide ones' time): an SM fills its shared memory with about
+//    100 KB/us whatever its neighbours do, and a K step of a narrow tile is 48 KB instead of 64.  8 experts of 256 rows, 2048 x 1536
+//    (96 narrow tiles) 20 / 28, 16 of 64 rows, 2048 x 1024 (128) 17 / 22, one of 300 rows, 7168 x 4096 (64) 46 / 71.
+//  * A second round of narrow tiles against one of wide tiles: 8 experts of 257 rows, 2048 x 1536 (192) 31 / 28, at k = 7168 88 / 75.
+//    Where it holds nothing but short tiles of the last row block, the narrow ones still gain with k up to 2048 (20 points, 0.78 to
+//    0.91): one expert of 1025 rows, 2048 x 4096 (160) 25 / 28, of 1100 rows at k = 7168 74 / 73.
+//  * More rounds: the wide ones.  They are the faster by more than 5 % at 1013 points behind this line, the narrow ones at 357, most of
+//    these three narrow rounds for two wide ones (4 experts of 1100 rows, 2048 x 2048, 39 / 49).
+__host__ __device__ inline bool gmm_narrow_tiles(long long row_tiles, long long last_rows, long long rows, long long k, long long n,
+                                                 long long blocks) {
+  const long long cols = (n + kGmmNarrowBN - 1) / kGmmNarrowBN, tiles = row_tiles * cols;
+  const bool short_end = tiles <= blocks + cols && last_rows <= kGmmBM && rows > kGmmBM * row_tiles && k <= 2048;   // some tile is full
+  return tiles <= blocks || short_end;
 }
 // Either op on one rank (world 1) whose x, output, gathered rows and weights do not overlap: p.r[0] with tmap_a over x.
 cudaError_t launch_gmm_local(const GmmParams& p, int blocks, cudaStream_t stream);
 
-// 2-D bf16 tensor map, `cols` contiguous, 128-byte swizzle, box {64 columns, box_rows}.
-bool encode_bf16_map(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows, const char** error);
+// Tensor map of bf16 [rows, cols], `cols` contiguous, 128-byte swizzle, box {64 columns, box_rows}.  `shared_rows`: the operand whose
+// boxes many blocks load at once, as a 3-D map with a second plane behind the first; boxes are taken at z = 0 alone, nothing of the
+// second plane is read.  It is there for the extent that the map states: boxes of a map over less than 128 KB came slowly when 60 blocks
+// or more loaded them at once.  8 experts of 1 row, 7168 x 1536, 112 KB of x, by the tensor's address and by the GPU: tiles of
+// 128 columns 70 to 81 us, of 256 columns 57 to 86; as planes 41 and 57, like 16 rows (229 KB) either way.
+constexpr unsigned long long kGmmMapBytes = 128 * 1024;
+bool encode_bf16_map(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows, bool shared_rows,
+                     const char** error);
 
 }  // namespace dep

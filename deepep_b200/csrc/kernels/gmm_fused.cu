@@ -13,7 +13,7 @@
 // GEMM: 256 x 256 tiles, K in steps of 64, A K-major and B (weights [K, N], N contiguous) MN-major, both moved by
 // TMA with the 128-byte swizzle; per stage two groups of four tcgen05.mma kind::f16 (M = 128, N = 256, K = 16), one
 // group per 128-row half of the tile, each half with its own fp32 accumulator in tensor memory (2 x 256 columns).
-// One rank with few tiles works on tiles of 128 columns and four stages (`gmm_use_narrow_tiles`).
+// One rank with few tiles works on tiles of 128 columns and four stages (`gmm_narrow_tiles`).
 // The two halves share every B stage: the kernel is bound by the rate at which one SM's shared memory is filled
 // from L2 (measured about 100 KB/us), and the shared B cuts the bytes per FLOP by a third against 128-row tiles.
 // Expert row blocks are not padded: a tile that reaches past its expert's rows computes rows that the epilogue drops.
@@ -57,7 +57,7 @@ struct GmmShared {
   int seg_src[kMaxExperts];        // [l * P + s] first row of the segment on its owner (staged x / returned output)
   int seg_dst[kMaxExperts + 1];    // [l * P + s] first row of the segment on this rank (exclusive prefix)
   int tile0[kMaxExperts + 1];      // [l] first tile of local expert l ([L]: number of tiles)
-  int alive, total_rows, num_tiles;
+  int alive, total_rows, num_tiles, last_rows;   // last_rows: rows of the last tile (single rank)
 };
 
 // Shared-memory descriptor of an MN-major operand: 64-value (128-byte) rows along N, 8 K-rows per 1024-byte swizzle
@@ -157,6 +157,7 @@ __device__ __forceinline__ void build_layout_local(const GmmArgs& a, GmmShared& 
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < 32) {
     long long rows = 0, tiles = 0;
+    int last = 0;
     for (int e0 = 0; e0 < a.E; e0 += 32) {
       const int e = e0 + lane, c = e < a.E ? max(a.counts[e], 0) : 0, t = c / kGmmTileRows + (c % kGmmTileRows != 0);
       long long row_sum = c, tile_sum = t;
@@ -165,6 +166,8 @@ __device__ __forceinline__ void build_layout_local(const GmmArgs& a, GmmShared& 
         if (lane >= d) { row_sum += r; tile_sum += q; }
       }
       if (e < a.E) { sh.seg_dst[e] = (int)(rows + row_sum - c); sh.tile0[e] = (int)(tiles + tile_sum - t); }
+      const unsigned filled = __ballot_sync(0xffffffffu, c > 0);
+      if (filled) last = __shfl_sync(0xffffffffu, c, 31 - __clz(filled));
       rows += __shfl_sync(0xffffffffu, row_sum, 31);
       tiles += __shfl_sync(0xffffffffu, tile_sum, 31);
     }
@@ -175,6 +178,7 @@ __device__ __forceinline__ void build_layout_local(const GmmArgs& a, GmmShared& 
       sh.tile0[a.E] = (int)tiles;
       sh.total_rows = sh.alive ? (int)rows : 0;
       sh.num_tiles = sh.alive ? (int)tiles : 0;
+      sh.last_rows = last > 0 ? (last - 1) % kGmmTileRows + 1 : 0;
     }
   }
   __syncthreads();
@@ -290,7 +294,7 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
           uint8_t* dst = tiles + (size_t)s * kStageBytes;
           mbar_expect_tx(&bars->full[s], halves * kGmmTileA + kLoadB);
           for (int m = 0; m < halves; ++m)        // rows past the end of the operand are filled with zeros
-            umma::tma_load_2d(dst + m * kGmmTileA, &a.tmap_a, ks * kGmmBK, info.y + m * kGmmBM, &bars->full[s]);
+            umma::tma_load_3d(dst + m * kGmmTileA, &a.tmap_a, ks * kGmmBK, info.y + m * kGmmBM, 0, &bars->full[s]);
 #pragma unroll
           for (int j = 0; j < kBN / 64; ++j)   // a box past the last column is filled with zeros
             umma::tma_load_2d(dst + kOffB + j * kGmmBoxB, &a.tmap_b, nb * kBN + j * 64, info.x * a.K + ks * kGmmBK, &bars->full[s]);
@@ -504,14 +508,16 @@ __global__ void __launch_bounds__(kGmmGemmThreads, 1) gmm_a2av_kernel(const __gr
 // kernels copy x twice and pass four grid barriers (a2av_gmm), or write the output into the receive area and copy it from
 // there (gmm_a2av); here x is the A operand and the epilogue writes the output.  32768 rows of 7168 x 4096, 4 experts: 1811 -> 1551 us;
 // 5003 rows of 2048 x 7168, 16 experts: 257 -> 213 us (of which a part is the second halves of short tiles left out).
-template <int kBN>
 __global__ void __launch_bounds__(kGmmGemmThreads + kGmmPullWarps * 32, 1) gmm_local_kernel(const __grid_constant__ GmmParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ GmmShared sh;
   const GmmArgs& a = p.r[0];
   build_layout_local(a, sh, min(min(a.rows_in, a.out_rows_cap), a.gathered_cap));
   if (threadIdx.x < kGmmGemmThreads) {
-    gmm_phase<false, true, kBN>(a, sh, nullptr, smem_raw, blockIdx.x, gridDim.x);
+    if (gmm_narrow_tiles(sh.num_tiles, sh.last_rows, sh.total_rows, a.K, a.N, gridDim.x))
+      gmm_phase<false, true, kGmmNarrowBN>(a, sh, nullptr, smem_raw, blockIdx.x, gridDim.x);
+    else
+      gmm_phase<false, true>(a, sh, nullptr, smem_raw, blockIdx.x, gridDim.x);
   } else {
     __syncthreads();                               // pairs with the set-up barrier inside gmm_phase
     if (a.gathered) {                              // the caller wants the all-to-all-v result as well
@@ -544,16 +550,13 @@ cudaError_t launch_gmm_a2av(const GmmParams& p, int nranks, int blocks, cudaStre
 }
 
 cudaError_t launch_gmm_local(const GmmParams& p, int blocks, cudaStream_t stream) {
-  const GmmArgs& a = p.r[0];
-  const void* fn = gmm_use_narrow_tiles(a.rows_in, a.E, a.N, blocks) ? (const void*)gmm_local_kernel<kGmmNarrowBN>
-                                                                     : (const void*)gmm_local_kernel<kGmmBN>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGmmSmemBytes);
+  cudaError_t e = cudaFuncSetAttribute(gmm_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGmmSmemBytes);
   if (e != cudaSuccess) return e;
-  void* args[] = {const_cast<GmmParams*>(&p)};
-  return cudaLaunchKernel(fn, dim3(blocks), dim3(kGmmGemmThreads + kGmmPullWarps * 32), args, kGmmSmemBytes, stream);
+  gmm_local_kernel<<<blocks, kGmmGemmThreads + kGmmPullWarps * 32, kGmmSmemBytes, stream>>>(p);
+  return cudaGetLastError();
 }
 
-bool encode_bf16_map(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows, const char** error) {
+bool encode_bf16_map(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows, bool shared_rows, const char** error) {
   typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -567,11 +570,12 @@ bool encode_bf16_map(CUtensorMap* map, const void* base, long long rows, long lo
     }
     encode = reinterpret_cast<EncodeFn>(fn);
   }
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-  cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
-  cuuint32_t elem[2] = {1, 1};
-  CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+  const cuuint64_t pitch = (cuuint64_t)cols * 2, bytes = pitch * rows;     // a plane; its pitch is a multiple of 16 as the rows' is
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 2};
+  cuuint64_t strides[2] = {pitch, bytes > kGmmMapBytes ? bytes : kGmmMapBytes};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+  cuuint32_t elem[3] = {1, 1, 1};
+  CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, shared_rows ? 3 : 2, const_cast<void*>(base), dims, strides, box, elem,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {

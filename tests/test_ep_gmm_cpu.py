@@ -220,3 +220,21 @@ def test_group_given_in_bytes_and_the_context_manager():
         G.init_group(None, max_rows=8)
     with pytest.raises(ValueError, match="1 MiB"):
         G.init_udma_group(heap_size=1000)
+
+
+@pytest.mark.parametrize("counts, k, n, narrow", [
+    ([256] * 8, 2048, 1536, True),       # 96 narrow tiles, all at once
+    ([257] * 8, 2048, 1536, False),      # 192, a second round, for 96 wide ones
+    ([1100], 7168, 4096, False),         # 160 for 80
+    ([1024], 7168, 4096, True),          # 128
+    ([148 * 256], 64, 128, True), ([148 * 256 + 129], 64, 128, False),
+    ([1025], 2048, 4096, True), ([1152], 2048, 4096, True), ([1153], 2048, 4096, False),     # 12 of 160 in a second round, 1 to 129 rows high
+    ([1025], 2112, 4096, False), ([1281], 2048, 4096, False), ([100] * 38, 2048, 512, False),
+    ([1] * 8, 7168, 1536, True), ([1] * 49, 2048, 384, True), ([1] * 50, 2048, 384, False), ([], 64, 64, True)])
+def test_width_of_a_single_ranks_tiles(counts, k, n, narrow):
+    """Tiles of 128 columns only where they all start at once on 148 blocks, but for short ones at the end."""
+    from deepep_b200.ops import load_native
+
+    row_tiles = sum(-(-c // 256) for c in counts)
+    last_rows = next(((c - 1) % 256 + 1 for c in reversed(counts) if c), 0)
+    assert load_native().gmm_narrow_tiles(row_tiles, last_rows, sum(counts), k, n, 148) is narrow

@@ -121,6 +121,37 @@ def test_tile_edges_on_a_single_rank(counts, K, N):
         session.close()
 
 
+def test_both_tile_widths_give_the_same_rows():
+    """Nine narrow tiles (one and two halves high): on nine blocks all at once, on eight and six the short ones of the last row block
+    are second tiles, behind 13 K steps in a pipeline of four; on five and two blocks the wide ones take their place."""
+    from deepep_b200.ops import load_native
+
+    C, dev, counts, K, N = load_native(), torch.device("cuda"), [200, 0, 256, 100], 832, 384
+    rows, gen = sum(counts), torch.Generator().manual_seed(4)
+    x = torch.randn((rows, K), generator=gen).to(torch.bfloat16)
+    w = (torch.randn((4, K, N), generator=gen) / K ** 0.5).to(torch.bfloat16)
+    ref = torch.cat([a.float() @ b.float() for a, b in zip(x.split(counts), w)])
+    layout = C.make_mega_layout(1, 1, 128, 1, G.GmmEngine.region_bytes(C, rows, K, N))
+    session = C.Session(0, 1, layout.total, 20.0)
+    session.attach_peers([session.workspace])
+    try:
+        d_x, d_w, d_c = x.to(dev), w.to(dev), torch.tensor(counts, dtype=torch.int32, device=dev)
+        outs = []
+        for blocks in (9, 8, 6, 5, 2):
+            assert C.gmm_narrow_tiles(3, counts[-1], rows, K, N, blocks) is (blocks >= 6)
+            eng = G.GmmEngine([session], layout, dev, rows, K, N, num_sms=blocks)
+            outs.append(torch.full((rows, N), float("nan"), dtype=torch.bfloat16, device=dev))
+            eng.a2av_gmm([d_x], [d_w], [d_c], [outs[-1]], num_experts=4)
+            torch.cuda.synchronize()
+            eng.check()
+        # one rounding to bf16 (2^-9 of the value) behind fp32 sums of K products
+        assert torch.allclose(outs[0].float().cpu(), ref, rtol=2.0 ** -8, atol=1e-4)
+        assert all(torch.equal(outs[0], o) for o in outs[1:])
+    finally:
+        torch.cuda.synchronize()
+        session.close()
+
+
 def test_two_ranks_odd_sizes():
     _world(2, 6, 192, 320, 500, seed=3, empty_expert=2)
 
