@@ -36,6 +36,7 @@ struct MegaGemmParams {
   CUtensorMap tmap_b;        // weights, tiled as [rows / 128][(K / 128) * 128][128 values]: e2m1 pairs that the copy engine widens
                              // to one byte per value, or e4m3 bytes (b_fp8); a box holds the 128 rows of a CTA of a pair, or 256
   CUtensorMap tmap_sfa, tmap_sfb;   // the chunked scales as [chunks][512 B], kSfGroup chunks a box
+  CUtensorMap tmap_b2, tmap_sfb2;   // weights and scales from row b_rows on (the shared experts), if any
   const int* mtile_expert;   // [max_mtiles] local expert of each 128-row tile
   const int* a_ready;        // optional: rows of each tile of A in place so far; a tile's loads start at 128
   const int* num_mtiles;     // device scalar: tiles in use
@@ -43,7 +44,7 @@ struct MegaGemmParams {
   int epi, b_tx_bytes;
   int pair, stages;          // stand-alone launch only: run as CTA pairs (the tile list must pair row blocks 2j, 2j + 1 of one expert);
                              // pipeline stages (0 = default)
-  int commit_every, pad3;    // stand-alone launch only: stages released per tcgen05.commit (0 = 1)
+  int commit_every, b_rows;  // stand-alone launch only: stages released per tcgen05.commit (0 = 1); first row of tmap_b2
   // kEpiStoreF32
   float* c;
   int ldc, b_fp8;            // b_fp8: the weights are e4m3 (A8W8) instead of e2m1 (A8W4)

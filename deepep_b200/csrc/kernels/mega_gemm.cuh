@@ -272,7 +272,11 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
         const MegaGemmParams& p = second ? *g2 : g1;
         const int local = second ? tile - tiles1 : tile;
         const int mt = kPair ? 2 * (local / p.n_tiles) + (int)crank : local / p.n_tiles, nb = local % p.n_tiles;
-        const int brow = p.mtile_expert[mt] * p.n_total + nb * kGemmBN;        // first of the tile's 256 weight rows
+        int brow = p.mtile_expert[mt] * p.n_total + nb * kGemmBN;        // first of the tile's 256 weight rows
+        const bool shared = brow >= p.b_rows;
+        if (shared) brow -= p.b_rows;
+        const CUtensorMap* tmap_b = shared ? &p.tmap_b2 : &p.tmap_b;
+        const CUtensorMap* tmap_sfb = shared ? &p.tmap_sfb2 : &p.tmap_sfb;
         if (second && ready) {
           if (!wait_rows_ready(ready + mt, g1.n_tiles, failed, kWaitRowBlockDone)) break;
           fence_proxy_async();          // rows written by other SMs' stores are about to be read by the copy engine
@@ -304,23 +308,23 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
             if (crank == 0) mbar_expect_tx(&bars->full[s], 2 * (kTileABytes + p.b_tx_bytes + sf_bytes));
             umma::tma_load_2d_pair(a_dst, &p.tmap_a, ks * kGemmBK, mt * kGemmBM, bar);
             // this CTA's half of the 256 weight rows, and the scales of all of them (each CTA of a pair needs them all)
-            umma::tma_load_3d_pair(a_dst + kTileABytes, &p.tmap_b, 0, ks * 128, brow / 128 + (int)crank, bar);
+            umma::tma_load_3d_pair(a_dst + kTileABytes, tmap_b, 0, ks * 128, brow / 128 + (int)crank, bar);
             if (group_start) {
               umma::tma_load_2d_pair(sf_dst, &p.tmap_sfa, 0, mt * p.k_steps + ks, bar);
 #pragma unroll
               for (int h = 0; h < kGemmBN / 128; ++h)
-                umma::tma_load_2d_pair(sf_dst + (1 + h) * kSfPart, &p.tmap_sfb, 0, (brow / 128 + h) * p.k_steps + ks, bar);
+                umma::tma_load_2d_pair(sf_dst + (1 + h) * kSfPart, tmap_sfb, 0, (brow / 128 + h) * p.k_steps + ks, bar);
             }
           } else {
             mbar_expect_tx(&bars->full[s], kTileABytes + kBBoxes * p.b_tx_bytes + sf_bytes);
             umma::tma_load_2d(a_dst, &p.tmap_a, ks * kGemmBK, mt * kGemmBM, &bars->full[s]);
             // both 128-row blocks of weights in one box; the second continues the swizzled tile of the first
-            umma::tma_load_3d(a_dst + kTileABytes, &p.tmap_b, 0, ks * 128, brow / 128, &bars->full[s]);
+            umma::tma_load_3d(a_dst + kTileABytes, tmap_b, 0, ks * 128, brow / 128, &bars->full[s]);
             if (group_start) {
               umma::tma_load_2d(sf_dst, &p.tmap_sfa, 0, mt * p.k_steps + ks, &bars->full[s]);
 #pragma unroll
               for (int h = 0; h < kGemmBN / 128; ++h)
-                umma::tma_load_2d(sf_dst + (1 + h) * kSfPart, &p.tmap_sfb, 0, (brow / 128 + h) * p.k_steps + ks, &bars->full[s]);
+                umma::tma_load_2d(sf_dst + (1 + h) * kSfPart, tmap_sfb, 0, (brow / 128 + h) * p.k_steps + ks, &bars->full[s]);
             }
           }
         }

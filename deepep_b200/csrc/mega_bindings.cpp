@@ -3,6 +3,7 @@
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
+#include <limits>
 #include <stdexcept>
 #include <string>
 
@@ -29,17 +30,21 @@ long long getl(const py::dict& d, const char* key, long long dflt = 0) { return 
 // One grouped GEMM launch.  `d` carries operand pointers and shapes; `session` is needed only by the
 // combine epilogue (peer workspaces).
 void fill_gemm(MegaGemmParams& p, const py::dict& d, py::object session) {
-  const long long rows_pad = getl(d, "rows_pad"), k = getl(d, "k"), b_rows = getl(d, "b_rows");
-  if (rows_pad % kGemmBM || k % kGemmBK || b_rows % kGemmBN) throw std::invalid_argument("rows and K must be multiples of 128, weight rows of 256");
+  const long long rows_pad = getl(d, "rows_pad"), k = getl(d, "k"), b_rows = getl(d, "b_rows"), b2_rows = getl(d, "b2_rows");
+  if (rows_pad % kGemmBM || k % kGemmBK || b_rows % kGemmBN || b2_rows % kGemmBN) throw std::invalid_argument("rows and K must be multiples of 128, weight rows of 256");
   const char* err = nullptr;
   if (!encode_operand_map(&p.tmap_a, ptr<const void>(d, "a"), rows_pad, k, &err)) throw std::runtime_error(err);
   // weights are stored tiled: every (128-row, 128-K) block is one contiguous run of 128 rows x 64 (e2m1) or 128 (e4m3) bytes
   p.b_fp8 = geti(d, "b_fp8", 0) ? 1 : 0;
   p.pair = geti(d, "pair", 0) ? 1 : 0;
-  if (!encode_weights_map(&p.tmap_b, ptr<const void>(d, "b"), b_rows / 128, k / kGemmBK, p.pair ? 1 : kGemmBN / 128, !p.b_fp8, &err))
-    throw std::runtime_error(err);
+  auto weights = [&](CUtensorMap* values, CUtensorMap* scales, const char* b, const char* sfb, long long rows) {
+    return encode_weights_map(values, ptr<const void>(d, b), rows / 128, k / kGemmBK, p.pair ? 1 : kGemmBN / 128, !p.b_fp8, &err) &&
+           encode_sf_map(scales, ptr<const void>(d, sfb), (rows / 128) * (k / kGemmBK), &err);
+  };
+  if (!weights(&p.tmap_b, &p.tmap_sfb, "b", "sfb", b_rows)) throw std::runtime_error(err);
+  if (b2_rows > 0 && !weights(&p.tmap_b2, &p.tmap_sfb2, "b2", "sfb2", b2_rows)) throw std::runtime_error(err);
+  p.b_rows = b2_rows > 0 ? (int)b_rows : std::numeric_limits<int>::max();     // without a second set every row is behind tmap_b
   if (!encode_sf_map(&p.tmap_sfa, ptr<const void>(d, "sfa"), (rows_pad / kGemmBM) * (k / kGemmBK), &err)) throw std::runtime_error(err);
-  if (!encode_sf_map(&p.tmap_sfb, ptr<const void>(d, "sfb"), (b_rows / 128) * (k / kGemmBK), &err)) throw std::runtime_error(err);
   p.mtile_expert = ptr<const int>(d, "mtile_expert"); p.num_mtiles = ptr<const int>(d, "num_mtiles");
   p.a_ready = ptr<const int>(d, "a_ready");
   p.max_mtiles = (int)(rows_pad / kGemmBM);

@@ -19,6 +19,7 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 import os
+import weakref
 from typing import Optional, Sequence, Tuple
 
 import torch
@@ -47,6 +48,38 @@ class MegaWeights:
     k: int
     fp8: bool = False           # e4m3 weights (mma_type "fp8xfp8") instead of e2m1 ("fp8xfp4")
     source: Optional[Tuple[torch.Tensor, torch.Tensor]] = None   # (weights, scales) as given; kept for CPU targets only
+
+
+class JoinedWeights:
+    """Routed experts followed by the shared ones, as the kernel numbers them.  Holds the two sets and no copy of them: the kernel
+    reads each from its own tensors, so weights that are changed in place or replaced are never stale."""
+
+    def __init__(self, routed: MegaWeights, shared: MegaWeights):
+        self.routed, self.shared = routed, shared
+        self.experts, self.n, self.k, self.fp8 = routed.experts + shared.experts, routed.n, routed.k, routed.fp8
+
+    def parts(self) -> Tuple[torch.Tensor, ...]:
+        return self.routed.packed, self.routed.sf_chunks, self.shared.packed, self.shared.sf_chunks
+
+    @property
+    def packed(self) -> torch.Tensor:
+        return torch.cat([self.routed.packed, self.shared.packed])
+
+    @property
+    def sf_chunks(self) -> torch.Tensor:
+        return torch.cat([self.routed.sf_chunks, self.shared.sf_chunks])
+
+
+def _weight_args(w, hold: list) -> dict:
+    """One projection's weights (``MegaWeights`` or ``JoinedWeights``) for the native launch; ``hold`` gets what has to outlive it."""
+    if isinstance(w, JoinedWeights) and all(t.is_contiguous() and t.data_ptr() % 32 == 0 for t in w.parts()):
+        b, sfb, b2, sfb2 = w.parts()
+        more = dict(b2=b2.data_ptr(), sfb2=sfb2.data_ptr(), b2_rows=w.shared.experts * w.n)
+    else:                       # one set, or two of which one lies where the copy engine cannot read it: copied into one
+        b, sfb, more = w.packed, w.sf_chunks, {}
+    hold += [b, sfb]
+    return dict(b=b.data_ptr(), sfb=sfb.data_ptr(), b_rows=(w.routed.experts if more else w.experts) * w.n, n_total=w.n,
+                b_fp8=int(w.fp8), **more)
 
 
 def _sf_chunks(sf: torch.Tensor) -> torch.Tensor:
@@ -157,12 +190,13 @@ class MegaEngine:
                 timer: Optional[torch.Tensor] = None) -> None:
         """Run the layer.  ``fused``: one persistent cooperative kernel (route -> GEMM1 -> GEMM2 -> finish); otherwise
         the same phases as four launches (kept for debugging and for comparing the two schedules).
-        ``l1`` / ``l2`` hold the routed experts followed by the shared ones when the engine has shared experts.
+        ``l1`` / ``l2`` hold the routed experts followed by the shared ones (in one set of tensors, or joined from two) when the
+        engine has shared experts.
         ``x_bf16[i]``: bf16 activations quantised to MXFP8 inside the kernel instead of pre-quantised inputs.
         ``timer``: int64 ``[SMs, mega_timer_words]`` that receives one record of phase stamps per CTA (fused, one rank)."""
         C, lay = self.C, self.layout
         s = (stream if stream is not None else torch.cuda.current_stream(self.device)).cuda_stream
-        route_args, finish_args, gemm1_args, gemm2_args = [], [], [], []
+        route_args, finish_args, gemm1_args, gemm2_args, hold = [], [], [], [], []
         for i in range(self.n):
             sc, w1, w2 = self.scratch[i], l1[i], l2[i]
             route_args.append(dict(in_off=self.in_off, T=tokens[i], E=self.E, K=self.K, H=self.H, max_tokens=self.M,
@@ -177,13 +211,9 @@ class MegaEngine:
                                     timer=None if timer is None else timer.data_ptr()))
             common = dict(mtile_expert=sc["mtile_expert"].data_ptr(), num_mtiles=sc["num_mtiles"].data_ptr(), rows_pad=self.rows_cap,
                           error_flag=sc["err"].data_ptr())
-            gemm1_args.append(dict(common, a=sc["a1"].data_ptr(), sfa=sc["a1_sf"].data_ptr(), b=w1.packed.data_ptr(),
-                                   sfb=w1.sf_chunks.data_ptr(), k=self.H, b_rows=w1.experts * w1.n, n_total=w1.n, epi=1,
-                                   b_fp8=int(w1.fp8),
+            gemm1_args.append(dict(common, **_weight_args(w1, hold), a=sc["a1"].data_ptr(), sfa=sc["a1_sf"].data_ptr(), k=self.H, epi=1,
                                    a2=sc["a2"].data_ptr(), a2_sf=sc["a2_sf"].data_ptr(), inter=self.I))
-            gemm2_args.append(dict(common, a=sc["a2"].data_ptr(), sfa=sc["a2_sf"].data_ptr(), b=w2.packed.data_ptr(),
-                                   sfb=w2.sf_chunks.data_ptr(), k=self.I, b_rows=w2.experts * w2.n, n_total=w2.n, epi=2,
-                                   b_fp8=int(w2.fp8),
+            gemm2_args.append(dict(common, **_weight_args(w2, hold), a=sc["a2"].data_ptr(), sfa=sc["a2_sf"].data_ptr(), k=self.I, epi=2,
                                    row_src=sc["row_src"].data_ptr(), comb_off=self.comb_off, max_tokens=self.M,
                                    topk=self.K + self.S, hidden=self.H))
         if fused:
@@ -301,7 +331,7 @@ class SymmBuffer:
         self.num_experts, self.num_topk, self.hidden, self.intermediate_hidden = num_experts, num_topk, hidden, intermediate_hidden
         self.num_max_tokens_per_rank = num_max_tokens_per_rank
         self.num_shared_experts, self.mma_type = int(num_shared_experts), mma_type
-        self._joined: dict = {}
+        self._joined = weakref.WeakValueDictionary()       # pairs of routed and shared weights that are in use
         self.batch_size = 0
         self._destroyed = False
         if not torch.cuda.is_available() or (device is not None and torch.device(device).type == "cpu"):
@@ -326,7 +356,6 @@ class SymmBuffer:
         self.runtime = Runtime(self.control, self.layout, float(num_gpu_timeout_secs), self.device)
         self.engine = MegaEngine([self.runtime.native], self.layout, self.device, num_experts, intermediate_hidden, num_sms,
                                  self.num_shared_experts)
-        # self._joined: routed + shared weights joined once per weight set
         self.x, self.x_sf, self.topk_idx, self.topk_weights = self.engine.input_views(0)
 
     def prepare(self, batch_size: int) -> "SymmBuffer":
@@ -371,17 +400,19 @@ class SymmBuffer:
         C = require_native("MegaMoE timer")
         return torch.zeros((self.engine.sm_count, C.mega_timer_words), dtype=torch.int64, device=self.device)
 
-    def joined_weights(self, routed: MegaWeights, shared: Optional[MegaWeights]) -> MegaWeights:
-        """Routed experts followed by the shared ones in one operand (the kernel sees them as extra local experts)."""
+    def joined_weights(self, routed: MegaWeights, shared: Optional[MegaWeights]):
+        """Routed experts followed by the shared ones as one operand (the kernel sees them as extra local experts)."""
         if shared is None:
             return routed
-        key = (routed.packed.data_ptr(), shared.packed.data_ptr())
-        if key not in self._joined:
-            if (shared.n, shared.k, shared.fp8) != (routed.n, routed.k, routed.fp8):
-                raise ValueError("shared experts must have the shapes and the weight type of the routed experts")
-            self._joined[key] = MegaWeights(torch.cat([routed.packed, shared.packed]), torch.cat([routed.sf_chunks, shared.sf_chunks]),
-                                            routed.experts + shared.experts, routed.n, routed.k, routed.fp8)
-        return self._joined[key]
+        if (shared.n, shared.k, shared.fp8) != (routed.n, routed.k, routed.fp8):
+            raise ValueError("shared experts must have the shapes and the weight type of the routed experts")
+        if len({t.device for t in (routed.packed, routed.sf_chunks, shared.packed, shared.sf_chunks)}) > 1:
+            raise RuntimeError("routed and shared weights must be on the same device")
+        key = (id(routed), id(shared))           # a live entry holds both objects, so their ids belong to them
+        joined = self._joined.get(key)
+        if joined is None:
+            self._joined[key] = joined = JoinedWeights(routed, shared)
+        return joined
 
     def validate_inputs(self, batch_size: int, *, x: Optional[torch.Tensor] = None) -> None:
         """Scan the inputs of the next call (synchronises; keep it outside timed regions).  ``x``: the bf16 override that

@@ -143,6 +143,34 @@ def test_shared_experts_are_joined_once_per_weight_set():
         MM.fp8_fp4_mega_moe(y, l1, l2, sym)
 
 
+def test_joined_weights_are_never_stale():
+    """The kernel gets the addresses of the tensors that hold the weights now: after a change in place (through ``.data`` too), after
+    a field was given another tensor, and for another set of weights."""
+    sym, (l1, _), (s1, _) = make_buffer(shared=1), weights(), weights(experts=1, seed=9)
+    first = sym.joined_weights(l1, s1)
+    l1.packed.add_(1)
+    s1.sf_chunks.data.add_(1)
+    j = sym.joined_weights(l1, s1)
+    assert torch.equal(j.packed, torch.cat([l1.packed, s1.packed])) and torch.equal(j.sf_chunks, torch.cat([l1.sf_chunks, s1.sf_chunks]))
+    l1.packed = l1.packed.clone()
+    hold = []
+    args = MM._weight_args(sym.joined_weights(l1, s1), hold)
+    assert (args["b"], args["sfb"], args["b_rows"]) == (l1.packed.data_ptr(), l1.sf_chunks.data_ptr(), E * 2 * I)
+    assert (args["b2"], args["sfb2"], args["b2_rows"]) == (s1.packed.data_ptr(), s1.sf_chunks.data_ptr(), 2 * I)
+    assert "b2" not in MM._weight_args(l1, hold) and MM._weight_args(l1, hold)["b"] == l1.packed.data_ptr()
+    # shared weights at an odd address, or strided, are copied for the launch as the copy engine cannot read them there
+    odd = MM.MegaWeights(torch.zeros(s1.packed.numel() + 8, dtype=torch.uint8)[8:].view_as(s1.packed).copy_(s1.packed), s1.sf_chunks, 1, s1.n, s1.k)
+    strided = MM.MegaWeights(s1.packed, torch.stack([s1.sf_chunks, s1.sf_chunks], 1)[:, 0], 1, s1.n, s1.k)
+    for w in (odd, strided):
+        args = MM._weight_args(sym.joined_weights(l1, w), hold)
+        assert "b2" not in args and (args["b"], args["sfb"], args["b_rows"]) == (hold[-2].data_ptr(), hold[-1].data_ptr(), (E + 1) * 2 * I)
+        assert torch.equal(hold[-2], torch.cat([l1.packed, s1.packed])) and torch.equal(hold[-1], torch.cat([l1.sf_chunks, s1.sf_chunks]))
+    other, _ = weights(experts=1, seed=10)
+    other.packed.set_(s1.packed)                                    # another set of weights at the same address
+    k = sym.joined_weights(l1, other)
+    assert k is not first and torch.equal(k.sf_chunks[-other.sf_chunks.numel():], other.sf_chunks)
+
+
 def test_weight_transform_shapes_and_rules():
     (w1, w1_sf), (w2, w2_sf) = O.make_weights(E, H, I, 0)
     l1, l2 = MM.transform_weights_for_mega_moe((w1, w1_sf), (w2, w2_sf))

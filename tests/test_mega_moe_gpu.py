@@ -136,6 +136,35 @@ def test_shared_experts_stats_bf16_input_and_timer():
         buf.destroy()
 
 
+@pytest.mark.parametrize("pairs", ["0", "1"])
+def test_weights_changed_in_place_take_effect(pairs):
+    """Routed and shared weights rewritten in place between two calls, as a program that reloads its weights does."""
+    from deepep_b200.models.mega_moe import SymmBuffer, fp8_fp4_mega_moe, transform_weights_for_mega_moe
+
+    dev = torch.device("cuda")
+    T, H, I, E, K, S = 150, 256, 128, 4, 2, 1
+    x = torch.randn((T, H), generator=torch.Generator().manual_seed(1)).bfloat16()
+    idx, w = make_routes("random", T, E, K, 1, 7), make_weights(T, K, 2)
+    buf = SymmBuffer(None, E, 256, K, H, I, num_shared_experts=S)
+    buf.engine.pairs = pairs
+    try:
+        buf.topk_idx[:T].copy_(idx.to(torch.int32)); buf.topk_weights[:T].copy_(w)
+        y, held = torch.zeros((T, H), dtype=torch.bfloat16, device=dev), None
+        for seed in (3, 4):
+            routed, shared = O.make_weights(E, H, I, seed), O.make_weights(S, H, I, 100 + seed)
+            new = transform_weights_for_mega_moe(*routed, device=dev) + transform_weights_for_mega_moe(*shared, device=dev)
+            if held is None:
+                held = new
+            for mine, theirs in zip(held, new):
+                mine.packed.copy_(theirs.packed); mine.sf_chunks.copy_(theirs.sf_chunks)
+            fp8_fp4_mega_moe(y, held[0], held[1], buf, held[2], held[3], x=x.to(dev), check=True)
+            ref = O.mega_moe_reference([O.quantize_mxfp8(x)], [idx], [w], *routed, E, *shared)[0]
+            ok, bad, worst = _mixed_error_ok(y.cpu(), ref)
+            assert ok, f"weights {seed}: {bad:.4f} of elements off, worst relative error {worst:.4f}"
+    finally:
+        buf.destroy()
+
+
 def test_shared_experts_on_two_virtual_ranks():
     """Shared experts next to routed ones on two ranks (engine level): rows of the shared experts never leave their rank."""
     from deepep_b200.models.mega_moe import MegaEngine, MegaWeights, transform_weights_for_mega_moe
