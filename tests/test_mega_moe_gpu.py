@@ -137,6 +137,45 @@ def test_shared_experts_stats_bf16_input_and_timer():
 
 
 @pytest.mark.parametrize("pairs", ["0", "1"])
+@pytest.mark.parametrize("E, S", [(32, 1), (33, 0), (64, 0), (70, 2)])
+def test_layout_of_more_than_32_local_experts(E, S, pairs):
+    """The scan over the experts takes a second and a third turn: empty experts at the turns and at both ends, one of more than a
+    tile in front of a turn and one behind it."""
+    from deepep_b200.models.mega_moe import SymmBuffer, fp8_fp4_mega_moe, transform_weights_for_mega_moe
+
+    dev = torch.device("cuda")
+    T, H, I, K = 300, 256, 128, 4
+    g = torch.Generator().manual_seed(E + S)
+    scores = torch.rand((T, E), generator=g)
+    for empty in (0, 30, 32, 33, E - 1):
+        scores[:, min(empty, E - 1)] = -1.0
+    scores[:150, 29] = 2.0
+    scores[20:290, 31] = 2.0
+    if E > 34:
+        scores[:200, 34] = 2.0
+    idx, w = torch.topk(scores, K, dim=1).indices, make_weights(T, K, 2)
+    l1, l2 = O.make_weights(E, H, I, 3)
+    shared = O.make_weights(S, H, I, 103) if S else (None, None)
+    x = torch.randn((T, H), generator=g).bfloat16()
+    ref = O.mega_moe_reference([O.quantize_mxfp8(x)], [idx], [w], l1, l2, E, *shared)[0]
+    buf = SymmBuffer(None, E, 320, K, H, I, num_shared_experts=S)
+    buf.engine.pairs = pairs
+    try:
+        weights = transform_weights_for_mega_moe(l1, l2, device=dev)
+        extra = transform_weights_for_mega_moe(*shared, device=dev) if S else (None, None)
+        buf.topk_idx[:T].copy_(idx.to(torch.int32)); buf.topk_weights[:T].copy_(w)
+        stats = torch.zeros(E, dtype=torch.int32, device=dev)
+        for fused in (True, False) if pairs == "0" else (True,):
+            y = torch.zeros((T, H), dtype=torch.bfloat16, device=dev)
+            fp8_fp4_mega_moe(y, *weights, buf, *extra, stats.zero_(), x=x.to(dev), fused=fused, check=True)
+            ok, bad, worst = _mixed_error_ok(y.cpu(), ref)
+            assert ok, f"fused={fused}: {bad:.4f} of elements off, worst relative error {worst:.4f}"
+            assert torch.equal(stats.cpu(), torch.bincount(idx.flatten(), minlength=E).int())
+    finally:
+        buf.destroy()
+
+
+@pytest.mark.parametrize("pairs", ["0", "1"])
 def test_weights_changed_in_place_take_effect(pairs):
     """Routed and shared weights rewritten in place between two calls, as a program that reloads its weights does."""
     from deepep_b200.models.mega_moe import SymmBuffer, fp8_fp4_mega_moe, transform_weights_for_mega_moe
