@@ -338,8 +338,8 @@ __device__ __forceinline__ void gmm_phase(const GmmArgs& a, const GmmShared& sh,
       const int4 info = tile_info(mt);
       // This warp drains its 32 lanes of an accumulator into registers as bf16, and hands tensor memory back before it stores
       // the last half, so that the next tile's MMAs overlap the stores.  Stored straight from each thread's row, 64 bytes
-      // at a time, with the accumulators held until then: 5003 rows of 2048 x 7168, 16 experts 167 us instead of 151, 32768 rows of
-      // 7168 x 4096, 4 experts 1330 instead of 1291.  Eight lanes exchange their rows' 16-byte pieces first:
+      // at a time, with the accumulators held until then, the kernel took 167 us instead of 151 for 5003 rows of 2048 x 7168, 16 experts,
+      // and 1330 instead of 1291 for 32768 rows of 7168 x 4096, 4 experts.  Eight lanes exchange their rows' 16-byte pieces first:
       // together they cover one row's 128-byte segment of this rank's output (a2av_gmm) or of the receive area of the rank
       // the row came from (gmm_a2av).
       if (!bounded_wait(&bars->acc_full, local_tile & 1u, failed)) break;
@@ -506,8 +506,9 @@ __global__ void __launch_bounds__(kGmmGemmThreads, 1) gmm_a2av_kernel(const __gr
 // ---------------------------------------------------------------- both ops on a single rank
 // Rows sorted by global expert are already grouped by local expert, and every result belongs to this rank.  The general
 // kernels copy x twice and pass four grid barriers (a2av_gmm), or write the output into the receive area and copy it from
-// there (gmm_a2av); here x is the A operand and the epilogue writes the output.  32768 rows of 7168 x 4096, 4 experts: 1811 -> 1551 us;
-// 5003 rows of 2048 x 7168, 16 experts: 257 -> 213 us (of which a part is the second halves of short tiles left out).
+// there (gmm_a2av); here x is the A operand and the epilogue writes the output.  A whole call, with what surrounds the kernel, when it took
+// their place: 32768 rows of 7168 x 4096, 4 experts, 1811 -> 1551 us; 5003 rows of 2048 x 7168, 16 experts, 257 -> 213 us (of which a
+// part is the second halves of short tiles left out).  With the epilogue above: 1517 and 194 us.
 __global__ void __launch_bounds__(kGmmGemmThreads + kGmmPullWarps * 32, 1) gmm_local_kernel(const __grid_constant__ GmmParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ GmmShared sh;

@@ -5,9 +5,10 @@
 // scales per 32.
 //
 // `gemm_phase` is run by a whole CTA of kGemmThreads threads, one CTA per SM, warp-specialised:
-//   warp 0     one lane issues the TMA tile loads (A, B) and bulk loads (scale chunks) of a stage
-//   warp 1     allocates tensor memory; one lane copies the scales smem -> TMEM (tcgen05.cp) and
-//              issues four tcgen05.mma (M=128, N=256, K=32) per stage; tcgen05.commit frees the stage
+//   warp 0     one elected lane issues the TMA loads: A and B of every stage, and every fourth K step the
+//              scales of four into one of two slots of their own
+//   warp 1     allocates tensor memory; one elected lane copies a step's scales smem -> TMEM (tcgen05.cp) and
+//              issues four tcgen05.mma (M=128, N=256, K=32) per stage; tcgen05.commit frees `commit_every` stages
 //   warps 2-9  epilogue (two warps per TMEM lane quadrant, each takes half of the columns):
 //              tcgen05.ld of the fp32 accumulator (one tile row per thread), then
 //              store fp32 | SwiGLU + MXFP8 requantisation | bf16 rows pushed into the source
@@ -26,7 +27,8 @@
 // it into registers as bf16, 64 a thread, before anything else, and the next tile's MMAs overlap the arithmetic and the stores.
 // Scales travel in groups of four K steps (kSfGroup), both 128-row blocks of weights in one box, and the rows of the combine
 // epilogue are turned in registers, which leaves shared memory for four stages instead of three.  32 experts, hidden 7168,
-// intermediate 2048, GEMM phases of the fused layer: 1264 -> 1158 us at 4096 tokens, 192 -> 169 us at 64.
+// intermediate 2048, GEMM phases of the fused layer when this came in: 1264 -> 1158 us at 4096 tokens, 192 -> 169 us at 64 (156 since
+// the rows arrive sooner).  Depth of the pipeline, 64 tokens' first GEMM alone: 208 us with two stages, 154 with three, 133 with four.
 // All waits are bounded; a wait that runs out sets an error flag, the CTA stops issuing work,
 // frees its tensor memory and returns.
 //
@@ -69,7 +71,7 @@ constexpr int kSchedRing = 8;   // tile ids in flight between the producer and t
 struct GemmBarriers {
   uint64_t full[kGemmMaxStages], acc_full, acc_empty, epi_done;
   uint64_t peer_acc_empty;         // CTA pairs: the odd CTA's acc_empty, forwarded to the even CTA
-  uint64_t released[kGroupRing];   // the MMAs of a group of kCommitEvery stages have completed
+  uint64_t released[kGroupRing];   // the MMAs of a group of `commit_every` stages have completed
   uint64_t sched[kSchedRing];      // the producer has published tile_id[slot]
   int tile_id[kSchedRing];
   uint32_t tmem_base;

@@ -267,7 +267,7 @@ __device__ __forceinline__ void finish_phase(const MegaFinishArgs& a, bool bump_
     const float* w = reinterpret_cast<const float*>(ctx.ws[me] + a.in_off + in.w);
     const uint8_t* comb = ctx.ws[me] + a.comb_off;
     // A work item is a span of 64 16-byte pieces of one token, dealt out statically: whole tokens were 2.3 waves of warps at
-    // 4096 tokens (the layer took 1978 us with them and takes 1973 in spans, hardly more than its runs differ).  Slot and weight
+    // 4096 tokens (1978 us for the layer as it was then, 1973 in spans, hardly more than its runs differ).  Slot and weight
     // of the next item are fetched while this one is summed.
     const int units = H / 8, spans = (units + 63) / 64, items = a.T * spans;
     // lane k holds slot k: its weight and whether it counts (shared experts: every token, weight one)
