@@ -14,10 +14,11 @@
 // What stays on the rank takes neither detour: its tokens are routed from the caller's table, its rows go
 // from the caller's tensor straight into the output rows (quantised on the way, cut into as many pieces as
 // there are warps), and the combine reads the rows of its own experts where they lie, through the row of
-// every (token, slot) that the dispatch leaves behind.  What bounds both kernels is the chain of dependent
-// steps, not bytes: on one GPU a captured round (hidden 7168, 256 experts, top-8, fp8) took 34.8 us for one
-// token while own rows went through flags and the staging area and one thread scanned the experts, 18.4 us
-// since; 93 bf16 tokens of 4096 (64 experts, top-6) 41.3 and 20.5 us.
+// every (token, slot) that the dispatch leaves behind.  A single rank, where that is all there is, has kernels of
+// its own (the *_local kernels).  What bounds all of them is the launch and the chain of dependent steps, not
+// bytes: on one GPU a captured round (hidden 7168, 256 experts, top-8, fp8) took 34.8 us for one token while own
+// rows went through flags and the staging area and one thread scanned the experts, 18.4 us in the kernels for
+// several ranks, 9.6 us in those for one; 93 bf16 tokens of 4096 (64 experts, top-6) 41.3, 20.5 and 10.3 us.
 //
 // Re-entrancy: epochs live in device memory and select one of two banks, flags hold epochs and
 // are never cleared, a bank is reused only after the peers acknowledged the call before last.
@@ -33,8 +34,10 @@
 namespace dep {
 
 constexpr int kLLThreads = 512;
+constexpr int kLLLocalThreads = 128; // combine of one rank
 constexpr int kLLSendWarps = 8;      // dispatch: warps that push rows; the other warps of the block derive the layout meanwhile
-constexpr int kLLWords = 8;  // 256 tokens as 8 x 32-bit masks
+constexpr int kLLMaxTokens = 256;
+constexpr int kLLWords = kLLMaxTokens / 32;  // a token set as 32-bit masks
 
 // A row travels as kLLParts column parts, each with its own flag, so that a row is spread over several warps on both
 // sides.  Parts are whole groups of 128 values (the granularity of the fp8 scales): part p covers values [v0, v1).
@@ -111,6 +114,52 @@ __device__ __forceinline__ LLPart ll_piece(int H, int p, int n) {
 }
 
 constexpr int kOwnUnroll = 4;   // 16-byte pieces per lane of an own row that are read ahead of the layout
+
+// One piece of token t of the caller's tensor, quantised on the way in mode 2, into the output rows of its slots: lane l of
+// `live` holds an output row.  `ahead`: the piece's first loads, when they were issued earlier.
+__device__ __forceinline__ void write_own_piece(const LLDispatchArgs& a, uint8_t* recv_x, int t, const LLPart& pr, int row, unsigned live,
+                                                int H, int nsf, int row_bytes, int src_bytes, const int4* ahead, int lane) {
+  const int4* src = reinterpret_cast<const int4*>(reinterpret_cast<const uint8_t*>(a.x) + (size_t)t * src_bytes);
+  const int lo = (a.mode == 1 ? pr.v0 : pr.v0 * 2) / 16, hi = (a.mode == 1 ? pr.v1 : pr.v1 * 2) / 16;
+  for (int u0 = lo; u0 < hi; u0 += 32 * kOwnUnroll) {
+    int4 v[kOwnUnroll];
+#pragma unroll
+    for (int i = 0; i < kOwnUnroll; ++i) {
+      const int u = u0 + i * 32 + lane;
+      if (ahead && u0 == lo) v[i] = ahead[i];
+      else v[i] = u < hi ? __ldg(src + u) : make_int4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int i = 0; i < kOwnUnroll; ++i) {
+      const int u = u0 + i * 32 + lane;
+      if (u0 + i * 32 >= hi) break;               // warp-uniform
+      if (a.mode == 2) {
+        float scale;
+        const uint2 q = quant8(v[i], scale);
+        for (unsigned m = live; m; m &= m - 1) {
+          const size_t o = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
+          if (u < hi) {
+            *reinterpret_cast<uint2*>(recv_x + o * H + (size_t)u * 8) = q;
+            if ((lane & 15) == 0) a.recv_sf[o * nsf + u / 16] = scale;
+          }
+        }
+      } else {
+        for (unsigned m = live; m; m &= m - 1) {
+          const size_t o = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
+          if (u < hi) reinterpret_cast<int4*>(recv_x + o * row_bytes)[u] = v[i];
+        }
+      }
+    }
+  }
+  if (a.mode == 1)
+    for (int b = pr.b0; b < pr.b1; b += 32) {
+      const float sf = b + lane < pr.b1 ? __ldg(a.x_sf + (size_t)t * nsf + b + lane) : 0.f;
+      for (unsigned m = live; m; m &= m - 1) {
+        const size_t o = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
+        if (b + lane < pr.b1) a.recv_sf[o * nsf + b + lane] = sf;
+      }
+    }
+}
 
 template <bool kProfile>
 __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid_constant__ LLDispatchParams p) {
@@ -289,7 +338,6 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
     int maxT = 1;
     for (int r = 0; r < P; ++r) maxT = max(maxT, min(s_T[r], M));
     const int words = (maxT + 31) >> 5;               // mask words in use
-    if (P > 1) {
     // one thread per (source, token) of the peers (this rank's masks are already set); the loads of four items are issued
     // before the first of them is used
     constexpr int kBatch = 4;
@@ -316,7 +364,6 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
       }
     }
     layout_sync();
-    }
     // rows per local expert and their exclusive prefix: every thread owns `per` consecutive experts, a warp scan and the
     // warps' totals give its first row (a serial scan by one thread took 6 us for 384 experts)
     const int per = (Lx + LT - 1) / LT, l0 = min(Lx, lt * per), l1 = min(Lx, l0 + per);
@@ -410,46 +457,7 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
       }
       const unsigned live = __ballot_sync(0xffffffffu, row >= 0);
       if (live == 0 || pr.v0 >= pr.v1) continue;
-      const int4* src = reinterpret_cast<const int4*>(reinterpret_cast<const uint8_t*>(a.x) + (size_t)t * src_bytes);
-      const int lo = (a.mode == 1 ? pr.v0 : pr.v0 * 2) / 16, hi = (a.mode == 1 ? pr.v1 : pr.v1 * 2) / 16;
-      for (int u0 = lo; u0 < hi; u0 += 32 * kOwnUnroll) {
-        int4 v[kOwnUnroll];
-#pragma unroll
-        for (int i = 0; i < kOwnUnroll; ++i) {
-          const int u = u0 + i * 32 + lane;
-          if (item == gw && u0 == lo) v[i] = ahead[i];
-          else v[i] = u < hi ? __ldg(src + u) : make_int4(0, 0, 0, 0);
-        }
-#pragma unroll
-        for (int i = 0; i < kOwnUnroll; ++i) {
-          const int u = u0 + i * 32 + lane;
-          if (u0 + i * 32 >= hi) break;               // warp-uniform
-          if (a.mode == 2) {
-            float scale;
-            const uint2 q = quant8(v[i], scale);
-            for (unsigned m = live; m; m &= m - 1) {
-              const size_t o = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
-              if (u < hi) {
-                *reinterpret_cast<uint2*>(recv_x + o * H + (size_t)u * 8) = q;
-                if ((lane & 15) == 0) a.recv_sf[o * nsf + u / 16] = scale;
-              }
-            }
-          } else {
-            for (unsigned m = live; m; m &= m - 1) {
-              const size_t o = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
-              if (u < hi) reinterpret_cast<int4*>(recv_x + o * row_bytes)[u] = v[i];
-            }
-          }
-        }
-      }
-      if (a.mode == 1)
-        for (int b = pr.b0; b < pr.b1; b += 32) {
-          const float sf = b + lane < pr.b1 ? __ldg(a.x_sf + (size_t)t * nsf + b + lane) : 0.f;
-          for (unsigned m = live; m; m &= m - 1) {
-            const size_t o = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
-            if (b + lane < pr.b1) a.recv_sf[o * nsf + b + lane] = sf;
-          }
-        }
+      write_own_piece(a, recv_x, t, pr, row, live, H, nsf, row_bytes, src_bytes, item == gw ? ahead : nullptr, lane);
     }
 
     // ---- rows of the peers: poll the part flags and write the output rows
@@ -514,7 +522,168 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
   }
 }
 
+// One rank: nothing is sent and nobody is waited for, so every block derives the layout from the caller's table by itself and
+// writes its share of the rows.  What bounds it is the launch and the chain routes -> masks -> scan -> rows; the table's and the
+// first row's loads are issued before anything else.  Because no block waits for another an ordinary launch will do: a captured
+// dispatch of one fp8 token (hidden 7168, 256 experts, top-8) took 12.4 us as a cooperative launch of the kernel above, of which 6.9
+// were spent inside, and takes 6.3 here (3.8 inside); 64 tokens 12.5 and 6.7 us, 128 tokens 14.7 and 8.7.
+template <bool kProfile>
+__global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_local_kernel(const __grid_constant__ LLDispatchParams p) {
+  const LLDispatchArgs& a = p.r[0];
+  const WsLayout& lay = p.lay;
+  const int K = lay.topk, H = lay.hidden, E = a.E, T = a.T, n = T * K;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int gw = warp * gridDim.x + blockIdx.x, total_warps = gridDim.x * (kLLThreads / 32);
+  const bool fp8 = a.mode != 0;
+  const int nsf = H / 128, row_bytes = fp8 ? H : H * 2, src_bytes = a.mode == 1 ? H : H * 2, words = (T + 31) >> 5;
+
+  __shared__ unsigned s_emask[kMaxExperts * kLLWords];    // [expert][words]: its tokens
+  __shared__ int s_off[kMaxExperts];                      // first output row of the expert
+  __shared__ short s_id[kLLMaxTokens * kMaxTopk];         // the table; -1: no expert
+  __shared__ int s_warp_rows[kLLThreads / 32];
+
+  Control* ctl = control_of(a.ctx.ws[0]);
+  unsigned long long t_start = 0;
+  if constexpr (kProfile) t_start = global_timer_ns();
+  auto stamp = [&](int i) {
+    if constexpr (kProfile)
+      if (blockIdx.x == 0 && threadIdx.x == 0) ctl->dbg[i] = global_timer_ns() - t_start;
+  };
+
+  // ---- the routes and this warp's first piece of a row (loops over the table stay rolled: a launch starts with a cold instruction
+  // cache, and copies of a loop's body cost more than its iterations)
+  constexpr int kIds = 4;
+#pragma unroll 1
+  for (int i0 = threadIdx.x; i0 < n; i0 += kLLThreads * kIds) {
+    long long v[kIds];
+#pragma unroll
+    for (int j = 0; j < kIds; ++j) v[j] = i0 + j * kLLThreads < n ? __ldg(a.topk_idx + i0 + j * kLLThreads) : -1;
+#pragma unroll
+    for (int j = 0; j < kIds; ++j)
+      if (i0 + j * kLLThreads < n) s_id[i0 + j * kLLThreads] = (short)((v[j] < 0 || v[j] >= E) ? -1 : (int)v[j]);
+  }
+  const int pieces = max(1, min((H + 127) / 128, total_warps / max(T, 1)));
+  int4 ahead[kOwnUnroll];
+  LLPart first_part = {0, 0, 0, 0};
+  if (gw < T * pieces) {
+    first_part = ll_piece(H, gw % pieces, pieces);
+    const int lo = (a.mode == 1 ? first_part.v0 : first_part.v0 * 2) / 16, hi = (a.mode == 1 ? first_part.v1 : first_part.v1 * 2) / 16;
+    const int4* src = reinterpret_cast<const int4*>(reinterpret_cast<const uint8_t*>(a.x) + (size_t)(gw / pieces) * src_bytes);
+#pragma unroll
+    for (int i = 0; i < kOwnUnroll; ++i) {
+      const int u = lo + i * 32 + lane;
+      ahead[i] = u < hi ? __ldg(src + u) : make_int4(0, 0, 0, 0);
+    }
+  }
+#pragma unroll 1
+  for (int i = threadIdx.x; i < E * words; i += kLLThreads) s_emask[i] = 0u;
+  const bool head = gw < T * pieces && gw % pieces == 0;      // this warp starts with the first piece of a token: its weights too
+  const float first_w = head && lane < K && a.topk_w ? __ldg(a.topk_w + (size_t)(gw / pieces) * K + lane) : 0.f;
+  __syncthreads();
+  stamp(0);
+
+  // ---- tokens of every expert: a repeated id sets the same bit again
+#pragma unroll 1
+  for (int i = threadIdx.x; i < n; i += kLLThreads) {
+    const int e = s_id[i], t = i / K;
+    if (e >= 0) atomicOr(&s_emask[e * words + (t >> 5)], 1u << (t & 31));
+  }
+  __syncthreads();
+  stamp(2);
+
+  // ---- first row of every expert: two consecutive experts per thread, a warp scan and the warps' totals
+  constexpr int kPer = kMaxExperts / kLLThreads;
+  const int per = E > kLLThreads ? kPer : 1;
+  int rows[kPer] = {}, tot = 0;
+  for (int j = 0; j < per; ++j) {
+    const int e = (int)threadIdx.x * per + j;
+    if (e < E)
+      for (int w = 0; w < words; ++w) rows[j] += __popc(s_emask[e * words + w]);
+    tot += rows[j];
+  }
+  int incl = tot;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += o;
+  }
+  if (lane == 31) s_warp_rows[warp] = incl;
+  __syncthreads();
+  int run = incl - tot, all = 0;
+#pragma unroll
+  for (int w = 0; w < kLLThreads / 32; ++w) {
+    const int r = s_warp_rows[w];
+    if (w < warp) run += r;
+    all += r;
+  }
+  for (int j = 0; j < per; ++j) {
+    const int e = (int)threadIdx.x * per + j;
+    if (e >= E) break;
+    s_off[e] = run;
+    if (blockIdx.x == 0) {
+      a.expert_offsets[e] = run;
+      a.expert_counts[e] = rows[j];
+      if (a.mailbox) a.mailbox[4 + e] = rows[j];
+    }
+    run += rows[j];
+  }
+  __syncthreads();
+  stamp(3);
+
+  // ---- the rows, each piece from the caller's tensor into every output row of its token
+  uint8_t* recv_x = reinterpret_cast<uint8_t*>(a.recv_x);
+  for (int item = gw; item < T * pieces; item += total_warps) {
+    const int piece = item % pieces, t = item / pieces;
+    const LLPart pr = item == gw ? first_part : ll_piece(H, piece, pieces);
+    const int e = lane < K ? s_id[t * K + lane] : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    int row = -1;
+    if (e >= 0 && (same & ((1u << lane) - 1u)) == 0) {
+      row = s_off[e] + below8(s_emask + e * words, t);
+      if (row >= a.capacity) row = -1;
+    }
+    if (piece == 0 && lane < K) {
+      a.local_row[(size_t)t * K + lane] = row;
+      if (row >= 0) {
+        a.recv_row_src[row] = t * K + lane;
+        a.recv_w[row] = item == gw ? first_w : a.topk_w ? __ldg(a.topk_w + (size_t)t * K + lane) : 0.f;
+      }
+    }
+    const unsigned live = __ballot_sync(0xffffffffu, row >= 0);
+    if (live == 0 || pr.v0 >= pr.v1) continue;
+    write_own_piece(a, recv_x, t, pr, row, live, H, nsf, row_bytes, src_bytes, item == gw ? ahead : nullptr, lane);
+  }
+  stamp(4);
+
+  // ---- the host's copy of the counts, and the epoch (nothing but this block reads it)
+  if (blockIdx.x == 0) {
+    if (a.mailbox) __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const unsigned long long epoch = ctl->epoch[kOpLLDispatch] + 1;
+      a.expert_offsets[E] = all;
+      *a.num_rows = all;
+      if (a.mailbox) {
+        a.mailbox[0] = all;
+        __threadfence_system();
+        a.mailbox[3] = (int)(epoch & 0x7fffffff);
+      }
+      ctl->ll_disp_ack[0] = epoch;
+      ctl->epoch[kOpLLDispatch] = epoch;
+    }
+    stamp(5);
+  }
+}
+
 cudaError_t launch_ll_dispatch(const LLDispatchParams& p, int nranks, int blocks, cudaStream_t stream) {
+  if (p.lay.world == 1 && nranks == 1) {
+    const LLDispatchArgs& a = p.r[0];
+    // no more blocks than pieces of 128 values: every block derives the whole layout
+    const int items = a.T * ((p.lay.hidden + 127) / 128), grid = max(1, min(blocks, items));
+    if (p.profile) ep_dispatch_ll_local_kernel<true><<<grid, kLLThreads, 0, stream>>>(p);
+    else ep_dispatch_ll_local_kernel<false><<<grid, kLLThreads, 0, stream>>>(p);
+    return cudaGetLastError();
+  }
   dim3 grid(blocks, nranks), block(kLLThreads);
   void* args[] = {const_cast<LLDispatchParams*>(&p)};
   const void* fn = p.profile ? (const void*)ep_dispatch_ll_kernel<true> : (const void*)ep_dispatch_ll_kernel<false>;
@@ -553,8 +722,7 @@ __global__ void __launch_bounds__(kLLThreads) ep_combine_ll_kernel(const __grid_
 
   if (alive) {
     // ---- return every expert row of a peer's token, part by part, to its (token, slot) slot there
-    int R = P > 1 ? min(*a.num_rows, a.x_rows) : 0;
-    if (aborted) R = 0;
+    const int R = aborted ? 0 : min(*a.num_rows, a.x_rows);
     PendingFlags pending;
     for (int item = gw; item < R * kLLParts; item += total_warps) {
       const int r = item / kLLParts, part = item % kLLParts;
@@ -668,7 +836,93 @@ __global__ void __launch_bounds__(kLLThreads) ep_combine_ll_kernel(const __grid_
   }
 }
 
+// One rank: every row is in x, so a warp takes 32 pieces of 16 bytes of a token and there is nothing to wait for.  Launch and two
+// dependent rounds of loads (slots, rows) bound it; small blocks, as many as there are pieces, in an ordinary launch.  A captured
+// combine of one token of 7168, top-8: 8.4 us as a cooperative launch of the kernel above (2.5 inside), 4.3 here (2.0 inside);
+// 128 tokens 10.4 and 6.4 us.
+template <bool kProfile>
+__global__ void __launch_bounds__(kLLLocalThreads) ep_combine_ll_local_kernel(const __grid_constant__ LLCombineParams p) {
+  const LLCombineArgs& a = p.r[0];
+  const int K = p.lay.topk, units = p.lay.hidden / 8, spans = (units + 31) / 32, lane = threadIdx.x & 31;
+  Control* ctl = control_of(a.ctx.ws[0]);
+  unsigned long long t_start = 0;
+  if constexpr (kProfile) t_start = global_timer_ns();
+  auto stamp = [&](int i) {
+    if constexpr (kProfile)
+      if (blockIdx.x == 0 && threadIdx.x == 0) ctl->dbg[8 + i] = global_timer_ns() - t_start;
+  };
+  const int aborted = ld_volatile_int(&ctl->abort);    // set: an earlier call gave up, the handle's tensors may never have been written
+  const int item = blockIdx.x * (kLLLocalThreads / 32) + (threadIdx.x >> 5), t = item / spans, u = (item - t * spans) * 32 + lane;
+  if (t < a.T) {
+    // lane k holds slot k: whether it counts (id in range, first occurrence), its weight, its row
+    int e = -1, local = -1;
+    float w = 0.f;
+    if (lane < K) {
+      const size_t at = (size_t)t * K + lane;
+      const long long v = __ldg(a.topk_idx + at);
+      w = __ldg(a.topk_w + at);
+      local = __ldg(a.local_row + at);
+      e = (v < 0 || v >= a.E) ? -1 : (int)v;
+    }
+    stamp(0);
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    const bool counts = e >= 0 && (same & ((1u << lane) - 1u)) == 0;
+    const unsigned valid = __ballot_sync(0xffffffffu, counts);
+    bool ok = !aborted;
+    if (ok && counts && (local < 0 || local >= a.x_rows)) {       // the handle and x do not belong together
+      report_failure(a.ctx, kStatusBadArgument, kOpLLCombine, 2, 0, a.x_rows, (unsigned long long)(long long)local);
+      ok = false;
+    }
+    stamp(1);
+    if (__all_sync(0xffffffffu, ok)) {
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      const int4* x = reinterpret_cast<const int4*>(a.x);
+      for (int kb = 0; kb < K; kb += 8) {    // eight slots' loads in flight at a time
+        int4 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (kb + k < K && ((valid >> (kb + k)) & 1u)) {
+            const int4* row = x + (size_t)__shfl_sync(0xffffffffu, local, kb + k) * units;
+            if (u < units) v[k] = __ldg(row + u);
+          }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (kb + k < K && ((valid >> (kb + k)) & 1u)) {         // warp-uniform
+            const float wk = __shfl_sync(0xffffffffu, w, kb + k);
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[k]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              // product and sum are rounded separately (no fused multiply-add), as the CPU oracle does
+              acc[2 * i] = __fadd_rn(acc[2 * i], __fmul_rn(wk, __low2float(h[i])));
+              acc[2 * i + 1] = __fadd_rn(acc[2 * i + 1], __fmul_rn(wk, __high2float(h[i])));
+            }
+          }
+      }
+      if (u < units) {
+        int4 o;
+        __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) oh[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
+        reinterpret_cast<int4*>(a.out)[(size_t)t * units + u] = o;
+      }
+    }
+  }
+  stamp(2);
+  if (item == 0 && lane == 0) {            // nothing but this thread reads the epoch
+    const unsigned long long epoch = ctl->epoch[kOpLLCombine] + 1;
+    ctl->ll_comb_ack[0] = epoch;
+    ctl->epoch[kOpLLCombine] = epoch;
+  }
+  stamp(3);
+}
+
 cudaError_t launch_ll_combine(const LLCombineParams& p, int nranks, int blocks, cudaStream_t stream) {
+  if (p.lay.world == 1 && nranks == 1) {
+    const int warps = max(1, p.r[0].T * ((p.lay.hidden / 8 + 31) / 32)), per = kLLLocalThreads / 32, grid = (warps + per - 1) / per;
+    if (p.profile) ep_combine_ll_local_kernel<true><<<grid, kLLLocalThreads, 0, stream>>>(p);
+    else ep_combine_ll_local_kernel<false><<<grid, kLLLocalThreads, 0, stream>>>(p);
+    return cudaGetLastError();
+  }
   dim3 grid(blocks, nranks), block(kLLThreads);
   void* args[] = {const_cast<LLCombineParams*>(&p)};
   const void* fn = p.profile ? (const void*)ep_combine_ll_kernel<true> : (const void*)ep_combine_ll_kernel<false>;

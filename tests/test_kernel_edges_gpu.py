@@ -24,6 +24,35 @@ def test_low_latency_splits(world, tokens, hidden, experts, topk, mode):
     ll_case(world, tokens, hidden, experts, topk, mode, routes="invalid", repeats=3)
 
 
+# one rank: mask words (32 tokens), batches of the table (2048 slots), one and two experts per thread, short last pieces
+@pytest.mark.parametrize("tokens,hidden,experts,topk,mode", [
+    (1, 8, 1, 1, 0), (1, 7168, 384, 8, 2), (31, 264, 513, 7, 0), (32, 256, 512, 16, 1), (33, 1032, 1024, 16, 0),
+    (129, 128, 511, 16, 2), (256, 640, 1024, 16, 0), (255, 8192, 9, 9, 2), (256, 1280, 40, 3, 1)])
+def test_low_latency_on_one_rank(monkeypatch, tokens, hidden, experts, topk, mode):
+    """Repeated and out-of-range ids among the slots; rows, scales, weights, counts and the combine against the oracle, for which
+    the later ones of repeated ids are empty slots."""
+    from types import SimpleNamespace
+
+    import test_ll_gpu
+
+    def routes(kind, t, E, K, world, seed):
+        g = torch.Generator().manual_seed(seed)
+        idx = torch.randint(-1, E + 1, (t, K), generator=g)
+        idx[::3, K // 2:] = idx[::3, :K - K // 2].clone()      # the second half repeats the first
+        idx[1::4] = idx[1::4, :1].clone()                       # one expert in every slot
+        return idx
+
+    def first_only(idx):
+        earlier = (idx.unsqueeze(2) == idx.unsqueeze(1)).tril(-1).any(2)
+        return torch.where(earlier, torch.full_like(idx, -1), idx)
+
+    monkeypatch.setattr(test_ll_gpu, "make_routes", routes)
+    monkeypatch.setattr(test_ll_gpu, "R", SimpleNamespace(
+        dispatch=lambda xs, idx, *args, **kw: R.dispatch(xs, [first_only(i) for i in idx], *args, **kw),
+        low_latency_combine=R.low_latency_combine))
+    test_ll_gpu._case(1, [tokens], hidden, experts, topk, mode)
+
+
 @pytest.mark.parametrize("world,tokens,hidden,experts,topk,kw", [
     (1, [1], 7168, 256, 8, dict(dmode=2)),             # one token, many pieces
     (1, [65], 8, 16, 9, {}),                           # rows of one 16-byte piece; two groups of operands per token
