@@ -69,8 +69,9 @@ void op_notify(const WsLayout& lay, const std::vector<py::object>& sessions, con
 }
 
 void op_dispatch(const WsLayout& lay, const std::vector<py::object>& sessions, const std::vector<py::dict>& args, int send_blocks,
-                 int recv_blocks, uintptr_t stream, bool local_direct, bool profile) {
+                 int recv_blocks, uintptr_t stream, bool local_direct, bool profile, bool whole_gpu) {
   DispatchParams p{};
+  p.whole_gpu = whole_gpu;
   p.lay = lay; p.send_blocks = send_blocks; p.recv_blocks = recv_blocks; p.local_direct = local_direct; p.profile = profile;
   const int n = (int)args.size();
   if (n < 1 || n > kMaxRanks || (int)sessions.size() != n) throw std::invalid_argument("1..8 rank argument blocks expected");
@@ -242,7 +243,8 @@ PYBIND11_MODULE(_C, m) {
   m.def("notify", &op_notify, py::arg("layout"), py::arg("sessions"), py::arg("args"), py::arg("blocks"), py::arg("stream"),
         py::arg("profile") = false);
   m.def("dispatch", &op_dispatch, py::arg("layout"), py::arg("sessions"), py::arg("args"), py::arg("send_blocks"),
-        py::arg("recv_blocks"), py::arg("stream"), py::arg("local_direct") = true, py::arg("profile") = false);
+        py::arg("recv_blocks"), py::arg("stream"), py::arg("local_direct") = true, py::arg("profile") = false,
+        py::arg("whole_gpu") = false);
   m.def("combine", &op_combine, py::arg("layout"), py::arg("sessions"), py::arg("args"), py::arg("send_blocks"),
         py::arg("recv_blocks"), py::arg("stream"), py::arg("local_direct") = true, py::arg("profile") = false,
         py::arg("t_begin") = 0, py::arg("t_end") = -1);

@@ -68,8 +68,14 @@ struct DispatchArgs {
 };
 // local_direct: rows whose destination is the sending rank itself are written straight into recv_x by the sender
 // blocks (no staging, no flag); 0 sends them through the staging area like remote rows.
-// pieces: column pieces per token when one rank keeps all its rows (set by the launcher); 0: groups of tokens with a flag each.
-struct DispatchParams { WsLayout lay; int send_blocks, recv_blocks, local_direct, profile, pieces; DispatchArgs r[kMaxRanks]; };
+// whole_gpu: the caller gave no number of blocks to stay within.
+// pieces: column pieces per token when one rank keeps all its rows; 0: groups of tokens with a flag each.  pad_blocks: blocks that
+// zero the padding rows.  (Both set by the launcher.)
+struct DispatchParams {
+  WsLayout lay;
+  int send_blocks, recv_blocks, local_direct, profile, whole_gpu, pieces, pad_blocks, pad;
+  DispatchArgs r[kMaxRanks];
+};
 // per block: role (0 sender, 1 receiver), start ns, end ns, then summed over the block's warps: cycles spent reading
 // routing records, waiting for flags, moving rows, publishing flags; rows moved
 constexpr int kDispatchProfWords = 8;

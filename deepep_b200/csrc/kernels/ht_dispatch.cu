@@ -37,19 +37,19 @@ __device__ __forceinline__ unsigned long long shfl_u64(unsigned long long v, int
 
 // Copies `units` 16-byte pieces from `src` to every destination in `mask`: lane l of the mask holds its
 // destination in `dst`.  All loads of a pass are issued before the first store.
-template <bool kPeerWritten>
+template <bool kPeerWritten, int U = kCopyUnroll>
 __device__ __forceinline__ void warp_fanout(const int4* src, int units, unsigned long long dst, unsigned mask, int lane) {
-  for (int u0 = 0; u0 < units; u0 += 32 * kCopyUnroll) {
-    int4 v[kCopyUnroll];
+  for (int u0 = 0; u0 < units; u0 += 32 * U) {
+    int4 v[U];
 #pragma unroll
-    for (int i = 0; i < kCopyUnroll; ++i) {
+    for (int i = 0; i < U; ++i) {
       const int u = u0 + i * 32 + lane;
       if (u < units) v[i] = kPeerWritten ? __ldcg(src + u) : __ldg(src + u);
     }
     for (unsigned m = mask; m; m &= m - 1) {
       int4* d = reinterpret_cast<int4*>(shfl_u64(dst, __ffs(m) - 1));
 #pragma unroll
-      for (int i = 0; i < kCopyUnroll; ++i) {
+      for (int i = 0; i < U; ++i) {
         const int u = u0 + i * 32 + lane;
         if (u < units) d[u] = v[i];
       }
@@ -357,10 +357,68 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) ep_dispatch_ht_kernel(con
   }
 }
 
+// One rank without a budget of SMs: no peer waits for a flag and no block for another, so every warp takes one piece of a token
+// (2 KB of a bf16 row) and is done, and the hardware deals the blocks out.  Written bytes bound it, and a loop over many pieces per
+// warp is slower at that whatever its items: SMs write at different speeds, and the slowest one ends last (4096 rows of 14 KB stored
+// eight times each, stand-alone: 86 to 88 us in pieces of 1 to 2 KB with 64 to 512 threads per block, 97 to 100 us as 148 blocks of
+// 512 threads that stride over the pieces, with plain, streaming or bulk stores alike; kernel above with tickets 94 us).
+// The first p.pad_blocks blocks zero the padding rows.
+constexpr int kLocalDispatchThreads = 256;
+constexpr int kLocalUnroll = 4;       // 16-byte pieces per lane and item
+
+__global__ void __launch_bounds__(kLocalDispatchThreads) ep_dispatch_local_kernel(const __grid_constant__ DispatchParams p) {
+  const DispatchArgs& a = p.r[0];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = kLocalDispatchThreads / 32, H = p.lay.hidden, K = a.K;
+  Control* ctl = control_of(a.ctx.ws[0]);
+  const bool aborted = ld_volatile_int(&ctl->abort) != 0;   // an earlier call gave up, the plan's tensors may never have been written
+  const bool fp8 = a.mode != kDispatchBf16;
+  const int nsf = fp8 ? H / 128 : 0, row_bytes = fp8 ? H : H * 2, units = row_bytes / 16;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {                // nothing else in this kernel reads the epoch
+    const unsigned long long epoch = ctl->epoch[kOpDispatch] + 1;
+    if (!aborted) ctl->disp_ack[0] = epoch;
+    ctl->epoch[kOpDispatch] = epoch;
+  }
+  if (aborted) return;
+  if ((int)blockIdx.x < p.pad_blocks) {
+    zero_padding(a, a.E, row_bytes, nsf, warp * p.pad_blocks + blockIdx.x, p.pad_blocks * nwarps, lane);
+    return;
+  }
+  const int item = ((int)blockIdx.x - p.pad_blocks) * nwarps + warp, t = item / p.pieces, piece = item - t * p.pieces;
+  if (t >= a.T) return;
+  const int per_piece = ((units + p.pieces - 1) / p.pieces + 31) / 32 * 32, u_begin = min(units, piece * per_piece);
+  const int u_count = min(units - u_begin, per_piece);
+  const uint8_t* src = reinterpret_cast<const uint8_t*>(a.x) + (size_t)t * (a.mode == kDispatchFp8Given ? H : H * 2);
+  // lane k: the output row of slot k (rank layout: lane 0, the token's one row)
+  int row = -1;
+  if (a.expand) { if (lane < K) row = __ldg(a.slot_row + (size_t)t * K + lane); }
+  else if (lane == 0) row = __ldg(a.send_slot + t);
+  if (row >= 0 && a.recv_rows > 0 && !DEP_INDEX_OK(a.ctx, row, a.recv_rows, kOpDispatch, 1)) row = -1;
+  const unsigned mask = __ballot_sync(0xffffffffu, row >= 0);
+  if (mask == 0) return;
+  const unsigned long long dst = reinterpret_cast<unsigned long long>(reinterpret_cast<uint8_t*>(a.recv_x) + (long long)row * row_bytes);
+  const unsigned long long dst_sf = reinterpret_cast<unsigned long long>(a.recv_sf + (long long)row * nsf);
+  if (a.mode == kDispatchFp8Fused) {
+    warp_quant_fanout(reinterpret_cast<const int4*>(src) + 2 * u_begin, u_count * 16, dst + (size_t)u_begin * 16,
+                      dst_sf + (size_t)u_begin / 2, mask, lane);      // 8 pieces of codes share a 4-byte scale
+  } else {
+    warp_fanout<false, kLocalUnroll>(reinterpret_cast<const int4*>(src) + u_begin, u_count, dst + (size_t)u_begin * 16, mask, lane);
+    if (fp8 && piece == 0) warp_fanout_f32<false>(a.x_sf + (size_t)t * nsf, nsf, dst_sf, mask, lane);
+  }
+}
+
 cudaError_t launch_dispatch(const DispatchParams& params, int nranks, cudaStream_t stream) {
   DispatchParams p = params;
   if (p.lay.hidden > 8192) return cudaErrorInvalidValue;   // the fused quantiser keeps at most 64 scales per row in registers
   p.pieces = 0;
+  if (p.lay.world == 1 && nranks == 1 && p.local_direct && p.whole_gpu && !p.profile) {
+    const DispatchArgs& a = p.r[0];
+    const int units = (a.mode == kDispatchBf16 ? 2 : 1) * p.lay.hidden / 16, warps = kLocalDispatchThreads / 32;
+    p.pieces = (units + 32 * kLocalUnroll - 1) / (32 * kLocalUnroll);
+    p.pad_blocks = a.pad_offsets ? std::min(592, (a.recv_rows + warps - 1) / warps) : 0;      // 592: four blocks per SM
+    const long long blocks = p.pad_blocks + ((long long)a.T * p.pieces + warps - 1) / warps;
+    ep_dispatch_local_kernel<<<(unsigned)std::max(1ll, blocks), kLocalDispatchThreads, 0, stream>>>(p);
+    return cudaGetLastError();
+  }
   if (p.lay.world == 1 && p.local_direct) {
     // No peer waits for a group's flag, so the items can be as small as balances the warps.  4096 rows of 14 KB stored eight times
     // each by 144 blocks: 101 us in whole rows, 98 in halves, 93 in quarters (a quarter is what a warp holds in registers);

@@ -113,6 +113,7 @@ class CudaEngine:
         # One block per SM.  The sender side of dispatch (expert side of combine) has to keep NVLink busy, which takes
         # 32 SMs or more; the other side moves the rows inside local memory.  With one rank every row is local and is
         # written (read) directly by the sender (source) side, so that side gets all the blocks.
+        self.sm_budget = num_sms
         budget = min(per_rank, num_sms) if num_sms else min(per_rank, max(2, self.sm_count - 4))
         self.dispatch_blocks = self.combine_blocks = self.default_blocks = budget
         self.dispatch_send_fraction = DISPATCH_SEND_FRACTION.get(self.world, 0.35)
@@ -356,8 +357,9 @@ class CudaEngine:
                              pad_offsets=plan.expert_offsets.data_ptr() if padded else None,
                              prof=self._prof_buffer("dispatch", i)))
         send, recv = split if split is not None else self.split_blocks(blocks, self.dispatch_send_fraction, self.dispatch_blocks)
+        whole = split is None and not blocks and not self.sm_budget       # nobody asked to leave SMs to other work
         self._timed("dispatch", stream, lambda: self.C.dispatch(lay, self.sessions, args, send, recv, self._stream(stream),
-                                                                self.local_direct, self._device_profile))
+                                                                self.local_direct, self._device_profile, whole))
         return outs
 
     def combine(self, xs: Sequence[torch.Tensor], plans: Sequence[RoutingPlan], ws: Sequence[Optional[torch.Tensor]],

@@ -67,6 +67,41 @@ def test_high_throughput_splits(world, tokens, hidden, experts, topk, kw):
     run_case(world, tokens, hidden, experts, topk, "invalid", repeats=2, **kw)
 
 
+@pytest.mark.parametrize("dmode", [0, 1, 2])
+@pytest.mark.parametrize("tokens,hidden,experts,topk,expand,alignment", [
+    (1, 128, 4, 1, True, 1), (9, 1152, 16, 2, True, 16), (70, 1024, 7, 7, True, 128), (33, 8192, 64, 16, True, 1),
+    (257, 2176, 48, 3, True, 1), (65, 4224, 32, 8, False, 1), (1, 128, 3, 3, False, 1)])
+def test_one_rank_with_and_without_a_budget_of_blocks(filled_outputs, tokens, hidden, experts, topk, expand, alignment, dmode):
+    """The kernels of one piece per warp (no budget) and those of a few persistent blocks give the same bits, rows, scales, zeroed
+    padding, sums, biases and values alike; empty and out-of-range slots among them."""
+    from deepep_b200.parallel.virtual import VirtualWorld
+    from deepep_b200.utils.math import per_token_cast_to_fp8
+
+    dev = torch.device("cuda")
+    x = torch.randn((tokens, hidden), generator=torch.Generator().manual_seed(3)).bfloat16()
+    idx = make_routes("empty" if tokens > 1 else "random", tokens, experts, topk, 1, 5)
+    idx[1::7] = experts + 3
+    w = make_weights(tokens, topk, 8).to(dev)
+    src = tuple(t.to(dev) for t in per_token_cast_to_fp8(x)) if dmode == 1 else x.to(dev)
+    bias = tuple(torch.randn((tokens, hidden), generator=torch.Generator().manual_seed(r)).bfloat16().to(dev) for r in (1, 2))
+    with VirtualWorld(1, tokens, hidden, topk, timeout=10.0) as vw:
+        eng = vw.engine
+        plan = eng.notify([idx.to(dev)], [w], experts, expand=expand, alignment=alignment)
+        got = [eng.dispatch([src], plan, dmode, blocks=blocks)[0] for blocks in (0, 5, 0)]
+        rows = torch.randn((plan[0].num_rows, hidden), generator=torch.Generator().manual_seed(4)).bfloat16().to(dev)
+        sums = []
+        for blocks in (0, 5, 0):
+            for b in (None, bias[0], bias):
+                sums += eng.combine([rows], plan, [plan[0].recv_w], bias=None if b is None else [b], blocks=blocks)
+            sums += eng.combine([rows], plan, [None], blocks=blocks)
+        torch.cuda.synchronize()
+        eng.check_status()
+    for out, sf in got[1:]:
+        assert bits_equal(out, got[0][0]) and (sf is None or bits_equal(sf, got[0][1]))
+    for i, (out, out_w) in enumerate(sums):
+        assert bits_equal(out, sums[i % 4][0]) and (out_w is None or bits_equal(out_w, sums[i % 4][1]))
+
+
 def _torch_activation(gate_up, grad):
     x = gate_up.detach().requires_grad_()
     gate, up = x.chunk(2, dim=-1)
