@@ -106,8 +106,9 @@ void op_dispatch(const WsLayout& lay, const std::vector<py::object>& sessions, c
 }
 
 void op_combine(const WsLayout& lay, const std::vector<py::object>& sessions, const std::vector<py::dict>& args, int send_blocks,
-                int recv_blocks, uintptr_t stream, bool local_direct, bool profile, int t_begin, int t_end) {
+                int recv_blocks, uintptr_t stream, bool local_direct, bool profile, int t_begin, int t_end, bool whole_gpu) {
   CombineParams p{};
+  p.whole_gpu = whole_gpu;
   p.lay = lay; p.send_blocks = send_blocks; p.recv_blocks = recv_blocks; p.local_direct = local_direct; p.profile = profile;
   p.t_begin = t_begin; p.t_end = t_end < 0 ? lay.max_tokens : t_end;
   if (p.t_begin < 0 || p.t_end < p.t_begin || p.t_end - p.t_begin > lay.partial_tokens)
@@ -124,7 +125,7 @@ void op_combine(const WsLayout& lay, const std::vector<py::object>& sessions, co
     a.x = ptr<const __nv_bfloat16>(d, "x"); a.w = ptr<const float>(d, "w");
     a.stage_meta = ptr<const int>(d, "stage_meta"); a.rank_rows = ptr<const int>(d, "rank_rows");
     a.rank_tokens = ptr<const int>(d, "rank_tokens"); a.send_slot = ptr<const int>(d, "send_slot");
-    a.topk_idx = ptr<const long long>(d, "topk_idx");
+    a.slot_row = ptr<const int>(d, "slot_row"); a.topk_idx = ptr<const long long>(d, "topk_idx");
     a.T = geti(d, "T"); a.meta_stride = geti(d, "meta_stride"); a.K = geti(d, "K"); a.E = geti(d, "E"); a.expand = geti(d, "expand", 1);
     a.x_rows = geti(d, "x_rows", 0);
     a.bias0 = ptr<const __nv_bfloat16>(d, "bias0"); a.bias1 = ptr<const __nv_bfloat16>(d, "bias1");
@@ -132,6 +133,7 @@ void op_combine(const WsLayout& lay, const std::vector<py::object>& sessions, co
     a.prof = ptr<unsigned long long>(d, "prof");
     if (!a.stage_meta || !a.rank_rows || !a.rank_tokens || !a.send_slot || ((!a.topk_idx || !a.out) && a.T > 0))
       throw std::invalid_argument("combine: a required pointer is missing");
+    if (whole_gpu && lay.world == 1 && a.expand && !a.slot_row && a.T > 0) throw std::invalid_argument("combine: slot_row is missing");
     if (a.E < a.ctx.world) throw std::invalid_argument("combine: num_experts is missing");
   }
   check(launch_combine(p, n, reinterpret_cast<cudaStream_t>(stream)), "ep_combine_ht launch");
@@ -247,7 +249,7 @@ PYBIND11_MODULE(_C, m) {
         py::arg("whole_gpu") = false);
   m.def("combine", &op_combine, py::arg("layout"), py::arg("sessions"), py::arg("args"), py::arg("send_blocks"),
         py::arg("recv_blocks"), py::arg("stream"), py::arg("local_direct") = true, py::arg("profile") = false,
-        py::arg("t_begin") = 0, py::arg("t_end") = -1);
+        py::arg("t_begin") = 0, py::arg("t_end") = -1, py::arg("whole_gpu") = false);
   m.attr("group_tokens") = kGroupTokens;
   m.attr("row_block") = kRowBlock;
   m.attr("dispatch_prof_words") = kDispatchProfWords;

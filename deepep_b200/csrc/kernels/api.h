@@ -94,6 +94,7 @@ struct CombineArgs {
   const int* rank_tokens;
   const int* rank_rows;        // [P + 1] exclusive prefix of the staged rows per source
   const int* send_slot;        // [T][P]
+  const int* slot_row;         // [T][K] as in DispatchArgs
   const long long* topk_idx;   // [T][K] of the source tokens (validity of returned weights)
   int T, meta_stride, K, E, expand, x_rows;   // x_rows: rows of x (only read by the optional index checks; 0 = unknown)
   const __nv_bfloat16* bias0;  // [T][H] or null
@@ -106,7 +107,7 @@ struct CombineArgs {
 // fp32), so no local partial is written and no flag is needed for it.
 // t_begin / t_end: the token window of this pass (all tokens unless the workspace holds the partials of fewer tokens than
 // num_max_tokens_per_rank: the combine then runs one launch per window, every rank with the same window).
-struct CombineParams { WsLayout lay; int send_blocks, recv_blocks, local_direct, profile; int t_begin, t_end; CombineArgs r[kMaxRanks]; };
+struct CombineParams { WsLayout lay; int send_blocks, recv_blocks, local_direct, profile, whole_gpu, pad, t_begin, t_end; CombineArgs r[kMaxRanks]; };
 // per block: role (0 expert side, 1 source side), start ns, end ns, then summed over the block's warps: cycles spent
 // reading routing records, waiting for flags, reducing rows, publishing flags; rows read
 constexpr int kCombineProfWords = 8;

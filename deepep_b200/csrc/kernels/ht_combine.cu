@@ -17,6 +17,8 @@
 // no gateway stage): same numeric contract (fp32 sum -> bf16 partial -> fp32 sum -> bf16), but no
 // entry/exit device barriers, no prepare kernel and no final device-to-device copy, because flags are
 // epochs and the output is written in place.
+#include <algorithm>
+
 #include "api.h"
 
 namespace dep {
@@ -408,8 +410,98 @@ __global__ void __launch_bounds__(kCombineThreads, 1) ep_combine_local_kernel(co
   clk.finish(a.prof ? a.prof + (size_t)blockIdx.x * kCombineProfWords : nullptr, 1);
 }
 
+// One rank without a budget of SMs: every warp takes U x 32 pieces of 16 bytes of one token and is done.  Memory bounds it, and
+// occupancy is what keeps memory busy: with few registers (B = 3 rows in flight, one piece per lane) an SM holds all its warps, and
+// the hardware deals blocks out as they finish.  Times in us right after a dispatch, kernel above / U = 1, B = 3 / U = 1, B = 8:
+// 4096 rows of 7168, top-8 97 / 89 / 94, 8192 of 4096, top-6 114 / 80 / 93, 1531 of 4096, top-6 28 / 20 / 22, 4096 of 4096,
+// top-2 37 / 24 / 36, top-16 123 / 99 / -.  With a single row per token U = 4, B = 1: rank layout, 2048 of 4096, 13.5 / 11.1 as
+// U = 1, B = 3 and 8.7; 4096 of 4096, top-1 30 / 20.5 and 17.2.
+constexpr int kLocalCombineThreads = 256;
+
+template <int U, int B>
+__global__ void __launch_bounds__(kLocalCombineThreads) ep_combine_items_kernel(const __grid_constant__ CombineParams p) {
+  const CombineArgs& a = p.r[0];
+  const int H = p.lay.hidden, K = a.K, lane = threadIdx.x & 31, units = H / 8;
+  const int spans = (units + 32 * U - 1) / (32 * U);
+  const int span_units = ((units + spans - 1) / spans + 31) / 32 * 32;
+  const int item = blockIdx.x * (kLocalCombineThreads / 32) + (threadIdx.x >> 5), t = p.t_begin + item / spans;
+  if (t >= min(a.T, p.t_end)) return;
+  const int u0 = item % spans * span_units, u_end = min(units, u0 + span_units);
+  // lane k: the row of slot k (rank layout: lane 0, the token's one row)
+  int row = -1;
+  if (a.expand) { if (lane < K) row = __ldg(a.slot_row + (size_t)t * K + lane); }
+  else if (lane == 0) row = __ldg(a.send_slot + t);
+  if (row >= 0 && a.x_rows > 0 && !DEP_INDEX_OK(a.ctx, row, a.x_rows, kOpCombine, 0)) row = 0;
+  const unsigned mask = __ballot_sync(0xffffffffu, row >= 0);
+  const int4* x = reinterpret_cast<const int4*>(a.x);
+  float sum[U][8];
+#pragma unroll
+  for (int i = 0; i < U; ++i)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) sum[i][e] = 0.f;
+  for (unsigned m = mask; m;) {          // B rows in flight, added in slot order
+    int4 v[B][U];
+    const int n = __popc(m);
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      if (q < n) {
+        const int4* src = x + (size_t)__shfl_sync(0xffffffffu, row, __ffs(m) - 1) * units;
+        m &= m - 1;
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+          const int u = u0 + i * 32 + lane;
+          if (u < u_end) v[q][i] = __ldg(src + u);
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      if (q < n) {
+#pragma unroll
+        for (int i = 0; i < U; ++i)
+          if (u0 + i * 32 + lane < u_end) add_bf16x8(sum[i], v[q][i]);
+      }
+    }
+  }
+  const int4* b0 = a.bias0 ? reinterpret_cast<const int4*>(a.bias0) + (size_t)t * units : nullptr;
+  const int4* b1 = a.bias1 ? reinterpret_cast<const int4*>(a.bias1) + (size_t)t * units : nullptr;
+#pragma unroll
+  for (int i = 0; i < U; ++i) {
+    const int u = u0 + i * 32 + lane;
+    if (u >= u_end) continue;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    add_bf16x8(acc, pack_bf16x8(sum[i]));               // the sum joins rounded to bf16, like a partial from a peer
+    if (b0) add_bf16x8(acc, __ldg(b0 + u));
+    if (b1) add_bf16x8(acc, __ldg(b1 + u));
+    reinterpret_cast<int4*>(a.out)[(size_t)t * units + u] = pack_bf16x8(acc);
+  }
+  if (a.out_w && u0 == 0) {      // the value channel: zero for empty and repeated slots
+    float value = 0.f;
+    if (a.expand) {
+      if (row >= 0 && a.w) value = __ldg(a.w + row);
+    } else {
+      const long long v = lane < K ? __ldg(a.topk_idx + (size_t)t * K + lane) : -1;
+      const int e = (v < 0 || v >= a.E) ? -1 : (int)v, row0 = __shfl_sync(0xffffffffu, row, 0);
+      const unsigned same = __match_any_sync(0xffffffffu, e);
+      if (e >= 0 && (same & ((1u << lane) - 1u)) == 0 && row0 >= 0 && a.w) value = __ldg(a.w + (size_t)row0 * K + lane);
+    }
+    if (lane < K) a.out_w[(size_t)t * K + lane] = value;
+  }
+}
+
+template <int U, int B>
+cudaError_t launch_items(const CombineParams& p, cudaStream_t stream) {
+  const int spans = (p.lay.hidden / 8 + 32 * U - 1) / (32 * U), per = kLocalCombineThreads / 32;
+  const long long items = (long long)std::max(0, std::min(p.r[0].T, p.t_end) - p.t_begin) * spans;
+  if (items == 0) return cudaSuccess;
+  ep_combine_items_kernel<U, B><<<(unsigned)((items + per - 1) / per), kLocalCombineThreads, 0, stream>>>(p);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_combine(const CombineParams& p, int nranks, cudaStream_t stream) {
   if (p.lay.world == 1 && p.local_direct && nranks == 1) {
+    if (p.whole_gpu && !p.profile)      // one row per token: nothing to sum, a wide piece keeps enough loads in flight
+      return p.r[0].expand && p.r[0].K > 1 ? launch_items<1, 3>(p, stream) : launch_items<4, 1>(p, stream);
     const int blocks = p.send_blocks + p.recv_blocks;
     if (p.profile) ep_combine_local_kernel<true><<<blocks, kCombineThreads, 0, stream>>>(p);
     else ep_combine_local_kernel<false><<<blocks, kCombineThreads, 0, stream>>>(p);

@@ -378,7 +378,8 @@ class CudaEngine:
             args.append(dict(x=xs[i].data_ptr(), w=_ptr(ws[i]), stage_meta=plan.stage_meta.data_ptr(),
                              rank_rows=plan.rank_rows.data_ptr(), rank_tokens=plan.rank_tokens.data_ptr(),
                              prof=self._prof_buffer("combine", i),
-                             send_slot=plan.send_slot.data_ptr(), topk_idx=plan.topk_idx.data_ptr(), T=T,
+                             send_slot=plan.send_slot.data_ptr(), slot_row=plan.slot_row.data_ptr(),
+                             topk_idx=plan.topk_idx.data_ptr(), T=T,
                              meta_stride=plan.meta_stride, K=K, E=plan.num_experts, expand=int(plan.expand),
                              bias0=_ptr(b0), bias1=_ptr(b1), out=out.data_ptr(), out_w=_ptr(out_w), x_rows=xs[i].shape[0]))
         send, recv = self.split_blocks(blocks, self.combine_send_fraction, self.combine_blocks)
@@ -387,13 +388,14 @@ class CudaEngine:
             send, recv = max(1, int(split[0])), max(1, int(split[1]))
             if send + recv > limit:
                 raise ValueError(f"combine_num_sms + reduce_num_sms must not exceed {limit} on this device")
+        whole = split is None and not blocks and not self.sm_budget
         # one launch per token window: all tokens at once unless the workspace holds the partials of fewer tokens
         window, most = lay.partial_tokens, max([plan.num_tokens for plan in plans] + [1])
         if self.n == 1 and self.world > 1 and window < lay.max_tokens:
             most = lay.max_tokens         # real ranks cannot see each other's token counts: every rank runs every pass
         for begin in range(0, most, window):
             self._timed("combine", stream, lambda b=begin: self.C.combine(lay, self.sessions, args, send, recv, self._stream(stream),
-                                                                          self.local_direct, self._device_profile, b, b + window))
+                                                                          self.local_direct, self._device_profile, b, b + window, whole))
         return outs
 
     # ------------------------------------------------------------------ low latency
