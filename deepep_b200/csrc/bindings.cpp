@@ -69,9 +69,8 @@ void op_notify(const WsLayout& lay, const std::vector<py::object>& sessions, con
 }
 
 void op_dispatch(const WsLayout& lay, const std::vector<py::object>& sessions, const std::vector<py::dict>& args, int send_blocks,
-                 int recv_blocks, uintptr_t stream, bool local_direct, bool profile, bool whole_gpu) {
+                 int recv_blocks, uintptr_t stream, bool local_direct, bool profile) {
   DispatchParams p{};
-  p.whole_gpu = whole_gpu;
   p.lay = lay; p.send_blocks = send_blocks; p.recv_blocks = recv_blocks; p.local_direct = local_direct; p.profile = profile;
   const int n = (int)args.size();
   if (n < 1 || n > kMaxRanks || (int)sessions.size() != n) throw std::invalid_argument("1..8 rank argument blocks expected");
@@ -90,6 +89,7 @@ void op_dispatch(const WsLayout& lay, const std::vector<py::object>& sessions, c
     a.meta_stride = geti(d, "meta_stride");
     a.K = geti(d, "K"); a.E = geti(d, "E"); a.expand = geti(d, "expand", 1);
     a.recv_rows = geti(d, "recv_rows", 0);
+    p.whole_gpu = geti(d, "whole", 0);
     a.pad_counts = ptr<const int>(d, "pad_counts"); a.pad_offsets = ptr<const int>(d, "pad_offsets");
     if (!a.pad_counts != !a.pad_offsets || (a.pad_offsets && a.E < a.ctx.world)) throw std::invalid_argument("dispatch: padding needs the expert counts, offsets and E");
     a.recv_x = ptr<void>(d, "recv_x"); a.recv_sf = ptr<float>(d, "recv_sf");
@@ -106,9 +106,8 @@ void op_dispatch(const WsLayout& lay, const std::vector<py::object>& sessions, c
 }
 
 void op_combine(const WsLayout& lay, const std::vector<py::object>& sessions, const std::vector<py::dict>& args, int send_blocks,
-                int recv_blocks, uintptr_t stream, bool local_direct, bool profile, int t_begin, int t_end, bool whole_gpu) {
+                int recv_blocks, uintptr_t stream, bool local_direct, bool profile, int t_begin, int t_end) {
   CombineParams p{};
-  p.whole_gpu = whole_gpu;
   p.lay = lay; p.send_blocks = send_blocks; p.recv_blocks = recv_blocks; p.local_direct = local_direct; p.profile = profile;
   p.t_begin = t_begin; p.t_end = t_end < 0 ? lay.max_tokens : t_end;
   if (p.t_begin < 0 || p.t_end < p.t_begin || p.t_end - p.t_begin > lay.partial_tokens)
@@ -128,12 +127,13 @@ void op_combine(const WsLayout& lay, const std::vector<py::object>& sessions, co
     a.slot_row = ptr<const int>(d, "slot_row"); a.topk_idx = ptr<const long long>(d, "topk_idx");
     a.T = geti(d, "T"); a.meta_stride = geti(d, "meta_stride"); a.K = geti(d, "K"); a.E = geti(d, "E"); a.expand = geti(d, "expand", 1);
     a.x_rows = geti(d, "x_rows", 0);
+    p.whole_gpu = geti(d, "whole", 0);
     a.bias0 = ptr<const __nv_bfloat16>(d, "bias0"); a.bias1 = ptr<const __nv_bfloat16>(d, "bias1");
     a.out = ptr<__nv_bfloat16>(d, "out"); a.out_w = ptr<float>(d, "out_w");
     a.prof = ptr<unsigned long long>(d, "prof");
     if (!a.stage_meta || !a.rank_rows || !a.rank_tokens || !a.send_slot || ((!a.topk_idx || !a.out) && a.T > 0))
       throw std::invalid_argument("combine: a required pointer is missing");
-    if (whole_gpu && lay.world == 1 && a.expand && !a.slot_row && a.T > 0) throw std::invalid_argument("combine: slot_row is missing");
+    if (p.whole_gpu && lay.world == 1 && a.expand && !a.slot_row && a.T > 0) throw std::invalid_argument("combine: slot_row is missing");
     if (a.E < a.ctx.world) throw std::invalid_argument("combine: num_experts is missing");
   }
   check(launch_combine(p, n, reinterpret_cast<cudaStream_t>(stream)), "ep_combine_ht launch");
@@ -245,11 +245,10 @@ PYBIND11_MODULE(_C, m) {
   m.def("notify", &op_notify, py::arg("layout"), py::arg("sessions"), py::arg("args"), py::arg("blocks"), py::arg("stream"),
         py::arg("profile") = false);
   m.def("dispatch", &op_dispatch, py::arg("layout"), py::arg("sessions"), py::arg("args"), py::arg("send_blocks"),
-        py::arg("recv_blocks"), py::arg("stream"), py::arg("local_direct") = true, py::arg("profile") = false,
-        py::arg("whole_gpu") = false);
+        py::arg("recv_blocks"), py::arg("stream"), py::arg("local_direct") = true, py::arg("profile") = false);
   m.def("combine", &op_combine, py::arg("layout"), py::arg("sessions"), py::arg("args"), py::arg("send_blocks"),
         py::arg("recv_blocks"), py::arg("stream"), py::arg("local_direct") = true, py::arg("profile") = false,
-        py::arg("t_begin") = 0, py::arg("t_end") = -1, py::arg("whole_gpu") = false);
+        py::arg("t_begin") = 0, py::arg("t_end") = -1);
   m.attr("group_tokens") = kGroupTokens;
   m.attr("row_block") = kRowBlock;
   m.attr("dispatch_prof_words") = kDispatchProfWords;

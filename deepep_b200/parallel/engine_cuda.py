@@ -99,6 +99,8 @@ COMBINE_SEND_FRACTION = {1: 0.0, 2: 0.5, 4: 0.6, 8: 0.6}
 
 
 class CudaEngine:
+    sm_budget = 0          # SMs that the dispatch and combine kernels stay within (0: no limit asked for)
+
     def __init__(self, sessions: Sequence, layout, device: torch.device, num_sms: int = 0, host_timeout: float = 300.0):
         self.C = require_native("ElasticBuffer")
         self.host_timeout = float(host_timeout)       # limit of the host's waits for a kernel whose results it reads back
@@ -335,6 +337,7 @@ class CudaEngine:
         ``split`` = (sender blocks, receiver blocks) overrides the default division."""
         lay, dev = self.layout, self.device
         H = lay.hidden
+        whole = split is None and not blocks and not self.sm_budget       # nobody asked to leave SMs to other work
         outs, args = [], []
         for i, plan in enumerate(plans):
             x, sf = (xs[i] if isinstance(xs[i], (tuple, list)) else (xs[i], None))
@@ -355,11 +358,10 @@ class CudaEngine:
                              recv_x=recv_x.data_ptr(), recv_sf=_ptr(recv_sf), recv_rows=recv_x.shape[0],
                              pad_counts=plan.expert_counts.data_ptr() if padded else None,
                              pad_offsets=plan.expert_offsets.data_ptr() if padded else None,
-                             prof=self._prof_buffer("dispatch", i)))
+                             prof=self._prof_buffer("dispatch", i), whole=int(whole)))
         send, recv = split if split is not None else self.split_blocks(blocks, self.dispatch_send_fraction, self.dispatch_blocks)
-        whole = split is None and not blocks and not self.sm_budget       # nobody asked to leave SMs to other work
         self._timed("dispatch", stream, lambda: self.C.dispatch(lay, self.sessions, args, send, recv, self._stream(stream),
-                                                                self.local_direct, self._device_profile, whole))
+                                                                self.local_direct, self._device_profile))
         return outs
 
     def combine(self, xs: Sequence[torch.Tensor], plans: Sequence[RoutingPlan], ws: Sequence[Optional[torch.Tensor]],
@@ -367,6 +369,7 @@ class CudaEngine:
         """``split`` = (expert-side sender blocks, source-side reducer blocks) overrides the default division."""
         lay, dev = self.layout, self.device
         H, K = lay.hidden, lay.topk
+        whole = split is None and not blocks and not self.sm_budget
         outs, args = [], []
         for i, plan in enumerate(plans):
             T = plan.num_tokens
@@ -378,24 +381,24 @@ class CudaEngine:
             args.append(dict(x=xs[i].data_ptr(), w=_ptr(ws[i]), stage_meta=plan.stage_meta.data_ptr(),
                              rank_rows=plan.rank_rows.data_ptr(), rank_tokens=plan.rank_tokens.data_ptr(),
                              prof=self._prof_buffer("combine", i),
-                             send_slot=plan.send_slot.data_ptr(), slot_row=plan.slot_row.data_ptr(),
+                             send_slot=plan.send_slot.data_ptr(), slot_row=plan.slot_row.data_ptr() if self.world == 1 else None,
                              topk_idx=plan.topk_idx.data_ptr(), T=T,
                              meta_stride=plan.meta_stride, K=K, E=plan.num_experts, expand=int(plan.expand),
-                             bias0=_ptr(b0), bias1=_ptr(b1), out=out.data_ptr(), out_w=_ptr(out_w), x_rows=xs[i].shape[0]))
+                             bias0=_ptr(b0), bias1=_ptr(b1), out=out.data_ptr(), out_w=_ptr(out_w), x_rows=xs[i].shape[0],
+                             whole=int(whole)))
         send, recv = self.split_blocks(blocks, self.combine_send_fraction, self.combine_blocks)
         if split is not None:
             limit = max(2, self.sm_count // self.n)
             send, recv = max(1, int(split[0])), max(1, int(split[1]))
             if send + recv > limit:
                 raise ValueError(f"combine_num_sms + reduce_num_sms must not exceed {limit} on this device")
-        whole = split is None and not blocks and not self.sm_budget
         # one launch per token window: all tokens at once unless the workspace holds the partials of fewer tokens
         window, most = lay.partial_tokens, max([plan.num_tokens for plan in plans] + [1])
         if self.n == 1 and self.world > 1 and window < lay.max_tokens:
             most = lay.max_tokens         # real ranks cannot see each other's token counts: every rank runs every pass
         for begin in range(0, most, window):
             self._timed("combine", stream, lambda b=begin: self.C.combine(lay, self.sessions, args, send, recv, self._stream(stream),
-                                                                          self.local_direct, self._device_profile, b, b + window, whole))
+                                                                          self.local_direct, self._device_profile, b, b + window))
         return outs
 
     # ------------------------------------------------------------------ low latency
