@@ -13,9 +13,12 @@
 //
 // The pass moves next to nothing; a chain of short phases between grid barriers bounds it, so each phase is cut over all
 // threads: one thread per (token, slot) reads a tile's ids once into shared memory, and the same tile serves the counts
-// and the records when every block has one.  One GPU, 1531 x 6 routes over 64 experts: 37.7 us with one thread per token,
-// 20.9 us since; 4096 x 8 over 256 experts in blocks of 128 rows: 78.9 us (one block wrote all padding marks), 26.9 us.
+// and the records when every block has one.  One rank on one GPU, before it had a kernel of its own, 1531 x 6 routes over 64
+// experts: 37.7 us with one thread per token, 20.9 us since; 4096 x 8 over 256 experts in blocks of 128 rows: 78.9 us (one block
+// wrote all padding marks), 26.9 us.
 #include <cooperative_groups.h>
+
+#include <algorithm>
 
 #include "api.h"
 
@@ -103,48 +106,41 @@ __global__ void __launch_bounds__(kNotifyThreads) ep_notify_kernel(const __grid_
   };
 
   // ---- A: publish my routing table into every peer (after they consumed the previous one).  My own tokens are read from
-  // the caller's tensors, so a single rank skips this phase and its grid barrier.
-  int alive = 1;
-  if (P > 1) {
-    int ok = 1;
-    if (threadIdx.x < P) ok = wait_flag_ge(&ctl->notify_ack[threadIdx.x], epoch - 1, ctx, kOpNotify, 0, threadIdx.x);
-    alive = __syncthreads_and(ok);
-    if (alive) {
-      const int n = a.T * K;
-      for (int i = gtid; i < (P - 1) * n; i += gstride) {
-        const int q = i / n, j = i - q * n, d = (me + 1 + q) % P;
-        long long v = a.topk_idx[j];
-        int e = (v < 0 || v >= E) ? -1 : (int)v;
-        reinterpret_cast<int*>(ctx.ws[d] + lay.gather_idx)[(size_t)me * Tmax * K + j] = e;
-        if (a.topk_w) reinterpret_cast<float*>(ctx.ws[d] + lay.gather_w)[(size_t)me * Tmax * K + j] = a.topk_w[j];
-      }
-      if (blockIdx.x == 0 && threadIdx.x < P) {
-        int* hdr = reinterpret_cast<int*>(ctx.ws[threadIdx.x] + lay.gather_hdr) + me * 4;
-        hdr[0] = a.T;
-        hdr[1] = a.topk_w != nullptr;
-      }
-      __threadfence_system();
+  // the caller's tensors.
+  int ok = 1;
+  if (threadIdx.x < P) ok = wait_flag_ge(&ctl->notify_ack[threadIdx.x], epoch - 1, ctx, kOpNotify, 0, threadIdx.x);
+  int alive = __syncthreads_and(ok);
+  if (alive) {
+    const int n = a.T * K;
+    for (int i = gtid; i < (P - 1) * n; i += gstride) {
+      const int q = i / n, j = i - q * n, d = (me + 1 + q) % P;
+      long long v = a.topk_idx[j];
+      int e = (v < 0 || v >= E) ? -1 : (int)v;
+      reinterpret_cast<int*>(ctx.ws[d] + lay.gather_idx)[(size_t)me * Tmax * K + j] = e;
+      if (a.topk_w) reinterpret_cast<float*>(ctx.ws[d] + lay.gather_w)[(size_t)me * Tmax * K + j] = a.topk_w[j];
     }
-    grid.sync();
-    if (alive && blockIdx.x == 0 && threadIdx.x < P)
-      st_release_sys(&control_of(ctx.ws[threadIdx.x])->notify_ready[me], epoch);
+    if (blockIdx.x == 0 && threadIdx.x < P) {
+      int* hdr = reinterpret_cast<int*>(ctx.ws[threadIdx.x] + lay.gather_hdr) + me * 4;
+      hdr[0] = a.T;
+      hdr[1] = a.topk_w != nullptr;
+    }
+    __threadfence_system();
   }
+  grid.sync();
+  if (alive && blockIdx.x == 0 && threadIdx.x < P)
+    st_release_sys(&control_of(ctx.ws[threadIdx.x])->notify_ready[me], epoch);
 
   stamp(0);
   // ---- B: wait for every rank's table
   const int* ghdr = reinterpret_cast<const int*>(ws + lay.gather_hdr);
   const int* gidx = reinterpret_cast<const int*>(ws + lay.gather_idx);
   const float* gw = reinterpret_cast<const float*>(ws + lay.gather_w);
-  if (P > 1) {
-    int ok = 1;
-    if (alive && threadIdx.x < P) ok = wait_flag_ge(&ctl->notify_ready[threadIdx.x], epoch, ctx, kOpNotify, 1, threadIdx.x);
-    alive = __syncthreads_and(ok) && alive;
-    if (threadIdx.x < kMaxRanks) s_T[threadIdx.x] = (alive && threadIdx.x < P) ? __ldcg(ghdr + threadIdx.x * 4) : 0;
-  } else if (threadIdx.x < kMaxRanks) {
-    s_T[threadIdx.x] = threadIdx.x == 0 ? a.T : 0;
-  }
+  ok = 1;
+  if (alive && threadIdx.x < P) ok = wait_flag_ge(&ctl->notify_ready[threadIdx.x], epoch, ctx, kOpNotify, 1, threadIdx.x);
+  alive = __syncthreads_and(ok) && alive;
+  if (threadIdx.x < kMaxRanks) s_T[threadIdx.x] = (alive && threadIdx.x < P) ? __ldcg(ghdr + threadIdx.x * 4) : 0;
   __syncthreads();
-  const bool has_w = alive && a.recv_w != nullptr && (P > 1 ? __ldcg(ghdr + 1) != 0 : a.topk_w != nullptr);
+  const bool has_w = alive && a.recv_w != nullptr && __ldcg(ghdr + 1) != 0;
   // the ids and weights of source r: this rank's own come from the caller's tensors
   auto own_ids = [&](int r) { return r == me ? a.topk_idx : nullptr; };
   auto weight_of = [&](int r, int i) {
@@ -169,7 +165,7 @@ __global__ void __launch_bounds__(kNotifyThreads) ep_notify_kernel(const __grid_
   }
   grid.sync();
   // a block whose wait ran out has counted nothing: all blocks give up together and leave an empty plan
-  if (P > 1 && __syncthreads_or(threadIdx.x == 0 && ld_volatile_int(&ctl->abort))) {
+  if (__syncthreads_or(threadIdx.x == 0 && ld_volatile_int(&ctl->abort))) {
     alive = 0;
     if (threadIdx.x < kMaxRanks) s_T[threadIdx.x] = 0;
     __syncthreads();
@@ -363,7 +359,260 @@ __global__ void __launch_bounds__(kNotifyThreads) ep_notify_kernel(const __grid_
   }
 }
 
+// ------------------------------------------------------------------------------------------ one rank
+// The same plan for a single rank, by clusters of 16 CTAs.  There is no table to exchange, so what is left is a chain of short steps
+// over the own table; the CTAs of a cluster pass their counts through distributed shared memory and meet at cluster barriers, and the
+// launch need not be cooperative.  Each CTA owns a range of tokens (whole 64-token tiles), keeps its ids and one bit per (expert,
+// token) in shared memory from the first step to the last, and no count passes through memory.  Sixteen SMs would write the records
+// of a large table slowly, so several clusters do the first steps alike and each writes its share of every range: clusters never wait
+// for one another.  Kernel times as one grid of 128 cooperative blocks (the kernel above) and here: 1531 x 6 routes over 64 experts 20.9
+// and 8.0 us, 4096 x 8 over 256 22.7 and 10.6 (13.2 with one cluster), in blocks of 128 rows 26.3 and 10.8, 16384 x 8 over 64 34.9 and
+// 16.3 (26.5 with one), 16384 x 16 over 1024 72 and 35 (60 with one, 50 with eight).
+constexpr int kLocalNotifyThreads = 1024;
+constexpr int kLocalNotifyCtas = 16;       // largest cluster of this device class
+constexpr int kLocalNotifyClusters = 4;    // at most, one per 16384 slots: eight do not all fit the GPU at once
+constexpr unsigned kRepeated = 1u << 31;   // in LocalTile::valid: two slots of the token name one expert
+
+// Shared memory of a CTA that owns `per` tokens.
+struct LocalTile {
+  unsigned* mask;      // [E][stride]: tokens of the expert, `stride` odd so that a column of it meets all banks
+  unsigned* hit;       // [words]: tokens with at least one slot that counts
+  int* cnt;            // [E + 1]: tokens per expert of this CTA, then tokens with a hit (read by the other CTAs)
+  int* tot;            // [E] rows of the expert
+  int* off;            // [E + 1] first row of the expert
+  int* base;           // [E] first row of this CTA's tokens
+  unsigned* valid;     // [per] bit k: slot k counts
+  short* id;           // [per][K], -1: no expert
+  __host__ __device__ static int stride(int per) { return per / 32 | 1; }
+  __host__ __device__ static size_t bytes(int per, int E, int K) {
+    return 4 * ((size_t)E * stride(per) + per / 32 + 4 * E + 2 + per) + 2 * (size_t)per * K;
+  }
+  __device__ LocalTile(void* smem, int per, int E) {
+    mask = reinterpret_cast<unsigned*>(smem);
+    hit = mask + (size_t)E * stride(per);
+    cnt = reinterpret_cast<int*>(hit + per / 32);
+    tot = cnt + E + 1; off = tot + E; base = off + E + 1;
+    valid = reinterpret_cast<unsigned*>(base + E);
+    id = reinterpret_cast<short*>(valid + per);
+  }
+};
+__host__ __device__ inline int local_tokens(int T, int ctas) {          // tokens per CTA: whole tiles
+  const int tiles = (T + kChunkTokens - 1) / kChunkTokens;
+  return (tiles > ctas ? (tiles + ctas - 1) / ctas : 1) * kChunkTokens;
+}
+__device__ __forceinline__ int below_words(const unsigned* m, int t) {   // bits of m below bit t
+  int n = 0;
+  for (int w = 0; w < t >> 5; ++w) n += __popc(m[w]);
+  return n + ((t & 31) ? __popc(m[t >> 5] & ((1u << (t & 31)) - 1u)) : 0);
+}
+
+template <bool kProfile>
+__global__ void __launch_bounds__(kLocalNotifyThreads) ep_notify_local_kernel(const __grid_constant__ NotifyParams p) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const NotifyArgs& a = p.r[0];
+  constexpr int C = kLocalNotifyCtas;
+  const int c = blockIdx.x % C, share = blockIdx.x / C, shares = gridDim.x / C;
+  const int T = a.T, K = a.K, E = a.E, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int per = local_tokens(T, C), words = per / 32, stride = LocalTile::stride(per);
+  const int t0 = min(T, c * per), live = min(per, T - t0), n = live * K;
+  const int NT = (p.lay.max_tokens + kChunkTokens - 1) / kChunkTokens;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const LocalTile s(smem, per, E);
+  __shared__ int s_warp[kLocalNotifyThreads / 32];
+  __shared__ int s_hits[2];                              // tokens with a hit: before this CTA, of all CTAs
+  Control* ctl = control_of(a.ctx.ws[0]);
+  unsigned long long t_start = 0;
+  if constexpr (kProfile) t_start = global_timer_ns();
+  auto stamp = [&](int i) {
+    if constexpr (kProfile)
+      if (blockIdx.x == 0 && tid == 0) ctl->dbg[16 + i] = global_timer_ns() - t_start;
+  };
+
+  // ---- the ids, and which tokens every expert gets
+  for (int i0 = tid; i0 < n; i0 += kLocalNotifyThreads * 4) {
+    long long v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = i0 + j * kLocalNotifyThreads < n ? __ldg(a.topk_idx + (size_t)t0 * K + i0 + j * kLocalNotifyThreads) : -1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + j * kLocalNotifyThreads < n) s.id[i0 + j * kLocalNotifyThreads] = (short)((v[j] < 0 || v[j] >= E) ? -1 : (int)v[j]);
+  }
+  for (int i = tid; i < E * stride; i += kLocalNotifyThreads) s.mask[i] = 0u;
+  for (int i = tid; i < words; i += kLocalNotifyThreads) s.hit[i] = 0u;
+  for (int i = tid; i < per; i += kLocalNotifyThreads) s.valid[i] = 0u;
+  stamp(0);
+  __syncthreads();
+  stamp(1);
+  for (int i = tid; i < n; i += kLocalNotifyThreads) {
+    const int tl = i / K, k = i - tl * K, e = s.id[i];
+    if (e < 0) continue;
+    const unsigned bit = 1u << (tl & 31);
+    const bool again = atomicOr(&s.mask[e * stride + (tl >> 5)], bit) & bit;
+    atomicOr(&s.valid[tl], 1u << k | (again ? kRepeated : 0u));
+  }
+  __syncthreads();
+  for (int i = tid; i < per; i += kLocalNotifyThreads) {          // per is a multiple of 64: whole warps
+    unsigned valid = s.valid[i];
+    if (valid & kRepeated) {                                      // only the first of a token's slots with one expert counts
+      valid &= ~kRepeated;
+      for (int k = 1; k < K; ++k)
+        for (int j = 0; j < k; ++j)
+          if (s.id[i * K + j] == s.id[i * K + k]) valid &= ~(1u << k);
+      s.valid[i] = valid;
+    }
+    const unsigned word = __ballot_sync(0xffffffffu, valid != 0u);
+    if (lane == 0) s.hit[i >> 5] = word;
+  }
+  for (int e = tid; e < E; e += kLocalNotifyThreads) {
+    int v = 0;
+    for (int w = 0; w < words; ++w) v += __popc(s.mask[e * stride + w]);
+    s.cnt[e] = v;
+  }
+  __syncthreads();
+  if (tid == 0) s.cnt[E] = below_words(s.hit, per - 1) + (int)(s.hit[words - 1] >> 31);
+  cluster.sync();
+  stamp(2);
+
+  // ---- rows of every expert, the blocks' first rows, and this CTA's first row in each
+  int before = 0, tot = 0;
+  if (tid <= E) {
+    int v[C];
+#pragma unroll
+    for (int r = 0; r < C; ++r) v[r] = cluster.map_shared_rank(s.cnt, r)[tid];
+#pragma unroll
+    for (int r = 0; r < C; ++r) {
+      if (r < c) before += v[r];
+      tot += v[r];
+    }
+  }
+  if (tid == E) { s_hits[0] = before; s_hits[1] = tot; }
+  if (E == kLocalNotifyThreads && warp == 0) {                     // no thread is left for the hits
+    int b = 0, v = lane < C ? cluster.map_shared_rank(s.cnt, lane)[E] : 0;
+    b = lane < c ? v : 0;
+    for (int d = 16; d > 0; d >>= 1) { b += __shfl_xor_sync(0xffffffffu, b, d); v += __shfl_xor_sync(0xffffffffu, v, d); }
+    if (lane == 0) { s_hits[0] = b; s_hits[1] = v; }
+  }
+  const int rows = tid < E ? (a.expand ? (tot + a.alignment - 1) / a.alignment * a.alignment : tot) : 0;
+  int incl = rows;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += o;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  int warps = lane < warp ? s_warp[lane] : 0;                      // rows of the experts of the warps before this one
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) warps += __shfl_xor_sync(0xffffffffu, warps, d);
+  const int first = warps + incl - rows;
+  if (tid < E) {
+    s.tot[tid] = tot; s.off[tid] = first; s.base[tid] = first + before;
+    if (tid == E - 1) s.off[E] = first + rows;
+    if (blockIdx.x == 0) {
+      a.expert_counts[tid] = tot; a.expert_offsets[tid] = first;
+      if (a.mailbox) a.mailbox[4 + tid] = tot;
+    }
+  }
+  __syncthreads();
+  const int hits_before = s_hits[0], hits = s_hits[1], all_rows = a.expand ? s.off[E] : hits;
+  if (blockIdx.x == 0) {
+    if (tid == 0) {
+      if (a.mailbox) { a.mailbox[0] = all_rows; a.mailbox[1] = hits; a.mailbox[2] = T; }
+      a.expert_offsets[E] = s.off[E];
+      a.rank_rows[0] = 0; a.rank_rows[1] = hits; a.rank_tokens[0] = T;
+      if (a.rank_matrix) a.rank_matrix[0] = hits;
+    }
+    const int nt = (T + kChunkTokens - 1) / kChunkTokens;
+    for (int i = nt + tid; i <= NT; i += kLocalNotifyThreads) a.chunk_start[i] = hits;
+    // The epoch word tells a host that polls it that the counts are there; the records are complete when the launch is.  The fence
+    // takes 2 us, which the others spend on the records.
+    __syncthreads();
+    if (tid == kLocalNotifyThreads - 1) {
+      const unsigned long long epoch = ctl->epoch[kOpNotify] + 1;
+      ctl->notify_ack[0] = epoch;
+      ctl->epoch[kOpNotify] = epoch;
+      if (a.mailbox) {
+        __threadfence_system();
+        a.mailbox[3] = (int)(epoch & 0x7fffffff);
+      }
+    }
+  }
+  stamp(3);
+
+  // ---- padding rows carry no source; the experts are dealt out to the CTAs
+  const bool has_w = a.recv_w != nullptr && a.topk_w != nullptr;
+  if (a.expand && a.alignment > 1)
+    for (int e = warp * (int)gridDim.x + blockIdx.x; e < E; e += gridDim.x * (kLocalNotifyThreads / 32))
+      for (int row = s.off[e] + s.tot[e] + lane; row < s.off[e + 1] && row < a.rcap; row += 32) {
+        a.recv_row_src[row] = -1;
+        if (a.recv_w) a.recv_w[row] = 0.f;
+      }
+
+  // ---- per-token records of this cluster's share, one thread per (token, slot)
+  const int tokens = (live + shares - 1) / shares, first_token = min(live, share * tokens), last_token = min(live, first_token + tokens);
+  for (int i = first_token * K + tid; i < last_token * K; i += kLocalNotifyThreads) {
+    const int tl = i / K, k = i - tl * K, e = s.id[i];
+    const unsigned valid = s.valid[tl];
+    const bool counts = (valid >> k) & 1u;
+    const int row = a.expand && counts ? s.base[e] + below_words(s.mask + e * stride, tl) : -1;
+    a.slot_row[(size_t)t0 * K + i] = row;
+    if (valid == 0) continue;
+    const int j = hits_before + below_words(s.hit, tl);
+    const float w = has_w && counts ? __ldg(a.topk_w + (size_t)t0 * K + i) : 0.f;
+    if (a.expand) {
+      if (!counts) continue;
+      a.stage_meta[(size_t)j * a.meta_stride + 2 + __popc(valid & ((1u << k) - 1u))] = row | (k << kRowSlotShift);
+      if (row < a.rcap) {
+        a.recv_row_src[row] = t0 * K + i;
+        if (a.recv_w) a.recv_w[row] = w;
+      }
+    } else if (j < a.rcap) {
+      if (k == 0) a.recv_row_src[j] = (t0 + tl) * K;
+      if (a.recv_idx) a.recv_idx[(size_t)j * K + k] = counts ? e : -1;
+      if (a.recv_w) a.recv_w[(size_t)j * K + k] = w;
+    }
+  }
+  for (int tl = first_token + tid; tl < last_token; tl += kLocalNotifyThreads) {
+    const unsigned valid = s.valid[tl];
+    const int j = hits_before + below_words(s.hit, tl);
+    a.send_slot[t0 + tl] = valid ? j : -1;
+    if (tl % kChunkTokens == 0) {
+      a.chunk_start[(t0 + tl) / kChunkTokens] = j;
+      a.own_hits[(t0 + tl) / kChunkTokens] = j;
+    }
+    if (valid == 0) continue;
+    int* rec = a.stage_meta + (size_t)j * a.meta_stride;
+    rec[0] = t0 + tl;
+    rec[1] = a.expand ? __popc(valid) : 1;
+    if (!a.expand) { rec[2] = j; rec[3] = (int)valid; }
+  }
+  stamp(4);
+  cluster.sync();           // nobody reads another CTA's counts any more
+  stamp(5);
+}
+
+static cudaError_t launch_notify_local(const NotifyParams& p, cudaStream_t stream) {
+  const NotifyArgs& a = p.r[0];
+  const void* fn = p.profile ? (const void*)ep_notify_local_kernel<true> : (const void*)ep_notify_local_kernel<false>;
+  const int ctas = kLocalNotifyCtas;
+  const size_t smem = LocalTile::bytes(local_tokens(a.T, ctas), a.E, a.K);
+  const int clusters = std::max(1, std::min(kLocalNotifyClusters, (a.T * a.K + ctas * kLocalNotifyThreads - 1) / (ctas * kLocalNotifyThreads)));
+  // attributes belong to the current device, so they are set on every launch (a process may drive several GPUs)
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess && smem > 48 * 1024) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas * clusters); cfg.blockDim = dim3(kLocalNotifyThreads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = ctas; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  void* args[] = {const_cast<NotifyParams*>(&p)};
+  return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 cudaError_t launch_notify(const NotifyParams& p, int nranks, int blocks, cudaStream_t stream) {
+  if (p.lay.world == 1 && nranks == 1) return launch_notify_local(p, stream);
   for (int i = 0; i < nranks; ++i) {
     const NotifyArgs& a = p.r[i];
     if (!a.rank_matrix) continue;

@@ -16,14 +16,8 @@ constexpr int kMaxTokens = DEEPEP_NOALLOC_MAX_TOKENS;
 constexpr int kTiles = kMaxTokens / kChunkTokens;
 
 // Layout of the scratch array (byte offsets).  The first part plays the role of a one-rank workspace.
-constexpr long long kOffHdr = kControlBytes;
-constexpr long long kOffIdx = kOffHdr + 1024;
-constexpr long long kOffW = kOffIdx + (long long)kMaxTokens * kMaxTopk * 4;
-constexpr long long kOffHist = kOffW + (long long)kMaxTokens * kMaxTopk * 4;
-constexpr long long kOffHits = kOffHist + (long long)kTiles * kMaxExperts * 4;
-constexpr long long kOffOwnHits = kOffHits + 1024;
-constexpr long long kOffCnt = kOffOwnHits + 1024;
-constexpr long long kOffRankTokens = kOffCnt + kMaxExperts * 4;
+constexpr long long kOffOwnHits = kControlBytes;
+constexpr long long kOffRankTokens = kOffOwnHits + kTiles * 4;
 constexpr long long kOffRankRows = kOffRankTokens + 64;
 constexpr long long kScratchUsed = kOffRankRows + 64;
 static_assert(kScratchUsed <= DEEPEP_NOALLOC_SCRATCH_BYTES, "scratch array is too small for the stated limits");
@@ -94,7 +88,6 @@ extern "C" __attribute__((visibility("default"))) int deepep_notify_layout_noall
 
   NotifyParams p{};
   p.lay.world = 1; p.lay.max_tokens = kMaxTokens; p.lay.hidden = 8; p.lay.topk = num_topk; p.lay.stage_row_bytes = 128;
-  p.lay.gather_hdr = kOffHdr; p.lay.gather_idx = kOffIdx; p.lay.gather_w = kOffW;
   p.lay.total = DEEPEP_NOALLOC_SCRATCH_BYTES;
   NotifyArgs& a = p.r[0];
   a.ctx.ws[0] = scratch; a.ctx.status = nullptr; a.ctx.timeout_ns = 2000000000ll; a.ctx.rank = 0; a.ctx.world = 1;
@@ -102,8 +95,7 @@ extern "C" __attribute__((visibility("default"))) int deepep_notify_layout_noall
   a.T = num_tokens; a.E = num_experts; a.K = num_topk; a.expand = 1; a.alignment = expert_alignment;
   const int per_token = num_topk < num_experts ? num_topk : num_experts;
   a.meta_stride = 2 + (per_token > 2 ? per_token : 2);
-  a.hist = reinterpret_cast<int*>(scratch + kOffHist); a.hits = reinterpret_cast<int*>(scratch + kOffHits);
-  a.own_hits = reinterpret_cast<int*>(scratch + kOffOwnHits); a.cnt = reinterpret_cast<int*>(scratch + kOffCnt);
+  a.own_hits = reinterpret_cast<int*>(scratch + kOffOwnHits);      // (the per-tile tables serve several ranks only)
   a.rank_tokens = reinterpret_cast<int*>(scratch + kOffRankTokens); a.rank_rows = reinterpret_cast<int*>(scratch + kOffRankRows);
   a.send_slot = send_slot; a.slot_row = slot_row; a.stage_meta = stage_meta; a.chunk_start = chunk_start;
   a.expert_counts = expert_counts; a.expert_offsets = expert_offsets; a.recv_row_src = recv_row_src; a.recv_w = recv_weights;

@@ -67,6 +67,63 @@ def test_high_throughput_splits(world, tokens, hidden, experts, topk, kw):
     run_case(world, tokens, hidden, experts, topk, "invalid", repeats=2, **kw)
 
 
+# one rank: tiles of 64 tokens, 16 ranges of them, one to four shares of a range, one thread per expert and none left for the hits
+@pytest.mark.parametrize("tokens,experts,topk,expand,alignment", [
+    (1, 1, 1, True, 1), (64, 5, 3, True, 16), (65, 1024, 16, True, 128), (1024, 1023, 8, True, 1), (1025, 64, 8, False, 1),
+    (2049, 1024, 8, False, 1), (3000, 300, 11, True, 128), (16384, 1024, 16, True, 1), (16321, 40, 1, True, 16)])
+def test_routing_plan_of_one_rank(tokens, experts, topk, expand, alignment):
+    """Every field of the plan against its definition, with empty, out-of-range and repeated slots; one expert gets most tokens."""
+    from deepep_b200.parallel.virtual import VirtualWorld
+
+    g = torch.Generator().manual_seed(tokens + experts)
+    idx = torch.randint(-1, experts + 1, (tokens, topk), generator=g)
+    idx[torch.rand((tokens, topk), generator=g) < 0.2] = 0
+    idx[5::9] = -1
+    w = torch.rand((tokens, topk), generator=g)
+    dev = torch.device("cuda")
+    with VirtualWorld(1, tokens, 8, topk, timeout=10.0) as vw:
+        plan = vw.engine.notify([idx.to(dev)], [w.to(dev)], experts, expand=expand, alignment=alignment, rank_matrix=True)[0]
+        torch.cuda.synchronize()
+
+    earlier = (idx.unsqueeze(2) == idx.unsqueeze(1)).tril(-1).any(2)
+    valid = (idx >= 0) & (idx < experts) & ~earlier
+    hit = valid.any(1)
+    staged = torch.where(hit, hit.cumsum(0) - 1, torch.full((tokens,), -1))
+    assert torch.equal(plan.send_slot[:, 0].cpu().long(), staged)
+    starts = torch.cat((torch.zeros(1, dtype=torch.long), hit.long().cumsum(0)))
+    tiles = -(-tokens // 64)
+    assert torch.equal(plan.chunk_start[0].cpu().long(), starts[torch.arange(tiles + 1).mul(64).clamp(max=tokens)])
+    assert torch.equal(plan.send_chunk_prefix[0].cpu().long(), starts[torch.arange(tiles) * 64])
+    assert plan.rank_rows.tolist() == [0, int(hit.sum())] and plan.rank_tokens.tolist() == [tokens]
+    assert plan.rank_matrix.tolist() == [[int(hit.sum())]] and plan.num_staged_rows == int(hit.sum())
+    t, k = valid.nonzero(as_tuple=True)
+    counts = torch.bincount(idx[t, k], minlength=experts)
+    assert plan.expert_counts.cpu().tolist() == counts.tolist() == plan.expert_counts_list
+    blocks = (counts + alignment - 1) // alignment * alignment if expand else counts
+    offsets = torch.cat((torch.zeros(1, dtype=torch.long), blocks.cumsum(0)))
+    assert torch.equal(plan.expert_offsets.cpu().long(), offsets)
+    meta, slot_row = plan.stage_meta.cpu().long(), torch.full((tokens, topk), -1)
+    src, row_w = plan.recv_row_src.cpu().long(), plan.recv_w.cpu()
+    mask = (valid.long() << torch.arange(topk)).sum(1)
+    if expand:
+        order = torch.argsort(idx[t, k], stable=True)
+        t, k = t[order], k[order]
+        e = idx[t, k]
+        row = offsets[e] + torch.arange(len(e)) - (counts.cumsum(0) - counts)[e]
+        slot_row[t, k] = row
+        want, want_w = torch.full((int(offsets[-1]),), -1), torch.zeros((int(offsets[-1]),))
+        want[row], want_w[row] = t * topk + k, w[t, k]
+        assert plan.num_rows == len(want) and torch.equal(src[:len(want)], want) and torch.equal(row_w[:len(want)], want_w)
+        at = valid.long().cumsum(1)[t, k] + 1
+        assert torch.equal(meta[staged[t], at], row | k << 27) and torch.equal(meta[staged[hit], 1], valid.sum(1)[hit])
+    else:
+        assert plan.num_rows == int(hit.sum()) and torch.equal(src[:plan.num_rows], hit.nonzero()[:, 0] * topk)
+        assert torch.equal(row_w[:plan.num_rows], torch.where(valid, w, torch.zeros(()))[hit])
+        assert torch.equal(plan.recv_idx[:plan.num_rows].cpu(), torch.where(valid, idx, torch.full_like(idx, -1))[hit])
+        assert torch.equal(meta[staged[hit], 2], staged[hit]) and torch.equal(meta[staged[hit], 3], mask[hit])
+    assert torch.equal(plan.slot_row.cpu().long(), slot_row) and torch.equal(meta[staged[hit], 0], hit.nonzero()[:, 0])
+
+
 @pytest.mark.parametrize("dmode", [0, 1, 2])
 @pytest.mark.parametrize("tokens,hidden,experts,topk,expand,alignment", [
     (1, 128, 4, 1, True, 1), (9, 1152, 16, 2, True, 16), (70, 1024, 7, 7, True, 128), (33, 8192, 64, 16, True, 1),
