@@ -47,7 +47,7 @@ void bind_expand(py::module_& m) {
     if ((a | out | b | prod) % 16) throw std::invalid_argument("row_scale: rows must start on a 16-byte boundary");
     check_launch(launch_row_scale(p, blocks, reinterpret_cast<cudaStream_t>(stream)), "row_scale");
   });
-  m.attr("expand_tile") = kExpandTile;
+  m.def("expand_scratch", &expand_scratch, py::arg("rows"), py::arg("experts"), py::arg("topk"));
   m.def("expand", [](const py::dict& d, int blocks, uintptr_t stream) {
     ExpandParams p{};
     p.x = eptr<const uint8_t>(d, "x"); p.x_sf = eptr<const float>(d, "x_sf");
@@ -61,13 +61,19 @@ void bind_expand(py::module_& m) {
     if (p.L < 1 || p.L > kMaxExperts) throw std::invalid_argument("1..1024 local experts are supported");
     if (p.row_bytes <= 0 || p.row_bytes % 16) throw std::invalid_argument("a row must be a positive multiple of 16 bytes");
     if (p.R < 0 || p.N < 0) throw std::invalid_argument("negative row count");
-    if (!p.expert_offsets || !p.actual_counts || !p.error_flag || (p.R > 0 && (!p.x || !p.mapping)) || (p.N > 0 && !p.out))
+    if (!p.expert_offsets || !p.actual_counts || (p.R > 0 && (!p.x || !p.mapping)) || (p.N > 0 && !p.out))
       throw std::invalid_argument("missing tensor");
-    if (!p.cached && p.R > 0 && (!p.topk_idx || !p.tile_counts)) throw std::invalid_argument("expand needs topk_idx and its scratch");
+    if (!p.cached) {
+      if (!p.error_flag || (p.R > 0 && (!p.topk_idx || (!p.tile_counts && expand_scratch(p.R, p.L, p.K) > 0))))
+        throw std::invalid_argument("expand needs topk_idx and its scratch");
+      const py::list caps = d["caps"];
+      if ((int)caps.size() != p.L) throw std::invalid_argument("expand needs a capacity per expert");
+      for (int e = 0; e < p.L; ++e) p.caps[e] = caps[e].cast<int>();
+    }
     if ((p.x_sf == nullptr) != (p.out_sf == nullptr)) throw std::invalid_argument("scales need an input and an output");
     check_launch(launch_expand(p, blocks, reinterpret_cast<cudaStream_t>(stream)), "expand launch");
   });
-  m.def("aggregate", [](const py::dict& d, int blocks, uintptr_t stream) {
+  m.def("aggregate", [](const py::dict& d, uintptr_t stream) {
     AggregateParams p{};
     p.x = eptr<const uint8_t>(d, "x"); p.row_w = eptr<const float>(d, "row_w"); p.values = eptr<const float>(d, "values");
     p.mapping = eptr<const int>(d, "mapping"); p.out = eptr<uint8_t>(d, "out"); p.out_values = eptr<float>(d, "out_values");
@@ -77,6 +83,6 @@ void bind_expand(py::module_& m) {
     if (p.H <= 0 || p.H % 8) throw std::invalid_argument("hidden must be a positive multiple of 8");
     if (p.R > 0 && (!p.mapping || !p.out || (p.N > 0 && !p.x))) throw std::invalid_argument("missing tensor");
     if (p.R == 0) return;
-    check_launch(launch_aggregate(p, blocks, reinterpret_cast<cudaStream_t>(stream)), "aggregate launch");
+    check_launch(launch_aggregate(p, reinterpret_cast<cudaStream_t>(stream)), "aggregate launch");
   });
 }

@@ -19,13 +19,17 @@ struct ExpandParams {
   uint8_t* out;                // [N][row_bytes]
   float* out_sf;               // [N][num_sf] or null
   float* out_w;                // [N] or null
-  int* expert_offsets;         // [L + 1] exclusive prefix of the capacities (input)
+  int* expert_offsets;         // [L + 1] exclusive prefix of the capacities (output; input in cached mode)
   int* actual_counts;          // [L] rows really routed to each expert (output; input in cached mode)
   int* mapping;                // [R][K] expanded row of every slot, -1 for empty (output; input in cached mode)
-  int* tile_counts;            // scratch [tiles][L]
-  int* error_flag;             // set to 1 when an expert receives more rows than its capacity
-  int R, K, L, N, row_bytes, num_sf, cached, pad;
+  int* tile_counts;            // scratch [tiles][L] of tables that do not fit a cluster's shared memory (expand_scratch)
+  int* error_flag;             // 1 when an expert receives more rows than its capacity, else 0 (not cached)
+  int R, K, L, N, row_bytes, num_sf, cached;
+  int pieces, pad_blocks;      // column pieces per row, blocks that zero padding rows (set by the launcher)
+  int caps[kMaxExperts];       // capacity of every expert (not cached): with the launch, so that no copy to the device is needed
 };
+// Ints of scratch that a plan needs.
+long long expand_scratch(int R, int L, int K);
 cudaError_t launch_expand(const ExpandParams& p, int blocks, cudaStream_t stream);
 
 struct AggregateParams {
@@ -37,6 +41,6 @@ struct AggregateParams {
   float* out_values;           // [R][K] or null
   int R, K, H, N, is_half, pad;
 };
-cudaError_t launch_aggregate(const AggregateParams& p, int blocks, cudaStream_t stream);
+cudaError_t launch_aggregate(const AggregateParams& p, cudaStream_t stream);
 
 }  // namespace dep

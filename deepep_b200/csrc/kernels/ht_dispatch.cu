@@ -26,50 +26,9 @@
 #include <algorithm>
 
 #include "api.h"
+#include "fanout.cuh"
 
 namespace dep {
-
-constexpr int kCopyUnroll = 7;    // 16-byte pieces per lane and pass: 3.5 KB in flight per warp
-
-__device__ __forceinline__ unsigned long long shfl_u64(unsigned long long v, int src) {
-  return __shfl_sync(0xffffffffu, v, src);
-}
-
-// Copies `units` 16-byte pieces from `src` to every destination in `mask`: lane l of the mask holds its
-// destination in `dst`.  All loads of a pass are issued before the first store.
-template <bool kPeerWritten, int U = kCopyUnroll>
-__device__ __forceinline__ void warp_fanout(const int4* src, int units, unsigned long long dst, unsigned mask, int lane) {
-  for (int u0 = 0; u0 < units; u0 += 32 * U) {
-    int4 v[U];
-#pragma unroll
-    for (int i = 0; i < U; ++i) {
-      const int u = u0 + i * 32 + lane;
-      if (u < units) v[i] = kPeerWritten ? __ldcg(src + u) : __ldg(src + u);
-    }
-    for (unsigned m = mask; m; m &= m - 1) {
-      int4* d = reinterpret_cast<int4*>(shfl_u64(dst, __ffs(m) - 1));
-#pragma unroll
-      for (int i = 0; i < U; ++i) {
-        const int u = u0 + i * 32 + lane;
-        if (u < units) d[u] = v[i];
-      }
-    }
-  }
-}
-
-// The same for a short run of floats (the scales of an fp8 row).
-template <bool kPeerWritten>
-__device__ __forceinline__ void warp_fanout_f32(const float* src, int n, unsigned long long dst, unsigned mask, int lane) {
-  for (int b0 = 0; b0 < n; b0 += 32) {   // the trip count is the same for every lane: all of them take part in the shuffles
-    const int b = b0 + lane;
-    float v = 0.f;
-    if (b < n) v = kPeerWritten ? __ldcg(src + b) : __ldg(src + b);
-    for (unsigned m = mask; m; m &= m - 1) {
-      float* d = reinterpret_cast<float*>(shfl_u64(dst, __ffs(m) - 1));
-      if (b < n) d[b] = v;
-    }
-  }
-}
 
 // 16 bf16 values (two 16-byte pieces) -> their absolute maximum.
 __device__ __forceinline__ float amax16(const int4& a, const int4& b, float v[16]) {
@@ -141,20 +100,12 @@ __device__ __forceinline__ void warp_quant_fanout(const int4* src, int H, unsign
 }
 
 // Zeroes the rows of this rank's output that no token fills: the padding of every expert's aligned block and the rows behind
-// the last block.  Warp `gw` of `warps`; the warps are dealt out to the experts in turn.  (4096 x 8 fp8 rows over 256 experts in
-// blocks of 128 rows: clearing the whole output first took a pass of 95 us, these rows add about 12 us to the kernel.)
+// the last block.  (4096 x 8 fp8 rows over 256 experts in blocks of 128 rows: clearing the whole output first took a pass of 95 us,
+// these rows add about 12 us to the kernel.)
 __device__ __forceinline__ void zero_padding(const DispatchArgs& a, int local_experts, int row_bytes, int nsf, int gw, int warps, int lane) {
-  auto zero_row = [&](int row) {
-    int4* x = reinterpret_cast<int4*>(reinterpret_cast<uint8_t*>(a.recv_x) + (size_t)row * row_bytes);
-    for (int u = lane; u < row_bytes / 16; u += 32) x[u] = make_int4(0, 0, 0, 0);
-    for (int b = lane; b < nsf; b += 32) a.recv_sf[(size_t)row * nsf + b] = 0.f;
-  };
-  const int per = max(1, warps / local_experts);            // warps per expert
-  for (int i = gw; i < local_experts * per; i += warps) {
-    const int l = i % local_experts, end = min(a.pad_offsets[l + 1], a.recv_rows);
-    for (int row = a.pad_offsets[l] + a.pad_counts[l] + i / local_experts; row < end; row += per) zero_row(row);
-  }
-  for (int row = a.pad_offsets[local_experts] + gw; row < a.recv_rows; row += warps) zero_row(row);
+  for_padding_rows(a.pad_offsets, a.pad_counts, local_experts, a.recv_rows, gw, warps, [&](int row) {
+    zero_row(reinterpret_cast<uint8_t*>(a.recv_x) + (size_t)row * row_bytes, row_bytes, a.recv_sf + (size_t)row * nsf, nsf, lane);
+  });
 }
 
 // kPieces: one rank that keeps all its rows, the work items are column pieces of tokens.  Several ranks run without: their items

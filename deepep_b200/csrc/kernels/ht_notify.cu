@@ -21,6 +21,7 @@
 #include <algorithm>
 
 #include "api.h"
+#include "local_tile.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -368,58 +369,21 @@ __global__ void __launch_bounds__(kNotifyThreads) ep_notify_kernel(const __grid_
 // for one another.  Kernel times as one grid of 128 cooperative blocks (the kernel above) and here: 1531 x 6 routes over 64 experts 20.9
 // and 8.0 us, 4096 x 8 over 256 22.7 and 10.6 (13.2 with one cluster), in blocks of 128 rows 26.3 and 10.8, 16384 x 8 over 64 34.9 and
 // 16.3 (26.5 with one), 16384 x 16 over 1024 72 and 35 (60 with one, 50 with eight).
-constexpr int kLocalNotifyThreads = 1024;
-constexpr int kLocalNotifyCtas = 16;       // largest cluster of this device class
 constexpr int kLocalNotifyClusters = 4;    // at most, one per 16384 slots: eight do not all fit the GPU at once
-constexpr unsigned kRepeated = 1u << 31;   // in LocalTile::valid: two slots of the token name one expert
-
-// Shared memory of a CTA that owns `per` tokens.
-struct LocalTile {
-  unsigned* mask;      // [E][stride]: tokens of the expert, `stride` odd so that a column of it meets all banks
-  unsigned* hit;       // [words]: tokens with at least one slot that counts
-  int* cnt;            // [E + 1]: tokens per expert of this CTA, then tokens with a hit (read by the other CTAs)
-  int* tot;            // [E] rows of the expert
-  int* off;            // [E + 1] first row of the expert
-  int* base;           // [E] first row of this CTA's tokens
-  unsigned* valid;     // [per] bit k: slot k counts
-  short* id;           // [per][K], -1: no expert
-  __host__ __device__ static int stride(int per) { return per / 32 | 1; }
-  __host__ __device__ static size_t bytes(int per, int E, int K) {
-    return 4 * ((size_t)E * stride(per) + per / 32 + 4 * E + 2 + per) + 2 * (size_t)per * K;
-  }
-  __device__ LocalTile(void* smem, int per, int E) {
-    mask = reinterpret_cast<unsigned*>(smem);
-    hit = mask + (size_t)E * stride(per);
-    cnt = reinterpret_cast<int*>(hit + per / 32);
-    tot = cnt + E + 1; off = tot + E; base = off + E + 1;
-    valid = reinterpret_cast<unsigned*>(base + E);
-    id = reinterpret_cast<short*>(valid + per);
-  }
-};
-__host__ __device__ inline int local_tokens(int T, int ctas) {          // tokens per CTA: whole tiles
-  const int tiles = (T + kChunkTokens - 1) / kChunkTokens;
-  return (tiles > ctas ? (tiles + ctas - 1) / ctas : 1) * kChunkTokens;
-}
-__device__ __forceinline__ int below_words(const unsigned* m, int t) {   // bits of m below bit t
-  int n = 0;
-  for (int w = 0; w < t >> 5; ++w) n += __popc(m[w]);
-  return n + ((t & 31) ? __popc(m[t >> 5] & ((1u << (t & 31)) - 1u)) : 0);
-}
 
 template <bool kProfile>
-__global__ void __launch_bounds__(kLocalNotifyThreads) ep_notify_local_kernel(const __grid_constant__ NotifyParams p) {
+__global__ void __launch_bounds__(kTileThreads) ep_notify_local_kernel(const __grid_constant__ NotifyParams p) {
   cg::cluster_group cluster = cg::this_cluster();
   const NotifyArgs& a = p.r[0];
-  constexpr int C = kLocalNotifyCtas;
+  constexpr int C = kTileCtas;
   const int c = blockIdx.x % C, share = blockIdx.x / C, shares = gridDim.x / C;
   const int T = a.T, K = a.K, E = a.E, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int per = local_tokens(T, C), words = per / 32, stride = LocalTile::stride(per);
+  const int per = LocalTile::tokens(T), stride = LocalTile::stride(per);
   const int t0 = min(T, c * per), live = min(per, T - t0), n = live * K;
   const int NT = (p.lay.max_tokens + kChunkTokens - 1) / kChunkTokens;
   extern __shared__ __align__(16) unsigned char smem[];
   const LocalTile s(smem, per, E);
-  __shared__ int s_warp[kLocalNotifyThreads / 32];
-  __shared__ int s_hits[2];                              // tokens with a hit: before this CTA, of all CTAs
+  __shared__ int s_warp[kTileThreads / 32], s_hits[2];
   Control* ctl = control_of(a.ctx.ws[0]);
   unsigned long long t_start = 0;
   if constexpr (kProfile) t_start = global_timer_ns();
@@ -428,83 +392,16 @@ __global__ void __launch_bounds__(kLocalNotifyThreads) ep_notify_local_kernel(co
       if (blockIdx.x == 0 && tid == 0) ctl->dbg[16 + i] = global_timer_ns() - t_start;
   };
 
-  // ---- the ids, and which tokens every expert gets
-  for (int i0 = tid; i0 < n; i0 += kLocalNotifyThreads * 4) {
-    long long v[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = i0 + j * kLocalNotifyThreads < n ? __ldg(a.topk_idx + (size_t)t0 * K + i0 + j * kLocalNotifyThreads) : -1;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (i0 + j * kLocalNotifyThreads < n) s.id[i0 + j * kLocalNotifyThreads] = (short)((v[j] < 0 || v[j] >= E) ? -1 : (int)v[j]);
-  }
-  for (int i = tid; i < E * stride; i += kLocalNotifyThreads) s.mask[i] = 0u;
-  for (int i = tid; i < words; i += kLocalNotifyThreads) s.hit[i] = 0u;
-  for (int i = tid; i < per; i += kLocalNotifyThreads) s.valid[i] = 0u;
+  // ---- the ids, which tokens every expert gets, and the counts of the other CTAs
   stamp(0);
-  __syncthreads();
+  s.count(a.topk_idx + (size_t)t0 * K, n, per, K, E);
   stamp(1);
-  for (int i = tid; i < n; i += kLocalNotifyThreads) {
-    const int tl = i / K, k = i - tl * K, e = s.id[i];
-    if (e < 0) continue;
-    const unsigned bit = 1u << (tl & 31);
-    const bool again = atomicOr(&s.mask[e * stride + (tl >> 5)], bit) & bit;
-    atomicOr(&s.valid[tl], 1u << k | (again ? kRepeated : 0u));
-  }
-  __syncthreads();
-  for (int i = tid; i < per; i += kLocalNotifyThreads) {          // per is a multiple of 64: whole warps
-    unsigned valid = s.valid[i];
-    if (valid & kRepeated) {                                      // only the first of a token's slots with one expert counts
-      valid &= ~kRepeated;
-      for (int k = 1; k < K; ++k)
-        for (int j = 0; j < k; ++j)
-          if (s.id[i * K + j] == s.id[i * K + k]) valid &= ~(1u << k);
-      s.valid[i] = valid;
-    }
-    const unsigned word = __ballot_sync(0xffffffffu, valid != 0u);
-    if (lane == 0) s.hit[i >> 5] = word;
-  }
-  for (int e = tid; e < E; e += kLocalNotifyThreads) {
-    int v = 0;
-    for (int w = 0; w < words; ++w) v += __popc(s.mask[e * stride + w]);
-    s.cnt[e] = v;
-  }
-  __syncthreads();
-  if (tid == 0) s.cnt[E] = below_words(s.hit, per - 1) + (int)(s.hit[words - 1] >> 31);
   cluster.sync();
   stamp(2);
-
-  // ---- rows of every expert, the blocks' first rows, and this CTA's first row in each
-  int before = 0, tot = 0;
-  if (tid <= E) {
-    int v[C];
-#pragma unroll
-    for (int r = 0; r < C; ++r) v[r] = cluster.map_shared_rank(s.cnt, r)[tid];
-#pragma unroll
-    for (int r = 0; r < C; ++r) {
-      if (r < c) before += v[r];
-      tot += v[r];
-    }
-  }
-  if (tid == E) { s_hits[0] = before; s_hits[1] = tot; }
-  if (E == kLocalNotifyThreads && warp == 0) {                     // no thread is left for the hits
-    int b = 0, v = lane < C ? cluster.map_shared_rank(s.cnt, lane)[E] : 0;
-    b = lane < c ? v : 0;
-    for (int d = 16; d > 0; d >>= 1) { b += __shfl_xor_sync(0xffffffffu, b, d); v += __shfl_xor_sync(0xffffffffu, v, d); }
-    if (lane == 0) { s_hits[0] = b; s_hits[1] = v; }
-  }
+  int before, tot;
+  s.gather(cluster, c, E, s_hits, before, tot);
   const int rows = tid < E ? (a.expand ? (tot + a.alignment - 1) / a.alignment * a.alignment : tot) : 0;
-  int incl = rows;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const int o = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += o;
-  }
-  if (lane == 31) s_warp[warp] = incl;
-  __syncthreads();
-  int warps = lane < warp ? s_warp[lane] : 0;                      // rows of the experts of the warps before this one
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) warps += __shfl_xor_sync(0xffffffffu, warps, d);
-  const int first = warps + incl - rows;
+  const int first = tile_prefix(rows, s_warp);
   if (tid < E) {
     s.tot[tid] = tot; s.off[tid] = first; s.base[tid] = first + before;
     if (tid == E - 1) s.off[E] = first + rows;
@@ -523,11 +420,11 @@ __global__ void __launch_bounds__(kLocalNotifyThreads) ep_notify_local_kernel(co
       if (a.rank_matrix) a.rank_matrix[0] = hits;
     }
     const int nt = (T + kChunkTokens - 1) / kChunkTokens;
-    for (int i = nt + tid; i <= NT; i += kLocalNotifyThreads) a.chunk_start[i] = hits;
+    for (int i = nt + tid; i <= NT; i += kTileThreads) a.chunk_start[i] = hits;
     // The epoch word tells a host that polls it that the counts are there; the records are complete when the launch is.  The fence
     // takes 2 us, which the others spend on the records.
     __syncthreads();
-    if (tid == kLocalNotifyThreads - 1) {
+    if (tid == kTileThreads - 1) {
       const unsigned long long epoch = ctl->epoch[kOpNotify] + 1;
       ctl->notify_ack[0] = epoch;
       ctl->epoch[kOpNotify] = epoch;
@@ -542,7 +439,7 @@ __global__ void __launch_bounds__(kLocalNotifyThreads) ep_notify_local_kernel(co
   // ---- padding rows carry no source; the experts are dealt out to the CTAs
   const bool has_w = a.recv_w != nullptr && a.topk_w != nullptr;
   if (a.expand && a.alignment > 1)
-    for (int e = warp * (int)gridDim.x + blockIdx.x; e < E; e += gridDim.x * (kLocalNotifyThreads / 32))
+    for (int e = warp * (int)gridDim.x + blockIdx.x; e < E; e += gridDim.x * (kTileThreads / 32))
       for (int row = s.off[e] + s.tot[e] + lane; row < s.off[e + 1] && row < a.rcap; row += 32) {
         a.recv_row_src[row] = -1;
         if (a.recv_w) a.recv_w[row] = 0.f;
@@ -550,14 +447,14 @@ __global__ void __launch_bounds__(kLocalNotifyThreads) ep_notify_local_kernel(co
 
   // ---- per-token records of this cluster's share, one thread per (token, slot)
   const int tokens = (live + shares - 1) / shares, first_token = min(live, share * tokens), last_token = min(live, first_token + tokens);
-  for (int i = first_token * K + tid; i < last_token * K; i += kLocalNotifyThreads) {
+  for (int i = first_token * K + tid; i < last_token * K; i += kTileThreads) {
     const int tl = i / K, k = i - tl * K, e = s.id[i];
     const unsigned valid = s.valid[tl];
     const bool counts = (valid >> k) & 1u;
-    const int row = a.expand && counts ? s.base[e] + below_words(s.mask + e * stride, tl) : -1;
+    const int row = a.expand && counts ? s.base[e] + LocalTile::below(s.mask + e * stride, tl) : -1;
     a.slot_row[(size_t)t0 * K + i] = row;
     if (valid == 0) continue;
-    const int j = hits_before + below_words(s.hit, tl);
+    const int j = hits_before + LocalTile::below(s.hit, tl);
     const float w = has_w && counts ? __ldg(a.topk_w + (size_t)t0 * K + i) : 0.f;
     if (a.expand) {
       if (!counts) continue;
@@ -572,9 +469,9 @@ __global__ void __launch_bounds__(kLocalNotifyThreads) ep_notify_local_kernel(co
       if (a.recv_w) a.recv_w[(size_t)j * K + k] = w;
     }
   }
-  for (int tl = first_token + tid; tl < last_token; tl += kLocalNotifyThreads) {
+  for (int tl = first_token + tid; tl < last_token; tl += kTileThreads) {
     const unsigned valid = s.valid[tl];
-    const int j = hits_before + below_words(s.hit, tl);
+    const int j = hits_before + LocalTile::below(s.hit, tl);
     a.send_slot[t0 + tl] = valid ? j : -1;
     if (tl % kChunkTokens == 0) {
       a.chunk_start[(t0 + tl) / kChunkTokens] = j;
@@ -594,21 +491,9 @@ __global__ void __launch_bounds__(kLocalNotifyThreads) ep_notify_local_kernel(co
 static cudaError_t launch_notify_local(const NotifyParams& p, cudaStream_t stream) {
   const NotifyArgs& a = p.r[0];
   const void* fn = p.profile ? (const void*)ep_notify_local_kernel<true> : (const void*)ep_notify_local_kernel<false>;
-  const int ctas = kLocalNotifyCtas;
-  const size_t smem = LocalTile::bytes(local_tokens(a.T, ctas), a.E, a.K);
-  const int clusters = std::max(1, std::min(kLocalNotifyClusters, (a.T * a.K + ctas * kLocalNotifyThreads - 1) / (ctas * kLocalNotifyThreads)));
-  // attributes belong to the current device, so they are set on every launch (a process may drive several GPUs)
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e == cudaSuccess && smem > 48 * 1024) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ctas * clusters); cfg.blockDim = dim3(kLocalNotifyThreads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-  cudaLaunchAttribute attr = {};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = ctas; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr; cfg.numAttrs = 1;
-  void* args[] = {const_cast<NotifyParams*>(&p)};
-  return cudaLaunchKernelExC(&cfg, fn, args);
+  constexpr int kSlots = kTileCtas * kTileThreads;
+  const int clusters = std::max(1, std::min(kLocalNotifyClusters, (a.T * a.K + kSlots - 1) / kSlots));
+  return launch_tiles(fn, &p, clusters, LocalTile::bytes(LocalTile::tokens(a.T), a.E, a.K), stream);
 }
 
 cudaError_t launch_notify(const NotifyParams& p, int nranks, int blocks, cudaStream_t stream) {

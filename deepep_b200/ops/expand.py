@@ -169,24 +169,22 @@ def expand(x: Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor]], recv_topk_
     out = torch.empty((total, data.shape[1]), dtype=data.dtype, device=dev)
     out_sf = torch.empty((total, scales.shape[1]), dtype=torch.float32, device=dev) if scales is not None else None
     out_w = torch.empty((total,), dtype=torch.float32, device=dev) if topk_weights is not None else None
-    err = torch.zeros((1,), **i32)
+    err = tile_counts = None
     if handle is None:
-        offsets = torch.zeros((L + 1,), dtype=torch.int32)
-        offsets[1:] = torch.tensor(caps, dtype=torch.int64).cumsum(0).to(torch.int32)
-        offsets = offsets.to(dev)
-        actual = torch.empty((L,), **i32)
-        mapping = torch.empty((R, K), **i32)
-        tiles = -(-R // C.expand_tile)
-        tile_counts = torch.empty((max(tiles, 1) * L,), **i32)
+        offsets, actual, mapping, err = (torch.empty(shape, **i32) for shape in ((L + 1,), (L,), (R, K), (1,)))
+        scratch = C.expand_scratch(R, L, K)
+        if scratch:
+            tile_counts = torch.empty((scratch,), **i32)
     else:
-        offsets, actual, mapping, tile_counts = handle.expert_offsets, handle.actual_expert_counts, handle.recv_to_expanded_idx, None
+        offsets, actual, mapping = handle.expert_offsets, handle.actual_expert_counts, handle.recv_to_expanded_idx
     C.expand(dict(x=data.data_ptr() if R else None, x_sf=scales.data_ptr() if scales is not None and R else (scales.data_ptr() if scales is not None else None),
                   topk_idx=recv_topk_idx.data_ptr() if recv_topk_idx is not None and R else None,
                   topk_w=topk_weights.data_ptr() if topk_weights is not None and R else None,
                   out=out.data_ptr() if total else None, out_sf=out_sf.data_ptr() if out_sf is not None else None,
                   out_w=out_w.data_ptr() if out_w is not None else None, expert_offsets=offsets.data_ptr(),
                   actual_counts=actual.data_ptr(), mapping=mapping.data_ptr() if R else None,
-                  tile_counts=tile_counts.data_ptr() if tile_counts is not None else None, err=err.data_ptr(), rows=R, topk=K,
+                  tile_counts=tile_counts.data_ptr() if tile_counts is not None else None,
+                  err=err.data_ptr() if err is not None else None, caps=caps if handle is None else None, rows=R, topk=K,
                   experts=L, expanded_rows=total, row_bytes=data.shape[1] * data.element_size(),
                   num_sf=scales.shape[1] if scales is not None else 0, cached=int(handle is not None)),
              _blocks(dev), stream.cuda_stream)
@@ -225,7 +223,7 @@ def aggregate(x: torch.Tensor, handle: ExpandHandle, topk_weights: Optional[torc
                      values=expanded_values.data_ptr() if expanded_values is not None and N else None,
                      mapping=handle.recv_to_expanded_idx.data_ptr() if R else None, out=out.data_ptr() if R else None,
                      out_values=out_values.data_ptr() if out_values is not None and R else None, rows=R, topk=K,
-                     hidden=x.shape[1], expanded_rows=N, is_half=int(x.dtype == torch.float16)), _blocks(dev), stream.cuda_stream)
+                     hidden=x.shape[1], expanded_rows=N, is_half=int(x.dtype == torch.float16)), stream.cuda_stream)
     return out, out_values
 
 

@@ -58,3 +58,37 @@ def test_capacity_overflow_is_reported():
     small = [max(c - 1, 0) for c in caps]
     with pytest.raises(ValueError, match="capacity"):
         X.expand(x.to(dev), idx.to(dev), None, small, 1)
+
+
+# a table that a cluster's shared memory holds, the largest such ranges, and one that takes the passes with grid barriers
+@pytest.mark.parametrize("R,K,L,H,align,slack", [(0, 2, 3, 64, 4, 4), (65, 1, 1, 8, 1, 0), (1025, 16, 1024, 24, 1, 0), (16384, 6, 128, 136, 1, 3),
+                                                 (131072, 8, 64, 8, 16, 16)])
+def test_expand_plan_against_its_definition(R, K, L, H, align, slack):
+    """Repeated and out-of-range ids, experts without rows, capacities above the counts: plan, rows, weights and zeroed padding."""
+    g = torch.Generator().manual_seed(R + L)
+    dev = torch.device("cuda")
+    idx = torch.randint(-1, L + 1, (R, K), generator=g)
+    idx[1::5] = idx[1::5, :1].clone()
+    earlier = (idx.unsqueeze(2) == idx.unsqueeze(1)).tril(-1).any(2)
+    r, k = ((idx >= 0) & (idx < L) & ~earlier).nonzero(as_tuple=True)
+    order = torch.argsort(idx[r, k], stable=True)
+    r, k = r[order], k[order]
+    e = idx[r, k]
+    counts = torch.bincount(e, minlength=L)
+    caps = (counts + slack + align - 1) // align * align
+    offsets = torch.cat((torch.zeros(1, dtype=torch.long), caps.cumsum(0)))
+    row = offsets[e] + torch.arange(len(e)) - (counts.cumsum(0) - counts)[e]
+    mapping = torch.full((R, K), -1, dtype=torch.int32)
+    mapping[r, k] = row.int()
+    x, w = torch.randn((R, H), generator=g).to(torch.bfloat16), torch.rand((R, K), generator=g)
+    want, want_w = torch.zeros((int(offsets[-1]), H), dtype=torch.bfloat16), torch.zeros((int(offsets[-1]),))
+    want[row], want_w[row] = x[r], w[r, k]
+    ex, ew, h = X.expand(x.to(dev), idx.to(dev), w.to(dev), caps.tolist(), align)
+    assert torch.equal(h.recv_to_expanded_idx.cpu(), mapping) and torch.equal(h.actual_expert_counts.cpu().long(), counts)
+    assert torch.equal(h.expert_offsets.cpu().long(), offsets)
+    assert torch.equal(ex.cpu().view(torch.int16), want.view(torch.int16)) and torch.equal(ew.cpu(), want_w)
+    if len(e):
+        busiest = int(counts.argmax())
+        caps[busiest] = (counts[busiest] - 1) // align * align
+        with pytest.raises(ValueError, match="capacity"):
+            X.expand(x.to(dev), idx.to(dev), w.to(dev), caps.tolist(), align)
