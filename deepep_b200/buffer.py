@@ -128,8 +128,8 @@ class Buffer:
 
             C = require_native("Buffer.get_dispatch_layout")
             dev = topk_idx.device
-            per_rank = torch.zeros((world,), dtype=torch.int32, device=dev)
-            per_expert = torch.zeros((num_experts,), dtype=torch.int32, device=dev)
+            per_rank = torch.empty((world,), dtype=torch.int32, device=dev)
+            per_expert = torch.empty((num_experts,), dtype=torch.int32, device=dev)
             in_rank = torch.empty((T, world), dtype=torch.bool, device=dev)
             C.layout(topk_idx.data_ptr(), T, K, num_experts, world, per_rank.data_ptr(), per_expert.data_ptr(), in_rank.data_ptr(),
                      torch.cuda.current_stream(dev).cuda_stream)
@@ -146,16 +146,14 @@ class Buffer:
     def _v1_handle(self, eh, in_rank: Optional[torch.Tensor], tokens: int) -> Handle:
         """Upstream's six handle tensors from the routing plan of the dispatch, bound to a slot."""
         plan = eh._plan
-        tmax, K = self._elastic.num_max_tokens_per_rank, self._elastic.num_topk
-        rank_prefix = torch.cumsum(plan.rank_matrix.to(torch.int64), dim=0).to(torch.int32)
-        recv_src_idx = (torch.div(plan.recv_row_src[:plan.num_rows], K, rounding_mode="floor") % tmax).to(torch.int32)
         send_head = plan.send_slot[:tokens]
         if in_rank is None:
             in_rank = send_head >= 0
         slot = self._slots.acquire()
         slot.move(SlotState.DISPATCH_IN_FLIGHT)
         slot.move(SlotState.DISPATCH_READY)
-        return Handle((rank_prefix, plan.send_chunk_prefix, plan.chunk_start, recv_src_idx, in_rank, send_head), slot, eh)
+        return Handle((plan.rank_prefix, plan.send_chunk_prefix, plan.chunk_start, plan.recv_src_idx[:plan.num_rows], in_rank,
+                       send_head), slot, eh)
 
     def dispatch(self, x, handle=None, num_tokens_per_rank=None, num_tokens_per_rdma_rank=None, is_token_in_rank=None,
                  num_tokens_per_expert=None, topk_idx=None, topk_weights=None, expert_alignment: int = 1, num_worst_tokens: int = 0,

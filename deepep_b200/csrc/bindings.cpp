@@ -57,7 +57,10 @@ void op_notify(const WsLayout& lay, const std::vector<py::object>& sessions, con
     a.chunk_start = ptr<int>(d, "chunk_start"); a.rank_tokens = ptr<int>(d, "rank_tokens"); a.rank_rows = ptr<int>(d, "rank_rows");
     a.expert_counts = ptr<int>(d, "expert_counts"); a.expert_offsets = ptr<int>(d, "expert_offsets");
     a.recv_row_src = ptr<int>(d, "recv_row_src"); a.recv_w = ptr<float>(d, "recv_w"); a.recv_idx = ptr<long long>(d, "recv_idx");
-    a.rank_matrix = ptr<int>(d, "rank_matrix");
+    a.rank_matrix = ptr<int>(d, "rank_matrix"); a.rank_prefix = ptr<int>(d, "rank_prefix");
+    a.send_prefix = ptr<int>(d, "send_prefix"); a.recv_src = ptr<int>(d, "recv_src");
+    if (!a.rank_matrix != !a.rank_prefix || !a.rank_matrix != !a.send_prefix || !a.rank_matrix != !a.recv_src)
+      throw std::invalid_argument("notify: the V1 handle's tensors come together");
     a.mailbox = sessions[i].cast<Session&>().mailbox_device();
     a.rcap = getl(d, "rcap");
     if (a.T < 0 || a.T > lay.max_tokens) throw std::invalid_argument("token count exceeds num_max_tokens_per_rank");

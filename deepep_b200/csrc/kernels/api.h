@@ -36,7 +36,13 @@ struct NotifyArgs {
   int* recv_row_src;           // [rcap] (source * Tmax + token) * K + slot of every output row, -1 for padding
   float* recv_w;               // [rcap] (expanded) or [rcap][K] (rank layout); may be null
   long long* recv_idx;         // [rcap][K] destination-local expert ids (rank layout) or null
-  int* rank_matrix;            // optional [P][P], cleared by the launcher: tokens that source i sends to rank j (every rank computes all of it)
+  // the V1 handle's tensors (all or none): tokens that source i sends to rank j, which every rank computes all of (cleared by the
+  // launcher), its inclusive prefix over the sources, this rank's sent tokens before each of its tiles, and, in the rank layout, the
+  // source token of every output row
+  int* rank_matrix;            // [P][P]
+  int* rank_prefix;            // [P][P]
+  int* send_prefix;            // [P][max(1, ceil(T / kChunkTokens))]
+  int* recv_src;               // [rcap]
   int* mailbox;                // mapped host memory: [0] rows, [1] staged rows, [2] max tokens, [3] epoch, [4..] counts
   long long rcap;
 };

@@ -211,11 +211,14 @@ __global__ void __launch_bounds__(kNotifyThreads) ep_notify_kernel(const __grid_
           if (lane_ >= q) incl += o;
         }
         if (tile < nt) {
-          if (own) a.own_hits[tile * P + d] = run + incl - v;
-          else a.chunk_start[r * (NT + 1) + tile] = run + incl - v;
+          if (own) {
+            a.own_hits[tile * P + d] = run + incl - v;
+            if (a.send_prefix) a.send_prefix[d * max(nt, 1) + tile] = run + incl - v;
+          } else a.chunk_start[r * (NT + 1) + tile] = run + incl - v;
         }
         run += __shfl_sync(0xffffffffu, incl, 31);
       }
+      if (own && nt == 0 && lane_ == 0 && a.send_prefix) a.send_prefix[d] = 0;
       if (!own)
         for (int tile = nt + lane_; tile <= NT; tile += 32) a.chunk_start[r * (NT + 1) + tile] = run;
     }
@@ -262,6 +265,11 @@ __global__ void __launch_bounds__(kNotifyThreads) ep_notify_kernel(const __grid_
   if (blockIdx.x == 0) {
     if (threadIdx.x <= P) a.rank_rows[threadIdx.x] = s_rank_base[threadIdx.x];
     if (threadIdx.x < P) a.rank_tokens[threadIdx.x] = s_T[threadIdx.x];
+    if (a.rank_matrix && threadIdx.x < P * P) {
+      int run = 0;
+      for (int i = threadIdx.x % P; i <= (int)threadIdx.x; i += P) run += a.rank_matrix[i];
+      a.rank_prefix[threadIdx.x] = run;
+    }
   }
   if (a.expand && a.alignment > 1) {    // padding rows carry no source; the experts are dealt out to the blocks
     for (int l = blockIdx.x; l < Lx; l += gridDim.x) {
@@ -311,7 +319,10 @@ __global__ void __launch_bounds__(kNotifyThreads) ep_notify_kernel(const __grid_
       } else {
         const long long out = (long long)s_rank_base[r] + j;
         if (out < a.rcap) {
-          if (k == 0) a.recv_row_src[out] = (r * Tmax + t0 + tl) * K;
+          if (k == 0) {
+            a.recv_row_src[out] = (r * Tmax + t0 + tl) * K;
+            if (a.recv_src) a.recv_src[out] = t0 + tl;
+          }
           if (a.recv_idx) a.recv_idx[(size_t)out * K + k] = here ? e - me * Lx : -1;
           if (a.recv_w) a.recv_w[(size_t)out * K + k] = here ? weight_of(r, t0 * K + i) : 0.f;
         }
@@ -417,7 +428,10 @@ __global__ void __launch_bounds__(kTileThreads) ep_notify_local_kernel(const __g
       if (a.mailbox) { a.mailbox[0] = all_rows; a.mailbox[1] = hits; a.mailbox[2] = T; }
       a.expert_offsets[E] = s.off[E];
       a.rank_rows[0] = 0; a.rank_rows[1] = hits; a.rank_tokens[0] = T;
-      if (a.rank_matrix) a.rank_matrix[0] = hits;
+      if (a.rank_matrix) {
+        a.rank_matrix[0] = a.rank_prefix[0] = hits;
+        if (T == 0) a.send_prefix[0] = 0;
+      }
     }
     const int nt = (T + kChunkTokens - 1) / kChunkTokens;
     for (int i = nt + tid; i <= NT; i += kTileThreads) a.chunk_start[i] = hits;
@@ -464,7 +478,10 @@ __global__ void __launch_bounds__(kTileThreads) ep_notify_local_kernel(const __g
         if (a.recv_w) a.recv_w[row] = w;
       }
     } else if (j < a.rcap) {
-      if (k == 0) a.recv_row_src[j] = (t0 + tl) * K;
+      if (k == 0) {
+        a.recv_row_src[j] = (t0 + tl) * K;
+        if (a.recv_src) a.recv_src[j] = t0 + tl;
+      }
       if (a.recv_idx) a.recv_idx[(size_t)j * K + k] = counts ? e : -1;
       if (a.recv_w) a.recv_w[(size_t)j * K + k] = w;
     }
@@ -475,7 +492,7 @@ __global__ void __launch_bounds__(kTileThreads) ep_notify_local_kernel(const __g
     a.send_slot[t0 + tl] = valid ? j : -1;
     if (tl % kChunkTokens == 0) {
       a.chunk_start[(t0 + tl) / kChunkTokens] = j;
-      a.own_hits[(t0 + tl) / kChunkTokens] = j;
+      if (a.send_prefix) a.send_prefix[(t0 + tl) / kChunkTokens] = j;
     }
     if (valid == 0) continue;
     int* rec = a.stage_meta + (size_t)j * a.meta_stride;

@@ -13,11 +13,9 @@ namespace {
 using namespace dep;
 
 constexpr int kMaxTokens = DEEPEP_NOALLOC_MAX_TOKENS;
-constexpr int kTiles = kMaxTokens / kChunkTokens;
 
 // Layout of the scratch array (byte offsets).  The first part plays the role of a one-rank workspace.
-constexpr long long kOffOwnHits = kControlBytes;
-constexpr long long kOffRankTokens = kOffOwnHits + kTiles * 4;
+constexpr long long kOffRankTokens = kControlBytes;
 constexpr long long kOffRankRows = kOffRankTokens + 64;
 constexpr long long kScratchUsed = kOffRankRows + 64;
 static_assert(kScratchUsed <= DEEPEP_NOALLOC_SCRATCH_BYTES, "scratch array is too small for the stated limits");
@@ -95,7 +93,6 @@ extern "C" __attribute__((visibility("default"))) int deepep_notify_layout_noall
   a.T = num_tokens; a.E = num_experts; a.K = num_topk; a.expand = 1; a.alignment = expert_alignment;
   const int per_token = num_topk < num_experts ? num_topk : num_experts;
   a.meta_stride = 2 + (per_token > 2 ? per_token : 2);
-  a.own_hits = reinterpret_cast<int*>(scratch + kOffOwnHits);      // (the per-tile tables serve several ranks only)
   a.rank_tokens = reinterpret_cast<int*>(scratch + kOffRankTokens); a.rank_rows = reinterpret_cast<int*>(scratch + kOffRankRows);
   a.send_slot = send_slot; a.slot_row = slot_row; a.stage_meta = stage_meta; a.chunk_start = chunk_start;
   a.expert_counts = expert_counts; a.expert_offsets = expert_offsets; a.recv_row_src = recv_row_src; a.recv_w = recv_weights;

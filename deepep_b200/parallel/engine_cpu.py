@@ -44,7 +44,9 @@ class CpuPlan:
     has_weights: bool = False
     low_latency: bool = False
     rank_matrix: Optional[torch.Tensor] = None
+    rank_prefix: Optional[torch.Tensor] = None
     send_chunk_prefix: Optional[torch.Tensor] = None
+    recv_src_idx: Optional[torch.Tensor] = None
     exact_rows: int = 0                 # rows that carry data; ``num_rows`` is larger when the counts were not read back
 
     def tensors(self):
@@ -113,6 +115,8 @@ class CpuEngine:
                 dst = torch.where(ok, torch.div(i.clamp(min=0), local, rounding_mode="floor"), torch.full_like(i, -1))
                 hits.append(torch.stack([(dst == d).any(dim=1) for d in range(self.world)], dim=1))      # [T_r, P]
             plan.rank_matrix = torch.stack([h.sum(0) for h in hits]).int()
+            plan.rank_prefix = torch.cumsum(plan.rank_matrix, dim=0).int()
+            plan.recv_src_idx = torch.div(plan.recv_row_src, k, rounding_mode="floor") % self.max_tokens
             mine = hits[self.rank]
             pos = torch.cumsum(mine.int(), 0) - 1
             plan.send_slot = torch.where(mine, pos, torch.full_like(pos, -1)).int()

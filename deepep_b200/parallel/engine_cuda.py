@@ -12,7 +12,6 @@ single host synchronisation of a fresh dispatch
 """
 from __future__ import annotations
 
-import contextlib
 from dataclasses import dataclass
 import os
 from typing import List, Optional, Sequence, Tuple
@@ -75,8 +74,11 @@ class RoutingPlan:
     local_row: Optional[torch.Tensor] = None
     local_row_ptr: int = 0
     topk_w: Optional[torch.Tensor] = None
+    # what the V1 handle is made of, written by the routing pass
     rank_matrix: Optional[torch.Tensor] = None
+    rank_prefix: Optional[torch.Tensor] = None
     send_chunk_prefix: Optional[torch.Tensor] = None
+    recv_src_idx: Optional[torch.Tensor] = None
 
     def tensors(self):
         return [t for t in (self.topk_idx, self.send_slot, self.slot_row, self.stage_meta, self.chunk_start, self.rank_tokens,
@@ -276,8 +278,9 @@ class CudaEngine:
                expand: bool = True, alignment: int = 1, cpu_sync: bool = True, blocks: int = 0, stream=None,
                rank_matrix: bool = False) -> List[RoutingPlan]:
         """``rank_matrix``: also count, on every rank, the tokens each source sends to each rank (``plan.rank_matrix
-        [P, P]``, what the V1 handle's ``rank_prefix_matrix`` is built from) and keep this rank's per-chunk send
-        prefixes (``plan.send_chunk_prefix [P, chunks]``)."""
+        [P, P]`` and its inclusive prefix over the sources, the V1 handle's ``rank_prefix_matrix``), this rank's per-chunk send
+        prefixes (``plan.send_chunk_prefix [P, chunks]``) and, in the rank layout, the source token of every row
+        (``plan.recv_src_idx``)."""
         C, lay, dev = self.C, self.layout, self.device
         P, K = self.world, lay.topk
         local = num_experts // P
@@ -300,7 +303,11 @@ class CudaEngine:
                         if topk_w[i] is not None else None),
                 recv_idx=None if expand else torch.empty((rcap, K), dtype=torch.int64, device=dev),
                 has_weights=topk_w[i] is not None)
-            plan.rank_matrix = torch.empty((P, P), **i32) if rank_matrix else None      # cleared by the launcher, on its stream
+            if rank_matrix:
+                tiles = -(-max(T, 1) // C.chunk_tokens)
+                parts = torch.empty((2 * P * P + P * tiles + rcap,), **i32).split([P * P, P * P, P * tiles, rcap])
+                plan.rank_matrix, plan.rank_prefix = parts[0].view(P, P), parts[1].view(P, P)
+                plan.send_chunk_prefix, plan.recv_src_idx = parts[2].view(P, tiles), parts[3]
             plans.append(plan)
             sc = self._scratch[i]
             args.append(dict(topk_idx=idx.data_ptr(), topk_w=_ptr(topk_w[i]), T=T, E=num_experts, K=K, expand=int(expand),
@@ -311,15 +318,11 @@ class CudaEngine:
                              rank_rows=plan.rank_rows.data_ptr(), expert_counts=plan.expert_counts.data_ptr(),
                              expert_offsets=plan.expert_offsets.data_ptr(), recv_row_src=plan.recv_row_src.data_ptr(),
                              recv_w=_ptr(plan.recv_w), recv_idx=_ptr(plan.recv_idx), rcap=rcap,
-                             rank_matrix=_ptr(plan.rank_matrix)))
+                             rank_matrix=_ptr(plan.rank_matrix), rank_prefix=_ptr(plan.rank_prefix),
+                             send_prefix=_ptr(plan.send_chunk_prefix), recv_src=_ptr(plan.recv_src_idx)))
         # the layout pass is a chain of short phases over (source, tile) tasks: P x T / 64 of them, a few microseconds each
         nblocks = blocks or max(1, min(128, self.sm_count // self.n))
         self._timed("notify", stream, lambda: C.notify(lay, self.sessions, args, nblocks, self._stream(stream), self._device_profile))
-        if rank_matrix:       # the scratch is reused by the next call: keep this rank's per-chunk send prefixes with the plan
-            for plan, sc in zip(plans, self._scratch):
-                tiles = -(-max(plan.num_tokens, 1) // C.chunk_tokens)
-                with torch.cuda.stream(stream) if stream is not None else contextlib.nullcontext():
-                    plan.send_chunk_prefix = sc["own_hits"][:tiles * P].view(tiles, P).t().contiguous()
         if cpu_sync:
             self._host_wait(stream, "the routing layout pass")
             self.check_status()

@@ -95,7 +95,7 @@ def test_routing_plan_of_one_rank(tokens, experts, topk, expand, alignment):
     assert torch.equal(plan.chunk_start[0].cpu().long(), starts[torch.arange(tiles + 1).mul(64).clamp(max=tokens)])
     assert torch.equal(plan.send_chunk_prefix[0].cpu().long(), starts[torch.arange(tiles) * 64])
     assert plan.rank_rows.tolist() == [0, int(hit.sum())] and plan.rank_tokens.tolist() == [tokens]
-    assert plan.rank_matrix.tolist() == [[int(hit.sum())]] and plan.num_staged_rows == int(hit.sum())
+    assert plan.rank_matrix.tolist() == plan.rank_prefix.tolist() == [[int(hit.sum())]] and plan.num_staged_rows == int(hit.sum())
     t, k = valid.nonzero(as_tuple=True)
     counts = torch.bincount(idx[t, k], minlength=experts)
     assert plan.expert_counts.cpu().tolist() == counts.tolist() == plan.expert_counts_list
@@ -118,10 +118,49 @@ def test_routing_plan_of_one_rank(tokens, experts, topk, expand, alignment):
         assert torch.equal(meta[staged[t], at], row | k << 27) and torch.equal(meta[staged[hit], 1], valid.sum(1)[hit])
     else:
         assert plan.num_rows == int(hit.sum()) and torch.equal(src[:plan.num_rows], hit.nonzero()[:, 0] * topk)
+        assert torch.equal(plan.recv_src_idx[:plan.num_rows].cpu().long(), hit.nonzero()[:, 0])
         assert torch.equal(row_w[:plan.num_rows], torch.where(valid, w, torch.zeros(()))[hit])
         assert torch.equal(plan.recv_idx[:plan.num_rows].cpu(), torch.where(valid, idx, torch.full_like(idx, -1))[hit])
         assert torch.equal(meta[staged[hit], 2], staged[hit]) and torch.equal(meta[staged[hit], 3], mask[hit])
     assert torch.equal(plan.slot_row.cpu().long(), slot_row) and torch.equal(meta[staged[hit], 0], hit.nonzero()[:, 0])
+
+
+def test_v1_tables_of_several_ranks():
+    """What the V1 handle is made of, with ranks of unequal size and one without tokens."""
+    from deepep_b200.parallel.virtual import VirtualWorld
+
+    world, tokens, experts, topk, dev = 4, [130, 0, 64, 201], 16, 3, torch.device("cuda")
+    idx = [make_routes("empty", t, experts, topk, world, r) for r, t in enumerate(tokens)]
+    with VirtualWorld(world, max(tokens), 64, topk, timeout=10.0) as vw:
+        plans = vw.engine.notify([i.to(dev) for i in idx], [make_weights(t, topk, 1).to(dev) for t in tokens], experts, expand=False,
+                                 rank_matrix=True)
+        torch.cuda.synchronize()
+        vw.engine.check_status()
+    hits = [torch.stack([((i >= 0) & (i // (experts // world) == d)).any(1) for d in range(world)], 1).long() for i in idx]   # [T, P]
+    matrix = torch.stack([h.sum(0) for h in hits])
+    for r, plan in enumerate(plans):
+        assert torch.equal(plan.rank_matrix.cpu().long(), matrix) and torch.equal(plan.rank_prefix.cpu().long(), matrix.cumsum(0))
+        starts = torch.cat((torch.zeros((1, world), dtype=torch.long), hits[r].cumsum(0)))
+        tiles = torch.arange(max(1, -(-tokens[r] // 64))) * 64
+        assert torch.equal(plan.send_chunk_prefix.cpu().long(), starts[tiles].t())
+        sources = torch.cat([h[:, r].nonzero()[:, 0] for h in hits])
+        assert torch.equal(plan.recv_src_idx[:plan.num_rows].cpu().long(), sources)
+
+
+@pytest.mark.parametrize("tokens,experts,topk,world", [(0, 8, 2, 2), (1, 1024, 16, 8), (40000, 24, 5, 1), (16385, 1000, 8, 4)])
+def test_v1_layout(tokens, experts, topk, world):
+    from deepep_b200.ops import load_native
+
+    dev = torch.device("cuda")
+    idx = torch.randint(-2, experts + 2, (tokens, topk), generator=torch.Generator().manual_seed(tokens)).to(dev)
+    per_rank, per_expert = (torch.full((n,), 77, dtype=torch.int32, device=dev) for n in (world, experts))
+    in_rank = torch.ones((tokens, world), dtype=torch.bool, device=dev)
+    load_native().layout(idx.data_ptr(), tokens, topk, experts, world, per_rank.data_ptr(), per_expert.data_ptr(), in_rank.data_ptr(),
+                         torch.cuda.current_stream().cuda_stream)
+    ok = (idx >= 0) & (idx < experts)
+    want = torch.stack([(ok & (idx // (experts // world) == r)).any(1) for r in range(world)], 1)
+    assert torch.equal(in_rank, want) and torch.equal(per_rank.long(), want.sum(0))
+    assert torch.equal(per_expert.long(), torch.bincount(idx[ok], minlength=experts))
 
 
 @pytest.mark.parametrize("dmode", [0, 1, 2])
