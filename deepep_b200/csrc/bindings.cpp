@@ -125,6 +125,7 @@ void op_combine(const WsLayout& lay, const std::vector<py::object>& sessions, co
     CombineArgs& a = p.r[i];
     a.ctx = ctx_of(sessions[i]);
     a.x = ptr<const __nv_bfloat16>(d, "x"); a.w = ptr<const float>(d, "w");
+    a.row_w = ptr<const float>(d, "row_w");
     a.stage_meta = ptr<const int>(d, "stage_meta"); a.rank_rows = ptr<const int>(d, "rank_rows");
     a.rank_tokens = ptr<const int>(d, "rank_tokens"); a.send_slot = ptr<const int>(d, "send_slot");
     a.slot_row = ptr<const int>(d, "slot_row"); a.topk_idx = ptr<const long long>(d, "topk_idx");
@@ -137,6 +138,8 @@ void op_combine(const WsLayout& lay, const std::vector<py::object>& sessions, co
     if (!a.stage_meta || !a.rank_rows || !a.rank_tokens || !a.send_slot || ((!a.topk_idx || !a.out) && a.T > 0))
       throw std::invalid_argument("combine: a required pointer is missing");
     if (p.whole_gpu && lay.world == 1 && a.expand && !a.slot_row && a.T > 0) throw std::invalid_argument("combine: slot_row is missing");
+    if (a.row_w && !(p.whole_gpu && lay.world == 1 && n == 1 && a.expand && local_direct && !profile))
+      throw std::invalid_argument("combine: rows are weighed by a single rank's kernel only");
     if (a.E < a.ctx.world) throw std::invalid_argument("combine: num_experts is missing");
   }
   check(launch_combine(p, n, reinterpret_cast<cudaStream_t>(stream)), "ep_combine_ht launch");

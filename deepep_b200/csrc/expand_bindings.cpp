@@ -47,6 +47,20 @@ void bind_expand(py::module_& m) {
     if ((a | out | b | prod) % 16) throw std::invalid_argument("row_scale: rows must start on a 16-byte boundary");
     check_launch(launch_row_scale(p, blocks, reinterpret_cast<cudaStream_t>(stream)), "row_scale");
   });
+  // `dy` and `dw` may be null, not both.
+  m.def("return_grad", [](uintptr_t g, uintptr_t y, uintptr_t w, uintptr_t slot_row, uintptr_t dy, uintptr_t dw, int tokens, int topk,
+                          long long rows, int width, uintptr_t stream) {
+    ReturnGradParams p{};
+    p.g = reinterpret_cast<const __nv_bfloat16*>(g); p.y = reinterpret_cast<const __nv_bfloat16*>(y);
+    p.w = reinterpret_cast<const float*>(w); p.slot_row = reinterpret_cast<const int*>(slot_row);
+    p.dy = reinterpret_cast<__nv_bfloat16*>(dy); p.dw = reinterpret_cast<float*>(dw);
+    p.rows = rows; p.tokens = tokens; p.topk = topk; p.width = width;
+    if (tokens < 0 || rows < 0 || topk < 1 || topk > kMaxTopk) throw std::invalid_argument("return_grad: tokens, rows or top-k out of range");
+    if (width < 8 || width % 8 || width > 8192) throw std::invalid_argument("return_grad: the width must be a multiple of 8 up to 8192");
+    if (tokens > 0 && rows > 0 && (!g || !w || !slot_row || (!dy && !dw) || (dw && !y))) throw std::invalid_argument("return_grad: a tensor is missing");
+    if ((g | y | dy) % 16) throw std::invalid_argument("return_grad: rows must start on a 16-byte boundary");
+    check_launch(launch_return_grad(p, reinterpret_cast<cudaStream_t>(stream)), "return_grad");
+  });
   m.def("expand_scratch", &expand_scratch, py::arg("rows"), py::arg("experts"), py::arg("topk"));
   m.def("expand", [](const py::dict& d, int blocks, uintptr_t stream) {
     ExpandParams p{};

@@ -96,6 +96,7 @@ struct CombineArgs {
   RankCtx ctx;
   const __nv_bfloat16* x;      // [R][H] expert outputs
   const float* w;              // [R] (expanded) / [R][K] (rank layout) value channel, or null
+  const float* row_w;          // [R] weights that the rows are multiplied by on the way (one rank, expanded, whole_gpu), or null
   const int* stage_meta;
   const int* rank_tokens;
   const int* rank_rows;        // [P + 1] exclusive prefix of the staged rows per source

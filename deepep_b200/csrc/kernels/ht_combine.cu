@@ -33,6 +33,14 @@ __device__ __forceinline__ void add_bf16x8(float acc[8], const int4& v) {
     acc[2 * i + 1] += __high2float(h[i]);
   }
 }
+__device__ __forceinline__ int4 scale_bf16x8(const int4& v, __nv_bfloat162 w) {     // (a product of two bf16 values is rounded once)
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+  int4 out;
+  __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&out);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) o[i] = __hmul2(h[i], w);
+  return out;
+}
 __device__ __forceinline__ int4 pack_bf16x8(const float acc[8]) {
   int4 out;
   __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&out);
@@ -418,7 +426,10 @@ __global__ void __launch_bounds__(kCombineThreads, 1) ep_combine_local_kernel(co
 // U = 1, B = 3 and 8.7; 4096 of 4096, top-1 30 / 20.5 and 17.2.
 constexpr int kLocalCombineThreads = 256;
 
-template <int U, int B>
+//
+// kWeighted (the training layer): every row is multiplied by its weight on the way, the weight and the product rounded to bf16, as if
+// a pass over the rows had done it before; that pass alone reads and writes every row once more.
+template <int U, int B, bool kWeighted>
 __global__ void __launch_bounds__(kLocalCombineThreads) ep_combine_items_kernel(const __grid_constant__ CombineParams p) {
   const CombineArgs& a = p.r[0];
   const int H = p.lay.hidden, K = a.K, lane = threadIdx.x & 31, units = H / 8;
@@ -434,6 +445,8 @@ __global__ void __launch_bounds__(kLocalCombineThreads) ep_combine_items_kernel(
   if (row >= 0 && a.x_rows > 0 && !DEP_INDEX_OK(a.ctx, row, a.x_rows, kOpCombine, 0)) row = 0;
   const unsigned mask = __ballot_sync(0xffffffffu, row >= 0);
   const int4* x = reinterpret_cast<const int4*>(a.x);
+  float weight = 1.f;
+  if constexpr (kWeighted) weight = row >= 0 ? __bfloat162float(__float2bfloat16_rn(__ldg(a.row_w + row))) : 0.f;
   float sum[U][8];
 #pragma unroll
   for (int i = 0; i < U; ++i)
@@ -441,11 +454,13 @@ __global__ void __launch_bounds__(kLocalCombineThreads) ep_combine_items_kernel(
     for (int e = 0; e < 8; ++e) sum[i][e] = 0.f;
   for (unsigned m = mask; m;) {          // B rows in flight, added in slot order
     int4 v[B][U];
+    float w[B];
     const int n = __popc(m);
 #pragma unroll
     for (int q = 0; q < B; ++q) {
       if (q < n) {
         const int4* src = x + (size_t)__shfl_sync(0xffffffffu, row, __ffs(m) - 1) * units;
+        if constexpr (kWeighted) w[q] = __shfl_sync(0xffffffffu, weight, __ffs(m) - 1);
         m &= m - 1;
 #pragma unroll
         for (int i = 0; i < U; ++i) {
@@ -459,7 +474,10 @@ __global__ void __launch_bounds__(kLocalCombineThreads) ep_combine_items_kernel(
       if (q < n) {
 #pragma unroll
         for (int i = 0; i < U; ++i)
-          if (u0 + i * 32 + lane < u_end) add_bf16x8(sum[i], v[q][i]);
+          if (u0 + i * 32 + lane < u_end) {
+            if constexpr (kWeighted) v[q][i] = scale_bf16x8(v[q][i], __float2bfloat162_rn(w[q]));
+            add_bf16x8(sum[i], v[q][i]);
+          }
       }
     }
   }
@@ -494,7 +512,9 @@ cudaError_t launch_items(const CombineParams& p, cudaStream_t stream) {
   const int spans = (p.lay.hidden / 8 + 32 * U - 1) / (32 * U), per = kLocalCombineThreads / 32;
   const long long items = (long long)std::max(0, std::min(p.r[0].T, p.t_end) - p.t_begin) * spans;
   if (items == 0) return cudaSuccess;
-  ep_combine_items_kernel<U, B><<<(unsigned)((items + per - 1) / per), kLocalCombineThreads, 0, stream>>>(p);
+  const unsigned grid = (unsigned)((items + per - 1) / per);
+  if (p.r[0].row_w) ep_combine_items_kernel<U, B, true><<<grid, kLocalCombineThreads, 0, stream>>>(p);
+  else ep_combine_items_kernel<U, B, false><<<grid, kLocalCombineThreads, 0, stream>>>(p);
   return cudaGetLastError();
 }
 

@@ -24,6 +24,19 @@ struct RowScaleParams {
   long long rows;
   int width, pad;              // width: a multiple of 8
 };
+// Backward of a combine with weighed rows: the gradient g of a token's sum goes to the rows of its slots, dy[row] = g * w[row], and
+// dw[row] = sum(g * y[row]).  The weight is rounded to bf16 first, every product once; the sum is taken in fp32 and rounded to bf16.
+struct ReturnGradParams {
+  const __nv_bfloat16* g;      // [tokens][width]
+  const __nv_bfloat16* y;      // [rows][width]
+  const float* w;              // [rows]
+  const int* slot_row;         // [tokens][topk] row of every slot, -1 for none
+  __nv_bfloat16* dy;           // [rows][width], or null
+  float* dw;                   // [rows], or null
+  long long rows;
+  int tokens, topk, width, pad;
+};
+cudaError_t launch_return_grad(const ReturnGradParams& p, cudaStream_t stream);
 cudaError_t launch_row_scale(const RowScaleParams& p, int blocks, cudaStream_t stream);
 cudaError_t launch_swiglu(const SwigluParams& p, bool backward, int blocks, cudaStream_t stream);
 

@@ -99,10 +99,43 @@ class _WeighRows(torch.autograd.Function):
         return out, None if terms is None else terms.sum(1, keepdim=True).to(weights.dtype).squeeze(1)
 
 
-def _launch(op: str, like: torch.Tensor, *args) -> None:
+class _WeighAndCombine(torch.autograd.Function):
+    """``_WeighRows`` and ``_Combine`` in one kernel each way, for a single rank: the products are never stored, and neither the rows
+    of the gradient nor the terms of the weights' gradients are.  The products are rounded as there."""
+
+    @staticmethod
+    def forward(ctx, buffer: ElasticBuffer, rows, weights, handle):
+        out, _, _ = buffer.combine(rows, handle, _row_weights=weights)
+        ctx.buffer, ctx.handle = buffer, handle
+        ctx.save_for_backward(rows, weights)
+        return out
+
+    @staticmethod
+    def backward(ctx, grad):
+        buffer, handle, (rows, weights) = ctx.buffer, ctx.handle, ctx.saved_tensors
+        need = ctx.needs_input_grad[1:3]
+        again = torch.is_grad_enabled()                  # the gradient will be differentiated itself
+        if again or not (_weighable(rows, weights, torch.bfloat16) and _ordinary(grad)):
+            grad_rows = buffer.dispatch(grad.to(torch.bfloat16).contiguous(), handle=handle)[0]
+            with torch.enable_grad():
+                out = rows * weights.unsqueeze(1).to(rows.dtype)
+            grads = iter(torch.autograd.grad(out, [t for t, n in zip((rows, weights), need) if n], grad_rows, create_graph=again))
+            return (None, *(next(grads) if n else None for n in need), None)
+        plan = buffer._live_plan(handle)
+        grad = _readable(grad.to(torch.bfloat16))
+        out = torch.empty_like(rows) if need[0] else None
+        grad_w = torch.empty_like(weights) if need[1] else None
+        _launch("return_grad", rows, grad.data_ptr(), rows.data_ptr(), weights.data_ptr(), plan.slot_row.data_ptr(),
+                0 if out is None else out.data_ptr(), 0 if grad_w is None else grad_w.data_ptr(), plan.num_tokens, plan.num_topk,
+                *rows.shape, blocks=False)
+        return None, out, grad_w, None
+
+
+def _launch(op: str, like: torch.Tensor, *args, blocks: bool = True) -> None:
     """Launches a kernel on the current stream of the device of ``like``."""
     kernel, index = getattr(require_native("the training layer"), op), like.get_device()
-    args += _blocks(index), torch._C._cuda_getCurrentRawStream(index)
+    args += (_blocks(index),) if blocks else ()
+    args += (torch._C._cuda_getCurrentRawStream(index),)
     if index == torch.cuda.current_device():
         kernel(*args)
     else:
@@ -151,14 +184,23 @@ def _activate(gate_up: torch.Tensor) -> torch.Tensor:
     return _separate_operations(gate_up)
 
 
-def _weigh(rows: torch.Tensor, weights: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
-    """``rows`` times their weights rounded to ``dtype``.  The kernel takes contiguous, 16-byte aligned bf16 rows of a multiple of
-    8 values and fp32 weights of the same number; anything else goes through torch, with the same results."""
-    if (_ordinary(rows, weights) and rows.is_cuda and rows.device == weights.device and rows.dtype == dtype == torch.bfloat16
+def _weighable(rows: torch.Tensor, weights: torch.Tensor, dtype: torch.dtype) -> bool:
+    """Contiguous, 16-byte aligned bf16 rows of a multiple of 8 values and fp32 weights of the same number, in an ordinary call."""
+    return (_ordinary(rows, weights) and rows.is_cuda and rows.device == weights.device and rows.dtype == dtype == torch.bfloat16
             and weights.dtype == torch.float32 and rows.dim() == 2 and weights.shape == rows.shape[:1] and rows.numel() > 0
-            and rows.shape[1] % 8 == 0 and rows.is_contiguous() and weights.is_contiguous() and rows.data_ptr() % 16 == 0):
-        return _WeighRows.apply(rows, weights)
-    return rows * weights.unsqueeze(1).to(dtype)
+            and rows.shape[1] % 8 == 0 and rows.is_contiguous() and weights.is_contiguous() and rows.data_ptr() % 16 == 0)
+
+
+def _weigh(rows: torch.Tensor, weights: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """``rows`` times their weights rounded to ``dtype``, by a kernel where it takes them, else through torch with the same results."""
+    return _WeighRows.apply(rows, weights) if _weighable(rows, weights, dtype) else rows * weights.unsqueeze(1).to(dtype)
+
+
+def _weigh_and_combine(buffer: ElasticBuffer, rows: torch.Tensor, weights: torch.Tensor, handle, dtype: torch.dtype) -> torch.Tensor:
+    weighs = getattr(buffer.engine, "weighs_rows", None)
+    if weighs is not None and _weighable(rows, weights, dtype) and weighs(handle._plan, buffer.num_sms):
+        return _WeighAndCombine.apply(buffer, rows, weights, handle)
+    return _Combine.apply(buffer, _weigh(rows, weights, dtype).contiguous(), handle)
 
 
 class ExpertParallelMoE(torch.nn.Module):
@@ -205,8 +247,8 @@ class ExpertParallelMoE(torch.nn.Module):
     def forward(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: torch.Tensor) -> torch.Tensor:
         holder = {}
         recv_x, recv_w, psum = _Dispatch.apply(self.buffer, x, topk_idx, topk_weights, self.num_experts, holder)
-        y = _weigh(self.experts(recv_x, psum, holder["handle"].num_recv_tokens_per_expert_list), recv_w, recv_x.dtype)
-        return _Combine.apply(self.buffer, y.contiguous(), holder["handle"])
+        y = self.experts(recv_x, psum, holder["handle"].num_recv_tokens_per_expert_list)
+        return _weigh_and_combine(self.buffer, y, recv_w, holder["handle"], recv_x.dtype)
 
 
 __all__ = ["ExpertParallelMoE"]

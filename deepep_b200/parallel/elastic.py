@@ -511,7 +511,7 @@ class ElasticBuffer:
     # ------------------------------------------------------------------ combine
     def combine(self, x, handle, topk_weights=None, bias=None, num_sms=0, num_qps=0, previous_event=None,
                 previous_event_before_epilogue=None, async_with_compute_stream=False, allocate_on_comm_stream=False,
-                combine_num_sms: int = 0, reduce_num_sms: int = 0):
+                combine_num_sms: int = 0, reduce_num_sms: int = 0, _row_weights=None):
         """Return every expert output row to its source token and reduce.
 
         ``combine_num_sms`` / ``reduce_num_sms`` (both or neither) set how many SMs return rows on the expert side and
@@ -561,8 +561,9 @@ class ElasticBuffer:
             else:
                 out, out_w = self.engine.combine([x], [plan], [topk_weights], bias=None if bias is None else [tuple(biases)],
                                                  blocks=num_sms or self.num_sms, stream=comm,
-                                                 **({"split": split} if split is not None else {}))[0]
-        event = self._leave(comm, async_with_compute_stream, [out, out_w, x, topk_weights] + [b for b in biases if b is not None],
+                                                 **({"split": split} if split is not None else {}),
+                                                 **({"row_weights": _row_weights} if _row_weights is not None else {}))[0]
+        event = self._leave(comm, async_with_compute_stream, [out, out_w, x, topk_weights, _row_weights] + [b for b in biases if b is not None],
                             handle, allocate_on_comm_stream)
         return out, out_w, event
 
@@ -577,6 +578,13 @@ class ElasticBuffer:
             raise TypeError("handle must be an EPHandle returned by dispatch")
         if handle._buffer_id != self._id:
             raise ValueError("the handle belongs to another buffer")
+
+    def _live_plan(self, handle):
+        """The plan of a handle of this buffer, checked like every call that takes one."""
+        self._alive()
+        self._own(handle)
+        handle._check_unchanged()
+        return handle._plan
 
     def _mode(self, x_data, x_sf) -> int:
         if x_sf is not None:

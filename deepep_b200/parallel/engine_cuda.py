@@ -367,9 +367,15 @@ class CudaEngine:
                                                                 self.local_direct, self._device_profile))
         return outs
 
+    def weighs_rows(self, plan: RoutingPlan, blocks: int = 0) -> bool:
+        """Whether ``combine`` takes ``row_weights`` for this plan, every row of which belongs to a slot."""
+        return (self.n == self.world == 1 and plan.expand and plan.alignment == 1 and plan.expert_counts_list is not None
+                and not plan.low_latency and self.local_direct and not blocks and not self.sm_budget and not self._device_profile)
+
     def combine(self, xs: Sequence[torch.Tensor], plans: Sequence[RoutingPlan], ws: Sequence[Optional[torch.Tensor]],
-                bias: Sequence = None, blocks: int = 0, stream=None, split: Optional[Tuple[int, int]] = None):
-        """``split`` = (expert-side sender blocks, source-side reducer blocks) overrides the default division."""
+                bias: Sequence = None, blocks: int = 0, stream=None, split: Optional[Tuple[int, int]] = None, row_weights=None):
+        """``split`` = (expert-side sender blocks, source-side reducer blocks) overrides the default division.  ``row_weights``
+        ``[rows]`` (``weighs_rows`` says when) multiply the rows, weight and product rounded to bf16."""
         lay, dev = self.layout, self.device
         H, K = lay.hidden, lay.topk
         whole = split is None and not blocks and not self.sm_budget
@@ -388,7 +394,7 @@ class CudaEngine:
                              topk_idx=plan.topk_idx.data_ptr(), T=T,
                              meta_stride=plan.meta_stride, K=K, E=plan.num_experts, expand=int(plan.expand),
                              bias0=_ptr(b0), bias1=_ptr(b1), out=out.data_ptr(), out_w=_ptr(out_w), x_rows=xs[i].shape[0],
-                             whole=int(whole)))
+                             row_w=_ptr(row_weights), whole=int(whole)))
         send, recv = self.split_blocks(blocks, self.combine_send_fraction, self.combine_blocks)
         if split is not None:
             limit = max(2, self.sm_count // self.n)

@@ -296,6 +296,49 @@ def test_weighted_rows(rows, width):
                 assert _same_values(a, b)
 
 
+@pytest.mark.parametrize("tokens,hidden,experts,topk", [(1, 8, 2, 1), (33, 264, 9, 3), (130, 2056, 40, 7), (64, 4096, 64, 6),
+                                                        (17, 8192, 32, 16), (300, 1024, 8, 1)])
+def test_weighed_combine(filled_outputs, tokens, hidden, experts, topk):
+    """Sums and row gradients as from the separate kernels bit for bit.  The weights' gradients are sums of the same bf16 terms in
+    another order, rounded to bf16: fp32 sums of n terms differ by at most 2 n 2^-24 of the sum of their magnitudes, and the rounding
+    adds half a step of 2^-8 on either side."""
+    from deepep_b200 import ElasticBuffer
+    from deepep_b200.models import moe_layer as M
+
+    dev = torch.device("cuda")
+    g = torch.Generator().manual_seed(tokens)
+    idx, w = make_routes("empty" if tokens > 1 else "random", tokens, experts, topk, 1, 3).to(dev), make_weights(tokens, topk, 4).to(dev)
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=max(tokens, 300), hidden=hidden, num_topk=topk, explicitly_destroy=True)
+    x = torch.zeros((tokens, hidden), dtype=torch.bfloat16, device=dev)
+    _, _, recv_w, handle, _ = buf.dispatch(x, topk_idx=idx, topk_weights=w, num_experts=experts, do_expand=True)
+    rows = torch.randn((handle._plan.num_rows, hidden), generator=g).bfloat16().to(dev)
+    grad = torch.randn((tokens, hidden), generator=g).bfloat16().to(dev)
+
+    def fused(a, b):
+        out = M._weigh_and_combine(buf, a, b, handle, torch.bfloat16)
+        assert type(out.grad_fn).__name__ == "_WeighAndCombineBackward"
+        return out
+
+    def separate(a, b):
+        return M._Combine.apply(buf, M._weigh(a, b, torch.bfloat16), handle)
+
+    for which in ((True, True), (True, False), (False, True)):
+        for again in (False, True):
+            got = []
+            for f in (fused, separate):
+                a, b = rows.clone().requires_grad_(which[0]), recv_w.clone().requires_grad_(which[1])
+                out = f(a, b)
+                got.append((out, *torch.autograd.grad(out, [t for t in (a, b) if t.requires_grad], grad, create_graph=again)))
+            for name, p, q in zip(["out"] + [n for n, need in zip(("rows", "weights"), which) if need], *got):
+                if name == "weights":
+                    token = handle._plan.recv_row_src[:rows.shape[0]].long() // topk
+                    size = (rows.float() * grad.float()[token]).abs().sum(1)
+                    assert bool(((p - q).abs() <= q.abs() * 2.0 ** -8 + size * hidden * 2.0 ** -23).all())
+                else:
+                    assert bits_equal(p, q), (name, which, again)
+    buf.destroy()
+
+
 @pytest.fixture
 def filled_outputs(monkeypatch):
     """Whatever the engine allocates holds 0x55 in every byte before a kernel sees it."""
