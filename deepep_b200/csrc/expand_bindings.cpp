@@ -23,7 +23,7 @@ void check_launch(cudaError_t e, const char* what) {
 
 void bind_expand(py::module_& m) {
   // `dh` null: h from gu; otherwise the gradient of gu.
-  m.def("swiglu", [](uintptr_t gu, uintptr_t dh, uintptr_t out, long long rows, int inter, int blocks, uintptr_t stream) {
+  m.def("swiglu", [](uintptr_t gu, uintptr_t dh, uintptr_t out, long long rows, int inter, uintptr_t stream) {
     SwigluParams p{};
     p.gu = reinterpret_cast<const __nv_bfloat16*>(gu);
     p.dh = reinterpret_cast<const __nv_bfloat16*>(dh);
@@ -32,7 +32,7 @@ void bind_expand(py::module_& m) {
     if (rows < 0 || inter < 8 || inter % 8) throw std::invalid_argument("swiglu: the width must be a positive multiple of 8");
     if (rows > 0 && (!gu || !out)) throw std::invalid_argument("swiglu: a tensor is missing");
     if ((gu | dh | out) % 16) throw std::invalid_argument("swiglu: rows must start on a 16-byte boundary");
-    check_launch(launch_swiglu(p, dh != 0, blocks, reinterpret_cast<cudaStream_t>(stream)), "swiglu");
+    check_launch(launch_swiglu(p, dh != 0, reinterpret_cast<cudaStream_t>(stream)), "swiglu");
   });
   // `out` and the pair `b`, `prod` may be null, not both.
   m.def("row_scale", [](uintptr_t a, uintptr_t w, uintptr_t out, uintptr_t b, uintptr_t prod, long long rows, int width, int blocks,

@@ -1,12 +1,14 @@
 // silu(gate) * up over rows of [gate | up], and its backward pass (see swiglu_api.h).
 //
 // The results are those of the separate bf16 operations, bit for bit: every intermediate that they would store (silu(gate),
-// dh * up) is rounded to bf16 here too, and the exponential and the division are the accurate ones.
+// dh * up) is rounded to bf16 here too.  silu(gate) is the gate times the reciprocal of 1 + exp(-gate), in the forward pass with the
+// fast exponential: a gate is one of 65536 values, and for every one of them the rounded product is that of the accurate exponential
+// and division (the tests go through all of them).  The backward pass needs the sigmoid in fp32 and takes the accurate exponential.
 //
-// One warp per row, 16-byte accesses: forward reads 4 and writes 2 bytes per value, backward reads 6 and writes 4.  The accurate
-// exponential and division bound it, not memory.  49152 rows of 1536: forward 99 us (4.6 TB/s; 75 us with the fast intrinsics,
-// whose results differ), backward 164 us (116 us).  As library passes over the two strided halves (silu, product, their gradients
-// and a concatenation): 382 and 575 us.
+// One 16-byte piece of every operand per thread, in as many blocks as that takes: forward reads 4 and writes 2 bytes per value,
+// backward reads 6 and writes 4.  Arithmetic and memory bound it about alike.  49152 rows of 1536: forward 85 us (5.3 TB/s), backward
+// 128 us (5.9 TB/s); with a division in either 99 and 146 us, and as warps that loop over rows 97 and 163 us.  As library passes over
+// the two strided halves (silu, product, their gradients and a concatenation): 382 and 575 us.
 #include "swiglu_api.h"
 
 namespace dep {
@@ -32,47 +34,32 @@ __device__ __forceinline__ float as_bf16(float v) { return __bfloat162float(__fl
 
 template <bool kBackward>
 __global__ void __launch_bounds__(kSwigluThreads) swiglu_kernel(const __grid_constant__ SwigluParams p) {
-  const int lane = threadIdx.x & 31, units = p.inter / 8;
-  const long long warps = (long long)gridDim.x * (kSwigluThreads / 32);
-  for (long long row = (long long)blockIdx.x * (kSwigluThreads / 32) + (threadIdx.x >> 5); row < p.rows; row += warps) {
-    const int4* gate = reinterpret_cast<const int4*>(p.gu) + row * 2 * units;
-    constexpr int U = 2;                       // 16-byte pieces of every operand in flight per lane
-    for (int u0 = lane; u0 < units; u0 += 32 * U) {
-      int4 g4[U], u4[U], d4[U];
+  const int units = p.inter / 8;
+  const long long i = (long long)blockIdx.x * kSwigluThreads + threadIdx.x, row = i / units;
+  if (row >= p.rows) return;
+  const int u = (int)(i - row * units);
+  const int4* gate = reinterpret_cast<const int4*>(p.gu) + row * 2 * units;
+  const int4 g4 = __ldg(gate + u), u4 = __ldg(gate + units + u);
+  int4 d4;
+  if (kBackward) d4 = __ldg(reinterpret_cast<const int4*>(p.dh) + i);
+  const Vec8 g = unpack8(g4), up = unpack8(u4);
+  if (!kBackward) {
+    Vec8 h;
 #pragma unroll
-      for (int i = 0; i < U; ++i) {
-        const int u = u0 + i * 32;
-        if (u < units) {
-          g4[i] = __ldg(gate + u);
-          u4[i] = __ldg(gate + units + u);
-          if (kBackward) d4[i] = __ldg(reinterpret_cast<const int4*>(p.dh) + row * units + u);
-        }
-      }
+    for (int e = 0; e < 8; ++e) h.v[e] = as_bf16(g.v[e] * __frcp_rn(1.f + __expf(-g.v[e]))) * up.v[e];
+    reinterpret_cast<int4*>(p.h)[i] = pack8(h);
+  } else {
+    const Vec8 d = unpack8(d4);
+    Vec8 dg, du;
 #pragma unroll
-      for (int i = 0; i < U; ++i) {
-        const int u = u0 + i * 32;
-        if (u >= units) break;
-        const Vec8 g = unpack8(g4[i]), up = unpack8(u4[i]);
-        if (!kBackward) {
-          Vec8 h;
-#pragma unroll
-          for (int e = 0; e < 8; ++e) h.v[e] = as_bf16(g.v[e] / (1.f + expf(-g.v[e]))) * up.v[e];
-          reinterpret_cast<int4*>(p.h)[row * units + u] = pack8(h);
-        } else {
-          const Vec8 d = unpack8(d4[i]);
-          Vec8 dg, du;
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float denom = 1.f + expf(-g.v[e]), s = 1.f / denom;
-            du.v[e] = d.v[e] * as_bf16(g.v[e] / denom);
-            dg.v[e] = as_bf16(d.v[e] * up.v[e]) * s * (1.f + g.v[e] * (1.f - s));
-          }
-          int4* out = reinterpret_cast<int4*>(p.dgu) + row * 2 * units;
-          out[u] = pack8(dg);
-          out[units + u] = pack8(du);
-        }
-      }
+    for (int e = 0; e < 8; ++e) {
+      const float s = __frcp_rn(1.f + expf(-g.v[e]));
+      du.v[e] = d.v[e] * as_bf16(g.v[e] * s);
+      dg.v[e] = as_bf16(d.v[e] * up.v[e]) * s * (1.f + g.v[e] * (1.f - s));
     }
+    int4* out = reinterpret_cast<int4*>(p.dgu) + row * 2 * units;
+    out[u] = pack8(dg);
+    out[units + u] = pack8(du);
   }
 }
 
@@ -212,10 +199,11 @@ cudaError_t launch_row_scale(const RowScaleParams& p, int blocks, cudaStream_t s
   return cudaGetLastError();
 }
 
-cudaError_t launch_swiglu(const SwigluParams& p, bool backward, int blocks, cudaStream_t stream) {
+cudaError_t launch_swiglu(const SwigluParams& p, bool backward, cudaStream_t stream) {
   if (p.rows == 0) return cudaSuccess;
-  if (backward) swiglu_kernel<true><<<blocks, kSwigluThreads, 0, stream>>>(p);
-  else swiglu_kernel<false><<<blocks, kSwigluThreads, 0, stream>>>(p);
+  const unsigned grid = (unsigned)((p.rows * (p.inter / 8) + kSwigluThreads - 1) / kSwigluThreads);
+  if (backward) swiglu_kernel<true><<<grid, kSwigluThreads, 0, stream>>>(p);
+  else swiglu_kernel<false><<<grid, kSwigluThreads, 0, stream>>>(p);
   return cudaGetLastError();
 }
 

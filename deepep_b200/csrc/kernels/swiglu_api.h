@@ -38,6 +38,6 @@ struct ReturnGradParams {
 };
 cudaError_t launch_return_grad(const ReturnGradParams& p, cudaStream_t stream);
 cudaError_t launch_row_scale(const RowScaleParams& p, int blocks, cudaStream_t stream);
-cudaError_t launch_swiglu(const SwigluParams& p, bool backward, int blocks, cudaStream_t stream);
+cudaError_t launch_swiglu(const SwigluParams& p, bool backward, cudaStream_t stream);
 
 }  // namespace dep

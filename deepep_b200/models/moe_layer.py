@@ -55,7 +55,7 @@ class _Swiglu(torch.autograd.Function):
         rows, width = gate_up.shape
         h = gate_up.new_empty((rows, width // 2))
         ctx.save_for_backward(gate_up)
-        _launch("swiglu", gate_up, gate_up.data_ptr(), 0, h.data_ptr(), rows, width // 2)
+        _launch("swiglu", gate_up, gate_up.data_ptr(), 0, h.data_ptr(), rows, width // 2, blocks=False)
         return h
 
     @staticmethod
@@ -67,7 +67,8 @@ class _Swiglu(torch.autograd.Function):
                 h = _separate_operations(gate_up)
             return torch.autograd.grad(h, gate_up, grad, create_graph=again)[0]
         grad, out = _readable(grad), torch.empty_like(gate_up)
-        _launch("swiglu", gate_up, gate_up.data_ptr(), grad.data_ptr(), out.data_ptr(), gate_up.shape[0], gate_up.shape[1] // 2)
+        _launch("swiglu", gate_up, gate_up.data_ptr(), grad.data_ptr(), out.data_ptr(), gate_up.shape[0], gate_up.shape[1] // 2,
+                blocks=False)
         return out
 
 
