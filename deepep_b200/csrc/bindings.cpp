@@ -3,6 +3,8 @@
 // Parity: csrc/bindings/module.cpp:17-95 of the reference (runtime factories + the
 // notify/dispatch/combine/low-latency op families, `runtime_protocol`).  Tensors cross this
 // boundary as raw device addresses (`tensor.data_ptr()`), so the module needs no libtorch.
+#include <atomic>
+#include <chrono>
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
@@ -61,8 +63,8 @@ void op_notify(const WsLayout& lay, const std::vector<py::object>& sessions, con
     a.send_prefix = ptr<int>(d, "send_prefix"); a.recv_src = ptr<int>(d, "recv_src");
     if (!a.rank_matrix != !a.rank_prefix || !a.rank_matrix != !a.send_prefix || !a.rank_matrix != !a.recv_src)
       throw std::invalid_argument("notify: the V1 handle's tensors come together");
-    a.mailbox = sessions[i].cast<Session&>().mailbox_device();
-    a.rcap = getl(d, "rcap");
+    a.rcap = getl(d, "rcap"); a.seq = geti(d, "seq");
+    a.mailbox = a.seq ? sessions[i].cast<Session&>().mailbox_device() : nullptr;    // nobody else's number appears in it
     if (a.T < 0 || a.T > lay.max_tokens) throw std::invalid_argument("token count exceeds num_max_tokens_per_rank");
     if (a.K != lay.topk) throw std::invalid_argument("top-k width differs from the buffer's num_topk");
     if (a.E < a.ctx.world || a.E > kMaxExperts || a.E % a.ctx.world) throw std::invalid_argument("num_experts must be a multiple of the world size and at most 1024");
@@ -151,6 +153,42 @@ void op_barrier(const std::vector<py::object>& sessions, uintptr_t stream) {
   if (n < 1 || n > kMaxRanks) throw std::invalid_argument("1..8 sessions expected");
   for (int i = 0; i < n; ++i) p.r[i] = ctx_of(sessions[i]);
   check(launch_barrier(p, n, reinterpret_cast<cudaStream_t>(stream)), "ep_barrier launch");
+}
+
+// `waiter` continues after what is queued on `waited` (streams of `device`).  One event per thread and device, recorded anew every
+// time: a wait refers to the record before it, so the event is free again as soon as both calls have returned.
+struct JoinEvents {
+  cudaEvent_t of[64] = {};
+  ~JoinEvents() {
+    for (cudaEvent_t e : of)
+      if (e) cudaEventDestroy(e);
+  }
+};
+void stream_join(uintptr_t waiter, uintptr_t waited, int device) {
+  static thread_local JoinEvents events;
+  if (device < 0 || device >= 64) throw std::invalid_argument("device index out of range");
+  int current = -1;
+  check(cudaGetDevice(&current), "current device");
+  if (current != device) check(cudaSetDevice(device), "device");
+  cudaEvent_t& e = events.of[device];
+  cudaError_t err = e ? cudaSuccess : cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+  if (err == cudaSuccess) err = cudaEventRecord(e, reinterpret_cast<cudaStream_t>(waited));
+  if (err == cudaSuccess) err = cudaStreamWaitEvent(reinterpret_cast<cudaStream_t>(waiter), e, 0);
+  if (current != device) cudaSetDevice(current);
+  check(err, "stream order");
+}
+
+// Polls the sessions' mailboxes for the call number `seq`; false when `microseconds` passed first.
+bool wait_mailbox(const std::vector<py::object>& sessions, int seq, int microseconds) {
+  std::vector<const volatile int*> words;
+  for (const auto& s : sessions) words.push_back(s.cast<Session&>().mailbox_host() + 3);
+  py::gil_scoped_release unlocked;
+  const auto end = std::chrono::steady_clock::now() + std::chrono::microseconds(microseconds);
+  for (const volatile int* word : words)
+    for (unsigned spins = 0; *word != seq; ++spins)
+      if ((spins & 63u) == 63u && std::chrono::steady_clock::now() > end) return false;
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return true;
 }
 
 }  // namespace
@@ -255,6 +293,8 @@ PYBIND11_MODULE(_C, m) {
   m.def("combine", &op_combine, py::arg("layout"), py::arg("sessions"), py::arg("args"), py::arg("send_blocks"),
         py::arg("recv_blocks"), py::arg("stream"), py::arg("local_direct") = true, py::arg("profile") = false,
         py::arg("t_begin") = 0, py::arg("t_end") = -1);
+  m.def("stream_join", &stream_join, py::arg("waiter"), py::arg("waited"), py::arg("device"));
+  m.def("wait_mailbox", &wait_mailbox, py::arg("sessions"), py::arg("seq"), py::arg("microseconds"));
   m.attr("group_tokens") = kGroupTokens;
   m.attr("row_block") = kRowBlock;
   m.attr("dispatch_prof_words") = kDispatchProfWords;

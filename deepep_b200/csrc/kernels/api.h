@@ -19,6 +19,7 @@ struct NotifyArgs {
   int expand;                  // 1: rows per (token, slot) sorted by local expert; 0: rows per (source, token)
   int alignment;               // every local expert's row block starts at a multiple of this
   int meta_stride;             // ints per stage_meta record: 2 + max(2, min(K, E / world))
+  int seq;                     // the host's number of this call, which it waits for in the mailbox (0: it does not)
   // scratch owned by the buffer
   int* hist;                   // [P][NT][E]
   int* hits;                   // [P][NT]
@@ -43,7 +44,7 @@ struct NotifyArgs {
   int* rank_prefix;            // [P][P]
   int* send_prefix;            // [P][max(1, ceil(T / kChunkTokens))]
   int* recv_src;               // [rcap]
-  int* mailbox;                // mapped host memory: [0] rows, [1] staged rows, [2] max tokens, [3] epoch, [4..] counts
+  int* mailbox;                // mapped host memory: [0] rows, [1] staged rows, [2] max tokens, [3] seq (0: the epoch), [4..] counts
   long long rcap;
 };
 struct NotifyParams { WsLayout lay; int profile, pad; NotifyArgs r[kMaxRanks]; };   // profile: block 0 stamps its phases into Control::dbg[16..23]

@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(kNotifyThreads) ep_notify_kernel(const __grid_
         a.mailbox[1] = s_rank_base[P];
         a.mailbox[2] = maxT;
         __threadfence_system();
-        a.mailbox[3] = (int)(epoch & 0x7fffffff);
+        a.mailbox[3] = a.seq ? a.seq : (int)(epoch & 0x7fffffff);
         __threadfence_system();
       }
     }
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(kTileThreads) ep_notify_local_kernel(const __g
     }
     const int nt = (T + kChunkTokens - 1) / kChunkTokens;
     for (int i = nt + tid; i <= NT; i += kTileThreads) a.chunk_start[i] = hits;
-    // The epoch word tells a host that polls it that the counts are there; the records are complete when the launch is.  The fence
+    // The last word tells a host that polls it that the counts are there; the records are complete when the launch is.  The fence
     // takes 2 us, which the others spend on the records.
     __syncthreads();
     if (tid == kTileThreads - 1) {
@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(kTileThreads) ep_notify_local_kernel(const __g
       ctl->epoch[kOpNotify] = epoch;
       if (a.mailbox) {
         __threadfence_system();
-        a.mailbox[3] = (int)(epoch & 0x7fffffff);
+        a.mailbox[3] = a.seq ? a.seq : (int)(epoch & 0x7fffffff);
       }
     }
   }

@@ -50,7 +50,7 @@ struct LLDispatchArgs {
   const float* x_sf;           // [T][H/128] (mode 1)
   const long long* topk_idx;   // [T][K]
   const float* topk_w;         // [T][K]
-  int T, E, mode, pad;
+  int T, E, mode, seq;         // seq: the host's number of this call, which it waits for in the mailbox
   void* recv_x;                // [C][H]
   float* recv_sf;              // [C][H/128] or null
   float* recv_w;               // [C]
@@ -59,7 +59,7 @@ struct LLDispatchArgs {
   int* expert_offsets;         // [L + 1]
   int* num_rows;               // [1] device copy of the row count
   int* local_row;              // [T][K] output row of every slot whose expert lives on this rank, -1 otherwise (read by the combine)
-  int* mailbox;                // mapped host memory (may be null): [0] rows, [3] epoch, [4..] counts
+  int* mailbox;                // mapped host memory (may be null): [0] rows, [3] seq, [4..] counts
   long long capacity;          // rows available in recv_x
 };
 struct LLDispatchParams { WsLayout lay; int profile, pad; LLDispatchArgs r[kMaxRanks]; };   // profile: block 0 stamps its phases into Control::dbg[0..7]

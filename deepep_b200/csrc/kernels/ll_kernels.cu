@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
         if (a.mailbox) {
           a.mailbox[0] = all;
           __threadfence_system();
-          a.mailbox[3] = (int)(epoch & 0x7fffffff);
+          a.mailbox[3] = a.seq;
         }
       }
     }
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_local_kernel(const 
       if (a.mailbox) {
         a.mailbox[0] = all;
         __threadfence_system();
-        a.mailbox[3] = (int)(epoch & 0x7fffffff);
+        a.mailbox[3] = a.seq;
       }
       ctl->ll_disp_ack[0] = epoch;
       ctl->epoch[kOpLLDispatch] = epoch;

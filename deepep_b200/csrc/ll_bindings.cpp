@@ -45,7 +45,7 @@ void op_ll_dispatch(const WsLayout& lay, const std::vector<py::object>& sessions
     a.ctx = s.ctx();
     a.x = ptr<const void>(d, "x"); a.x_sf = ptr<const float>(d, "x_sf");
     a.topk_idx = ptr<const long long>(d, "topk_idx"); a.topk_w = ptr<const float>(d, "topk_w");
-    a.T = geti(d, "T"); a.E = geti(d, "E"); a.mode = geti(d, "mode");
+    a.T = geti(d, "T"); a.E = geti(d, "E"); a.mode = geti(d, "mode"); a.seq = geti(d, "seq");
     a.recv_x = ptr<void>(d, "recv_x"); a.recv_sf = ptr<float>(d, "recv_sf"); a.recv_w = ptr<float>(d, "recv_w");
     a.recv_row_src = ptr<int>(d, "recv_row_src"); a.expert_counts = ptr<int>(d, "expert_counts");
     a.expert_offsets = ptr<int>(d, "expert_offsets"); a.num_rows = ptr<int>(d, "num_rows"); a.local_row = ptr<int>(d, "local_row");

@@ -62,7 +62,7 @@ class EPHandle:
         # private: set by the buffer that created the handle
         self.metadata_version = METADATA_VERSION
         self.dedup_group_size = 1          # rank-level dedup: a token crosses the link once per destination GPU
-        self._plan = None
+        self._plan: Any = None
         self._buffer_id = None
         self._tokens = 0
         self._hidden = 0
@@ -90,6 +90,31 @@ class EPHandle:
         now = tuple(self._stamp(t) for t in self._tracked())
         if now != self._snapshots:
             raise RuntimeError("handle metadata (or its topk_idx) was modified in place after dispatch")
+
+
+class _FromPlan:
+    """A tensor of a handle that is made from its plan when somebody asks for it."""
+
+    def __init__(self, name: str, make):
+        self.name, self.make = name, make
+
+    def __get__(self, handle, owner=None):
+        if handle is None:
+            return self
+        made = handle.__dict__[self.name] = self.make(handle._plan)
+        return made
+
+
+_FROM_PLAN = dict(
+    psum_num_recv_tokens_per_scaleup_rank=lambda p: None if p.rank_rows is None else p.rank_rows[1:],
+    psum_num_recv_tokens_per_expert=lambda p: p.expert_offsets[1:],
+    num_unaligned_recv_tokens_per_expert=lambda p: p.expert_counts,
+    recv_src_metadata=lambda p: p.recv_row_src,
+    dst_buffer_slot_idx=lambda p: getattr(p, "slot_row", None),
+    token_metadata_at_forward=lambda p: getattr(p, "stage_meta", None),
+    channel_linked_list=lambda p: getattr(p, "chunk_start", None))
+for _name, _make in _FROM_PLAN.items():
+    setattr(EPHandle, _name, _FromPlan(_name, _make))
 
 
 def _timeout_seconds(default: float) -> float:
@@ -301,7 +326,7 @@ class ElasticBuffer:
         """The comm stream starts after ``previous_event`` (or after everything queued on the current stream)."""
         if self.runtime is None:
             return None
-        comm, cur = self.runtime.stream, torch.cuda.current_stream(self.device)
+        comm = self.runtime.stream
         waited = False
         for ev in (previous_event, previous_event_before_epilogue):
             h = _as_event(ev)
@@ -309,8 +334,19 @@ class ElasticBuffer:
                 comm.wait_event(h.event)
                 waited = True
         if not waited:
-            comm.wait_stream(cur)
+            self._order(comm, first_is_current=True)
         return comm
+
+    def _order(self, comm, first_is_current: bool) -> None:
+        """The communication stream continues after what is queued on the current stream, or the other way round."""
+        if isinstance(comm, torch.cuda.Stream):            # two native calls in place of an event object and five
+            index = self.device.index if self.device.index is not None else torch.cuda.current_device()
+            cur = torch._C._cuda_getCurrentRawStream(index)
+            self.engine.C.stream_join(*((comm.cuda_stream, cur) if first_is_current else (cur, comm.cuda_stream)), index)
+        elif first_is_current:
+            comm.wait_stream(torch.cuda.current_stream(self.device))
+        else:
+            torch.cuda.current_stream(self.device).wait_stream(comm)
 
     @staticmethod
     def _allocates_on_comm(allocate_on_comm_stream: bool, *events) -> bool:
@@ -326,11 +362,11 @@ class ElasticBuffer:
         ``resources`` and the tensors of ``handle``."""
         if comm is None:
             return EventOverlap()
-        cur = torch.cuda.current_stream(self.device)
         if async_with_compute_stream:
             return EventOverlap._from_resources(EventHandle(comm), (*resources, *handle._kept()))
-        cur.wait_stream(comm)
+        self._order(comm, first_is_current=False)
         if allocated_on_comm:
+            cur = torch.cuda.current_stream(self.device)
             resources = (*resources, *handle._kept())
             # The outputs belong to the communication stream's memory pool but will be used on the current stream: tell
             # the allocator, or it could hand a dropped block to the next communication kernel while compute still reads it.
@@ -497,12 +533,10 @@ class ElasticBuffer:
         return out_x, None, recv_w, h, event
 
     def _make_handle(self, plan, expand, num_experts, alignment, num_sms, topk_idx, tokens, low_latency) -> EPHandle:
-        counts = plan.expert_counts_list
         h = EPHandle(expand, num_experts, alignment, self.num_max_tokens_per_rank, num_sms, topk_idx,
-                     plan.num_staged_rows, plan.num_rows, counts,
-                     None if plan.rank_rows is None else plan.rank_rows[1:], plan.expert_offsets[1:],
-                     plan.expert_counts, plan.recv_row_src, getattr(plan, "slot_row", None),
-                     getattr(plan, "stage_meta", None), getattr(plan, "chunk_start", None), is_low_latency=low_latency)
+                     plan.num_staged_rows, plan.num_rows, plan.expert_counts_list, *[None] * len(_FROM_PLAN), is_low_latency=low_latency)
+        for name in _FROM_PLAN:
+            del h.__dict__[name]
         h._plan, h._buffer_id, h._tokens, h._hidden = plan, self._id, tokens, self.hidden
         h._owner = self      # a live handle keeps its buffer alive (replacing the caller's variable does not end the buffer)
         h._snapshot()

@@ -13,6 +13,8 @@ single host synchronisation of a fresh dispatch
 from __future__ import annotations
 
 from dataclasses import dataclass
+from functools import lru_cache
+import math
 import os
 from typing import List, Optional, Sequence, Tuple
 
@@ -43,9 +45,35 @@ class CommunicationError(RuntimeError):
     pass
 
 
+class _View:
+    """A tensor of a plan that lies in its ``slab``, made when somebody asks for it; the kernels get its address (``_address``)."""
+
+    def __init__(self, name: str):
+        self.name = name
+
+    def __get__(self, plan, owner=None):
+        if plan is None:
+            return self
+        if plan.slab is None:
+            return None
+        begin, shape = plan.views[self.name]
+        made = plan.slab[begin:begin + math.prod(shape)].view(shape)
+        plan.__dict__[self.name] = made
+        return made
+
+
+def _address(plan, name: str) -> int:
+    """Where the kernels find a tensor of the plan."""
+    views = getattr(plan, "views", None)
+    return getattr(plan, name).data_ptr() if views is None else plan.slab_ptr + 4 * views[name][0]
+
+
 @dataclass
 class RoutingPlan:
-    """Device-side routing metadata of one dispatch (what an ``EPHandle`` owns)."""
+    """Device-side routing metadata of one dispatch (what an ``EPHandle`` owns).  The int32 tables of the routing pass lie in one
+    allocation, ``slab``: ``send_slot [T, P]``, ``slot_row [T, K]``, ``stage_meta``, ``chunk_start``, ``rank_tokens [P]``,
+    ``rank_rows [P + 1]``, ``expert_counts [L]``, ``expert_offsets [L + 1]``, ``recv_row_src`` and, for the V1 handle,
+    ``rank_matrix``, ``rank_prefix``, ``send_chunk_prefix`` and ``recv_src_idx``."""
     num_tokens: int
     num_experts: int
     num_topk: int
@@ -56,15 +84,6 @@ class RoutingPlan:
     num_staged_rows: int
     expert_counts_list: Optional[List[int]]
     topk_idx: torch.Tensor
-    send_slot: Optional[torch.Tensor]
-    slot_row: Optional[torch.Tensor]
-    stage_meta: Optional[torch.Tensor]
-    chunk_start: Optional[torch.Tensor]
-    rank_tokens: Optional[torch.Tensor]
-    rank_rows: Optional[torch.Tensor]
-    expert_counts: torch.Tensor
-    expert_offsets: torch.Tensor
-    recv_row_src: torch.Tensor
     recv_w: Optional[torch.Tensor]
     recv_idx: Optional[torch.Tensor]
     has_weights: bool = False
@@ -74,21 +93,38 @@ class RoutingPlan:
     local_row: Optional[torch.Tensor] = None
     local_row_ptr: int = 0
     topk_w: Optional[torch.Tensor] = None
-    # what the V1 handle is made of, written by the routing pass
-    rank_matrix: Optional[torch.Tensor] = None
-    rank_prefix: Optional[torch.Tensor] = None
-    send_chunk_prefix: Optional[torch.Tensor] = None
-    recv_src_idx: Optional[torch.Tensor] = None
+    slab: Optional[torch.Tensor] = None
+    slab_ptr: int = 0
+    views: Optional[dict] = None        # name -> (first int, shape)
 
     def tensors(self):
-        return [t for t in (self.topk_idx, self.send_slot, self.slot_row, self.stage_meta, self.chunk_start, self.rank_tokens,
-                            self.rank_rows, self.expert_counts, self.expert_offsets, self.recv_row_src, self.recv_w,
-                            self.recv_idx) if t is not None]
+        """What the handle watches for changes (the tables of the slab share one version counter)."""
+        tables = (self.slab,) if self.slab is not None else (self.expert_counts, self.expert_offsets, self.recv_row_src)
+        return [t for t in (self.topk_idx, *tables, self.recv_w, self.recv_idx) if t is not None]
 
     def private_tensors(self):
         """What the kernels use besides: kept alive with the others, but not watched for changes."""
         own = None if self.local_row is self.num_rows_dev else self.local_row
-        return [t for t in (self.num_rows_dev, own, self.topk_w, self.rank_matrix) if t is not None]
+        return [t for t in (self.num_rows_dev, own, self.topk_w) if t is not None]
+
+
+for _name in ("send_slot", "slot_row", "stage_meta", "chunk_start", "rank_tokens", "rank_rows", "expert_counts", "expert_offsets",
+              "recv_row_src", "rank_matrix", "rank_prefix", "send_chunk_prefix", "recv_src_idx"):
+    setattr(RoutingPlan, _name, _View(_name))
+
+
+@lru_cache(maxsize=64)
+def _slab_layout(T: int, P: int, K: int, tokens: int, stride: int, tiles: int, local: int, rcap: int, v1_tiles: int):
+    """(ints in all, name -> (first int, shape)) of a plan's tables, each on a 16-byte boundary."""
+    shapes = dict(send_slot=(max(T, 1), P), slot_row=(max(T, 1), K), stage_meta=(P * tokens, stride), chunk_start=(P, tiles + 1),
+                  rank_tokens=(P,), rank_rows=(P + 1,), expert_counts=(local,), expert_offsets=(local + 1,), recv_row_src=(rcap,))
+    if v1_tiles:
+        shapes.update(rank_matrix=(P, P), rank_prefix=(P, P), send_chunk_prefix=(P, v1_tiles), recv_src_idx=(rcap,))
+    at, views = 0, {}
+    for name, shape in shapes.items():
+        views[name] = (at, shape)
+        at += -(-math.prod(shape) // 4) * 4
+    return at, views
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -101,6 +137,7 @@ COMBINE_SEND_FRACTION = {1: 0.0, 2: 0.5, 4: 0.6, 8: 0.6}
 
 
 class CudaEngine:
+    _calls = 0             # number of the last call whose counts the host waited for
     sm_budget = 0          # SMs that the dispatch and combine kernels stay within (0: no limit asked for)
 
     def __init__(self, sessions: Sequence, layout, device: torch.device, num_sms: int = 0, host_timeout: float = 300.0):
@@ -232,6 +269,18 @@ class CudaEngine:
         self._timings.clear()
         return out
 
+    def _next_call(self, awaited: bool) -> int:
+        """The number by which the host recognises a call's counts in the mailbox (0: it does not read them)."""
+        if awaited:
+            self._calls = self._calls % 0x3fffffff + 1
+        return self._calls if awaited else 0
+
+    def _await_counts(self, seq: int, stream, what: str) -> None:
+        """The host needs the counts of call ``seq``: they are in the mailbox before the kernel is done, so that is polled first
+        (the kernels take tens of microseconds); what takes longer is waited for with an event, and not for ever."""
+        if not self.C.wait_mailbox(self.sessions, seq, 5000):
+            self._host_wait(stream, what)
+
     def _host_wait(self, stream, what: str) -> None:
         """The host needs the results of what was just queued on ``stream``: wait for it, but not for ever."""
         from ..utils.hostwait import HostTimeout, wait_for_event
@@ -286,45 +335,40 @@ class CudaEngine:
         local = num_experts // P
         stride = 2 + max(2, min(K, local))
         rcap = self.row_capacity(num_experts, alignment, expand)
+        seq = self._next_call(cpu_sync)
         plans, args = [], []
         for i in range(self.n):
             idx = topk_idx[i]
             T = idx.shape[0]
-            i32 = dict(dtype=torch.int32, device=dev)
+            ints, views = _slab_layout(T, P, K, lay.max_tokens, stride, self._nt, local, rcap,
+                                       -(-max(T, 1) // C.chunk_tokens) if rank_matrix else 0)
+            slab = torch.empty((ints,), dtype=torch.int32, device=dev)
+            base = slab.data_ptr()
             plan = RoutingPlan(
                 num_tokens=T, num_experts=num_experts, num_topk=K, expand=expand, alignment=alignment, meta_stride=stride,
                 num_rows=rcap, num_staged_rows=0, expert_counts_list=None, topk_idx=idx,
-                send_slot=torch.empty((max(T, 1), P), **i32), slot_row=torch.empty((max(T, 1), K), **i32),
-                stage_meta=torch.empty((P * lay.max_tokens, stride), **i32),
-                chunk_start=torch.empty((P, self._nt + 1), **i32), rank_tokens=torch.empty((P,), **i32),
-                rank_rows=torch.empty((P + 1,), **i32), expert_counts=torch.empty((local,), **i32),
-                expert_offsets=torch.empty((local + 1,), **i32), recv_row_src=torch.empty((rcap,), **i32),
                 recv_w=(torch.empty((rcap,) if expand else (rcap, K), dtype=torch.float32, device=dev)
                         if topk_w[i] is not None else None),
                 recv_idx=None if expand else torch.empty((rcap, K), dtype=torch.int64, device=dev),
-                has_weights=topk_w[i] is not None)
-            if rank_matrix:
-                tiles = -(-max(T, 1) // C.chunk_tokens)
-                parts = torch.empty((2 * P * P + P * tiles + rcap,), **i32).split([P * P, P * P, P * tiles, rcap])
-                plan.rank_matrix, plan.rank_prefix = parts[0].view(P, P), parts[1].view(P, P)
-                plan.send_chunk_prefix, plan.recv_src_idx = parts[2].view(P, tiles), parts[3]
+                has_weights=topk_w[i] is not None, slab=slab, slab_ptr=base, views=views)
             plans.append(plan)
+            at = lambda name: base + 4 * views[name][0]
+            v1 = at if rank_matrix else lambda name: None       # (cleared by the launcher, on its stream, where that is needed)
             sc = self._scratch[i]
             args.append(dict(topk_idx=idx.data_ptr(), topk_w=_ptr(topk_w[i]), T=T, E=num_experts, K=K, expand=int(expand),
                              alignment=alignment, meta_stride=stride, hist=sc["hist"].data_ptr(), hits=sc["hits"].data_ptr(),
-                             own_hits=sc["own_hits"].data_ptr(), cnt=sc["cnt"].data_ptr(), send_slot=plan.send_slot.data_ptr(),
-                             slot_row=plan.slot_row.data_ptr(), stage_meta=plan.stage_meta.data_ptr(),
-                             chunk_start=plan.chunk_start.data_ptr(), rank_tokens=plan.rank_tokens.data_ptr(),
-                             rank_rows=plan.rank_rows.data_ptr(), expert_counts=plan.expert_counts.data_ptr(),
-                             expert_offsets=plan.expert_offsets.data_ptr(), recv_row_src=plan.recv_row_src.data_ptr(),
-                             recv_w=_ptr(plan.recv_w), recv_idx=_ptr(plan.recv_idx), rcap=rcap,
-                             rank_matrix=_ptr(plan.rank_matrix), rank_prefix=_ptr(plan.rank_prefix),
-                             send_prefix=_ptr(plan.send_chunk_prefix), recv_src=_ptr(plan.recv_src_idx)))
+                             own_hits=sc["own_hits"].data_ptr(), cnt=sc["cnt"].data_ptr(), send_slot=at("send_slot"),
+                             slot_row=at("slot_row"), stage_meta=at("stage_meta"), chunk_start=at("chunk_start"),
+                             rank_tokens=at("rank_tokens"), rank_rows=at("rank_rows"), expert_counts=at("expert_counts"),
+                             expert_offsets=at("expert_offsets"), recv_row_src=at("recv_row_src"),
+                             recv_w=_ptr(plan.recv_w), recv_idx=_ptr(plan.recv_idx), rcap=rcap, rank_matrix=v1("rank_matrix"),
+                             rank_prefix=v1("rank_prefix"), send_prefix=v1("send_chunk_prefix"), recv_src=v1("recv_src_idx"),
+                             seq=seq))
         # the layout pass is a chain of short phases over (source, tile) tasks: P x T / 64 of them, a few microseconds each
         nblocks = blocks or max(1, min(128, self.sm_count // self.n))
         self._timed("notify", stream, lambda: C.notify(lay, self.sessions, args, nblocks, self._stream(stream), self._device_profile))
         if cpu_sync:
-            self._host_wait(stream, "the routing layout pass")
+            self._await_counts(seq, stream, "the routing layout pass")
             self.check_status()
             for plan, s in zip(plans, self.sessions):
                 box = s.mailbox(4 + local)
@@ -353,14 +397,14 @@ class CudaEngine:
                 recv_sf = torch.empty((rows, H // 128), dtype=torch.float32, device=dev)
             padded = plan.expand and plan.alignment > 1      # the kernel zeroes the rows that no token fills
             outs.append((recv_x, recv_sf))
-            args.append(dict(x=x.data_ptr(), x_sf=_ptr(sf), T=plan.num_tokens, mode=mode, send_slot=plan.send_slot.data_ptr(),
-                             slot_row=plan.slot_row.data_ptr(), topk_idx=plan.topk_idx.data_ptr(),
-                             stage_meta=plan.stage_meta.data_ptr(),
-                             rank_tokens=plan.rank_tokens.data_ptr(), rank_rows=plan.rank_rows.data_ptr(),
+            args.append(dict(x=x.data_ptr(), x_sf=_ptr(sf), T=plan.num_tokens, mode=mode, send_slot=_address(plan, "send_slot"),
+                             slot_row=_address(plan, "slot_row"), topk_idx=plan.topk_idx.data_ptr(),
+                             stage_meta=_address(plan, "stage_meta"),
+                             rank_tokens=_address(plan, "rank_tokens"), rank_rows=_address(plan, "rank_rows"),
                              meta_stride=plan.meta_stride, K=plan.num_topk, E=plan.num_experts, expand=int(plan.expand),
                              recv_x=recv_x.data_ptr(), recv_sf=_ptr(recv_sf), recv_rows=recv_x.shape[0],
-                             pad_counts=plan.expert_counts.data_ptr() if padded else None,
-                             pad_offsets=plan.expert_offsets.data_ptr() if padded else None,
+                             pad_counts=_address(plan, "expert_counts") if padded else None,
+                             pad_offsets=_address(plan, "expert_offsets") if padded else None,
                              prof=self._prof_buffer("dispatch", i), whole=int(whole)))
         send, recv = split if split is not None else self.split_blocks(blocks, self.dispatch_send_fraction, self.dispatch_blocks)
         self._timed("dispatch", stream, lambda: self.C.dispatch(lay, self.sessions, args, send, recv, self._stream(stream),
@@ -387,10 +431,10 @@ class CudaEngine:
             b = bias[i] if bias is not None else None
             b0, b1 = (b if isinstance(b, (tuple, list)) else (b, None)) if b is not None else (None, None)
             outs.append((out, out_w))
-            args.append(dict(x=xs[i].data_ptr(), w=_ptr(ws[i]), stage_meta=plan.stage_meta.data_ptr(),
-                             rank_rows=plan.rank_rows.data_ptr(), rank_tokens=plan.rank_tokens.data_ptr(),
+            args.append(dict(x=xs[i].data_ptr(), w=_ptr(ws[i]), stage_meta=_address(plan, "stage_meta"),
+                             rank_rows=_address(plan, "rank_rows"), rank_tokens=_address(plan, "rank_tokens"),
                              prof=self._prof_buffer("combine", i),
-                             send_slot=plan.send_slot.data_ptr(), slot_row=plan.slot_row.data_ptr() if self.world == 1 else None,
+                             send_slot=_address(plan, "send_slot"), slot_row=_address(plan, "slot_row") if self.world == 1 else None,
                              topk_idx=plan.topk_idx.data_ptr(), T=T,
                              meta_stride=plan.meta_stride, K=K, E=plan.num_experts, expand=int(plan.expand),
                              bias0=_ptr(b0), bias1=_ptr(b1), out=out.data_ptr(), out_w=_ptr(out_w), x_rows=xs[i].shape[0],
@@ -425,6 +469,7 @@ class CudaEngine:
         P, K, H = self.world, lay.topk, lay.hidden
         local = num_experts // P
         cap = P * lay.max_tokens * min(K, local)
+        seq = self._next_call(cpu_sync)
         res, args = [], []
         for i in range(self.n):
             x, sf = (xs[i] if isinstance(xs[i], (tuple, list)) else (xs[i], None))
@@ -439,10 +484,9 @@ class CudaEngine:
                          recv_row_src=torch.empty((cap,), **i32), expert_counts=torch.empty((local,), **i32),
                          expert_offsets=torch.empty((local + 1,), **i32), num_rows=torch.empty((1 + T * K,), **i32))
             plan = RoutingPlan(num_tokens=T, num_experts=num_experts, num_topk=K, expand=True, alignment=1, meta_stride=0,
-                               num_rows=cap, num_staged_rows=0, expert_counts_list=None, topk_idx=topk_idx[i], send_slot=None,
-                               slot_row=None, stage_meta=None, chunk_start=None, rank_tokens=None, rank_rows=None,
-                               expert_counts=o["expert_counts"], expert_offsets=o["expert_offsets"],
-                               recv_row_src=o["recv_row_src"], recv_w=o["recv_w"], recv_idx=None, has_weights=True)
+                               num_rows=cap, num_staged_rows=0, expert_counts_list=None, topk_idx=topk_idx[i],
+                               recv_w=o["recv_w"], recv_idx=None, has_weights=True)
+            plan.expert_counts, plan.expert_offsets, plan.recv_row_src = o["expert_counts"], o["expert_offsets"], o["recv_row_src"]
             plan.num_rows_dev, plan.topk_w, plan.low_latency = o["num_rows"], topk_w[i], True
             if outputs is None:      # behind the row count: a small eager call is bound by the host, and an allocation of its own costs it 2 us
                 plan.local_row = o["num_rows"]
@@ -456,11 +500,11 @@ class CudaEngine:
                              recv_w=o["recv_w"].data_ptr(), recv_row_src=o["recv_row_src"].data_ptr(),
                              expert_counts=o["expert_counts"].data_ptr(), expert_offsets=o["expert_offsets"].data_ptr(),
                              num_rows=o["num_rows"].data_ptr(),
-                             local_row=plan.local_row_ptr, use_mailbox=int(cpu_sync), capacity=cap))
+                             local_row=plan.local_row_ptr, use_mailbox=int(cpu_sync), seq=seq, capacity=cap))
         self._timed("ll_dispatch", stream, lambda: self.C.ll_dispatch(lay, self.sessions, args, self.ll_blocks(), self._stream(stream),
                                                                              self._device_profile))
         if cpu_sync:
-            self._host_wait(stream, "the low-latency dispatch")
+            self._await_counts(seq, stream, "the low-latency dispatch")
             self.check_status()
             out = []
             for (plan, rx, rsf), s in zip(res, self.sessions):

@@ -413,6 +413,34 @@ def test_device_profile_counts_every_row_once(hidden, expand, alignment):
         assert sum(b["rows"] for b in prof[op, 0]) == lays[0].row_index.numel(), op
 
 
+def test_counts_of_an_awaited_call_and_tables_made_on_demand():
+    """The host reads the counts of the call it waits for, also behind calls that it does not wait for, whose counts differ; the
+    tables of a handle appear when asked for, and changing one in place through its view is noticed."""
+    from deepep_b200 import ElasticBuffer
+
+    dev, T, E, K = torch.device("cuda"), 200, 24, 3
+    x = torch.randn((T, 256), generator=torch.Generator().manual_seed(1)).bfloat16().to(dev)
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=256, hidden=256, num_topk=K, explicitly_destroy=True)
+    for low_latency in (False, True):
+        for seed in range(12):
+            idx = make_routes("empty", T, E, K, 1, seed).to(dev)
+            args = dict(topk_weights=make_weights(T, K, seed).to(dev), num_experts=E, do_expand=not low_latency)
+            if seed % 3:
+                buf.dispatch(x, topk_idx=make_routes("random", T, E, K, 1, 100 + seed).to(dev), do_cpu_sync=False, **args)
+            handle = buf.dispatch(x, topk_idx=idx, **args)[3]
+            assert handle.is_low_latency == low_latency
+            assert handle.num_recv_tokens_per_expert_list == torch.bincount(idx[idx >= 0], minlength=E).tolist()
+            psum = handle.psum_num_recv_tokens_per_expert
+            assert psum is handle.psum_num_recv_tokens_per_expert
+            assert psum.tolist() == torch.tensor(handle.num_recv_tokens_per_expert_list).cumsum(0).tolist()
+        rows = torch.zeros((handle.num_expanded_tokens, 256), dtype=torch.bfloat16, device=dev)
+        buf.combine(rows, handle)
+        handle.recv_src_metadata.add_(1)
+        with pytest.raises(RuntimeError, match="modified in place"):
+            buf.combine(rows, handle)
+    buf.destroy()
+
+
 @pytest.mark.parametrize("counts,k,n", [
     ([1], 64, 64),                                   # one row, one step, a quarter of a tile
     ([128, 0, 129, 256, 257, 0, 127], 192, 320),     # both sides of a half tile and of a tile, empty experts, a short last tile
