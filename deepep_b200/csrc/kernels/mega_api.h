@@ -14,6 +14,8 @@ constexpr int kGemmBM = 128;   // token rows per tile (TMEM lanes)
 constexpr int kGemmBN = 256;   // output columns per tile
 constexpr int kGemmBK = 128;   // K elements per pipeline stage (one 128-byte swizzle row of fp8)
 constexpr int kSfChunk = 512;  // bytes of block scales of 128 rows x 128 K-elements (ue8m0 per 32)
+constexpr int kSwapRows = 32;  // a tile of at most this many rows multiplies the weights by the rows instead (mega_gemm.cuh)
+constexpr int kTileRowsShift = 16;   // MegaGemmParams::mtile_expert
 constexpr int kSfGroup = 4;    // chunks of consecutive K steps that one copy brings
 
 // Scale factors of a [rows, K] operand are stored as 512-byte chunks, one per (128-row block, 128-K block):
@@ -33,15 +35,17 @@ enum GemmEpilogue : int {
 
 struct MegaGemmParams {
   CUtensorMap tmap_a;        // activations [rows_pad, K] e4m3, box 128 x 128, 128-byte swizzle
+  CUtensorMap tmap_a_short;  // the same in boxes of 16 rows
   CUtensorMap tmap_b;        // weights, tiled as [rows / 128][(K / 128) * 128][128 values]: e2m1 pairs that the copy engine widens
                              // to one byte per value, or e4m3 bytes (b_fp8); a box holds the 128 rows of a CTA of a pair, or 256
   CUtensorMap tmap_sfa, tmap_sfb;   // the chunked scales as [chunks][512 B], kSfGroup chunks a box
   CUtensorMap tmap_b2, tmap_sfb2;   // weights and scales from row b_rows on (the shared experts), if any
-  const int* mtile_expert;   // [max_mtiles] local expert of each 128-row tile
+  const int* mtile_expert;   // [max_mtiles] local expert of each 128-row tile; with `swap` also its rows, above kTileRowsShift (0: all 128)
   const int* a_ready;        // optional: rows of each tile of A in place so far; a tile's loads start at 128
   const int* num_mtiles;     // device scalar: tiles in use
   int max_mtiles, n_tiles, k_steps, n_total;
   int epi, b_tx_bytes;
+  int swap, pad3;            // tiles of few rows swap their operands (kSwap in mega_gemm.cuh)
   int pair, stages;          // stand-alone launch only: run as CTA pairs (the tile list must pair row blocks 2j, 2j + 1 of one expert);
                              // pipeline stages (0 = default)
   int commit_every, b_rows;  // stand-alone launch only: stages released per tcgen05.commit (0 = 1); first row of tmap_b2
@@ -62,8 +66,8 @@ struct MegaGemmParams {
 };
 cudaError_t launch_mega_gemm(const MegaGemmParams& p, int blocks, cudaStream_t stream);
 
-// Encodes e4m3 activations [rows, k] as a 2-D tensor map with a {128 (K), 128 (rows)} box and the 128-byte swizzle.
-bool encode_operand_map(CUtensorMap* map, const void* base, long long rows, long long k, const char** error);
+// Encodes e4m3 activations [rows, k] as a 2-D tensor map with a {128 (K), box_rows} box and the 128-byte swizzle.
+bool encode_operand_map(CUtensorMap* map, const void* base, long long rows, long long k, int box_rows, const char** error);
 // Encodes tiled weights [row_blocks][k_steps * 128][128 values] as a 3-D map with a {128, 128, box_blocks} box, 128-byte swizzle.
 // fp4 = true: elements are packed e2m1 pairs that the copy engine widens to one byte each in shared memory.
 bool encode_weights_map(CUtensorMap* map, const void* base, long long row_blocks, long long k_steps, int box_blocks, bool fp4,
@@ -83,6 +87,7 @@ struct MegaRouteArgs {
   long long in_off;            // byte offset of the input block (x, x_sf, topk_idx, topk_w) in a workspace
   int T, E, K, H;              // tokens of this rank, experts, top-k, hidden
   int max_tokens, max_mtiles;
+  int tile_rows, pad;          // mtile_expert says the tiles' rows too
   int S, tile_pairs;           // tile_pairs: every expert's rows start at a multiple of 256 (pairs of 128-row tiles of one expert)
                                // S: shared experts of this rank: local experts E / world .. E / world + S - 1, fed with all of its own tokens
   const __nv_bfloat16* x_bf16; // optional [T, H]: quantised to MXFP8 into the input block at the start of the kernel
@@ -91,7 +96,7 @@ struct MegaRouteArgs {
   uint8_t* a1;                 // [rows_pad, H] e4m3
   uint8_t* a1_sf;              // chunked scales
   int* row_src;                // [rows_pad]
-  int* mtile_expert;           // [max_mtiles]
+  int* mtile_expert;           // [max_mtiles] see MegaGemmParams
   int* num_mtiles;             // [1]
   int* expert_rows;            // [L] rows per local expert
   int* expert_list;            // [L][world * max_tokens] scratch: routed slots of each local expert

@@ -23,7 +23,7 @@ constexpr int kPullWarps = 2;                                    // warps beside
 constexpr int kStages = 4, kPairStages = 5;                      // operand pipeline (a CTA of a pair holds half of the weights tile)
 constexpr int kFusedThreads = kGemmThreads + kPullWarps * 32;
 
-template <bool kPair>
+template <bool kPair, bool kSwap>
 __global__ void __launch_bounds__(kFusedThreads, 1) mega_moe_kernel(const __grid_constant__ MegaFusedParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ RouteShared sh;
@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) mega_moe_kernel(const __grid
   if (warp < kGemmThreads / 32) {
     unsigned long long* stats = a.route.timer ? a.route.timer + (size_t)blockIdx.x * kMegaTimerWords + kTimMmaThread : nullptr;
     if constexpr (kPair) gemm_phase<true>(a.g1, &a.g2, a.ready, smem_raw, kPairStages, blockIdx.x / 2, gridDim.x / 2, a.tile_counter, a.interleave, 1, stats);
-    else gemm_phase<false>(a.g1, &a.g2, a.ready, smem_raw, kStages, blockIdx.x, gridDim.x, a.tile_counter, a.interleave, 1, stats);
+    else gemm_phase<false, kSwap>(a.g1, &a.g2, a.ready, smem_raw, kStages, blockIdx.x, gridDim.x, a.tile_counter, a.interleave, 1, stats);
   } else {
     // the pull warps take part in the block (and, for CTA pairs, cluster) barriers of gemm_phase's set-up and tear-down
     if constexpr (kPair) { __syncthreads(); umma::cluster_sync_all(); }
@@ -60,7 +60,12 @@ cudaError_t launch_mega_fused(const MegaFusedParams& p, int nranks, int blocks, 
   const size_t smem = gemm_smem_bytes(pair ? kPairStages : kStages, pair);
   for (int i = 0; i < nranks; ++i)
     if ((p.r[i].pair != 0) != pair || (p.r[i].route.tile_pairs != 0) != pair) return cudaErrorInvalidValue;
-  const void* fn = pair ? (const void*)mega_moe_kernel<true> : (const void*)mega_moe_kernel<false>;
+  const bool swap = p.r[0].g1.swap != 0;
+  for (int i = 0; i < nranks; ++i)
+    if ((p.r[i].g1.swap != 0) != swap || (p.r[i].g2.swap != 0) != swap || (p.r[i].route.tile_rows != 0) != swap || (swap && pair))
+      return cudaErrorInvalidValue;
+  const void* fn = pair ? (const void*)mega_moe_kernel<true, false>
+                        : swap ? (const void*)mega_moe_kernel<false, true> : (const void*)mega_moe_kernel<false, false>;
   // the attribute belongs to the current device, so it is set on every launch (a process may drive several GPUs)
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;

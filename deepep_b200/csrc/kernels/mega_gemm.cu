@@ -3,9 +3,10 @@
 
 namespace dep {
 
+template <bool kSwap>
 __global__ void __launch_bounds__(kGemmThreads, 1) mega_gemm_kernel(const __grid_constant__ MegaGemmParams p) {
   extern __shared__ uint8_t smem_raw[];
-  gemm_phase<false>(p, nullptr, nullptr, smem_raw, p.stages ? p.stages : 4, blockIdx.x, gridDim.x, nullptr, 0,
+  gemm_phase<false, kSwap>(p, nullptr, nullptr, smem_raw, p.stages ? p.stages : 4, blockIdx.x, gridDim.x, nullptr, 0,
                     p.commit_every ? p.commit_every : 1);
 }
 // The same as CTA pairs: launched as clusters of two CTAs.
@@ -19,7 +20,8 @@ cudaError_t launch_mega_gemm(const MegaGemmParams& p, int blocks, cudaStream_t s
   const int stages = p.stages ? p.stages : 4;
   const size_t smem = gemm_smem_bytes(stages, p.pair);
   if (smem > 227 * 1024) return cudaErrorInvalidValue;
-  const void* fn = p.pair ? (const void*)mega_gemm_pair_kernel : (const void*)mega_gemm_kernel;
+  const void* fn = p.pair ? (const void*)mega_gemm_pair_kernel
+                          : p.swap ? (const void*)mega_gemm_kernel<true> : (const void*)mega_gemm_kernel<false>;
   // the attribute belongs to the current device, so it is set on every launch (a process may drive several GPUs)
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -87,9 +89,9 @@ static bool encode_values(CUtensorMap* map, const void* base, int rank, const cu
   return true;
 }
 
-bool encode_operand_map(CUtensorMap* map, const void* base, long long rows, long long k, const char** error) {
+bool encode_operand_map(CUtensorMap* map, const void* base, long long rows, long long k, int box_rows, const char** error) {
   const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)k};
-  const cuuint32_t box[2] = {kGemmBK, 128};
+  const cuuint32_t box[2] = {kGemmBK, (cuuint32_t)box_rows};
   return encode_values(map, base, 2, dims, strides, box, false, error);
 }
 

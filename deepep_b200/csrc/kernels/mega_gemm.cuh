@@ -146,6 +146,72 @@ __device__ __forceinline__ void transpose_pieces(uint32_t (&w)[32], int lane) {
   }
 }
 __device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+// silu(gate) * up of two accumulators, rounded like the separate steps.
+__device__ __forceinline__ float swiglu_bf16(float g, float up) {
+  // div.approx: the IEEE division has a slow path for huge / non-finite operands, which padding rows (whatever
+  // the row buffer held) do contain; it made this epilogue, and with it the whole tile, measurably slower
+  return bf16_round(__fdividef(g, 1.0f + __expf(fminf(fmaxf(-g, -80.f), 80.f))) * up);
+}
+// Exponent of the MX scale of a block: 2^(floor(log2(amax)) - 8), at least 2^-127; values saturate at 448.  2^-e is exact.
+__device__ __forceinline__ int mx_exponent(float amax) {
+  return max((int)((__float_as_uint(fmaxf(amax, 1.1754944e-38f)) >> 23) & 0xff) - 127 - 8, -127);
+}
+
+// The epilogue of a tile whose operands are swapped: a lane of tensor memory is a row of the weights, so a warp holds 32 neighbouring
+// output columns (twice: rows 0 to 127 of the tile's weights, and 128 to 255), and the accumulators' columns are `n` tokens, of which
+// this warp takes its half.
+__device__ __forceinline__ void swapped_epilogue(const MegaGemmParams& p, int mt, int nb, int quad, int part, int n, uint32_t taddr,
+                                                 uint64_t* acc_empty) {
+  constexpr int kTokens = kSwapRows / 2;           // of one warp; 16 at most
+  const int lane = threadIdx.x & 31, live = n / 2, t0 = part * live;
+  const long long row0 = (long long)mt * kGemmBM + t0;
+  uint32_t v[2][16];
+  umma::tmem_ld16(taddr + t0, v[0]);
+  umma::tmem_ld16(taddr + kSwapRows + t0, v[1]);
+  umma::tmem_ld_wait();
+  umma::fence_before_sync();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(acc_empty);
+  if (p.epi == kEpiSwigluQuant) {
+    const long long col = (long long)nb * (kGemmBN / 2) + quad * 32;
+    uint8_t* to = p.a2 + row0 * p.inter + col + lane;
+    uint8_t* sf = p.a2_sf + sf_offset(row0, col, p.inter);       // the scales of 32 rows are 16 bytes apart
+#pragma unroll
+    for (int j = 0; j < kTokens; ++j) {
+      if (j >= live) break;
+      const float h = swiglu_bf16(bf16_round(__uint_as_float(v[0][j])), bf16_round(__uint_as_float(v[1][j])));
+      // positive floats compare like their bits; a NaN does not count, as in fmaxf
+      const int e = mx_exponent(__uint_as_float(__reduce_max_sync(0xffffffffu, h == h ? __float_as_uint(fabsf(h)) : 0u)));
+      const float inv = __uint_as_float((uint32_t)(127 - e) << 23);
+      *to = (uint8_t)__nv_cvt_float_to_fp8(h * inv, __NV_SATFINITE, __NV_E4M3);
+      to += p.inter;
+      if (lane == 0) sf[j * 16] = (uint8_t)(e + 127);
+    }
+  } else if (p.epi == kEpiCombine) {
+    const int code = lane < live ? p.row_src[row0 + lane] : -1;
+    unsigned long long dst = 0;
+    if (code >= 0) {
+      const int src = code / (p.max_tokens * p.topk), rem = code - src * p.max_tokens * p.topk;
+      dst = reinterpret_cast<unsigned long long>(p.ws[src] + p.comb_off + ((size_t)rem * p.hidden + (size_t)nb * kGemmBN) * 2);
+    }
+#pragma unroll
+    for (int j = 0; j < kTokens; ++j) {
+      if (j >= live) break;
+      __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(__shfl_sync(0xffffffffu, dst, j));
+      if (!to) continue;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) to[h * 128 + quad * 32 + lane] = __float2bfloat16_rn(__uint_as_float(v[h][j]));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < kTokens; ++j) {
+      if (j >= live) break;
+      float* to = p.c + (row0 + j) * p.ldc + nb * kGemmBN + quad * 32 + lane;
+      to[0] = __uint_as_float(v[0][j]);
+      to[128] = __uint_as_float(v[1][j]);
+    }
+  }
+}
 
 // Position in the fused schedule -> tile id (ids below num_mtiles * n1 are GEMM1 tiles, the rest GEMM2 tiles).
 // The schedule interleaves the two GEMMs in waves of `wave` row blocks: GEMM1 of wave 0, then for every later wave its
@@ -169,6 +235,9 @@ __device__ __forceinline__ int schedule_to_tile(int pos, int num_mtiles, int n1,
   return -1;
 }
 
+// kSwap: a published tile id carries the number of rows, in sixteens, of a tile whose operands are swapped.
+constexpr int kSwapShift = 28;
+
 // Next tile of this CTA: the producer publishes it to the MMA and epilogue warps through a small ring.
 __device__ __forceinline__ int fetch_tile(GemmBarriers* bars, uint32_t local_tile, volatile int* failed, bool from_peer = false) {
   const uint32_t slot = local_tile % kSchedRing;
@@ -191,7 +260,13 @@ __device__ __forceinline__ int fetch_tile(GemmBarriers* bars, uint32_t local_til
 // "stage full" barrier; the odd CTA's MMA warp forwards its "accumulator drained" barrier; the even CTA's commits arrive
 // on both CTAs' barriers.  `cta` / `num_ctas` count pairs then, and all threads of both CTAs must
 // make this call (cluster barriers).
-template <bool kPair>
+//
+// kSwap: tiles of at most kSwapRows rows, which the tile list says, multiply 128 rows of weights by the tile's rows, twice, instead of
+// the tile's rows by 256 rows of weights.  A decode step's tiles hold a handful of rows; the other way round the tensor pipe works for
+// 128 of them and 16 KB of A are loaded for every step, beside 16 KB of weights.  32 experts, hidden 7168, intermediate 2048, GEMM phases:
+// 64 tokens 156 -> 144 us, 16 tokens 152 -> 140, where the weights alone take 115 of a copy's time.  As a branch of the other instance
+// the same tiles cost the large batches 1 to 4 % (registers); tiles of up to 64 rows swapped lost at 64 tokens and more.
+template <bool kPair, bool kSwap = false>
 __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaGemmParams* g2, int* ready, uint8_t* smem_raw,
                                            int stages, int cta, int num_ctas, int* tile_counter = nullptr, int interleave = 0,
                                            int commit_every = 1, unsigned long long* mma_stats = nullptr) {
@@ -252,7 +327,7 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
       const bool takes_tickets = tile_counter != nullptr && !(kPair && crank != 0);
       int ticket = takes_tickets ? atomicAdd(tile_counter, 1) : 0;
       for (uint32_t local_tile = 0;; ++local_tile) {
-        int tile;
+        int tile, swapped = 0;
         if (kPair && crank != 0) {
           tile = fetch_tile(bars, local_tile, failed, true);      // the even CTA hands out the pair's tiles
         } else {
@@ -261,8 +336,15 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
           if (tile >= total_tiles || *failed) tile = -1;
           else if (g2 && ready && interleave > 0)   // wave = row blocks whose GEMM1 tiles fill `2 * interleave` rounds of the CTAs
             tile = schedule_to_tile(tile, num_mtiles, g1.n_tiles, g2->n_tiles, (2 * interleave * num_ctas + g1.n_tiles - 1) / g1.n_tiles);
+          if constexpr (kSwap) {
+            if (tile >= 0) {
+              const bool second = tile >= tiles1;
+              const int rows = (second ? g2->mtile_expert[(tile - tiles1) / g2->n_tiles] : g1.mtile_expert[tile / g1.n_tiles]) >> kTileRowsShift;
+              swapped = rows > 0 && rows <= kSwapRows ? (rows + 15) / 16 : 0;
+            }
+          }
           const uint32_t slot = local_tile % kSchedRing;
-          bars->tile_id[slot] = tile;
+          bars->tile_id[slot] = tile < 0 ? tile : tile | swapped << kSwapShift;
           mbar_arrive(&bars->sched[slot]);      // release: the id is visible to whoever passes the wait
           if constexpr (kPair) {
             umma::remote_store_u32(umma::map_to_cta(smem_u32(&bars->tile_id[slot]), 1), (uint32_t)tile);
@@ -274,7 +356,7 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
         const MegaGemmParams& p = second ? *g2 : g1;
         const int local = second ? tile - tiles1 : tile;
         const int mt = kPair ? 2 * (local / p.n_tiles) + (int)crank : local / p.n_tiles, nb = local % p.n_tiles;
-        int brow = p.mtile_expert[mt] * p.n_total + nb * kGemmBN;        // first of the tile's 256 weight rows
+        int brow = (kSwap ? p.mtile_expert[mt] & ((1 << kTileRowsShift) - 1) : p.mtile_expert[mt]) * p.n_total + nb * kGemmBN;        // first of the tile's 256 weight rows
         const bool shared = brow >= p.b_rows;
         if (shared) brow -= p.b_rows;
         const CUtensorMap* tmap_b = shared ? &p.tmap_b2 : &p.tmap_b;
@@ -318,8 +400,13 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
                 umma::tma_load_2d_pair(sf_dst + (1 + h) * kSfPart, tmap_sfb, 0, (brow / 128 + h) * p.k_steps + ks, bar);
             }
           } else {
-            mbar_expect_tx(&bars->full[s], kTileABytes + kBBoxes * p.b_tx_bytes + sf_bytes);
-            umma::tma_load_2d(a_dst, &p.tmap_a, ks * kGemmBK, mt * kGemmBM, &bars->full[s]);
+            mbar_expect_tx(&bars->full[s], (kSwap && swapped ? swapped * 16 * kGemmBK : kTileABytes) + kBBoxes * p.b_tx_bytes + sf_bytes);
+            if (kSwap && swapped) {
+              for (int i = 0; i < swapped; ++i)
+                umma::tma_load_2d(a_dst + i * 16 * kGemmBK, &p.tmap_a_short, ks * kGemmBK, mt * kGemmBM + i * 16, &bars->full[s]);
+            } else {
+              umma::tma_load_2d(a_dst, &p.tmap_a, ks * kGemmBK, mt * kGemmBM, &bars->full[s]);
+            }
             // both 128-row blocks of weights in one box; the second continues the swizzled tile of the first
             umma::tma_load_3d(a_dst + kTileABytes, tmap_b, 0, ks * 128, brow / 128, &bars->full[s]);
             if (group_start) {
@@ -353,8 +440,9 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
       long long waited = 0;                      // cycles spent waiting for operands (only counted when asked for)
       const long long loop_start = mma_stats ? clock64() : 0;
       for (uint32_t local_tile = 0;; ++local_tile) {
-        const int tile = fetch_tile(bars, local_tile, failed);
-        if (tile < 0) break;
+        const int id = fetch_tile(bars, local_tile, failed);
+        if (id < 0) break;
+        const int tile = kSwap ? id & ((1 << kSwapShift) - 1) : id, swapped = kSwap ? id >> kSwapShift : 0;
         const int k_steps = tile >= tiles1 ? g2->k_steps : g1.k_steps;
         const uint32_t idesc = tile >= tiles1 ? idesc2 : idesc1;
         if (!bounded_wait(&bars->acc_empty, (local_tile & 1u) ^ 1u, failed, kWaitAccEmpty)) break;
@@ -383,6 +471,15 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
               umma::copy_sf_to_tmem(tsfb + 4 * h, umma::smem_desc_sf(sf_addr + (1 + h) * kSfPart));
           }
           const uint64_t da = umma::smem_desc_sw128(a_addr), db = umma::smem_desc_sw128(a_addr + kTileABytes);
+          if (kSwap && swapped) {
+            const uint32_t d = umma::instr_desc_mxf8f6f4(kGemmBM, swapped * 16, (tile >= tiles1 ? g2->b_fp8 : g1.b_fp8) ? 0 : 5, 0);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+              for (int h = 0; h < kGemmBN / 128; ++h)
+                umma::mma_block_scaled(tmem + h * kSwapRows, db + h * (128 * kGemmBK / 16) + 2 * k, da + 2 * k, umma::with_sf_ids(d, k, k),
+                                       tsfb + 4 * h, tsfa, ks > 0 || k > 0);
+          } else
 #pragma unroll
           for (int k = 0; k < 4; ++k) {   // 32 K-values = 32 bytes = 2 descriptor units per step inside the swizzle row
             if constexpr (kPair)
@@ -415,8 +512,9 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
     const int row_in_tile = quad * 32 + lane;
     uint32_t first_done = 0;
     for (uint32_t local_tile = 0;; ++local_tile) {
-      const int tile = fetch_tile(bars, local_tile, failed, kPair && crank != 0);
-      if (tile < 0) break;
+      const int id = fetch_tile(bars, local_tile, failed, kPair && crank != 0);
+      if (id < 0) break;
+      const int tile = kSwap ? id & ((1 << kSwapShift) - 1) : id, swapped = kSwap ? id >> kSwapShift : 0;
       const bool second = tile >= tiles1;
       const MegaGemmParams& p = second ? *g2 : g1;
       const int local = second ? tile - tiles1 : tile;
@@ -425,7 +523,9 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
       umma::fence_after_sync();
       const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
       const long long row = (long long)mt * kGemmBM + row_in_tile;
-      if (p.epi != kEpiStoreF32) {
+      if (kSwap && swapped) {
+        swapped_epilogue(p, mt, nb, quad, part, swapped * 16, taddr, &bars->acc_empty);
+      } else if (p.epi != kEpiStoreF32) {
         // Both epilogues round the accumulator to bf16 first, so this warp's 32 x 128 block fits into 64 registers a thread: it
         // is drained at once and tensor memory handed back, and the next tile's MMAs overlap everything that follows.
         uint32_t held[2][32];      // SwiGLU: [32-column group][16 words of gate, 16 of up]; combine: [64-column half][words]
@@ -478,15 +578,10 @@ __device__ __forceinline__ void gemm_phase(const MegaGemmParams& g1, const MegaG
               const __nv_bfloat162 bg = *reinterpret_cast<const __nv_bfloat162*>(&held[hh][i / 2]);
               const __nv_bfloat162 bu = *reinterpret_cast<const __nv_bfloat162*>(&held[hh][16 + i / 2]);
               const float g = i & 1 ? __high2float(bg) : __low2float(bg), up = i & 1 ? __high2float(bu) : __low2float(bu);
-              // div.approx: the IEEE division has a slow path for huge / non-finite operands, which padding rows (whatever
-              // the row buffer held) do contain; it made this epilogue, and with it the whole tile, measurably slower
-              const float act = __fdividef(g, 1.0f + __expf(fminf(fmaxf(-g, -80.f), 80.f))) * up;
-              h[i] = bf16_round(act);
+              h[i] = swiglu_bf16(g, up);
               amax = fmaxf(amax, fabsf(h[i]));
             }
-            // MX scale: 2^(floor(log2(amax)) - 8), at least 2^-127; values saturate at 448
-            int e = (int)((__float_as_uint(fmaxf(amax, 1.1754944e-38f)) >> 23) & 0xff) - 127 - 8;
-            e = max(e, -127);
+            const int e = mx_exponent(amax);
             const float inv = __uint_as_float((uint32_t)(127 - e) << 23);   // 2^-e, exact (e in [-127, 120])
             uint32_t q[8];
 #pragma unroll

@@ -186,7 +186,8 @@ __device__ __forceinline__ void route_layout_phase(const MegaRouteArgs& a, cg::g
       const int mid = (lo + hi) >> 1;
       if (sh.base[mid] <= t * kGemmBM) lo = mid; else hi = mid;
     }
-    a.mtile_expert[t] = lo;
+    const int rows = a.tile_rows ? max(0, min(kGemmBM, sh.rows[lo] - (t * kGemmBM - sh.base[lo]))) : 0;
+    a.mtile_expert[t] = lo | rows << kTileRowsShift;
   }
   __syncthreads();
   mega_stamp(a.timer, kTimLayout);
@@ -208,7 +209,7 @@ __device__ __forceinline__ void route_pull_phase(const MegaRouteArgs& a, const R
     // lane j < kPullChunk looks up row row0 + j * kPullStride
     int entry = -1;
     if (lane < kPullChunk) {
-      const int row = row0 + lane * kPullStride, l = __ldcg(a.mtile_expert + tile), j = row - sh.base[l];
+      const int row = row0 + lane * kPullStride, l = __ldcg(a.mtile_expert + tile) & ((1 << kTileRowsShift) - 1), j = row - sh.base[l];
       if (j < sh.rows[l]) entry = __ldcg(a.expert_list + (size_t)l * cap + j);
       a.row_src[row] = entry;
     }

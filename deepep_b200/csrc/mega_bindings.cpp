@@ -33,10 +33,13 @@ void fill_gemm(MegaGemmParams& p, const py::dict& d, py::object session) {
   const long long rows_pad = getl(d, "rows_pad"), k = getl(d, "k"), b_rows = getl(d, "b_rows"), b2_rows = getl(d, "b2_rows");
   if (rows_pad % kGemmBM || k % kGemmBK || b_rows % kGemmBN || b2_rows % kGemmBN) throw std::invalid_argument("rows and K must be multiples of 128, weight rows of 256");
   const char* err = nullptr;
-  if (!encode_operand_map(&p.tmap_a, ptr<const void>(d, "a"), rows_pad, k, &err)) throw std::runtime_error(err);
+  if (!encode_operand_map(&p.tmap_a, ptr<const void>(d, "a"), rows_pad, k, kGemmBM, &err)) throw std::runtime_error(err);
   // weights are stored tiled: every (128-row, 128-K) block is one contiguous run of 128 rows x 64 (e2m1) or 128 (e4m3) bytes
   p.b_fp8 = geti(d, "b_fp8", 0) ? 1 : 0;
   p.pair = geti(d, "pair", 0) ? 1 : 0;
+  p.swap = geti(d, "swap", 0) ? 1 : 0;
+  if (p.swap && p.pair) throw std::invalid_argument("CTA pairs do not swap their operands");
+  if (p.swap && !encode_operand_map(&p.tmap_a_short, ptr<const void>(d, "a"), rows_pad, k, 16, &err)) throw std::runtime_error(err);
   auto weights = [&](CUtensorMap* values, CUtensorMap* scales, const char* b, const char* sfb, long long rows) {
     return encode_weights_map(values, ptr<const void>(d, b), rows / 128, k / kGemmBK, p.pair ? 1 : kGemmBN / 128, !p.b_fp8, &err) &&
            encode_sf_map(scales, ptr<const void>(d, sfb), (rows / 128) * (k / kGemmBK), &err);
@@ -83,6 +86,7 @@ void fill_route(MegaRouteArgs& a, const py::dict& d, py::object session) {
   a.pulled = ptr<int>(d, "pulled");
   a.S = geti(d, "S", 0);
   a.tile_pairs = geti(d, "tile_pairs", 0) ? 1 : 0;
+  a.tile_rows = geti(d, "tile_rows", 0) ? 1 : 0;
   a.x_bf16 = ptr<const __nv_bfloat16>(d, "x_bf16");
   a.timer = ptr<unsigned long long>(d, "timer");
   if (a.S < 0 || a.K + a.S > kMaxTopk || a.E / a.ctx.world + a.S > kMaxExperts)
@@ -146,6 +150,7 @@ void op_mega_finish(const WsLayout& lay, const std::vector<py::object>& sessions
 }  // namespace
 
 void bind_mega(py::module_& m) {
+  m.attr("mega_tile_rows_shift") = kTileRowsShift;
   m.attr("gemm_tile") = kGemmBM;
   m.attr("gemm_tile_n") = kGemmBN;
   m.attr("sf_chunk") = kSfChunk;

@@ -218,12 +218,14 @@ class MegaEngine:
                                    topk=self.K + self.S, hidden=self.H))
         if fused:
             pair = self.use_pairs(tokens)
+            swap = not pair and self.use_swap(tokens)
             for i in range(self.n):    # the fused kernel overlaps the pull with the GEMMs through per-tile counters
                 sc = self.scratch[i]
                 route_args[i]["pulled"] = sc["pulled"].data_ptr()
                 route_args[i]["tile_pairs"] = int(pair)
                 gemm1_args[i]["a_ready"] = sc["pulled"].data_ptr()
                 gemm1_args[i]["pair"] = gemm2_args[i]["pair"] = int(pair)
+                route_args[i]["tile_rows"] = gemm1_args[i]["swap"] = gemm2_args[i]["swap"] = int(swap)
             blocks = max(1, min(self.gemm_blocks, self.sm_count // self.n))
             C.mega_fused(lay, self.sessions, [dict(route=route_args[i], finish=finish_args[i], gemm1=gemm1_args[i],
                                                   gemm2=gemm2_args[i], ready=self.scratch[i]["ready"].data_ptr(),
@@ -247,6 +249,12 @@ class MegaEngine:
         # expected rows per local expert if every rank sends what this one does, spread evenly over the experts
         per_expert = self.world * max(tokens) * self.K / max(self.E, 1) if self.L else 0
         return per_expert >= 384
+
+    def use_swap(self, tokens: Sequence[int]) -> bool:
+        """Whether tiles of few rows multiply the weights by the rows (``kSwap`` in ``mega_gemm.cuh``).  The line is at 32 rows per
+        expert, if every rank sends what this one does: up to there most tiles are that short.  32 experts, hidden 7168,
+        intermediate 2048, us with and without: 1 token 84 / 91, 16 157 / 169, 64 162 / 174, 128 (32 rows) 175 / 181, 160 184 / 183."""
+        return self.world * max(tokens) * self.K <= 32 * self.E
 
     WAIT_SITES = {1: "a pipeline barrier", 2: "the tile ticket from the producer warp", 3: "the first projection of a row block",
                   4: "rows pulled from the peers", 5: "the release of a group of operand stages", 6: "the drain of an accumulator",

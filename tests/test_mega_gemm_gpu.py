@@ -7,7 +7,7 @@ from deepep_b200.oracle import megamoe as O
 pytestmark = pytest.mark.gpu
 
 
-def _run(rows_per_expert, n_total, k, seed=0, b_tx=None, pair=False, stages=0, commit_every=0, blocks=148):
+def _run(rows_per_expert, n_total, k, seed=0, b_tx=None, pair=False, stages=0, commit_every=0, blocks=148, swap=False):
     from deepep_b200.ops import load_native
 
     C = load_native()
@@ -23,10 +23,17 @@ def _run(rows_per_expert, n_total, k, seed=0, b_tx=None, pair=False, stages=0, c
     mtile_expert = torch.tensor([e for e, t in enumerate(tiles) for _ in range(t)], dtype=torch.int32)
     ref = torch.empty((rows_pad, n_total))
     a_f, b_f = O.dequantize_mxfp8(a_codes, a_sf), O.unpack_fp4(packed, b_sf)
+    short = torch.zeros((rows_pad,), dtype=torch.bool)              # rows behind the end of a tile that is told its rows
+    told = mtile_expert.clone()
+    if swap:
+        rows = [min(128, r - 128 * t) for r, n in zip(rows_per_expert, tiles) for t in range(n)]
+        told |= torch.tensor(rows, dtype=torch.int32) << C.mega_tile_rows_shift
+        for mt, r in enumerate(rows):
+            short[mt * 128 + r:(mt + 1) * 128] = True
     for mt, e in enumerate(mtile_expert.tolist()):
         ref[mt * 128:(mt + 1) * 128] = a_f[mt * 128:(mt + 1) * 128] @ b_f[e * n_total:(e + 1) * n_total].t()
     d = dict(a=a_codes.view(torch.uint8).to(dev), b=O.tile_fp4_rows(packed).to(dev), sfa=O.to_sf_chunks(a_sf).to(dev), sfb=O.to_sf_chunks(b_sf).to(dev),
-             mt=mtile_expert.to(dev), n=torch.tensor([len(mtile_expert)], dtype=torch.int32, device=dev),
+             mt=told.to(dev), n=torch.tensor([len(mtile_expert)], dtype=torch.int32, device=dev),
              c=torch.zeros((rows_pad, n_total), dtype=torch.float32, device=dev), err=torch.zeros(1, dtype=torch.int32, device=dev))
     args = dict(a=d["a"].data_ptr(), b=d["b"].data_ptr(), sfa=d["sfa"].data_ptr(), sfb=d["sfb"].data_ptr(),
                 mtile_expert=d["mt"].data_ptr(), num_mtiles=d["n"].data_ptr(), rows_pad=rows_pad, k=k, b_rows=experts * n_total,
@@ -35,6 +42,8 @@ def _run(rows_per_expert, n_total, k, seed=0, b_tx=None, pair=False, stages=0, c
         args["b_tx_bytes"] = b_tx
     if pair:
         args["pair"] = 1
+    if swap:
+        args["swap"] = 1
     if stages:
         args["stages"] = stages
     if commit_every:
@@ -43,6 +52,7 @@ def _run(rows_per_expert, n_total, k, seed=0, b_tx=None, pair=False, stages=0, c
     torch.cuda.synchronize()
     assert d["err"].item() == 0, "a pipeline wait ran out inside the GEMM kernel"
     out = d["c"].cpu()
+    ref[short], out[short] = 0.0, 0.0
     err = (out - ref).abs().max().item()
     scale = ref.abs().max().item()
     assert err <= 2e-3 * scale + 1e-3, f"max abs error {err} (reference scale {scale})"
@@ -58,6 +68,14 @@ def test_k_loop_and_tiles():
 
 def test_grouped_shapes():
     _run([100, 1, 300, 128], 512, 2048, seed=3)
+
+
+@pytest.mark.parametrize("rows", [[1], [16], [17, 32, 33, 128], [31, 5, 150, 48, 300], [32] * 40])
+def test_swapped_operands(rows):
+    """Tiles of few rows multiply the weights by the rows: next to tiles that do not, short and whole scale groups, one and several
+    tiles a block."""
+    _run(rows, 256, 128, seed=1, swap=True)
+    _run(rows, 512, 896, seed=2, swap=True, blocks=3)
 
 
 def test_cta_pairs_single_pair():
