@@ -30,7 +30,7 @@ bool fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session
   a.table_off = lay.mega + (gather ? g.table_a : g.table_b);
   a.data_off = lay.mega + (gather ? g.stage : g.recv);
   a.x = gptr<const __nv_bfloat16>(d, "x");
-  a.counts = gptr<const int>(d, "counts");
+  a.counts = gptr<const void>(d, "counts"); a.counts64 = gint(d, "counts64");
   a.out = gptr<__nv_bfloat16>(d, "out");
   a.gathered = gptr<__nv_bfloat16>(d, "gathered");
   a.rows_in = gint(d, "rows_in"); a.E = gint(d, "experts"); a.K = gint(d, "k"); a.N = gint(d, "n");
@@ -55,11 +55,12 @@ bool fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session
   };
   const bool keep = gather && a.gathered;
   const long long x_bytes = (long long)a.rows_in * a.K * 2, out_bytes = (long long)a.out_rows_cap * a.N * 2,
-                  g_bytes = keep ? (long long)a.gathered_cap * a.K * 2 : 0, w_bytes = L * a.K * a.N * 2;
+                  g_bytes = keep ? (long long)a.gathered_cap * a.K * 2 : 0, w_bytes = L * a.K * a.N * 2,
+                  c_bytes = a.E * (a.counts64 ? 8ll : 4ll);
   const bool local = a.ctx.world == 1 && !overlap(a.out, out_bytes, a.x, x_bytes) && !overlap(a.out, out_bytes, weight, w_bytes) &&
                      !overlap(a.gathered, g_bytes, a.x, x_bytes) && !overlap(a.gathered, g_bytes, weight, w_bytes) &&
                      !overlap(a.gathered, g_bytes, a.out, out_bytes) &&
-                     !overlap(a.counts, a.E * 4ll, a.out, out_bytes) && !overlap(a.counts, a.E * 4ll, a.gathered, g_bytes) &&
+                     !overlap(a.counts, c_bytes, a.out, out_bytes) && !overlap(a.counts, c_bytes, a.gathered, g_bytes) &&
                      ((uintptr_t)a.x | (uintptr_t)a.out | (keep ? (uintptr_t)a.gathered : 0)) % 16 == 0;
   const char* err = nullptr;
   const void* a_base = gather && !local ? (const void*)a.gathered : (const void*)a.x;

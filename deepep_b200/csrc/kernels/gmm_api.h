@@ -42,14 +42,15 @@ struct GmmArgs {
   RankCtx ctx;
   long long table_off, data_off;   // absolute byte offsets in a workspace: this op's table, its stage / recv area
   const __nv_bfloat16* x;          // a2av_gmm: [rows_in, K] sorted by global expert; gmm_a2av: [rows_in, K] grouped by (local expert, source)
-  const int* counts;               // [E] rows this rank sends to (a2av_gmm) / gets back from (gmm_a2av) every global expert
+  const void* counts;              // [E] int, or long long (counts64): rows this rank sends to (a2av_gmm) / gets back from (gmm_a2av)
+                                   // every global expert, as the caller holds them
   __nv_bfloat16* out;              // a2av_gmm: [out_rows_cap, N] on the expert rank; gmm_a2av: [out_rows_cap, N] on the source rank
   __nv_bfloat16* gathered;         // a2av_gmm: [gathered_cap, K] the all-to-all-v result, A operand of the GEMM
                                    // (single-rank form: a copy for the caller, or null)
   CUtensorMap tmap_a;              // A operand [rows, K] bf16, 3-D with z = 0: box 64 x 128, 128-byte swizzle
   CUtensorMap tmap_b;              // weights [L * K, N] bf16 (N contiguous): box 64 (N) x 64 (K), 128-byte swizzle
   int rows_in, E, K, N;
-  int out_rows_cap, gathered_cap, max_tiles, pad;
+  int out_rows_cap, gathered_cap, max_tiles, counts64;
   int* tile_info;                  // scratch [max_tiles][4]: local expert, first row, rows, -
   int* num_tiles;                  // [2]: tiles in use, rows on the expert side
   int* pulled;                     // scratch [max_tiles]: rows of each tile that have arrived (a2av_gmm)

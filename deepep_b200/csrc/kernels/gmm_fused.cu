@@ -90,13 +90,20 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64
 }
 
 // ---------------------------------------------------------------- tables and layout
+// Rows of expert e; a count that does not fit an int fits no buffer either.
+__device__ __forceinline__ int count_of(const GmmArgs& a, int e) {
+  if (!a.counts64) return max(reinterpret_cast<const int*>(a.counts)[e], 0);
+  const long long c = reinterpret_cast<const long long*>(a.counts)[e];
+  return c < 0 ? 0 : c > 0x7fffffff ? 0x7fffffff : (int)c;
+}
+
 // Exclusive prefix of this rank's per-expert row counts into its table (one warp).
 // table[0] = total rows, table[1] = `limit` (rows the owner's area really holds), table[4 + e] = first row of expert e.
 __device__ __forceinline__ void publish_table(const GmmArgs& a, int* table, int limit, int lane) {
   int run = 0;
   for (int e0 = 0; e0 < a.E; e0 += 32) {
     const int e = e0 + lane;
-    const int c = e < a.E ? max(a.counts[e], 0) : 0;
+    const int c = e < a.E ? count_of(a, e) : 0;
     int inc = c;
     for (int d = 1; d < 32; d <<= 1) {
       const int o = __shfl_up_sync(0xffffffffu, inc, d);
@@ -159,7 +166,7 @@ __device__ __forceinline__ void build_layout_local(const GmmArgs& a, GmmShared& 
     long long rows = 0, tiles = 0;
     int last = 0;
     for (int e0 = 0; e0 < a.E; e0 += 32) {
-      const int e = e0 + lane, c = e < a.E ? max(a.counts[e], 0) : 0, t = c / kGmmTileRows + (c % kGmmTileRows != 0);
+      const int e = e0 + lane, c = e < a.E ? count_of(a, e) : 0, t = c / kGmmTileRows + (c % kGmmTileRows != 0);
       long long row_sum = c, tile_sum = t;
       for (int d = 1; d < 32; d <<= 1) {
         const long long r = __shfl_up_sync(0xffffffffu, row_sum, d), q = __shfl_up_sync(0xffffffffu, tile_sum, d);

@@ -132,7 +132,7 @@ class GmmEngine:
     def _common(self, i, x, weight, counts, out, num_experts):
         sc = self.scratch[i]
         return dict(max_rows=self.max_rows, max_k=self.max_k, max_n=self.max_n, x=x.data_ptr() if x.numel() else None,
-                    counts=counts.data_ptr(), out=out.data_ptr(), weight=weight.data_ptr(), rows_in=x.shape[0],
+                    counts=counts.data_ptr(), counts64=int(counts.dtype == torch.int64), out=out.data_ptr(), weight=weight.data_ptr(), rows_in=x.shape[0],
                     experts=num_experts, k=weight.shape[1], n=weight.shape[2], out_rows_cap=out.shape[0],
                     max_tiles=self.max_tiles, tile_info=sc["tile_info"].data_ptr(), num_tiles=sc["num_tiles"].data_ptr(),
                     pulled=sc["pulled"].data_ptr(), err=sc["err"].data_ptr())
@@ -418,14 +418,15 @@ def build_rank_route_tensors(m: int, rank: int, ep_size: int, expert_num: int, d
 
 # ------------------------------------------------------------------------------------------------ ops
 def _normalize_route(route: RouteInput, name: str, expert_num: int, device) -> Tuple[torch.Tensor, Optional[List[int]]]:
-    """Returns (int32 tensor on ``device``, host values or None when the route lives on a device)."""
+    """Returns (int32 or int64 tensor on ``device``, host values or None when the route lives on a device).  The kernels read either
+    type, so a route that is on the device already is passed as it is."""
     if isinstance(route, torch.Tensor):
         if route.dim() != 1 or route.numel() != expert_num:
             raise ValueError(f"{name} must be a flat tensor with expert_num={expert_num} elements")
         if route.dtype not in (torch.int64, torch.int32):
             raise TypeError(f"{name} must be an int64 or int32 tensor")
         host = route.tolist() if route.device.type == "cpu" else None
-        return route.to(device=device, dtype=torch.int32), host
+        return route.to(device=device).contiguous(), host
     values = [int(v) for v in route]
     if len(values) != expert_num:
         raise ValueError(f"{name} must have expert_num={expert_num} elements")

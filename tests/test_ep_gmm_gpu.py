@@ -121,6 +121,51 @@ def test_tile_edges_on_a_single_rank(counts, K, N):
         session.close()
 
 
+@pytest.mark.parametrize("world", [1, 2])
+def test_counts_of_either_integer_type(world):
+    """Counts in 64 bits are read where they lie and give the bits of counts in 32 bits; negative ones count as none, and a count
+    beyond any buffer is reported."""
+    from deepep_b200.ops import load_native
+
+    C, dev, E, K, N = load_native(), torch.device("cuda"), 6, 128, 192
+    counts = _counts(world, E, 400, 9)
+    xs = [torch.randn((sum(c), K), generator=torch.Generator().manual_seed(r)).bfloat16().to(dev) for r, c in enumerate(counts)]
+    ws = [torch.randn((E // world, K, N), generator=torch.Generator().manual_seed(7 + r)).bfloat16().to(dev) for r in range(world)]
+    received = [sum(c[e] for c in counts for e in range(r * E // world, (r + 1) * E // world)) for r in range(world)]
+    layout = C.make_mega_layout(world, 1, 128, 1, G.GmmEngine.region_bytes(C, 800, K, N))
+    sessions = [C.Session(r, world, layout.total, 20.0) for r in range(world)]
+    for s in sessions:
+        s.attach_peers([q.workspace for q in sessions])
+    try:
+        eng, results = G.GmmEngine(sessions, layout, dev, 800, K, N), []
+        for dtype in (torch.int32, torch.int64):
+            c = [torch.tensor(v, dtype=dtype, device=dev) for v in counts]
+            outs = [torch.zeros((r, N), dtype=torch.bfloat16, device=dev) for r in received]
+            gathered = [torch.zeros((r, K), dtype=torch.bfloat16, device=dev) for r in received]
+            eng.a2av_gmm(xs, ws, c, outs, gathered, num_experts=E)
+            back = [torch.zeros((x.shape[0], N), dtype=torch.bfloat16, device=dev) for x in xs]
+            eng.gmm_a2av(gathered, ws, c, back, num_experts=E)
+            torch.cuda.synchronize()
+            eng.check()
+            results.append(outs + gathered + back)
+        assert all(torch.equal(a, b) for a, b in zip(*results)) and all(bool(t.any()) for t in results[0] if t.numel())
+        if world == 1:
+            few = torch.tensor([3, -5, 0, 0, 0, -(1 << 40)], device=dev)
+            out = torch.zeros((3, N), dtype=torch.bfloat16, device=dev)
+            eng.a2av_gmm([xs[0][:3].contiguous()], ws, [few], [out], num_experts=E)
+            eng.check()
+            # one rounding to bf16 behind an fp32 sum of 128 products of size one
+            assert torch.allclose(out.float(), xs[0][:3].float() @ ws[0][0].float(), rtol=2.0 ** -8, atol=1e-3)
+            eng.a2av_gmm(xs, ws, [torch.tensor([1 << 40] * E, device=dev)], [torch.empty((received[0], N), dtype=torch.bfloat16, device=dev)],
+                         num_experts=E)
+            with pytest.raises(RuntimeError, match="row counts"):
+                eng.check()
+    finally:
+        torch.cuda.synchronize()
+        for s in sessions:
+            s.close()
+
+
 def test_both_tile_widths_give_the_same_rows():
     """Nine narrow tiles (one and two halves high): on nine blocks all at once, on eight and six the short ones of the last row block
     are second tiles, behind 13 K steps in a pipeline of four; on five and two blocks the wide ones take their place."""
