@@ -109,12 +109,26 @@ cudaError_t launch_mega_route(const MegaRouteParams& p, int nranks, int blocks, 
 long long mega_input_bytes(int max_tokens, int hidden, int topk);
 void mega_input_offsets(int max_tokens, int hidden, int topk, long long* out6);
 
+// One batch into the symmetric input block: codes, block scales, expert ids (of either integer type) and weights.
+struct MegaLoadArgs {
+  const int4* x; int4* x_to;               // [T][H] bytes; null: the fused kernel will quantise the rows, and the scales come with them
+  const int2* sf; int2* sf_to;             // [T][H / 32] bytes
+  const void* idx; int* idx_to;            // [T][K] int, or long long (idx64)
+  const float* w; float* w_to;             // [T][K]
+  int T, H, K, idx64;
+};
+cudaError_t launch_mega_load(const MegaLoadArgs& a, cudaStream_t stream);
+
 struct MegaFinishArgs {
   RankCtx ctx;
   long long in_off, comb_off;
   int T, E, K, H, max_tokens, S;   // S shared experts: combine slots K .. K + S - 1 of a token carry their rows (weight 1)
   unsigned long long* timer;
   __nv_bfloat16* y;            // [T, H]
+  // fused kernel only: rows of every routed local expert, added to what `stats` holds (or stored, stats_set), or null
+  const int* expert_rows;
+  int* stats;
+  int stats_set, pad;
 };
 struct MegaFinishParams { WsLayout lay; MegaFinishArgs r[kMaxRanks]; };
 cudaError_t launch_mega_finish(const MegaFinishParams& p, int nranks, int blocks, cudaStream_t stream);

@@ -333,6 +333,8 @@ __device__ __forceinline__ void finish_phase(const MegaFinishArgs& a, bool bump_
       }
     }
   }
+  if (blockIdx.x == 0 && a.stats)
+    for (int l = threadIdx.x; l < a.E / P; l += (int)blockDim.x) a.stats[l] = (a.stats_set ? 0 : a.stats[l]) + __ldcg(a.expert_rows + l);
   mega_stamp(a.timer, kTimEnd);
   if (bump_epoch && last_block_of_rank(ctl, kOpMega, gridDim.x)) {
     if (threadIdx.x == 0) ctl->epoch[kOpMega] = epoch;

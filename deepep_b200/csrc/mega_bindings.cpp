@@ -101,6 +101,8 @@ void fill_finish(MegaFinishArgs& a, const py::dict& d, py::object session) {
   a.y = ptr<__nv_bfloat16>(d, "y");
   a.S = geti(d, "S", 0);
   a.timer = ptr<unsigned long long>(d, "timer");
+  a.expert_rows = ptr<const int>(d, "expert_rows"); a.stats = ptr<int>(d, "stats"); a.stats_set = geti(d, "stats_set", 0);
+  if (a.stats && !a.expert_rows) throw std::invalid_argument("statistics need the row counts");
 }
 
 // One persistent launch for the whole layer: args[i] = {"route": {...}, "gemm1": {...}, "gemm2": {...}, "finish": {...}, "ready": ptr}
@@ -159,6 +161,17 @@ void bind_mega(py::module_& m) {
     long long o[6];
     mega_input_offsets(max_tokens, hidden, topk, o);
     return std::vector<long long>(o, o + 6);
+  });
+  // x and x_sf (or neither), topk_idx and topk_weights of `tokens` tokens into the input block; codes 16-byte, scales 8-byte aligned
+  m.def("mega_load", [](uintptr_t x, uintptr_t sf, uintptr_t idx, bool idx64, uintptr_t w, uintptr_t x_to, uintptr_t sf_to, uintptr_t idx_to,
+                        uintptr_t w_to, int tokens, int hidden, int topk, uintptr_t stream) {
+    if (tokens < 0 || hidden < 256 || hidden % 256 || topk < 1 || topk > kMaxTopk) throw std::invalid_argument("mega_load: sizes out of range");
+    if ((x | x_to) % 16 || (sf | sf_to) % 8 || idx % (idx64 ? 8 : 4) || (idx_to | w | w_to) % 4) throw std::invalid_argument("mega_load: misaligned tensor");
+    if (tokens > 0 && (!x != !sf || !idx || !w || !x_to || !sf_to || !idx_to || !w_to)) throw std::invalid_argument("mega_load: a tensor is missing");
+    MegaLoadArgs a = {reinterpret_cast<const int4*>(x), reinterpret_cast<int4*>(x_to), reinterpret_cast<const int2*>(sf),
+                      reinterpret_cast<int2*>(sf_to), reinterpret_cast<const void*>(idx), reinterpret_cast<int*>(idx_to),
+                      reinterpret_cast<const float*>(w), reinterpret_cast<float*>(w_to), tokens, hidden, topk, idx64 ? 1 : 0};
+    check(launch_mega_load(a, reinterpret_cast<cudaStream_t>(stream)), "mega_load launch");
   });
   m.def("mega_gemm", &op_mega_gemm);
   m.def("mega_route", &op_mega_route);

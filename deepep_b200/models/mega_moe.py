@@ -187,12 +187,14 @@ class MegaEngine:
 
     def forward(self, ys: Sequence[torch.Tensor], tokens: Sequence[int], l1: Sequence[MegaWeights], l2: Sequence[MegaWeights],
                 stream=None, fused: bool = True, x_bf16: Optional[Sequence[Optional[torch.Tensor]]] = None,
-                timer: Optional[torch.Tensor] = None) -> None:
+                timer: Optional[torch.Tensor] = None, stats: Optional[torch.Tensor] = None, stats_set: bool = False) -> None:
         """Run the layer.  ``fused``: one persistent cooperative kernel (route -> GEMM1 -> GEMM2 -> finish); otherwise
         the same phases as four launches (kept for debugging and for comparing the two schedules).
         ``l1`` / ``l2`` hold the routed experts followed by the shared ones (in one set of tensors, or joined from two) when the
         engine has shared experts.
         ``x_bf16[i]``: bf16 activations quantised to MXFP8 inside the kernel instead of pre-quantised inputs.
+        ``stats``: int32 ``[L]`` of a single local rank, to which the kernel adds the rows of every routed local expert (or stores
+        them there: ``stats_set``); fused only.
         ``timer``: int64 ``[SMs, mega_timer_words]`` that receives one record of phase stamps per CTA (fused, one rank)."""
         C, lay = self.C, self.layout
         s = (stream if stream is not None else torch.cuda.current_stream(self.device)).cuda_stream
@@ -208,7 +210,8 @@ class MegaEngine:
                                    expert_list=sc["expert_list"].data_ptr()))
             finish_args.append(dict(in_off=self.in_off, comb_off=self.comb_off, T=tokens[i], E=self.E, K=self.K, H=self.H,
                                     max_tokens=self.M, y=ys[i].data_ptr(), S=self.S,
-                                    timer=None if timer is None else timer.data_ptr()))
+                                    timer=None if timer is None else timer.data_ptr(), expert_rows=sc["expert_rows"].data_ptr(),
+                                    stats=None if stats is None or not fused else stats.data_ptr(), stats_set=int(stats_set)))
             common = dict(mtile_expert=sc["mtile_expert"].data_ptr(), num_mtiles=sc["num_mtiles"].data_ptr(), rows_pad=self.rows_cap,
                           error_flag=sc["err"].data_ptr())
             gemm1_args.append(dict(common, **_weight_args(w1, hold), a=sc["a1"].data_ptr(), sfa=sc["a1_sf"].data_ptr(), k=self.H, epi=1,
@@ -393,11 +396,30 @@ class SymmBuffer:
             codes = (exponent - 1 + 127).to(torch.uint8).repeat_interleave(4, dim=1)
         else:
             raise ValueError("x_sf must be uint8 [batch, hidden / 32] (ue8m0) or fp32 [batch, hidden / 128] (powers of two)")
-        self.x.view(torch.uint8)[:bs].copy_(x.view(torch.uint8))
-        self.x_sf[:bs].copy_(codes)
+        self._copy_inputs(x, codes, topk_idx, topk_weights)
+        return self.prepare(bs)
+
+    def _copy_inputs(self, x: Optional[torch.Tensor], codes: Optional[torch.Tensor], topk_idx: torch.Tensor,
+                     topk_weights: torch.Tensor) -> None:
+        """Codes and ue8m0 scales (or neither), expert ids and weights into the input block: one kernel where they lie as it reads them."""
+        bs = topk_idx.shape[0] if x is None else x.shape[0]
+        given = [t for t in (x, codes, topk_idx, topk_weights) if t is not None]
+        if (isinstance(self.engine, MegaEngine) and bs <= self.num_max_tokens_per_rank
+                and (x is None or x.dtype == torch.float8_e4m3fn and tuple(x.shape) == (bs, self.hidden) and x.data_ptr() % 16 == 0
+                     and codes.dtype == torch.uint8 and tuple(codes.shape) == (bs, self.hidden // 32) and codes.data_ptr() % 8 == 0)
+                and topk_idx.dtype in (torch.int32, torch.int64) and topk_weights.dtype == torch.float32
+                and tuple(topk_idx.shape) == tuple(topk_weights.shape) == (bs, self.num_topk)
+                and all(t.is_contiguous() and t.device == self.x.device for t in given)):
+            self.engine.C.mega_load(0 if x is None else x.data_ptr(), 0 if x is None else codes.data_ptr(), topk_idx.data_ptr(),
+                                    topk_idx.dtype == torch.int64, topk_weights.data_ptr(), self.x.data_ptr(), self.x_sf.data_ptr(),
+                                    self.topk_idx.data_ptr(), self.topk_weights.data_ptr(), bs, self.hidden, self.num_topk,
+                                    torch.cuda.current_stream(self.device).cuda_stream)
+            return
+        if x is not None:
+            self.x.view(torch.uint8)[:bs].copy_(x.to(torch.float8_e4m3fn).view(torch.uint8))
+            self.x_sf[:bs].copy_(codes)
         self.topk_idx[:bs].copy_(topk_idx.to(torch.int32))
         self.topk_weights[:bs].copy_(topk_weights.float())
-        return self.prepare(bs)
 
     def allocate_timer(self) -> torch.Tensor:
         """A zeroed int64 ``[SMs, words]`` tensor for ``fp8_fp4_mega_moe(..., timer=...)``: the kernel writes one record
@@ -449,7 +471,7 @@ def fp8_fp4_mega_moe(y: torch.Tensor, l1_weights: MegaWeights, l2_weights: MegaW
                      shared_l1_weights: Optional[MegaWeights] = None, shared_l2_weights: Optional[MegaWeights] = None,
                      cumulative_local_expert_recv_stats: Optional[torch.Tensor] = None, recipe=(1, 1, 32),
                      activation: str = "swiglu", activation_clamp=None, fast_math: bool = True, *, x: Optional[torch.Tensor] = None,
-                     timer: Optional[torch.Tensor] = None, fused: bool = True, check: bool = False) -> None:
+                     timer: Optional[torch.Tensor] = None, fused: bool = True, check: bool = False, _stats_set: bool = False) -> None:
     """Fused MoE forward; overwrites ``y`` (bf16 ``[bs, hidden]``, ``bs = y.shape[0]``) in place and returns ``None``.
 
     The positional parameters follow the reference (``api.py:520-535``).  Inputs are read from ``sym_buffer.x`` /
@@ -499,10 +521,11 @@ def fp8_fp4_mega_moe(y: torch.Tensor, l1_weights: MegaWeights, l2_weights: MegaW
             raise ValueError("timer must come from SymmBuffer.allocate_timer() and needs the fused kernel")
         engine.forward(y, sym_buffer, l1_weights, l2_weights, shared_l1_weights, shared_l2_weights, x, stats)
         return None
+    counted = stats is not None and fused and isinstance(engine, MegaEngine)       # the fused kernel counts by itself
     engine.forward([y], [bs], [sym_buffer.joined_weights(l1_weights, shared_l1_weights)],
                    [sym_buffer.joined_weights(l2_weights, shared_l2_weights)], fused=fused,
-                   x_bf16=None if x is None else [x], timer=timer)
-    if stats is not None:
+                   x_bf16=None if x is None else [x], timer=timer, **(dict(stats=stats, stats_set=_stats_set) if counted else {}))
+    if stats is not None and not counted:
         stats.add_(engine.scratch[0]["expert_rows"][:local])
     if check:
         torch.cuda.synchronize(sym_buffer.device)
@@ -518,18 +541,20 @@ def mega_moe(x, topk_idx: torch.Tensor, topk_weights: torch.Tensor, l1_weights: 
     to MXFP8 here) or an ``(e4m3, ue8m0)`` pair that is copied as is; fills the symmetric inputs and runs the fused forward.
     Returns ``(y, per_call_counts)`` as the reference does: the output and, int32 ``[experts per rank]``, the rows every
     routed local expert received in this call."""
-    if isinstance(x, (tuple, list)):
-        codes, sf = x
+    on_gpu = isinstance(sym_buffer.engine, MegaEngine)          # its kernel stores the counts, the CPU engine adds them up
+    inside = (on_gpu and isinstance(x, torch.Tensor) and x.dtype == torch.bfloat16 and x.is_contiguous() and x.device == sym_buffer.x.device
+              and tuple(x.shape) == (topk_idx.shape[0], sym_buffer.hidden) and x.data_ptr() % 16 == 0)
+    if inside:                                                  # the fused kernel quantises the rows, with the same bits
+        codes = sf = None
     else:
-        codes, sf = quantize_mxfp8_cuda(x)
-    bs = codes.shape[0]
-    sym_buffer.x[:bs].copy_(codes)
-    sym_buffer.x_sf[:bs].copy_(sf)
-    sym_buffer.topk_idx[:bs].copy_(topk_idx.to(torch.int32))
-    sym_buffer.topk_weights[:bs].copy_(topk_weights.float())
-    y = torch.empty((bs, sym_buffer.hidden), dtype=torch.bfloat16, device=codes.device) if out is None else out
-    counts = torch.zeros(sym_buffer.num_experts // sym_buffer.world_size, dtype=torch.int32, device=y.device)
-    fp8_fp4_mega_moe(y, l1_weights, l2_weights, sym_buffer.prepare(bs), shared_l1_weights, shared_l2_weights, counts, timer=timer)
+        codes, sf = x if isinstance(x, (tuple, list)) else quantize_mxfp8_cuda(x)
+    rows = x if inside else codes
+    bs = rows.shape[0]
+    sym_buffer._copy_inputs(codes, sf, topk_idx, topk_weights)
+    y = torch.empty((bs, sym_buffer.hidden), dtype=torch.bfloat16, device=rows.device) if out is None else out
+    counts = (torch.empty if on_gpu else torch.zeros)(sym_buffer.num_experts // sym_buffer.world_size, dtype=torch.int32, device=y.device)
+    fp8_fp4_mega_moe(y, l1_weights, l2_weights, sym_buffer.prepare(bs), shared_l1_weights, shared_l2_weights, counts, timer=timer,
+                     x=x if inside else None, _stats_set=on_gpu)
     return y, counts
 
 

@@ -136,6 +136,37 @@ def test_shared_experts_stats_bf16_input_and_timer():
         buf.destroy()
 
 
+@pytest.mark.parametrize("T,H,K", [(1, 256, 1), (7, 512, 3), (65, 1024, 16), (300, 256, 5)])
+def test_inputs_of_a_call_are_copied_whole(T, H, K):
+    """What ``mega_moe`` puts into the symmetric block: ids of either type, in whatever layout, codes and scales; bf16 rows give the
+    bits of rows quantised outside, counts are those of the call."""
+    from deepep_b200.models.mega_moe import SymmBuffer, mega_moe, transform_weights_for_mega_moe
+
+    dev, E, I = torch.device("cuda"), 16, 128
+    x = torch.randn((T, H), generator=torch.Generator().manual_seed(T)).bfloat16()
+    idx, w = make_routes("invalid" if T > 1 else "random", T, E, K, 1, 5), make_weights(T, K, 3)
+    codes, sf = (t.to(dev) for t in O.quantize_mxfp8(x))
+    buf, results = SymmBuffer(None, E, T + 3, K, H, I), []
+    try:
+        weights = transform_weights_for_mega_moe(*O.make_weights(E, H, I, 2), device=dev)
+        wide = torch.full((T, 2 * K), 3, dtype=torch.int64, device=dev)
+        wide[:, ::2] = idx.to(dev)
+        for ids, source in ((idx.to(dev), (codes, sf)), (idx.int().to(dev), (codes, sf)), (wide[:, ::2], (codes, sf)), (idx.to(dev), x.to(dev))):
+            for t in (buf.x.view(torch.uint8), buf.x_sf, buf.topk_idx, buf.topk_weights):
+                t.fill_(9)
+            y, counts = mega_moe(source, ids, w.to(dev), *weights, buf)
+            torch.cuda.synchronize()
+            buf.engine.check()
+            assert torch.equal(buf.x[:T].view(torch.uint8), codes.view(torch.uint8)) and torch.equal(buf.x_sf[:T], sf)
+            assert torch.equal(buf.topk_idx[:T].cpu(), idx.int()) and torch.equal(buf.topk_weights[:T].cpu(), w)
+            assert bool((buf.topk_idx[T:] == 9).all()) and bool((buf.x_sf[T:] == 9).all()) and bool((buf.x[T:].view(torch.uint8) == 9).all())
+            assert torch.equal(counts.cpu(), torch.bincount(idx[idx >= 0], minlength=E).int())
+            results.append(y)
+        assert all(torch.equal(y, results[0]) for y in results[1:])
+    finally:
+        buf.destroy()
+
+
 @pytest.mark.parametrize("pairs", ["0", "1"])
 @pytest.mark.parametrize("E, S", [(32, 1), (33, 0), (64, 0), (70, 2)])
 def test_layout_of_more_than_32_local_experts(E, S, pairs):
