@@ -2,6 +2,7 @@
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
+#include <chrono>
 #include <stdexcept>
 #include <string>
 
@@ -60,6 +61,15 @@ void bind_expand(py::module_& m) {
     if (tokens > 0 && rows > 0 && (!g || !w || !slot_row || (!dy && !dw) || (dw && !y))) throw std::invalid_argument("return_grad: a tensor is missing");
     if ((g | y | dy) % 16) throw std::invalid_argument("return_grad: rows must start on a 16-byte boundary");
     check_launch(launch_return_grad(p, reinterpret_cast<cudaStream_t>(stream)), "return_grad");
+  });
+  // Polls a word of host memory until it is not negative; false when `microseconds` passed first.
+  m.def("wait_word", [](uintptr_t word, int microseconds) {
+    py::gil_scoped_release unlocked;
+    const volatile int* w = reinterpret_cast<const volatile int*>(word);
+    const auto end = std::chrono::steady_clock::now() + std::chrono::microseconds(microseconds);
+    for (unsigned spins = 0; *w < 0; ++spins)
+      if ((spins & 63u) == 63u && std::chrono::steady_clock::now() > end) return false;
+    return true;
   });
   m.def("expand_scratch", &expand_scratch, py::arg("rows"), py::arg("experts"), py::arg("topk"));
   m.def("expand", [](const py::dict& d, int blocks, uintptr_t stream) {

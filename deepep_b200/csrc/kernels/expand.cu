@@ -25,6 +25,9 @@ namespace dep {
 
 constexpr int kExpandThreads = 256;
 
+// The host polls this word, which is in its memory, while the copies of the rows are queued behind the plan.
+__device__ __forceinline__ void report(int* flag, int value) { *reinterpret_cast<volatile int*>(flag) = value; }
+
 // The plan, by one cluster that keeps the table in shared memory.
 __global__ void __launch_bounds__(kTileThreads) ep_expand_plan_kernel(const __grid_constant__ ExpandParams p) {
   cg::cluster_group cluster = cg::this_cluster();
@@ -43,7 +46,10 @@ __global__ void __launch_bounds__(kTileThreads) ep_expand_plan_kernel(const __gr
   const int over = __syncthreads_or(tid < L && tot > cap);
   if (blockIdx.x == 0) {
     if (tid < L) { p.expert_offsets[tid] = first; p.actual_counts[tid] = tot; }
-    if (tid == 0) { p.expert_offsets[L] = s.off[L]; *p.error_flag = over != 0; }
+    if (tid == 0) {
+      p.expert_offsets[L] = s.off[L];
+      report(p.error_flag, over != 0);
+    }
   }
   const int rows = (live + shares - 1) / shares, begin = min(live, share * rows), end = min(live, begin + rows);
   for (int i = begin * K + tid; i < end * K; i += kTileThreads) {
@@ -67,7 +73,6 @@ __global__ void __launch_bounds__(kExpandThreads) ep_expand_plan_grid_kernel(con
     int run = 0;
     for (int e = 0; e < L; ++e) { p.expert_offsets[e] = run; run += p.caps[e]; }
     p.expert_offsets[L] = run;
-    *p.error_flag = 0;
   }
   // ---- pass 1: rows per (tile, expert)
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -85,12 +90,17 @@ __global__ void __launch_bounds__(kExpandThreads) ep_expand_plan_grid_kernel(con
   }
   __threadfence();
   grid.sync();
-  // ---- pass 2: exclusive scan over the tiles, one thread per expert
-  for (int e = blockIdx.x * kExpandThreads + threadIdx.x; e < L; e += gridDim.x * kExpandThreads) {
-    int run = 0;
-    for (int t = 0; t < tiles; ++t) { const int c = p.tile_counts[(size_t)t * L + e]; p.tile_counts[(size_t)t * L + e] = run; run += c; }
-    p.actual_counts[e] = run;
-    if (run > p.expert_offsets[e + 1] - p.expert_offsets[e]) *p.error_flag = 1;
+  // ---- pass 2: exclusive scan over the tiles, one thread per expert of the first block
+  if (blockIdx.x == 0) {
+    int over = 0;
+    for (int e = threadIdx.x; e < L; e += kExpandThreads) {
+      int run = 0;
+      for (int t = 0; t < tiles; ++t) { const int c = p.tile_counts[(size_t)t * L + e]; p.tile_counts[(size_t)t * L + e] = run; run += c; }
+      p.actual_counts[e] = run;
+      over |= run > p.caps[e];
+    }
+    over = __syncthreads_or(over);
+    if (threadIdx.x == 0) report(p.error_flag, over != 0);
   }
   __threadfence();
   grid.sync();

@@ -23,7 +23,7 @@ struct ExpandParams {
   int* actual_counts;          // [L] rows really routed to each expert (output; input in cached mode)
   int* mapping;                // [R][K] expanded row of every slot, -1 for empty (output; input in cached mode)
   int* tile_counts;            // scratch [tiles][L] of tables that do not fit a cluster's shared memory (expand_scratch)
-  int* error_flag;             // 1 when an expert receives more rows than its capacity, else 0 (not cached)
+  int* error_flag;             // host memory: 1 when an expert receives more rows than its capacity, else 0 (not cached)
   int R, K, L, N, row_bytes, num_sf, cached;
   int pieces, pad_blocks;      // column pieces per row, blocks that zero padding rows (set by the launcher)
   int caps[kMaxExperts];       // capacity of every expert (not cached): with the launch, so that no copy to the device is needed

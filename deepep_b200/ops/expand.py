@@ -171,7 +171,8 @@ def expand(x: Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor]], recv_topk_
     out_w = torch.empty((total,), dtype=torch.float32, device=dev) if topk_weights is not None else None
     err = tile_counts = None
     if handle is None:
-        offsets, actual, mapping, err = (torch.empty(shape, **i32) for shape in ((L + 1,), (L,), (R, K), (1,)))
+        offsets, actual, mapping = (torch.empty(shape, **i32) for shape in ((L + 1,), (L,), (R, K)))
+        err = torch.full((1,), -1, dtype=torch.int32, pin_memory=True)
         scratch = C.expand_scratch(R, L, K)
         if scratch:
             tile_counts = torch.empty((scratch,), **i32)
@@ -189,6 +190,9 @@ def expand(x: Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor]], recv_topk_
                   num_sf=scales.shape[1] if scales is not None else 0, cached=int(handle is not None)),
              _blocks(dev), stream.cuda_stream)
     if handle is None:
+        # the plan reports while the rows are still being copied; what takes long is waited for on the stream
+        if not C.wait_word(err.data_ptr(), 5000):
+            stream.synchronize()
         if int(err.item()):
             raise ValueError("an expert received more rows than its capacity in num_tokens_per_expert")
         handle = ExpandHandle(offsets, actual, mapping, caps, R, total, K, expert_alignment)
