@@ -132,6 +132,8 @@ struct MegaFinishArgs {
 };
 struct MegaFinishParams { WsLayout lay; MegaFinishArgs r[kMaxRanks]; };
 cudaError_t launch_mega_finish(const MegaFinishParams& p, int nranks, int blocks, cudaStream_t stream);
+// The same reduction of a single rank, which waits for nobody, behind the layer's kernel and on the whole GPU.
+cudaError_t launch_mega_reduce(const MegaFinishArgs& a, cudaStream_t stream);
 
 // ---------------------------------------------------------------- the fused layer (one persistent kernel)
 struct MegaFusedArgs {
@@ -140,6 +142,7 @@ struct MegaFusedArgs {
   MegaFinishArgs finish;
   int* ready;                  // [max_mtiles] finished GEMM1 tiles per row block (zeroed by the kernel)
   int* tile_counter;           // [1] next tile of the GEMM1 + GEMM2 tile list (zeroed by the kernel); null: static round-robin
+  int reduce_apart, pad;       // a single rank: the layer's kernel ends with the GEMMs, launch_mega_reduce follows it
   int interleave, pair;        // pair: CTA pairs share the weights tile (cluster of two; needs route.tile_pairs)
                                // interleave k > 0: GEMM2 tiles follow their GEMM1 wave (waves of 2k rounds of GEMM1 tiles); 0: all GEMM1 tiles first
 };

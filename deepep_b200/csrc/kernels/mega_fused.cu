@@ -5,7 +5,8 @@
 //   phase 2  gemm_phase    GEMM1 (+SwiGLU + MXFP8 requant) and GEMM2 (+ bf16 rows stored into the source
 //                          ranks' combine slots over NVLink) as one tile list on tcgen05 / TMEM; a GEMM2
 //                          tile starts as soon as the GEMM1 tiles of its row block are done
-//   phase 3  finish_phase  handshake, y[t] = sum_k w[t, k] * row[t, k]
+//   phase 3  finish_phase  handshake, y[t] = sum_k w[t, k] * row[t, k]; a single rank that has the whole GPU leaves it to a
+//                          kernel of its own (launch_mega_reduce)
 // One CTA per SM stays resident for all three phases; the phases are separated by grid barriers on this
 // GPU and by flag words in peer memory across GPUs.
 //
@@ -49,13 +50,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) mega_moe_kernel(const __grid
     __syncthreads();
     if constexpr (kPair) umma::cluster_sync_all();
   }
+  if (a.reduce_apart) return;
   mega_stamp(a.route.timer, kTimGemm);             // this CTA ran out of tiles (or of rows to pull)
   fence_for_peers(a.route.ctx.world);
   grid.sync();
   finish_phase(a.finish, true);
 }
 
-cudaError_t launch_mega_fused(const MegaFusedParams& p, int nranks, int blocks, cudaStream_t stream) {
+static cudaError_t launch_layer(const MegaFusedParams& p, int nranks, int blocks, cudaStream_t stream) {
   bool pair = p.r[0].pair != 0;
   const size_t smem = gemm_smem_bytes(pair ? kPairStages : kStages, pair);
   for (int i = 0; i < nranks; ++i)
@@ -83,6 +85,11 @@ cudaError_t launch_mega_fused(const MegaFusedParams& p, int nranks, int blocks, 
   attr[1].val.cooperative = 1;
   cfg.attrs = attr; cfg.numAttrs = 2;
   return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
+cudaError_t launch_mega_fused(const MegaFusedParams& p, int nranks, int blocks, cudaStream_t stream) {
+  const cudaError_t e = launch_layer(p, nranks, blocks, stream);
+  return e == cudaSuccess && p.r[0].reduce_apart ? launch_mega_reduce(p.r[0].finish, stream) : e;
 }
 
 }  // namespace dep

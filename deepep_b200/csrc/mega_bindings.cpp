@@ -122,6 +122,9 @@ void op_mega_fused(const WsLayout& lay, const std::vector<py::object>& sessions,
     p.r[i].ready = ptr<int>(d, "ready");
     p.r[i].tile_counter = ptr<int>(d, "tile_counter");
     p.r[i].interleave = geti(d, "interleave", 1);
+    p.r[i].reduce_apart = geti(d, "reduce_apart", 0) ? 1 : 0;
+    if (p.r[i].reduce_apart && (n > 1 || p.r[i].route.ctx.world > 1 || p.r[i].route.timer))
+      throw std::invalid_argument("the reduction is a kernel of its own on a single rank only, and without a timer");
     p.r[i].pair = geti(d, "pair", 0) ? 1 : 0;
     if (p.r[i].pair != p.r[i].g1.pair || p.r[i].pair != p.r[i].g2.pair) throw std::invalid_argument("the GEMMs' boxes disagree about CTA pairs");
     if (p.r[i].pair && n > 1) throw std::invalid_argument("CTA pairs are for one rank per GPU (virtual ranks share the SMs)");

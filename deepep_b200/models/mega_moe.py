@@ -230,10 +230,11 @@ class MegaEngine:
                 gemm1_args[i]["pair"] = gemm2_args[i]["pair"] = int(pair)
                 route_args[i]["tile_rows"] = gemm1_args[i]["swap"] = gemm2_args[i]["swap"] = int(swap)
             blocks = max(1, min(self.gemm_blocks, self.sm_count // self.n))
+            apart = self.world == 1 and blocks == self.sm_count and timer is None     # a kernel on the whole GPU: only without a budget
             C.mega_fused(lay, self.sessions, [dict(route=route_args[i], finish=finish_args[i], gemm1=gemm1_args[i],
                                                   gemm2=gemm2_args[i], ready=self.scratch[i]["ready"].data_ptr(),
                                                   tile_counter=self.scratch[i]["tile_counter"].data_ptr() if self.dynamic_tiles else None,
-                                                  interleave=int(self.interleave), pair=int(pair))
+                                                  interleave=int(self.interleave), pair=int(pair), reduce_apart=int(apart))
                                              for i in range(self.n)], blocks, s)
             return
         aux_blocks = max(1, min(self.sm_count // self.n, 128))

@@ -167,6 +167,41 @@ def test_inputs_of_a_call_are_copied_whole(T, H, K):
         buf.destroy()
 
 
+@pytest.mark.parametrize("T,H,I,E,K,S", [(1, 256, 128, 4, 1, 0), (9, 512, 128, 4, 3, 1), (33, 768, 128, 8, 4, 2),
+                                         (70, 1024, 256, 16, 15, 1), (300, 256, 128, 8, 5, 0)])
+def test_reduction_behind_the_layer_and_inside_it(T, H, I, E, K, S):
+    """The kernel that follows the layer gives the bits of the phase inside it (which a call with a timer takes): one to sixteen
+    slots, not multiples of those in flight, masked and foreign ids; and the same statistics."""
+    from deepep_b200.models.mega_moe import SymmBuffer, fp8_fp4_mega_moe, transform_weights_for_mega_moe
+
+    dev = torch.device("cuda")
+    l1, l2 = O.make_weights(E, H, I, 7)
+    w1, w2 = transform_weights_for_mega_moe(l1, l2, device=dev)
+    sw1, sw2 = transform_weights_for_mega_moe(*O.make_weights(S, H, I, 8), device=dev, shared=True) if S else (None, None)
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn((T, H), generator=g).bfloat16().to(dev)
+    idx = torch.rand((T, E), generator=g).topk(K, 1).indices.int()
+    idx[torch.rand((T, K), generator=g) < 0.2] = -1
+    if T > 3:
+        idx[1] = -1
+        idx[2, 0] = E
+    w = torch.randn((T, K), generator=g)
+    buf = SymmBuffer(None, E, max(T, 8), K, H, I, num_shared_experts=S)
+    try:
+        buf.topk_idx[:T].copy_(idx); buf.topk_weights[:T].copy_(w)
+        got = []
+        for timer in (None, buf.allocate_timer(), None):
+            y = torch.full((T, H), 7.0, dtype=torch.bfloat16, device=dev)
+            counts = torch.ones(E, dtype=torch.int32, device=dev)
+            fp8_fp4_mega_moe(y, w1, w2, buf, sw1, sw2, counts, x=x, timer=timer, check=True)
+            got.append((y, counts))
+        for y, counts in got[1:]:
+            assert torch.equal(y.view(torch.int16), got[0][0].view(torch.int16)) and torch.equal(counts, got[0][1])
+        assert bool(got[0][0].isfinite().all()) and (S or T <= 3 or not bool(got[0][0][1].any()))
+    finally:
+        buf.destroy()
+
+
 @pytest.mark.parametrize("pairs", ["0", "1"])
 @pytest.mark.parametrize("E, S", [(32, 1), (33, 0), (64, 0), (70, 2)])
 def test_layout_of_more_than_32_local_experts(E, S, pairs):
