@@ -82,12 +82,16 @@ enum MegaTimerSlot : int { kTimStart = 0, kTimHandshake = 1, kTimLayout = 2, kTi
                             kTimMmaThread = 7 };   // word 7: the MMA thread's cycles / 16, (waiting for operands) << 32 | (whole tile loop)
 
 // ---------------------------------------------------------------- routing + token pull
+// Tokens x (top-k + shared experts) up to which every block of a single rank derives the layout by itself, which costs a block more
+// the longer the table is.  The layer in captured graphs, 32 experts, hidden 7168, intermediate 2048, top-8, us with counts
+// over the grid / by every block: 1 token 76.4 / 71.3, 8 144.8 / 140.6, 32 151.9 / 148.6, 64 155.4 / 153.9, 128 166.8 / 166.2, 256 187.9 / 189.9.
+constexpr int kAloneSlots = 1024;
 struct MegaRouteArgs {
   RankCtx ctx;
   long long in_off;            // byte offset of the input block (x, x_sf, topk_idx, topk_w) in a workspace
   int T, E, K, H;              // tokens of this rank, experts, top-k, hidden
   int max_tokens, max_mtiles;
-  int tile_rows, pad;          // mtile_expert says the tiles' rows too
+  int tile_rows, alone;        // mtile_expert says the tiles' rows too; every block derives the layout (route_layout_alone)
   int S, tile_pairs;           // tile_pairs: every expert's rows start at a multiple of 256 (pairs of 128-row tiles of one expert)
                                // S: shared experts of this rank: local experts E / world .. E / world + S - 1, fed with all of its own tokens
   const __nv_bfloat16* x_bf16; // optional [T, H]: quantised to MXFP8 into the input block at the start of the kernel
@@ -128,7 +132,9 @@ struct MegaFinishArgs {
   // fused kernel only: rows of every routed local expert, added to what `stats` holds (or stored, stats_set), or null
   const int* expert_rows;
   int* stats;
-  int stats_set, pad;
+  int stats_set, max_mtiles;
+  // launch_mega_reduce only, or null: counters of the layer's kernel, left zero for the next call ([max_mtiles] each, and one)
+  int* ready; int* pulled; int* tile_counter;
 };
 struct MegaFinishParams { WsLayout lay; MegaFinishArgs r[kMaxRanks]; };
 cudaError_t launch_mega_finish(const MegaFinishParams& p, int nranks, int blocks, cudaStream_t stream);
@@ -140,8 +146,8 @@ struct MegaFusedArgs {
   MegaGemmParams g1, g2;       // GEMM1 (SwiGLU + requant epilogue) and GEMM2 (combine epilogue)
   MegaRouteArgs route;
   MegaFinishArgs finish;
-  int* ready;                  // [max_mtiles] finished GEMM1 tiles per row block (zeroed by the kernel)
-  int* tile_counter;           // [1] next tile of the GEMM1 + GEMM2 tile list (zeroed by the kernel); null: static round-robin
+  int* ready;                  // [max_mtiles] finished GEMM1 tiles per row block (zeroed by the kernel; with route.alone zero already)
+  int* tile_counter;           // [1] next tile of the GEMM1 + GEMM2 tile list (likewise); null: static round-robin
   int reduce_apart, pad;       // a single rank: the layer's kernel ends with the GEMMs, launch_mega_reduce follows it
   int interleave, pair;        // pair: CTA pairs share the weights tile (cluster of two; needs route.tile_pairs)
                                // interleave k > 0: GEMM2 tiles follow their GEMM1 wave (waves of 2k rounds of GEMM1 tiles); 0: all GEMM1 tiles first

@@ -23,6 +23,7 @@ namespace dep {
 constexpr int kPullWarps = 2;                                    // warps beside the GEMM roles that pull tokens from peers
 constexpr int kStages = 4, kPairStages = 5;                      // operand pipeline (a CTA of a pair holds half of the weights tile)
 constexpr int kFusedThreads = kGemmThreads + kPullWarps * 32;
+static_assert(kFusedThreads == kRouteWarps * 32, "route_layout_alone deals its slots out over the block's warps");
 
 template <bool kPair, bool kSwap>
 __global__ void __launch_bounds__(kFusedThreads, 1) mega_moe_kernel(const __grid_constant__ MegaFusedParams p) {
@@ -30,12 +31,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1) mega_moe_kernel(const __grid
   __shared__ RouteShared sh;
   cg::grid_group grid = cg::this_grid();
   const MegaFusedArgs& a = p.r[blockIdx.y];
-  if (blockIdx.x == 0)
-  {
-    for (int i = threadIdx.x; i < a.route.max_mtiles; i += blockDim.x) { a.ready[i] = 0; a.route.pulled[i] = 0; }
-    if (threadIdx.x == 0 && a.tile_counter) *a.tile_counter = 0;
+  if (a.route.alone) {                            // the counters are zero: nothing here waits for another block to clear them
+    route_layout_alone(a.route, grid, sh, reinterpret_cast<int*>(smem_raw));
+  } else {
+    if (blockIdx.x == 0) {
+      for (int i = threadIdx.x; i < a.route.max_mtiles; i += blockDim.x) { a.ready[i] = 0; a.route.pulled[i] = 0; }
+      if (threadIdx.x == 0 && a.tile_counter) *a.tile_counter = 0;
+    }
+    route_layout_phase(a.route, grid, sh);        // handshake, counts, tile layout (grid barriers inside)
   }
-  route_layout_phase(a.route, grid, sh);          // handshake, counts, tile layout (grid barriers inside)
   // The token pull overlaps the GEMMs: rows are pulled tile by tile, a GEMM1 tile starts once its rows have arrived.
   const int warp = threadIdx.x >> 5;
   if (warp < kGemmThreads / 32) {

@@ -62,6 +62,10 @@ __global__ void __launch_bounds__(kReduceThreads) mega_reduce_kernel(const __gri
     if (a.stats)
       for (int l = threadIdx.x; l < a.E; l += kReduceThreads) a.stats[l] = (a.stats_set ? 0 : a.stats[l]) + __ldg(a.expert_rows + l);
   }
+  if (a.ready && blockIdx.x == gridDim.x - 1) {
+    for (int i = threadIdx.x; i < a.max_mtiles; i += kReduceThreads) a.ready[i] = a.pulled[i] = 0;
+    if (threadIdx.x == 0 && a.tile_counter) *a.tile_counter = 0;
+  }
   const int item = blockIdx.x * (kReduceThreads / 32) + (threadIdx.x >> 5), t = item / spans;
   if (t >= a.T) return;
   const int u = (item - t * spans) * 32 + lane;

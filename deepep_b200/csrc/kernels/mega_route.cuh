@@ -102,6 +102,40 @@ __device__ __forceinline__ void quantize_inputs_phase(const MegaRouteArgs& a, ui
   }
 }
 
+// Every expert starts at a multiple of 128 rows (256 with CTA pairs).  Every block derives the whole layout from `sh.rows` and
+// writes the same tile list, so no block waits for another one's (the writes race with equal values).
+__device__ __forceinline__ void lay_out_tiles(const MegaRouteArgs& a, RouteShared& sh, int experts) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x, unit = a.tile_pairs ? 2 * kGemmBM : kGemmBM;      // with CTA pairs an expert owns whole pairs of tiles
+    int run = 0;
+    for (int l0 = 0; l0 < experts; l0 += 32) {
+      const int l = l0 + lane, rows = l < experts ? (sh.rows[l] + unit - 1) / unit * unit : 0;
+      int sum = rows;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, sum, d);
+        if (lane >= d) sum += o;
+      }
+      if (l < experts) sh.base[l] = run + sum - rows;
+      run += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (lane == 0) {
+      sh.total_rows = min(run, a.max_mtiles * kGemmBM);
+      *a.num_mtiles = sh.total_rows / kGemmBM;
+    }
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < sh.total_rows / kGemmBM; t += (int)blockDim.x) {
+    int lo = 0, hi = experts;       // the last expert that starts at this tile or before it (empty ones share a start and are skipped)
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (sh.base[mid] <= t * kGemmBM) lo = mid; else hi = mid;
+    }
+    const int rows = a.tile_rows ? max(0, min(kGemmBM, sh.rows[lo] - (t * kGemmBM - sh.base[lo]))) : 0;
+    a.mtile_expert[t] = lo | rows << kTileRowsShift;
+  }
+  __syncthreads();
+}
+
 // Handshake, per-expert entry lists, 128-row tile layout (tile -> expert).
 // expert_list[l * cap + j] (cap = world * max_tokens) = (source * M + token) * (K + S) + slot of the j-th routed slot of
 // local expert l, in arrival order; the S shared experts follow the routed ones and take every token of this rank
@@ -156,41 +190,62 @@ __device__ __forceinline__ void route_layout_phase(const MegaRouteArgs& a, cg::g
   }
   __threadfence();
   grid.sync();
-
-  // ---- tile layout: every expert starts at a multiple of 128 rows (256 with CTA pairs).  Every block derives all of it and
-  // writes the same tile list, so no block waits for another one's (the writes race with equal values).
   for (int l = threadIdx.x; l < Lx + S; l += (int)blockDim.x) sh.rows[l] = min(__ldcg(a.expert_rows + l), cap);
   __syncthreads();
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x, unit = a.tile_pairs ? 2 * kGemmBM : kGemmBM;      // with CTA pairs an expert owns whole pairs of tiles
-    int run = 0;
-    for (int l0 = 0; l0 < Lx + S; l0 += 32) {
-      const int l = l0 + lane, rows = l < Lx + S ? (sh.rows[l] + unit - 1) / unit * unit : 0;
-      int sum = rows;
-      for (int d = 1; d < 32; d <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, sum, d);
-        if (lane >= d) sum += o;
-      }
-      if (l < Lx + S) sh.base[l] = run + sum - rows;
-      run += __shfl_sync(0xffffffffu, sum, 31);
-    }
-    if (lane == 0) {
-      sh.total_rows = min(run, a.max_mtiles * kGemmBM);
-      *a.num_mtiles = sh.total_rows / kGemmBM;
-    }
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < sh.total_rows / kGemmBM; t += (int)blockDim.x) {
-    int lo = 0, hi = Lx + S;       // the last expert that starts at this tile or before it (empty ones share a start and are skipped)
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (sh.base[mid] <= t * kGemmBM) lo = mid; else hi = mid;
-    }
-    const int rows = a.tile_rows ? max(0, min(kGemmBM, sh.rows[lo] - (t * kGemmBM - sh.base[lo]))) : 0;
-    a.mtile_expert[t] = lo | rows << kTileRowsShift;
-  }
-  __syncthreads();
+  lay_out_tiles(a, sh, Lx + S);
   mega_stamp(a.timer, kTimLayout);
+}
+
+// The same for a single rank and a short routing table (MegaRouteArgs::alone): every block derives the lists from the table by itself,
+// in the order of the table, and writes the same ones, so no block waits for another one; rows that are quantised here are the
+// exception.  `scratch`: kRouteWarps * (experts + S) + kAloneSlots ints of shared memory.  The grid-wide counts above take two grid
+// barriers and an atomic with a returned value, 7.5 us until the layout is there.
+constexpr int kRouteWarps = 12;
+__device__ __forceinline__ void route_layout_alone(const MegaRouteArgs& a, cg::grid_group& grid, RouteShared& sh, int* scratch) {
+  const int K = a.K, Lx = a.E, S = a.S, M = a.max_tokens, Kp = K + S, n = a.T * K, experts = Lx + S;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const MegaInput in = mega_input_layout(M, a.H, K);
+  uint8_t* block = a.ctx.ws[0] + a.in_off;
+  if (a.x_bf16 != nullptr) quantize_inputs_phase(a, block + in.x, block + in.x_sf);
+  if (blockIdx.x == 0 && threadIdx.x == 0) reinterpret_cast<int*>(block + in.hdr)[0] = a.T;
+  int* seen = scratch;                               // [warp][expert]: slots that this warp has met, then those of the warps before it
+  int* place = scratch + kRouteWarps * experts;      // [slot]: its place among its warp's
+  const int* idx = reinterpret_cast<const int*>(block + in.idx);
+  for (int i = threadIdx.x; i < kRouteWarps * experts; i += (int)blockDim.x) seen[i] = 0;
+  if (threadIdx.x == 0) sh.alive = 1;
+  __syncthreads();
+  const int share = (n + kRouteWarps * 32 - 1) / (kRouteWarps * 32) * 32, first = warp * share, last = min(n, first + share);
+  for (int i0 = first; i0 < last; i0 += 32) {
+    const int i = i0 + lane, id = i < last ? __ldcg(idx + i) : -1, e = id >= 0 && id < Lx ? id : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    const int before = __popc(same & ((1u << lane) - 1u));
+    const int met = e >= 0 ? seen[warp * experts + e] : 0;
+    __syncwarp();
+    if (e >= 0 && before == 0) seen[warp * experts + e] = met + __popc(same);
+    __syncwarp();
+    if (i < last) place[i] = met + before;
+  }
+  __syncthreads();
+  for (int l = threadIdx.x; l < experts; l += (int)blockDim.x) {
+    int run = 0;
+    for (int w = 0; w < kRouteWarps; ++w) { const int c = seen[w * experts + l]; seen[w * experts + l] = run; run += c; }
+    sh.rows[l] = l < Lx ? min(run, M) : a.T;
+    if (blockIdx.x == 0) a.expert_rows[l] = l < Lx ? run : a.T;      // for the statistics
+  }
+  __syncthreads();
+  for (int i = first + lane; i < last; i += 32) {
+    const int e = __ldcg(idx + i);
+    if (e < 0 || e >= Lx) continue;
+    const int j = seen[warp * experts + e] + place[i];
+    if (j < M) a.expert_list[(size_t)e * M + j] = i / K * Kp + i % K;
+  }
+  for (int i = threadIdx.x; i < S * a.T; i += (int)blockDim.x) {
+    const int s = i / a.T, t = i - s * a.T;
+    a.expert_list[(size_t)(Lx + s) * M + t] = t * Kp + K + s;
+  }
+  fence_proxy_async();                               // the scratch becomes operand stages, which the copy engine writes
+  lay_out_tiles(a, sh, experts);                     // ends with a block barrier: the lists are there for the block's pull warps
+  if (a.x_bf16 != nullptr) { __threadfence(); grid.sync(); }
 }
 
 // Pulls the routed tokens from their owners (tile by tile, so that the first tiles are complete first); warp `gw` of

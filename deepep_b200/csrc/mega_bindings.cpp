@@ -87,6 +87,7 @@ void fill_route(MegaRouteArgs& a, const py::dict& d, py::object session) {
   a.S = geti(d, "S", 0);
   a.tile_pairs = geti(d, "tile_pairs", 0) ? 1 : 0;
   a.tile_rows = geti(d, "tile_rows", 0) ? 1 : 0;
+  a.alone = geti(d, "alone", 0) ? 1 : 0;
   a.x_bf16 = ptr<const __nv_bfloat16>(d, "x_bf16");
   a.timer = ptr<unsigned long long>(d, "timer");
   if (a.S < 0 || a.K + a.S > kMaxTopk || a.E / a.ctx.world + a.S > kMaxExperts)
@@ -125,6 +126,12 @@ void op_mega_fused(const WsLayout& lay, const std::vector<py::object>& sessions,
     p.r[i].reduce_apart = geti(d, "reduce_apart", 0) ? 1 : 0;
     if (p.r[i].reduce_apart && (n > 1 || p.r[i].route.ctx.world > 1 || p.r[i].route.timer))
       throw std::invalid_argument("the reduction is a kernel of its own on a single rank only, and without a timer");
+    if (p.r[i].route.alone) {          // the reduction leaves the counters zero for the next such call
+      if (!p.r[i].reduce_apart || (long long)p.r[i].route.T * (p.r[i].route.K + p.r[i].route.S) > kAloneSlots)
+        throw std::invalid_argument("every block derives the layout of a short table on a single rank only, before a reduction of its own");
+      p.r[i].finish.ready = p.r[i].ready; p.r[i].finish.pulled = p.r[i].route.pulled; p.r[i].finish.tile_counter = p.r[i].tile_counter;
+      p.r[i].finish.max_mtiles = p.r[i].route.max_mtiles;
+    }
     p.r[i].pair = geti(d, "pair", 0) ? 1 : 0;
     if (p.r[i].pair != p.r[i].g1.pair || p.r[i].pair != p.r[i].g2.pair) throw std::invalid_argument("the GEMMs' boxes disagree about CTA pairs");
     if (p.r[i].pair && n > 1) throw std::invalid_argument("CTA pairs are for one rank per GPU (virtual ranks share the SMs)");
@@ -156,6 +163,7 @@ void op_mega_finish(const WsLayout& lay, const std::vector<py::object>& sessions
 
 void bind_mega(py::module_& m) {
   m.attr("mega_tile_rows_shift") = kTileRowsShift;
+  m.attr("mega_alone_slots") = kAloneSlots;
   m.attr("gemm_tile") = kGemmBM;
   m.attr("gemm_tile_n") = kGemmBN;
   m.attr("sf_chunk") = kSfChunk;

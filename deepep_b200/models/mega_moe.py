@@ -169,7 +169,9 @@ class MegaEngine:
                 row_src=torch.empty((self.rows_cap,), **i32), mtile_expert=torch.zeros((self.max_mtiles,), **i32),
                 num_mtiles=torch.zeros((1,), **i32), expert_rows=torch.zeros((self.L + self.S,), **i32),
                 expert_list=torch.empty(((self.L + self.S) * self.world * self.M,), **i32), err=torch.zeros((1,), **i32),
-                ready=torch.zeros((self.max_mtiles,), **i32), pulled=torch.zeros((self.max_mtiles,), **i32), tile_counter=torch.zeros((1,), **i32)))
+                ready=torch.zeros((self.max_mtiles,), **i32), pulled=torch.zeros((self.max_mtiles,), **i32), tile_counter=torch.zeros((1,), **i32),
+                # the same three for calls that find them zero and leave them zero
+                clean=torch.zeros((2 * self.max_mtiles + 1,), **i32)))
 
     @staticmethod
     def mega_bytes(C, max_tokens: int, hidden: int, topk: int, num_shared_experts: int = 0) -> int:
@@ -222,20 +224,25 @@ class MegaEngine:
         if fused:
             pair = self.use_pairs(tokens)
             swap = not pair and self.use_swap(tokens)
-            for i in range(self.n):    # the fused kernel overlaps the pull with the GEMMs through per-tile counters
-                sc = self.scratch[i]
-                route_args[i]["pulled"] = sc["pulled"].data_ptr()
-                route_args[i]["tile_pairs"] = int(pair)
-                gemm1_args[i]["a_ready"] = sc["pulled"].data_ptr()
-                gemm1_args[i]["pair"] = gemm2_args[i]["pair"] = int(pair)
-                route_args[i]["tile_rows"] = gemm1_args[i]["swap"] = gemm2_args[i]["swap"] = int(swap)
             blocks = max(1, min(self.gemm_blocks, self.sm_count // self.n))
             apart = self.world == 1 and blocks == self.sm_count and timer is None     # a kernel on the whole GPU: only without a budget
-            C.mega_fused(lay, self.sessions, [dict(route=route_args[i], finish=finish_args[i], gemm1=gemm1_args[i],
-                                                  gemm2=gemm2_args[i], ready=self.scratch[i]["ready"].data_ptr(),
-                                                  tile_counter=self.scratch[i]["tile_counter"].data_ptr() if self.dynamic_tiles else None,
-                                                  interleave=int(self.interleave), pair=int(pair), reduce_apart=int(apart))
-                                             for i in range(self.n)], blocks, s)
+            alone = apart and tokens[0] * (self.K + self.S) <= C.mega_alone_slots
+            fused_args = []
+            for i in range(self.n):    # the fused kernel overlaps the pull with the GEMMs through per-tile counters
+                sc = self.scratch[i]
+                counters = [sc[name].data_ptr() for name in ("ready", "pulled", "tile_counter")]
+                if alone:
+                    counters = [sc["clean"].data_ptr() + at * 4 for at in (0, self.max_mtiles, 2 * self.max_mtiles)]
+                ready, pulled, ticket = counters
+                route_args[i]["pulled"] = gemm1_args[i]["a_ready"] = pulled
+                route_args[i]["tile_pairs"] = int(pair)
+                route_args[i]["alone"] = int(alone)
+                gemm1_args[i]["pair"] = gemm2_args[i]["pair"] = int(pair)
+                route_args[i]["tile_rows"] = gemm1_args[i]["swap"] = gemm2_args[i]["swap"] = int(swap)
+                fused_args.append(dict(route=route_args[i], finish=finish_args[i], gemm1=gemm1_args[i], gemm2=gemm2_args[i], ready=ready,
+                                       tile_counter=ticket if self.dynamic_tiles else None, interleave=int(self.interleave),
+                                       pair=int(pair), reduce_apart=int(apart)))
+            C.mega_fused(lay, self.sessions, fused_args, blocks, s)
             return
         aux_blocks = max(1, min(self.sm_count // self.n, 128))
         C.mega_route(lay, self.sessions, route_args, aux_blocks, s)
@@ -257,7 +264,8 @@ class MegaEngine:
     def use_swap(self, tokens: Sequence[int]) -> bool:
         """Whether tiles of few rows multiply the weights by the rows (``kSwap`` in ``mega_gemm.cuh``).  The line is at 32 rows per
         expert, if every rank sends what this one does: up to there most tiles are that short.  32 experts, hidden 7168,
-        intermediate 2048, us with and without: 1 token 84 / 91, 16 157 / 169, 64 162 / 174, 128 (32 rows) 175 / 181, 160 184 / 183."""
+        intermediate 2048, us with and without, both with longer phases around the GEMMs than now: 1 token 84 / 91, 16 157 / 169,
+        64 162 / 174, 128 (32 rows) 175 / 181, 160 184 / 183."""
         return self.world * max(tokens) * self.K <= 32 * self.E
 
     WAIT_SITES = {1: "a pipeline barrier", 2: "the tile ticket from the producer warp", 3: "the first projection of a row block",

@@ -168,10 +168,12 @@ def test_inputs_of_a_call_are_copied_whole(T, H, K):
 
 
 @pytest.mark.parametrize("T,H,I,E,K,S", [(1, 256, 128, 4, 1, 0), (9, 512, 128, 4, 3, 1), (33, 768, 128, 8, 4, 2),
-                                         (70, 1024, 256, 16, 15, 1), (300, 256, 128, 8, 5, 0)])
-def test_reduction_behind_the_layer_and_inside_it(T, H, I, E, K, S):
-    """The kernel that follows the layer gives the bits of the phase inside it (which a call with a timer takes): one to sixteen
-    slots, not multiples of those in flight, masked and foreign ids; and the same statistics."""
+                                         (70, 1024, 256, 16, 15, 1), (300, 256, 128, 8, 5, 0), (256, 256, 128, 40, 4, 0),
+                                         (257, 256, 128, 8, 3, 1)])
+def test_one_rank_with_and_without_barriers(T, H, I, E, K, S):
+    """A layout that every block derives and a reduction that follows the layer give the bits of the phases with grid barriers
+    (which a call with a timer takes): one to sixteen slots, not multiples of those in flight, masked and foreign ids, tables up to the
+    limit and behind it, rows quantised here or before; and the same statistics."""
     from deepep_b200.models.mega_moe import SymmBuffer, fp8_fp4_mega_moe, transform_weights_for_mega_moe
 
     dev = torch.device("cuda")
@@ -190,10 +192,11 @@ def test_reduction_behind_the_layer_and_inside_it(T, H, I, E, K, S):
     try:
         buf.topk_idx[:T].copy_(idx); buf.topk_weights[:T].copy_(w)
         got = []
-        for timer in (None, buf.allocate_timer(), None):
+        timer = buf.allocate_timer()
+        for stamps, rows in ((None, x), (timer, x), (None, None), (timer, None), (None, x), (None, None)):
             y = torch.full((T, H), 7.0, dtype=torch.bfloat16, device=dev)
             counts = torch.ones(E, dtype=torch.int32, device=dev)
-            fp8_fp4_mega_moe(y, w1, w2, buf, sw1, sw2, counts, x=x, timer=timer, check=True)
+            fp8_fp4_mega_moe(y, w1, w2, buf, sw1, sw2, counts, x=rows, timer=stamps, check=True)
             got.append((y, counts))
         for y, counts in got[1:]:
             assert torch.equal(y.view(torch.int16), got[0][0].view(torch.int16)) and torch.equal(counts, got[0][1])
