@@ -52,10 +52,11 @@ cudaError_t launch_mega_finish(const MegaFinishParams& p, int nranks, int blocks
 
 // One span of 32 16-byte pieces of a token per warp, three slots in flight: the loads of 2048 threads an SM instead of the layer's
 // 384, and a kernel's end instead of a grid barrier before it.  Inside the layer's kernel the barrier took 4.5 us and the reduction
-// 5 to 10 (4096 tokens of 7168: 113 for 530 MB, memory).  32 experts, top-8, intermediate 2048, the layer in captured graphs, us inside /
-// behind: 1 token 82.3 / 76.4, 8 149.7 / 144.8, 64 158.4 / 155.4, 128 173.0 / 166.8, 512 267 / 258; 4096 with a shared expert 1743 / 1722.
+// 5 to 10 (4096 tokens of 7168: 113).  32 experts, top-8, intermediate 2048, the layer in captured graphs, us inside / behind: 1 token
+// 82.3 / 76.4, 8 149.7 / 144.8, 64 158.4 / 155.4, 128 173.0 / 166.8, 512 267 / 258.  This kernel by itself, 4096 tokens of 7168, 8 slots:
+// 88 us, 6.0 TB/s (memory); with the 40 registers that the compiler takes unasked, 1536 threads an SM, 92.
 constexpr int kReduceThreads = 256, kReduceSlots = 3;
-__global__ void __launch_bounds__(kReduceThreads) mega_reduce_kernel(const __grid_constant__ MegaFinishArgs a) {
+__global__ void __launch_bounds__(kReduceThreads, 8) mega_reduce_kernel(const __grid_constant__ MegaFinishArgs a) {
   const int K = a.K, Kp = K + a.S, units = a.H / 8, spans = (units + 31) / 32, lane = threadIdx.x & 31;
   if (blockIdx.x == 0) {
     if (threadIdx.x == 0) ++control_of(a.ctx.ws[0])->epoch[kOpMega];
@@ -77,29 +78,26 @@ __global__ void __launch_bounds__(kReduceThreads) mega_reduce_kernel(const __gri
     e = __ldg(reinterpret_cast<const int*>(a.ctx.ws[0] + a.in_off + in.idx) + (size_t)t * K + lane);
     weight = __ldg(reinterpret_cast<const float*>(a.ctx.ws[0] + a.in_off + in.w) + (size_t)t * K + lane);
   }
-  const int4* rows = reinterpret_cast<const int4*>(a.ctx.ws[0] + a.comb_off) + (size_t)t * Kp * units + u;
+  const int4* rows = reinterpret_cast<const int4*>(a.ctx.ws[0] + a.comb_off) + (size_t)t * Kp * units + min(u, units - 1);
   float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (unsigned m = __ballot_sync(0xffffffffu, lane < K ? e >= 0 && e < a.E : lane < Kp); m;) {
     int4 v[kReduceSlots];
-    float w[kReduceSlots];
-    const int n = __popc(m);
+    unsigned taken = m;
 #pragma unroll
     for (int q = 0; q < kReduceSlots; ++q) {
-      if (q < n) {
-        const int k = __ffs(m) - 1;
-        m &= m - 1;
-        w[q] = __shfl_sync(0xffffffffu, weight, k);
-        if (u < units) v[q] = __ldg(rows + (size_t)k * units);
-      }
+      if (m) v[q] = __ldg(rows + (__ffs(m) - 1) * units);
+      m &= m - 1;
     }
 #pragma unroll
     for (int q = 0; q < kReduceSlots; ++q) {
-      if (q < n && u < units) {
+      if (taken) {
+        const float w = __shfl_sync(0xffffffffu, weight, __ffs(taken) - 1);
+        taken &= taken - 1;
         const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[q]);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {   // product and sum rounded separately, as the CPU oracle does
-          sum[2 * i] = __fadd_rn(sum[2 * i], __fmul_rn(w[q], __low2float(h[i])));
-          sum[2 * i + 1] = __fadd_rn(sum[2 * i + 1], __fmul_rn(w[q], __high2float(h[i])));
+          sum[2 * i] = __fadd_rn(sum[2 * i], __fmul_rn(w, __low2float(h[i])));
+          sum[2 * i + 1] = __fadd_rn(sum[2 * i + 1], __fmul_rn(w, __high2float(h[i])));
         }
       }
     }
