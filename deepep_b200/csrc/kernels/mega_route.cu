@@ -1,4 +1,5 @@
-// Stand-alone launches of the MegaMoE routing/pull and finishing phases (see mega_route.cuh).
+// Stand-alone launches of the MegaMoE routing/pull and finishing phases (see mega_route.cuh), the copy of a call's inputs, and the
+// final reduction of a single rank.
 #include "mega_route.cuh"
 
 namespace dep {
