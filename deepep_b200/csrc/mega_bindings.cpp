@@ -20,12 +20,15 @@ void check(cudaError_t e, const char* what) {
     throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
   }
 }
+// An entry, or null.  One look at the dictionary per argument: a launch has a hundred, and a call of a few tokens takes the kernels
+// less time than the host.
+py::handle find(const py::dict& d, const char* key) { return PyDict_GetItemString(d.ptr(), key); }
 template <class T> T* ptr(const py::dict& d, const char* key) {
-  if (!d.contains(key) || d[key].is_none()) return nullptr;
-  return reinterpret_cast<T*>(d[key].cast<uintptr_t>());
+  const py::handle v = find(d, key);
+  return !v || v.is_none() ? nullptr : reinterpret_cast<T*>(v.cast<uintptr_t>());
 }
-int geti(const py::dict& d, const char* key, int dflt = 0) { return d.contains(key) ? d[key].cast<int>() : dflt; }
-long long getl(const py::dict& d, const char* key, long long dflt = 0) { return d.contains(key) ? d[key].cast<long long>() : dflt; }
+int geti(const py::dict& d, const char* key, int dflt = 0) { const py::handle v = find(d, key); return v ? v.cast<int>() : dflt; }
+long long getl(const py::dict& d, const char* key, long long dflt = 0) { const py::handle v = find(d, key); return v ? v.cast<long long>() : dflt; }
 
 // One grouped GEMM launch.  `d` carries operand pointers and shapes; `session` is needed only by the
 // combine epilogue (peer workspaces).

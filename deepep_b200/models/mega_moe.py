@@ -172,6 +172,20 @@ class MegaEngine:
                 ready=torch.zeros((self.max_mtiles,), **i32), pulled=torch.zeros((self.max_mtiles,), **i32), tile_counter=torch.zeros((1,), **i32),
                 # the same three for calls that find them zero and leave them zero
                 clean=torch.zeros((2 * self.max_mtiles + 1,), **i32)))
+        self._fixed = [self._fixed_args(sc) for sc in self.scratch]
+
+    def _fixed_args(self, sc: dict):
+        """What every launch says about the engine's own sizes and tensors, which live as long as the engine: the arguments of routing,
+        final reduction and the two GEMMs."""
+        at = {name: t.data_ptr() for name, t in sc.items()}
+        pick = lambda *names: {name: at[name] for name in names}
+        sizes = dict(in_off=self.in_off, E=self.E, K=self.K, H=self.H, max_tokens=self.M, S=self.S, expert_rows=at["expert_rows"])
+        route = dict(sizes, max_mtiles=self.max_mtiles, **pick("a1", "a1_sf", "row_src", "mtile_expert", "num_mtiles", "expert_list"))
+        gemm = dict(pick("mtile_expert", "num_mtiles"), rows_pad=self.rows_cap, error_flag=at["err"])
+        return (route, dict(sizes, comb_off=self.comb_off),
+                dict(gemm, a=at["a1"], sfa=at["a1_sf"], k=self.H, epi=1, inter=self.I, **pick("a2", "a2_sf")),
+                dict(gemm, a=at["a2"], sfa=at["a2_sf"], k=self.I, epi=2, row_src=at["row_src"], comb_off=self.comb_off,
+                     max_tokens=self.M, topk=self.K + self.S, hidden=self.H))
 
     @staticmethod
     def mega_bytes(C, max_tokens: int, hidden: int, topk: int, num_shared_experts: int = 0) -> int:
@@ -199,28 +213,20 @@ class MegaEngine:
         them there: ``stats_set``); fused only.
         ``timer``: int64 ``[SMs, mega_timer_words]`` that receives one record of phase stamps per CTA (fused, one rank)."""
         C, lay = self.C, self.layout
-        s = (stream if stream is not None else torch.cuda.current_stream(self.device)).cuda_stream
+        if stream is not None:
+            s = stream.cuda_stream
+        else:
+            s = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if self.device.index is None else self.device.index)
         route_args, finish_args, gemm1_args, gemm2_args, hold = [], [], [], [], []
+        stamps = None if timer is None else timer.data_ptr()
         for i in range(self.n):
-            sc, w1, w2 = self.scratch[i], l1[i], l2[i]
-            route_args.append(dict(in_off=self.in_off, T=tokens[i], E=self.E, K=self.K, H=self.H, max_tokens=self.M,
-                                   S=self.S, x_bf16=None if x_bf16 is None or x_bf16[i] is None else x_bf16[i].data_ptr(),
-                                   timer=None if timer is None else timer.data_ptr(),
-                                   max_mtiles=self.max_mtiles, a1=sc["a1"].data_ptr(), a1_sf=sc["a1_sf"].data_ptr(),
-                                   row_src=sc["row_src"].data_ptr(), mtile_expert=sc["mtile_expert"].data_ptr(),
-                                   num_mtiles=sc["num_mtiles"].data_ptr(), expert_rows=sc["expert_rows"].data_ptr(),
-                                   expert_list=sc["expert_list"].data_ptr()))
-            finish_args.append(dict(in_off=self.in_off, comb_off=self.comb_off, T=tokens[i], E=self.E, K=self.K, H=self.H,
-                                    max_tokens=self.M, y=ys[i].data_ptr(), S=self.S,
-                                    timer=None if timer is None else timer.data_ptr(), expert_rows=sc["expert_rows"].data_ptr(),
+            route, finish, gemm1, gemm2 = self._fixed[i]
+            route_args.append(dict(route, T=tokens[i], x_bf16=None if x_bf16 is None or x_bf16[i] is None else x_bf16[i].data_ptr(),
+                                   timer=stamps))
+            finish_args.append(dict(finish, T=tokens[i], y=ys[i].data_ptr(), timer=stamps,
                                     stats=None if stats is None or not fused else stats.data_ptr(), stats_set=int(stats_set)))
-            common = dict(mtile_expert=sc["mtile_expert"].data_ptr(), num_mtiles=sc["num_mtiles"].data_ptr(), rows_pad=self.rows_cap,
-                          error_flag=sc["err"].data_ptr())
-            gemm1_args.append(dict(common, **_weight_args(w1, hold), a=sc["a1"].data_ptr(), sfa=sc["a1_sf"].data_ptr(), k=self.H, epi=1,
-                                   a2=sc["a2"].data_ptr(), a2_sf=sc["a2_sf"].data_ptr(), inter=self.I))
-            gemm2_args.append(dict(common, **_weight_args(w2, hold), a=sc["a2"].data_ptr(), sfa=sc["a2_sf"].data_ptr(), k=self.I, epi=2,
-                                   row_src=sc["row_src"].data_ptr(), comb_off=self.comb_off, max_tokens=self.M,
-                                   topk=self.K + self.S, hidden=self.H))
+            gemm1_args.append(dict(gemm1, **_weight_args(l1[i], hold)))
+            gemm2_args.append(dict(gemm2, **_weight_args(l2[i], hold)))
         if fused:
             pair = self.use_pairs(tokens)
             swap = not pair and self.use_swap(tokens)
@@ -230,10 +236,11 @@ class MegaEngine:
             fused_args = []
             for i in range(self.n):    # the fused kernel overlaps the pull with the GEMMs through per-tile counters
                 sc = self.scratch[i]
-                counters = [sc[name].data_ptr() for name in ("ready", "pulled", "tile_counter")]
                 if alone:
-                    counters = [sc["clean"].data_ptr() + at * 4 for at in (0, self.max_mtiles, 2 * self.max_mtiles)]
-                ready, pulled, ticket = counters
+                    ready = sc["clean"].data_ptr()
+                    pulled, ticket = ready + 4 * self.max_mtiles, ready + 8 * self.max_mtiles
+                else:
+                    ready, pulled, ticket = (sc[name].data_ptr() for name in ("ready", "pulled", "tile_counter"))
                 route_args[i]["pulled"] = gemm1_args[i]["a_ready"] = pulled
                 route_args[i]["tile_pairs"] = int(pair)
                 route_args[i]["alone"] = int(alone)
