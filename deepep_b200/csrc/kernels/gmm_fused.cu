@@ -99,20 +99,23 @@ __device__ __forceinline__ int count_of(const GmmArgs& a, int e) {
 
 // Exclusive prefix of this rank's per-expert row counts into its table (one warp).
 // table[0] = total rows, table[1] = `limit` (rows the owner's area really holds), table[4 + e] = first row of expert e.
+// Sums are taken in 64 bits and held at the largest int, which is behind every area: the entries never decrease, and the owner of
+// each expert from there on finds that its rows are not held.
 __device__ __forceinline__ void publish_table(const GmmArgs& a, int* table, int limit, int lane) {
-  int run = 0;
+  auto entry = [](long long rows) { return (int)min(rows, 0x7fffffffll); };
+  long long run = 0;
   for (int e0 = 0; e0 < a.E; e0 += 32) {
     const int e = e0 + lane;
-    const int c = e < a.E ? count_of(a, e) : 0;
-    int inc = c;
+    const long long c = e < a.E ? count_of(a, e) : 0;
+    long long inc = c;
     for (int d = 1; d < 32; d <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, inc, d);
+      const long long o = __shfl_up_sync(0xffffffffu, inc, d);
       if (lane >= d) inc += o;
     }
-    if (e < a.E) table[4 + e] = run + inc - c;
+    if (e < a.E) table[4 + e] = entry(run + inc - c);
     run += __shfl_sync(0xffffffffu, inc, 31);
   }
-  if (lane == 0) { table[4 + a.E] = run; table[0] = run; table[1] = limit; }
+  if (lane == 0) { table[4 + a.E] = table[0] = entry(run); table[1] = limit; }
 }
 
 // Segments (local expert, source rank) of this rank's gathered order, from every rank's table.  Run by all threads
@@ -126,7 +129,7 @@ __device__ __forceinline__ void build_layout(const GmmArgs& a, GmmShared& sh, in
     const int* table = reinterpret_cast<const int*>(ctx.ws[s] + a.table_off);
     int first = 0, cnt = 0;
     if (alive) { first = __ldcg(table + 4 + e); cnt = __ldcg(table + 4 + e + 1) - first; }
-    if (cnt < 0 || first < 0 || (alive && first + cnt > __ldcg(table + 1))) { bad = 1; cnt = 0; }   // the owner does not hold these rows
+    if (cnt < 0 || first < 0 || (alive && (long long)first + cnt > __ldcg(table + 1))) { bad = 1; cnt = 0; }   // the owner does not hold these rows
     sh.seg_src[i] = first;
     sh.seg_dst[i + 1] = cnt;
   }

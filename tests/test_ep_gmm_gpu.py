@@ -166,6 +166,39 @@ def test_counts_of_either_integer_type(world):
             s.close()
 
 
+@pytest.mark.parametrize("op", ["a2av_gmm", "gmm_a2av"])
+@pytest.mark.parametrize("dtype,most", [(torch.int32, 2 ** 31 - 1), (torch.int64, 1 << 40)])
+@pytest.mark.parametrize("oversized", [(0, 3), (2, 3), (0, 5), (4, 5), tuple(range(6))])
+def test_counts_whose_sum_fits_no_int_are_reported_by_every_owner(op, dtype, most, oversized):
+    """Two ranks of three experts each, both of which name more rows than an int holds: the owners of those experts, and of any
+    behind the first of them, report it (a sum that wrapped round would look like one that fits)."""
+    from deepep_b200.ops import load_native
+
+    C, dev, world, E, K, N = load_native(), torch.device("cuda"), 2, 6, 64, 64
+    layout = C.make_mega_layout(world, 1, 128, 1, G.GmmEngine.region_bytes(C, 64, K, N))
+    sessions = [C.Session(r, world, layout.total, 20.0) for r in range(world)]
+    for s in sessions:
+        s.attach_peers([q.workspace for q in sessions])
+    try:
+        eng = G.GmmEngine(sessions, layout, dev, 64, K, N)
+        counts = [most if e in oversized else 2 for e in range(E)]
+        rows = [torch.ones((16, K), dtype=torch.bfloat16, device=dev) for _ in range(world)]
+        weights = [torch.ones((E // world, K, N), dtype=torch.bfloat16, device=dev) for _ in range(world)]
+        outs = [torch.zeros((16, N), dtype=torch.bfloat16, device=dev) for _ in range(world)]
+        getattr(eng, op)(rows, weights, [torch.tensor(counts, dtype=dtype, device=dev) for _ in range(world)], outs, num_experts=E)
+        torch.cuda.synchronize()
+        codes = [int(sc["err"].item()) for sc in eng.scratch]
+        first = min(oversized)
+        assert codes == [2 if first < 3 else 0, 2] and all(s.status()["code"] == 0 for s in sessions)
+        if first >= 3:                      # the first rank's experts are served as ever: two rows from, or back to, either rank
+            done, rows = (outs[:1], 12) if op == "a2av_gmm" else (outs, 6)
+            assert all(bool((out[:rows] == K).all()) for out in done)
+    finally:
+        torch.cuda.synchronize()
+        for s in sessions:
+            s.close()
+
+
 def test_both_tile_widths_give_the_same_rows():
     """Nine narrow tiles (one and two halves high): on nine blocks all at once, on eight and six the short ones of the last row block
     are second tiles, behind 13 K steps in a pipeline of four; on five and two blocks the wide ones take their place."""
