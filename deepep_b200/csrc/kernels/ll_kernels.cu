@@ -398,16 +398,11 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
       }
     }
     if (blockIdx.x == 0) {
-      if (a.mailbox) __threadfence_system();
-      layout_sync();
+      if (a.mailbox) __threadfence_system();     // the last block of the launch publishes the call's number
       if (lt == 0) {
         a.expert_offsets[Lx] = all;
         *a.num_rows = all;
-        if (a.mailbox) {
-          a.mailbox[0] = all;
-          __threadfence_system();
-          a.mailbox[3] = a.seq;
-        }
+        if (a.mailbox) { a.mailbox[0] = all; __threadfence_system(); }
       }
     }
     }
@@ -518,7 +513,15 @@ __global__ void __launch_bounds__(kLLThreads) ep_dispatch_ll_kernel(const __grid
     stamp(5);
     if (!ld_volatile_int(&ctl->abort) && threadIdx.x < P)
       st_release_sys(&control_of(ctx.ws[threadIdx.x])->ll_disp_ack[me], epoch);
-    if (threadIdx.x == 0) ctl->epoch[kOpLLDispatch] = epoch;
+    if (threadIdx.x == 0) {
+      ctl->epoch[kOpLLDispatch] = epoch;
+      // A host that waits for the counts goes on when the rows of the peers are in place too: a wait for them that ran out is in the
+      // status by now (the blocks arrive behind their own waits), and the host looks there next.
+      if (a.mailbox) {
+        __threadfence_system();
+        a.mailbox[3] = a.seq;
+      }
+    }
   }
 }
 

@@ -276,8 +276,10 @@ class CudaEngine:
         return self._calls if awaited else 0
 
     def _await_counts(self, seq: int, stream, what: str) -> None:
-        """The host needs the counts of call ``seq``: they are in the mailbox before the kernel is done, so that is polled first
-        (the kernels take tens of microseconds); what takes longer is waited for with an event, and not for ever."""
+        """The host needs the counts of call ``seq``: the mailbox is polled first (the kernels take tens of microseconds), what takes
+        longer is waited for with an event, and not for ever.  A single rank's kernels publish the counts while they still write
+        records or rows: nothing in them can fail after that.  Those of several ranks publish behind the last of their waits, so that
+        a wait that ran out is in the status when this returns."""
         if not self.C.wait_mailbox(self.sessions, seq, 5000):
             self._host_wait(stream, what)
 

@@ -242,3 +242,41 @@ def test_ll_dispatch_that_gives_up_leaves_no_rows_behind():
         torch.cuda.synchronize()
         for s in ranks:
             s.close()
+
+
+@pytest.mark.parametrize("limit", [0.002, 0.05])
+def test_ll_dispatch_reports_rows_that_never_came(limit):
+    """One of two ranks runs alone and finds the peer's routing table, but none of the rows that it announces: the dispatch that
+    reads its counts back raises itself, whether its kernel gives up while the host still polls or later."""
+    from deepep_b200.models.mega_moe import _view
+    from deepep_b200.ops import load_native
+    from deepep_b200.parallel.engine_cuda import CommunicationError, CudaEngine
+
+    C, T, H, E, K, P = load_native(), 24, 512, 16, 4, 2
+    region = C.ll_region_bytes(P, T, K, H)
+    layout = C.make_layout(P, T, H, K, region, 0, 0)
+    ranks = [C.Session(r, P, layout.total, limit) for r in range(P)]
+    try:
+        for s in ranks:
+            s.attach_peers([r.workspace for r in ranks])
+        # what the peer would have written for the first call: header, table, weights and flag, in this order and 1024-byte aligned
+        sizes = dict(hdr=P * 16, idx=P * T * K * 4, w=P * T * K * 4, flag=P * 8)
+        at, dev = ranks[0].workspace + layout.ll + region // 2, torch.device("cuda", torch.cuda.current_device())
+        part = {}
+        for name, nbytes in sizes.items():
+            part[name] = _view(at, nbytes, dev)
+            at += -(-nbytes // 1024) * 1024
+        part["hdr"].view(torch.int32).view(P, 4)[1, 0] = 5
+        part["idx"].view(torch.int32).view(P, T, K)[1, :5] = torch.arange(K, dtype=torch.int32, device=dev)
+        part["w"].view(torch.float32).view(P, T, K)[1, :5] = 0.25
+        part["flag"].view(torch.int64)[1] = 1
+        torch.cuda.synchronize()
+        eng = CudaEngine(ranks[:1], layout, dev)
+        x = torch.randn((T, H), generator=torch.Generator().manual_seed(1)).bfloat16().cuda()
+        idx, w = make_routes("random", T, E, K, P, 2).cuda(), make_weights(T, K, 3).cuda()
+        with pytest.raises(CommunicationError, match=r"ll_dispatch timeout at wait site 2 \(a part of a row from a source rank\) on peer 1"):
+            eng.ll_dispatch([x], [idx], [w], E, 0)
+    finally:
+        torch.cuda.synchronize()
+        for s in ranks:
+            s.close()
