@@ -59,8 +59,9 @@ __device__ __forceinline__ void fence_for_peers(int world) {
 }
 
 // bf16 [T, H] -> e4m3 codes and one ue8m0 exponent per 32 values, written into this rank's symmetric input block.
-// Block scale 2^(floor(log2(amax)) - 8) (amax clamped to 2^-119, exponent to -127), values clamped to +-448: the
+// Block scale 2^(floor(log2(amax)) - 8) (amax clamped to 2^-119, exponent to -127), values saturated at +-448: the
 // quantiser of the reference's token-quant stage (stage/mega_moe_token_quant.hpp; oracle: reference.py:44-54).
+// What is not finite shows: a NaN makes its whole block NaN, an infinity becomes NaN and the others of its block zeros (scale 2^-127).
 // One lane per 32-value block.
 __device__ __forceinline__ void quantize_inputs_phase(const MegaRouteArgs& a, uint8_t* x_out, uint8_t* sf_out) {
   const int blocks_per_row = a.H / 32;
@@ -71,28 +72,26 @@ __device__ __forceinline__ void quantize_inputs_phase(const MegaRouteArgs& a, ui
 #pragma unroll
     for (int i = 0; i < 4; ++i) raw[i] = __ldg(src + i);
     float v[32];
-    float amax = 0.f;
+    unsigned amax = (127u - 119u) << 23;       // bits of 2^-119; magnitudes compare like their bits, NaN above infinity
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[i]);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         v[8 * i + 2 * j] = __low2float(h[j]); v[8 * i + 2 * j + 1] = __high2float(h[j]);
-        amax = fmaxf(amax, fmaxf(fabsf(v[8 * i + 2 * j]), fabsf(v[8 * i + 2 * j + 1])));
+        amax = max(amax, max(__float_as_uint(fabsf(v[8 * i + 2 * j])), __float_as_uint(fabsf(v[8 * i + 2 * j + 1]))));
       }
     }
-    amax = fmaxf(amax, __uint_as_float((127u - 119u) << 23));                       // 2^-119
-    const int exponent = max((int)((__float_as_uint(amax) >> 23) & 0xffu) - 127 - 8, -127);
-    const float inv = __uint_as_float((unsigned)(127 - exponent) << 23);          // 2^-exponent, exact
+    constexpr unsigned kInfinity = 0x7f800000u;
+    const int exponent = amax < kInfinity ? max((int)(amax >> 23) - 127 - 8, -127) : -127;
+    // 2^-exponent, exact; the reciprocal of an infinite or NaN maximum otherwise
+    const float inv = __uint_as_float(amax < kInfinity ? (unsigned)(127 - exponent) << 23 : amax == kInfinity ? 0u : 0x7fffffffu);
     uint32_t w[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       uint32_t word = 0;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float scaled = fminf(fmaxf(v[4 * i + j] * inv, -448.f), 448.f);
-        word |= (uint32_t)__nv_cvt_float_to_fp8(scaled, __NV_SATFINITE, __NV_E4M3) << (8 * j);
-      }
+      for (int j = 0; j < 4; ++j) word |= (uint32_t)__nv_cvt_float_to_fp8(v[4 * i + j] * inv, __NV_SATFINITE, __NV_E4M3) << (8 * j);
       w[i] = word;
     }
     int4* dst = reinterpret_cast<int4*>(x_out) + b * 2;

@@ -167,6 +167,45 @@ def test_inputs_of_a_call_are_copied_whole(T, H, K):
         buf.destroy()
 
 
+@pytest.mark.parametrize("T", [5, 300])
+def test_rows_that_are_not_finite_stay_visible(T):
+    """bf16 rows with NaN and infinities: the kernel's quantiser writes the codes of the torch quantiser, and exactly these tokens'
+    outputs are NaN, through both entry points."""
+    from deepep_b200.models.mega_moe import SymmBuffer, fp8_fp4_mega_moe, mega_moe, transform_weights_for_mega_moe
+
+    dev, H, I, E, K = torch.device("cuda"), 512, 128, 8, 2
+    x = torch.randn((T, H), generator=torch.Generator().manual_seed(T)).bfloat16()
+    clean = x.clone()
+    nan, inf = float("nan"), float("inf")
+    x[0, 3], x[1, 70], x[1, 71], x[2, H - 1] = nan, inf, -inf, -inf
+    x[3, 32:64] = torch.tensor([nan, inf] * 16).bfloat16()
+    x[4, 9], x[4, 40], x[4, 64:96] = 3.3e38, -3.3e38, 0.0         # the largest finite values and a block of zeros are ordinary rows
+    clean[4] = x[4]
+    if T > 5:
+        x[T - 1, 1] = -nan
+    odd = ~x.isfinite().all(1)
+    idx, w = make_routes("random", T, E, K, 1, 5), make_weights(T, K, 3)
+    codes, sf = O.quantize_mxfp8(x)
+    finite = x.view(T, H // 32, 32).isfinite().all(2)
+    buf = SymmBuffer(None, E, T + 3, K, H, I)
+    try:
+        weights = transform_weights_for_mega_moe(*O.make_weights(E, H, I, 2), device=dev)
+        ref = mega_moe(clean.to(dev), idx.to(dev), w.to(dev), *weights, buf)[0]
+        y = mega_moe(x.to(dev), idx.to(dev), w.to(dev), *weights, buf)[0]
+        again = torch.empty_like(y)
+        fp8_fp4_mega_moe(again, *weights, buf, x=x.to(dev), check=True)
+        got = buf.x[:T].cpu().float()
+        assert torch.equal(got.isnan(), codes.float().isnan())
+        assert torch.equal(got.nan_to_num(nan=0.0), codes.float().nan_to_num(nan=0.0))
+        assert torch.equal(buf.x_sf[:T].cpu()[finite], sf[finite])
+        for out in (y, again):
+            assert bool(out[odd.to(dev)].isnan().all())
+            assert torch.equal(out.cpu()[~odd].view(torch.int16), ref.cpu()[~odd].view(torch.int16))     # (token 4's overflow behind the codes)
+            assert bool(out[5:].cpu()[~odd[5:]].isfinite().all())
+    finally:
+        buf.destroy()
+
+
 @pytest.mark.parametrize("T,H,I,E,K,S", [(1, 256, 128, 4, 1, 0), (9, 512, 128, 4, 3, 1), (33, 768, 128, 8, 4, 2),
                                          (70, 1024, 256, 16, 15, 1), (300, 256, 128, 8, 5, 0), (256, 256, 128, 40, 4, 0),
                                          (257, 256, 128, 8, 3, 1)])
