@@ -426,10 +426,16 @@ class SymmBuffer:
                 and topk_idx.dtype in (torch.int32, torch.int64) and topk_weights.dtype == torch.float32
                 and tuple(topk_idx.shape) == tuple(topk_weights.shape) == (bs, self.num_topk)
                 and all(t.is_contiguous() and t.device == self.x.device for t in given)):
-            self.engine.C.mega_load(0 if x is None else x.data_ptr(), 0 if x is None else codes.data_ptr(), topk_idx.data_ptr(),
-                                    topk_idx.dtype == torch.int64, topk_weights.data_ptr(), self.x.data_ptr(), self.x_sf.data_ptr(),
-                                    self.topk_idx.data_ptr(), self.topk_weights.data_ptr(), bs, self.hidden, self.num_topk,
-                                    torch.cuda.current_stream(self.device).cuda_stream)
+            index = self.x.device.index
+            args = (0 if x is None else x.data_ptr(), 0 if x is None else codes.data_ptr(), topk_idx.data_ptr(),
+                    topk_idx.dtype == torch.int64, topk_weights.data_ptr(), self.x.data_ptr(), self.x_sf.data_ptr(),
+                    self.topk_idx.data_ptr(), self.topk_weights.data_ptr(), bs, self.hidden, self.num_topk,
+                    torch.cuda.current_stream(index).cuda_stream)
+            if index == torch.cuda.current_device():
+                self.engine.C.mega_load(*args)
+            else:
+                with torch.cuda.device(index):
+                    self.engine.C.mega_load(*args)
             return
         if x is not None:
             self.x.view(torch.uint8)[:bs].copy_(x.to(torch.float8_e4m3fn).view(torch.uint8))

@@ -3,6 +3,9 @@ block scales), the argument rules of ``fp8_fp4_mega_moe`` in the order the refer
 (``experiments/megamoe/python/deep_ep_experimental/megamoe/api.py:520-567``), shared-expert weight joining and the
 statistics update.  The buffer object is assembled by hand around a recording engine; no kernel runs.
 """
+import contextlib
+import types
+
 import pytest
 import torch
 
@@ -84,6 +87,37 @@ def test_load_inputs_converts_power_of_two_block_scales():
     sym.topk_weights[1, 1] = float("nan")
     with pytest.raises(ValueError, match="finite"):
         sym.validate_inputs(5)
+
+
+def test_inputs_are_copied_on_the_buffers_device(monkeypatch):
+    """The copy kernel is launched with the buffer's device current, whichever device the caller works on."""
+    log, current = [], [0]
+
+    @contextlib.contextmanager
+    def device(index):
+        before, current[0] = current[0], index
+        yield
+        current[0] = before
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current[0])
+    monkeypatch.setattr(torch.cuda, "device", device)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d: types.SimpleNamespace(cuda_stream=100 + getattr(d, "index", d)))
+
+    def tensor(dtype, *shape):
+        return types.SimpleNamespace(dtype=dtype, shape=shape, device=torch.device("cuda", 1), data_ptr=lambda: 4096, is_contiguous=lambda: True)
+
+    sym = object.__new__(MM.SymmBuffer)
+    sym.engine = object.__new__(MM.MegaEngine)
+    sym.engine.C = types.SimpleNamespace(mega_load=lambda *args: log.append((current[0], args[-1])))
+    sym.num_max_tokens_per_rank, sym.hidden, sym.num_topk, sym.device = 8, 256, 2, torch.device("cuda", 1)
+    sym.x, sym.x_sf = tensor(torch.float8_e4m3fn, 8, 256), tensor(torch.uint8, 8, 8)
+    sym.topk_idx, sym.topk_weights = tensor(torch.int32, 8, 2), tensor(torch.float32, 8, 2)
+    given = tensor(torch.float8_e4m3fn, 3, 256), tensor(torch.uint8, 3, 8), tensor(torch.int64, 3, 2), tensor(torch.float32, 3, 2)
+    for here in (0, 1):
+        current[0] = here
+        sym._copy_inputs(*given)
+        assert current[0] == here
+    assert log == [(1, 101), (1, 101)]
 
 
 def test_forward_argument_rules_and_what_reaches_the_engine():
