@@ -46,10 +46,11 @@ class CommunicationError(RuntimeError):
 
 
 class _View:
-    """A tensor of a plan that lies in its ``slab``, made when somebody asks for it; the kernels get its address (``_address``)."""
+    """A tensor of a plan that lies in its ``slab``, made when somebody asks for it; the kernels get its address (``_address``).
+    One that no kernel reads again (not ``watched``) counts its changes by itself: they are the owner's business."""
 
-    def __init__(self, name: str):
-        self.name = name
+    def __init__(self, name: str, watched: bool):
+        self.name, self.watched = name, watched
 
     def __get__(self, plan, owner=None):
         if plan is None:
@@ -57,7 +58,8 @@ class _View:
         if plan.slab is None:
             return None
         begin, shape = plan.views[self.name]
-        made = plan.slab.as_strided(shape, (shape[1], 1) if len(shape) == 2 else (1,), begin)
+        slab = plan.slab if self.watched else plan.slab.data
+        made = slab.as_strided(shape, (shape[1], 1) if len(shape) == 2 else (1,), begin)
         plan.__dict__[self.name] = made
         return made
 
@@ -98,7 +100,7 @@ class RoutingPlan:
     views: Optional[dict] = None        # name -> (first int, shape)
 
     def tensors(self):
-        """What the handle watches for changes (the tables of the slab share one version counter)."""
+        """What the handle watches for changes (the watched tables of the slab share one version counter)."""
         tables = (self.slab,) if self.slab is not None else (self.expert_counts, self.expert_offsets, self.recv_row_src)
         return [t for t in (self.topk_idx, *tables, self.recv_w, self.recv_idx) if t is not None]
 
@@ -108,9 +110,10 @@ class RoutingPlan:
         return [t for t in (self.num_rows_dev, own, self.topk_w) if t is not None]
 
 
-for _name in ("send_slot", "slot_row", "stage_meta", "chunk_start", "rank_tokens", "rank_rows", "expert_counts", "expert_offsets",
-              "recv_row_src", "rank_matrix", "rank_prefix", "send_chunk_prefix", "recv_src_idx"):
-    setattr(RoutingPlan, _name, _View(_name))
+for _names, _watched in ((("send_slot", "slot_row", "stage_meta", "chunk_start", "rank_tokens", "rank_rows", "expert_counts", "expert_offsets",
+                           "recv_row_src"), True), (("rank_matrix", "rank_prefix", "send_chunk_prefix", "recv_src_idx"), False)):
+    for _name in _names:
+        setattr(RoutingPlan, _name, _View(_name, _watched))
 
 
 @lru_cache(maxsize=64)

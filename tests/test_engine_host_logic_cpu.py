@@ -74,6 +74,30 @@ def test_combine_runs_one_pass_per_token_window():
         eng.combine([x], [plan_for(4, 8)], [None], split=(100, 60))
 
 
+def test_a_handle_watches_the_tables_that_kernels_read_again():
+    """The V1 handle's prefix tables and source tokens lie beside the routing tables, but changing them in place is the caller's
+    business, as it is with a tensor of its own; a changed routing table is refused."""
+    from deepep_b200.parallel.elastic import EPHandle
+
+    ints, views = EC._slab_layout(5, 1, 2, 64, 4, 1, 8, 10, 1)
+    slab = torch.zeros((ints,), dtype=torch.int32)
+    for name, write in [(n, lambda t: t.add_(1)) for n in views] + [("recv_src_idx", lambda t: t[:3].fill_(7))]:
+        plan = EC.RoutingPlan(num_tokens=5, num_experts=8, num_topk=2, expand=False, alignment=1, meta_stride=4, num_rows=10,
+                              num_staged_rows=10, expert_counts_list=[0] * 8, topk_idx=torch.zeros((5, 2), dtype=torch.int64), recv_w=None,
+                              recv_idx=None, slab=slab, slab_ptr=slab.data_ptr(), views=views)
+        handle = EPHandle(False, 8, 1, 64, 0, plan.topk_idx, 10, 10, [0] * 8, *[None] * 7)
+        handle._plan = plan
+        handle._snapshot()
+        table = getattr(plan, name)
+        assert table.shape == torch.Size(views[name][1]) and table.data_ptr() == slab.data_ptr() + 4 * views[name][0]
+        write(table)
+        if name in ("rank_matrix", "rank_prefix", "send_chunk_prefix", "recv_src_idx"):
+            handle._check_unchanged()
+        else:
+            with pytest.raises(RuntimeError, match="modified in place"):
+                handle._check_unchanged()
+
+
 def test_status_block_becomes_a_readable_error():
     class Session:
         def __init__(self, **status):
