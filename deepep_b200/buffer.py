@@ -148,7 +148,7 @@ class Buffer:
         plan = eh._plan
         send_head = plan.send_slot[:tokens]
         if in_rank is None:
-            in_rank = send_head >= 0
+            in_rank = plan.token_in_rank
         slot = self._slots.acquire()
         slot.move(SlotState.DISPATCH_IN_FLIGHT)
         slot.move(SlotState.DISPATCH_READY)
@@ -196,7 +196,8 @@ class Buffer:
         rx, ridx, rw, h, ev = eb.dispatch(x, topk_idx=topk_idx, topk_weights=topk_weights, num_experts=num_tokens_per_expert.numel(),
                                           num_sms=sms, previous_event=previous_event, async_with_compute_stream=async_finish,
                                           allocate_on_comm_stream=allocate_on_comm_stream, do_expand=False,
-                                          do_cpu_sync=(num_worst_tokens == 0), num_max_tokens_per_rank=10 ** 9, _rank_matrix=True)
+                                          do_cpu_sync=(num_worst_tokens == 0), num_max_tokens_per_rank=10 ** 9, _rank_matrix=True,
+                                          _token_in_rank=is_token_in_rank is None)
         counts = h.num_recv_tokens_per_expert_list
         if counts is not None and expert_alignment > 1:
             counts = [-(-c // expert_alignment) * expert_alignment for c in counts]

@@ -413,7 +413,7 @@ class ElasticBuffer:
                  num_max_tokens_per_rank=None, expert_alignment=None, num_sms=0, num_qps=0, previous_event=None,
                  previous_event_before_epilogue=None, async_with_compute_stream=False, allocate_on_comm_stream=False,
                  handle=None, do_handle_copy=True, do_cpu_sync=None, do_expand=False, do_zero_padding=False,
-                 use_tma_aligned_col_major_sf=False, _rank_matrix=False):
+                 use_tma_aligned_col_major_sf=False, _rank_matrix=False, _token_in_rank=False):
         """Send every token to the ranks that own its experts.
 
         Returns ``(recv_x | (recv_x, recv_x_sf), recv_topk_idx, recv_topk_weights, handle, event)``.
@@ -470,6 +470,10 @@ class ElasticBuffer:
                                           cpu_sync=cpu_sync, stream=comm, **({"rank_matrix": True} if _rank_matrix else {}))[0]
                 recv_x, recv_sf = self.engine.dispatch([x if x_sf is not None else x_data], [plan], mode,
                                                        blocks=num_sms or self.num_sms, stream=comm)[0]
+                if _token_in_rank:         # where the routing pass wrote the table: the host does not wait for all of it
+                    plan.token_in_rank = torch.empty((tokens, self.world_size), dtype=torch.bool, device=plan.send_slot.device)
+                    with self._on(comm):
+                        torch.ge(plan.send_slot[:tokens], 0, out=plan.token_in_rank)
                 if stats is not None:
                     with self._on(comm):   # the counts are produced on the communication stream
                         stats.add_(plan.expert_counts.to(stats.dtype).to(stats.device))

@@ -47,6 +47,7 @@ class CpuPlan:
     rank_prefix: Optional[torch.Tensor] = None
     send_chunk_prefix: Optional[torch.Tensor] = None
     recv_src_idx: Optional[torch.Tensor] = None
+    token_in_rank: Optional[torch.Tensor] = None
     exact_rows: int = 0                 # rows that carry data; ``num_rows`` is larger when the counts were not read back
 
     def tensors(self):

@@ -95,6 +95,7 @@ class RoutingPlan:
     local_row: Optional[torch.Tensor] = None
     local_row_ptr: int = 0
     topk_w: Optional[torch.Tensor] = None
+    token_in_rank: Optional[torch.Tensor] = None      # V1 handle: [T, P], when the caller did not bring it
     slab: Optional[torch.Tensor] = None
     slab_ptr: int = 0
     views: Optional[dict] = None        # name -> (first int, shape)
@@ -107,7 +108,7 @@ class RoutingPlan:
     def private_tensors(self):
         """What the kernels use besides: kept alive with the others, but not watched for changes."""
         own = None if self.local_row is self.num_rows_dev else self.local_row
-        return [t for t in (self.num_rows_dev, own, self.topk_w) if t is not None]
+        return [t for t in (self.num_rows_dev, own, self.topk_w, self.token_in_rank) if t is not None]
 
 
 for _names, _watched in ((("send_slot", "slot_row", "stage_meta", "chunk_start", "rank_tokens", "rank_rows", "expert_counts", "expert_offsets",

@@ -126,3 +126,37 @@ def test_barrier_and_stream_getters(wired):
     with pytest.raises(RuntimeError, match="destroyed"):
         buf.get_comm_stream()
     buf.runtime.closed = False
+
+
+@pytest.mark.parametrize("worst", [0, 64])
+def test_v1_token_in_rank_is_made_behind_the_routing_pass(wired, monkeypatch, worst):
+    """An asynchronous V1 dispatch to which the caller brought no ``is_token_in_rank`` derives it from a table that the routing pass
+    writes on the communication stream: the comparison is queued there, in front of the event that the caller waits for."""
+    buf, log, contexts, (x, idx, w, E) = wired
+    v1 = object.__new__(deep_ep.Buffer)
+    v1.group, v1._elastic = None, buf
+    from deepep_b200.resources import SlotPool
+
+    v1._slots = SlotPool(2)
+    ran, on = [], buf._on
+
+    @contextlib.contextmanager
+    def recording(comm):
+        with on(comm):
+            ran.append(comm)
+            yield
+            ran.pop()
+
+    ge, leave = torch.ge, buf._leave
+    monkeypatch.setattr(buf, "_on", recording)
+    monkeypatch.setattr(torch, "ge", lambda *a, **k: (log.append(("ge", ran[-1] and ran[-1].name)), ge(*a, **k))[1])
+    monkeypatch.setattr(buf, "_leave", lambda *a, **k: (log.append(("leave",)), leave(*a, **k))[1])
+    counts = torch.bincount(idx[idx >= 0], minlength=E).int()
+    handle, event = v1.dispatch(x, topk_idx=idx, topk_weights=w, num_tokens_per_expert=counts, num_worst_tokens=worst, async_finish=True)[4:]
+    assert log == [("comm", "wait_stream", "cur"), ("ge", "comm"), ("leave",)] and event.event is not None
+    assert torch.equal(handle[4], (idx >= 0).any(1, keepdim=True))
+    given = torch.ones((x.shape[0], 1), dtype=torch.bool)
+    del log[:]
+    handle = v1.dispatch(x, topk_idx=idx, topk_weights=w, num_tokens_per_expert=counts, is_token_in_rank=given)[4]
+    assert handle[4] is given and ("ge", "comm") not in log
+    v1._elastic = None

@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from deepep_b200.oracle import reference as R
-from helpers import bits_equal, group_limited_routes, make_weights
+from helpers import bits_equal, group_limited_routes, make_routes, make_weights
 
 pytestmark = pytest.mark.gpu
 
@@ -43,6 +43,33 @@ def test_previous_event_async_and_comm_stream_allocation():
     # synchronous cached dispatch after an EventOverlap: the result is usable on the current stream at return
     again, _, _, _, ev = buf.dispatch(x2, handle=handle, previous_event=deep_ep.EventOverlap(deep_ep.EventHandle()))
     assert ev.event is None and bits_equal(again, rx)
+    torch.cuda.synchronize()
+    buf.destroy()
+
+
+@pytest.mark.parametrize("worst", [False, True])
+def test_v1_token_in_rank_of_an_asynchronous_call(worst):
+    """The communication stream is far behind when the call returns (``worst``: nothing is read back): every tensor of the handle is
+    right once the event has been waited for."""
+    import deepep_b200 as deep_ep
+
+    dev = torch.device("cuda")
+    T, H, E, K = 300, 256, 16, 3
+    x = torch.randn((T, H), generator=torch.Generator().manual_seed(2)).bfloat16().to(dev)
+    idx, w = make_routes("invalid", T, E, K, 1, 4).to(dev), make_weights(T, K, 5).to(dev)
+    buf = deep_ep.Buffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K, explicitly_destroy=True)
+    per_expert = buf.get_dispatch_layout(idx, E)[2]
+    want = ((idx >= 0) & (idx < E)).any(1, keepdim=True)
+    for _ in range(3):
+        torch.cuda._sleep(20_000_000)
+        late = deep_ep.EventHandle()
+        handle, event = buf.dispatch(x, topk_idx=idx, topk_weights=w, num_tokens_per_expert=per_expert, num_worst_tokens=T if worst else 0,
+                                     previous_event=late, async_finish=True)[4:]
+        event.current_stream_wait()
+        rows = int(want.sum())
+        assert torch.equal(handle[4], want) and torch.equal(handle[5] >= 0, want)
+        assert torch.equal(handle[3][:rows].long(), want[:, 0].nonzero()[:, 0]) and int(handle[0]) == rows
+        del handle
     torch.cuda.synchronize()
     buf.destroy()
 
