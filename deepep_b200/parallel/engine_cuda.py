@@ -285,9 +285,9 @@ class CudaEngine:
         records or rows: nothing in them can fail after that.  Those of several ranks publish behind the last of their waits, so that
         a wait that ran out is in the status when this returns."""
         if not self.C.wait_mailbox(self.sessions, seq, 5000):
-            self._host_wait(stream, what)
+            self._host_wait(stream, what, spin_seconds=0.0)        # polled without pause long enough
 
-    def _host_wait(self, stream, what: str) -> None:
+    def _host_wait(self, stream, what: str, spin_seconds: float = 0.005) -> None:
         """The host needs the results of what was just queued on ``stream``: wait for it, but not for ever."""
         from ..utils.hostwait import HostTimeout, wait_for_event
 
@@ -295,7 +295,7 @@ class CudaEngine:
         done = torch.cuda.Event()
         done.record(st)
         try:
-            wait_for_event(done, self.host_timeout, what)
+            wait_for_event(done, self.host_timeout, what, spin_seconds)
         except HostTimeout as exc:
             raise CommunicationError(f"{exc}; restart the distributed job") from None
         st.synchronize()                               # returns at once: everything before the event is complete

@@ -95,3 +95,34 @@ def test_the_engine_turns_a_host_timeout_into_a_communication_error(monkeypatch)
     engine.host_timeout = 0.05
     with pytest.raises(EC.CommunicationError, match=r"\[DEEPEP_CPU_TIMEOUT\] the routing layout pass .* restart the distributed job"):
         EC.CudaEngine._host_wait(engine, FakeStream(), "the routing layout pass")
+
+
+@pytest.mark.parametrize("polled", [True, False])
+def test_the_host_polls_without_pause_once(monkeypatch, polled):
+    """``_await_counts``: the mailbox is polled for 5 ms; when the counts are not there by then, the event behind the kernel is waited
+    for with pauses from the start, not for another 5 ms without."""
+    import types
+
+    import torch
+
+    from deepep_b200.parallel import engine_cuda as EC
+
+    clock, log = Clock(0.0001), []
+
+    class FakeEvent:
+        left = 20
+
+        def record(self, stream): ...
+
+        def query(self):
+            self.left -= 1
+            return self.left < 0
+
+    monkeypatch.setattr(torch.cuda, "Event", FakeEvent)
+    wait = HW.wait_for_event
+    monkeypatch.setattr(HW, "wait_for_event", lambda *a, **k: wait(*a, **k, clock=clock, sleep=clock.sleep))
+    engine = object.__new__(EC.CudaEngine)
+    engine.device, engine.host_timeout, engine.sessions = torch.device("cpu"), 5.0, []
+    engine.C = types.SimpleNamespace(wait_mailbox=lambda sessions, seq, us: (log.append((seq, us)), polled)[1])
+    engine._await_counts(7, types.SimpleNamespace(synchronize=lambda: None), "the routing layout pass")
+    assert log == [(7, 5000)] and len(clock.sleeps) == (0 if polled else 20)
