@@ -269,11 +269,15 @@ class MegaEngine:
         return per_expert >= 384
 
     def use_swap(self, tokens: Sequence[int]) -> bool:
-        """Whether tiles of few rows multiply the weights by the rows (``kSwap`` in ``mega_gemm.cuh``).  The line is at 32 rows per
-        expert, if every rank sends what this one does: up to there most tiles are that short.  32 experts, hidden 7168,
-        intermediate 2048, us with and without, both with longer phases around the GEMMs than now: 1 token 84 / 91, 16 157 / 169,
-        64 162 / 174, 128 (32 rows) 175 / 181, 160 184 / 183."""
-        return self.world * max(tokens) * self.K <= 32 * self.E
+        """Whether tiles of few rows multiply the weights by the rows (``kSwap`` in ``mega_gemm.cuh``).  Up to 24 rows per expert, if
+        every rank sends what this one does, next to all tiles are that short (32 rows).  Up to 32 about half of them are: what the
+        others lose in this instance is hidden while the rank's weights, more than the L2 holds (126 MB as e2m1), stream from memory,
+        and not below.  us plain / swapped, cold L2, one rank unless said: 24 rows per expert, 8 experts of 4096 x 1536, 16 rows,
+        59 / 54, 32 of 2048 x 768, 57 / 49, 64 of 7168 x 2048 329 / 311, four emulated ranks, 64 of 4096 x 1536, 200 / 191; 32 rows, 64 of
+        2048 x 768 (151 MB) 77 / 76, 32 of 7168 x 2048 180 / 176, two ranks, 32 of 4096 x 1536, 125 / 121, but 12 of 4096 x 1536 (113 MB)
+        66.8 / 67.4, 32 of 2048 x 768 (75 MB) 60 / 62, 8 of 1024 x 512 36 / 41, four ranks, 16 of 4096 x 1024, 102 / 105."""
+        rows, values = self.world * max(tokens) * self.K, 3 * self.L * self.H * self.I
+        return rows <= (32 if values > 2 * 126e6 else 24) * self.E
 
     WAIT_SITES = {1: "a pipeline barrier", 2: "the tile ticket from the producer warp", 3: "the first projection of a row block",
                   4: "rows pulled from the peers", 5: "the release of a group of operand stages", 6: "the drain of an accumulator",

@@ -120,6 +120,18 @@ def test_inputs_are_copied_on_the_buffers_device(monkeypatch):
     assert log == [(1, 101), (1, 101)]
 
 
+@pytest.mark.parametrize("world,experts,hidden,inter,topk,tokens,swapped", [
+    (1, 8, 1024, 512, 2, 96, True), (1, 8, 1024, 512, 2, 100, False), (1, 8, 1024, 512, 2, 128, False),      # 24, 25 and 32 rows per expert
+    (1, 32, 2048, 768, 4, 192, True), (1, 32, 2048, 768, 4, 256, False),                                      # 75 MB of weights
+    (1, 64, 2048, 768, 8, 256, True), (1, 32, 7168, 2048, 8, 128, True), (1, 32, 7168, 2048, 8, 129, False),  # more than the L2 holds
+    (4, 16, 4096, 1024, 2, 48, True), (4, 16, 4096, 1024, 2, 64, False), (2, 32, 4096, 1536, 4, 128, True)])
+def test_when_operands_are_swapped(world, experts, hidden, inter, topk, tokens, swapped):
+    """Both sides of the line, which depends on the weights that one rank holds."""
+    engine = object.__new__(MM.MegaEngine)
+    engine.world, engine.E, engine.L, engine.H, engine.I, engine.K = world, experts, experts // world, hidden, inter, topk
+    assert engine.use_swap([tokens] * world) is swapped
+
+
 def test_forward_argument_rules_and_what_reaches_the_engine():
     sym, (l1, l2) = make_buffer(), weights()
     y = torch.zeros((6, H), dtype=torch.bfloat16)
