@@ -82,10 +82,9 @@ enum MegaTimerSlot : int { kTimStart = 0, kTimHandshake = 1, kTimLayout = 2, kTi
                             kTimMmaThread = 7 };   // word 7: the MMA thread's cycles / 16, (waiting for operands) << 32 | (whole tile loop)
 
 // ---------------------------------------------------------------- routing + token pull
-// Tokens x (top-k + shared experts) up to which every block of a single rank derives the layout by itself, which costs a block more
-// the longer the table is.  The layer in captured graphs, 32 experts, hidden 7168, intermediate 2048, top-8, us with counts
-// over the grid / by every block: 1 token 76.4 / 71.3, 8 144.8 / 140.6, 32 151.9 / 148.6, 64 155.4 / 153.9, 128 166.8 / 166.2, 256 187.9 / 189.9.
-constexpr int kAloneSlots = 1024;
+// Tokens x (top-k + shared experts) up to which every block of a single rank can derive the layout by itself, which costs a block
+// more the longer the table is; MegaEngine.use_alone says when it does, with both sides measured.
+constexpr int kAloneSlots = 512;
 struct MegaRouteArgs {
   RankCtx ctx;
   long long in_off;            // byte offset of the input block (x, x_sf, topk_idx, topk_w) in a workspace

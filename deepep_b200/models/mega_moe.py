@@ -232,7 +232,7 @@ class MegaEngine:
             swap = not pair and self.use_swap(tokens)
             blocks = max(1, min(self.gemm_blocks, self.sm_count // self.n))
             apart = self.world == 1 and blocks == self.sm_count and timer is None     # a kernel on the whole GPU: only without a budget
-            alone = apart and tokens[0] * (self.K + self.S) <= C.mega_alone_slots
+            alone = apart and self.use_alone(tokens)
             fused_args = []
             for i in range(self.n):    # the fused kernel overlaps the pull with the GEMMs through per-tile counters
                 sc = self.scratch[i]
@@ -278,6 +278,16 @@ class MegaEngine:
         66.8 / 67.4, 32 of 2048 x 768 (75 MB) 60 / 62, 8 of 1024 x 512 36 / 41, four ranks, 16 of 4096 x 1024, 102 / 105."""
         rows, values = self.world * max(tokens) * self.K, 3 * self.L * self.H * self.I
         return rows <= (32 if values > 2 * 126e6 else 24) * self.E
+
+    def use_alone(self, tokens: Sequence[int]) -> bool:
+        """Whether every block of a single rank derives the layout by itself (``route_layout_alone`` in ``mega_route.cuh``): what a
+        block pays grows with the routing table and with the experts, and is set against two grid barriers.  us with counts over the
+        grid / by every block, cold L2: 32 experts of 7168 x 2048, top-8, 8 tokens 137.8 / 133.1, 64 (512 slots) 164.6 / 162.2, 128 175.3 /
+        176.8; 32 of 2048 x 768, top-4, 128 tokens (512) 50 / 47, 224 60 / 61, 256 60 / 62.5; 64 of 7168 x 2048, top-8, 64 tokens 302 / 300,
+        128 310 / 313; 1024 of 1024 x 256, 16 tokens 52 / 48, 64 (512) 100 / 97; 256 of 7168 x 2048, 8 tokens 291 / 289, 32 (256) 725 / 727,
+        64 1042 / 1056, 128 1194 / 1229."""
+        slots = max(tokens) * (self.K + self.S)
+        return slots <= (self.C.mega_alone_slots if self.E <= 128 else self.C.mega_alone_slots // 2)
 
     WAIT_SITES = {1: "a pipeline barrier", 2: "the tile ticket from the producer warp", 3: "the first projection of a row block",
                   4: "rows pulled from the peers", 5: "the release of a group of operand stages", 6: "the drain of an accumulator",

@@ -132,6 +132,15 @@ def test_when_operands_are_swapped(world, experts, hidden, inter, topk, tokens, 
     assert engine.use_swap([tokens] * world) is swapped
 
 
+@pytest.mark.parametrize("experts,topk,shared,tokens,alone", [(32, 8, 0, 64, True), (32, 8, 0, 65, False), (128, 7, 1, 64, True), (8, 1, 0, 513, False),
+                                                               (129, 8, 0, 32, True), (129, 8, 1, 32, False), (1024, 8, 0, 64, False)])
+def test_when_every_block_derives_the_layout(experts, topk, shared, tokens, alone):
+    """Both sides of the line: 512 slots, 256 with more than 128 experts."""
+    engine = object.__new__(MM.MegaEngine)
+    engine.C, engine.E, engine.K, engine.S = types.SimpleNamespace(mega_alone_slots=512), experts, topk, shared
+    assert engine.use_alone([tokens]) is alone
+
+
 def test_forward_argument_rules_and_what_reaches_the_engine():
     sym, (l1, l2) = make_buffer(), weights()
     y = torch.zeros((6, H), dtype=torch.bfloat16)

@@ -208,7 +208,8 @@ def test_rows_that_are_not_finite_stay_visible(T):
 
 @pytest.mark.parametrize("T,H,I,E,K,S", [(1, 256, 128, 4, 1, 0), (9, 512, 128, 4, 3, 1), (33, 768, 128, 8, 4, 2),
                                          (70, 1024, 256, 16, 15, 1), (300, 256, 128, 8, 5, 0), (256, 256, 128, 40, 4, 0),
-                                         (257, 256, 128, 8, 3, 1)])
+                                         (257, 256, 128, 8, 3, 1), (128, 256, 128, 40, 4, 0), (32, 256, 128, 16, 15, 1), (129, 256, 128, 8, 3, 1),
+                                         (64, 256, 128, 136, 4, 0), (64, 256, 128, 136, 4, 1)])
 def test_one_rank_with_and_without_barriers(T, H, I, E, K, S):
     """A layout that every block derives and a reduction that follows the layer give the bits of the phases with grid barriers
     (which a call with a timer takes): one to sixteen slots, not multiples of those in flight, masked and foreign ids, tables up to the
