@@ -172,6 +172,8 @@ class MegaEngine:
                 ready=torch.zeros((self.max_mtiles,), **i32), pulled=torch.zeros((self.max_mtiles,), **i32), tile_counter=torch.zeros((1,), **i32),
                 # the same three for calls that find them zero and leave them zero
                 clean=torch.zeros((2 * self.max_mtiles + 1,), **i32)))
+        # calls may be made on any stream, and what is zero here was zeroed on this one
+        torch.cuda.current_stream(device).synchronize()
         self._fixed = [self._fixed_args(sc) for sc in self.scratch]
 
     def _fixed_args(self, sc: dict):

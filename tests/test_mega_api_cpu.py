@@ -120,6 +120,20 @@ def test_inputs_are_copied_on_the_buffers_device(monkeypatch):
     assert log == [(1, 101), (1, 101)]
 
 
+def test_an_engine_is_ready_for_any_stream(monkeypatch):
+    """The counters that calls find zero are zeroed on the stream on which the engine is made; it is waited for before a call on
+    another stream can read them."""
+    log = []
+    zeros = torch.zeros
+    monkeypatch.setattr(torch, "zeros", lambda *a, **k: (log.append("zeros"), zeros(*a, **k))[1])
+    monkeypatch.setattr(MM, "require_native", lambda name: types.SimpleNamespace(mega_input_offsets=lambda *a: [0] * 6))
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda device: types.SimpleNamespace(multi_processor_count=148))
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device: types.SimpleNamespace(synchronize=lambda: log.append("synchronize")))
+    layout = types.SimpleNamespace(world=1, max_tokens=4, hidden=256, topk=2, mega=0)
+    engine = MM.MegaEngine([None], layout, torch.device("cpu"), 4, 128)
+    assert "clean" in engine.scratch[0] and log.count("synchronize") == 1 and log[-1] == "synchronize"
+
+
 @pytest.mark.parametrize("world,experts,hidden,inter,topk,tokens,swapped", [
     (1, 8, 1024, 512, 2, 96, True), (1, 8, 1024, 512, 2, 100, False), (1, 8, 1024, 512, 2, 128, False),      # 24, 25 and 32 rows per expert
     (1, 32, 2048, 768, 4, 192, True), (1, 32, 2048, 768, 4, 256, False),                                      # 75 MB of weights

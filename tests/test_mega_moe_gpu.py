@@ -245,6 +245,29 @@ def test_one_rank_with_and_without_barriers(T, H, I, E, K, S):
         buf.destroy()
 
 
+def test_first_call_on_another_stream():
+    """A buffer made while its stream is still busy, and used on a stream that waits for nothing but the inputs."""
+    from deepep_b200.models.mega_moe import SymmBuffer, mega_moe, transform_weights_for_mega_moe
+
+    dev, T, H, I, E, K = torch.device("cuda"), 20, 256, 128, 8, 2
+    weights = transform_weights_for_mega_moe(*O.make_weights(E, H, I, 2), device=dev)
+    x = torch.randn((T, H), generator=torch.Generator().manual_seed(1)).bfloat16().to(dev)
+    idx, w = make_routes("random", T, E, K, 1, 5).to(dev), make_weights(T, K, 3).to(dev)
+    torch.full((1 << 20,), 5, dtype=torch.int32, device=dev)          # what the allocator hands out next is not zero
+    torch.cuda.synchronize()
+    side, got = torch.cuda.Stream(), []
+    for busy in (True, False):
+        if busy:
+            torch.cuda._sleep(20_000_000)
+        buf = SymmBuffer(None, E, T, K, H, I)
+        with torch.cuda.stream(side):
+            got.append(mega_moe(x, idx, w, *weights, buf)[0])
+            side.synchronize()
+        buf.engine.check()
+        buf.destroy()
+    assert torch.equal(got[0], got[1]) and bool(got[0].any())
+
+
 @pytest.mark.parametrize("pairs", ["0", "1"])
 @pytest.mark.parametrize("E, S", [(32, 1), (33, 0), (64, 0), (70, 2)])
 def test_layout_of_more_than_32_local_experts(E, S, pairs):
