@@ -200,25 +200,32 @@ class CudaEngine:
         kernels stamp the phases of their block 0 (read with ``phase_stamps``); in the high-throughput dispatch /
         combine every block records its role, its start and end time, the time its first warp spent waiting for
         flags and the rows that warp moved.  The production instantiation carries none of that code.
+        With one rank the records of dispatch and combine come from the persistent kernels, which a call with a budget of SMs
+        runs: without one, dispatch and combine launch a warp per piece of a token, which has no phases to record (and a combine
+        weighs no rows while records are on).  ``enable_profiling`` times what a call without them launches.
         Parity: the reference's ``template <bool Profile>`` kernels (``csrc/kernels/dispatch/profile.hpp``,
         ``csrc/kernels/combine/profile.hpp``)."""
         self._device_profile = bool(on)
         self._prof.clear()
 
-    PHASE_STAMPS = {"ll_dispatch": (0, ("routes_read", "rows_sent", "tables_in", "layout_done", "rows_out", "last_block", "table_sent",
-                                        "first_row_stored")),
-                    "ll_combine": (8, ("entered", "rows_returned", "reduced", "last_block")),
-                    "notify": (16, ("table_sent", "tables_in", "histograms", "scans", "records", "done"))}
+    # operation -> phase -> word that its end is stamped into
+    PHASE_STAMPS = {"ll_dispatch": dict(routes_read=0, rows_sent=1, tables_in=2, layout_done=3, rows_out=4, last_block=5, table_sent=6,
+                                        first_row_stored=7),
+                    "ll_combine": dict(entered=8, rows_returned=9, reduced=10, last_block=11),
+                    "notify": dict(table_sent=16, tables_in=17, histograms=18, scans=19, records=20, done=21)}
+    # the kernels of a single rank, which exchange nothing
+    PHASE_STAMPS_ONE_RANK = {"ll_dispatch": dict(routes_read=0, tokens_marked=2, layout_done=3, rows_out=4, counts_published=5),
+                             "ll_combine": dict(slots_read=8, slots_checked=9, reduced=10, done=11),
+                             "notify": dict(entered=16, counted=17, counts_exchanged=18, layout_done=19, records=20, done=21)}
 
     def phase_stamps(self, op: str, i: int = 0) -> dict:
         """Phase stamps of block 0 of the last profiled launch of ``op`` (``"notify"``, ``"ll_dispatch"`` or
         ``"ll_combine"``) on rank index ``i``: microseconds since the kernel started at which each phase was complete.
         Only the profile instantiations of these kernels write stamps (``enable_device_profile``)."""
-        first, names = self.PHASE_STAMPS[op]
+        phases = (self.PHASE_STAMPS_ONE_RANK if self.world == 1 else self.PHASE_STAMPS)[op]
         torch.cuda.synchronize(self.device)
         words = torch.frombuffer(bytearray(self.sessions[i].read_control()), dtype=torch.int64)
-        at = self.C.control_dbg_offset // 8 + first
-        return {name: int(words[at + k]) / 1e3 for k, name in enumerate(names)}
+        return {name: int(words[self.C.control_dbg_offset // 8 + word]) / 1e3 for name, word in phases.items()}
 
     def _prof_buffer(self, op: str, i: int):
         if not self._device_profile:

@@ -266,3 +266,26 @@ def test_phase_stamps_of_the_profile_instantiations():
             assert blocks and all(b["end_us"] >= b["start_us"] >= 0 for b in blocks) and sum(b["rows"] for b in blocks) > 0
         eng.enable_device_profile(False)
         eng.check_status()
+
+
+def test_phase_stamps_of_one_rank():
+    """The kernels of a single rank stamp phases of their own: every one that has a name, in the order of the names."""
+    from deepep_b200.ops import load_native
+    from deepep_b200.parallel.virtual import VirtualWorld
+
+    T, H, E, K = 96, 256, 8, 2
+    x = torch.randn((T, H), generator=torch.Generator().manual_seed(1)).bfloat16().cuda()
+    idx, w = make_routes("random", T, E, K, 1, 2).cuda(), make_weights(T, K, 3).cuda()
+    with VirtualWorld(1, T, H, K, timeout=10.0, ll_bytes=load_native().ll_region_bytes(1, T, K, H)) as vw:
+        eng = vw.engine
+        eng.enable_device_profile(True)
+        eng.notify([idx], [w], E)
+        (plan, rows, _), = eng.ll_dispatch([x], [idx], [w], E, 0)
+        eng.ll_combine([rows], [plan])
+        for op, names in (("notify", ("entered", "counted", "counts_exchanged", "layout_done", "records", "done")),
+                          ("ll_dispatch", ("routes_read", "tokens_marked", "layout_done", "rows_out", "counts_published")),
+                          ("ll_combine", ("slots_read", "slots_checked", "reduced", "done"))):
+            stamps = eng.phase_stamps(op)
+            order = [stamps[name] for name in names]
+            assert tuple(stamps) == names and order == sorted(order) and 0 < order[-1] < 1e5, stamps
+        eng.check_status()
