@@ -65,6 +65,7 @@ void op_notify(const WsLayout& lay, const std::vector<py::object>& sessions, con
       throw std::invalid_argument("notify: the V1 handle's tensors come together");
     a.rcap = getl(d, "rcap"); a.seq = geti(d, "seq");
     a.mailbox = a.seq ? sessions[i].cast<Session&>().mailbox_device() : nullptr;    // nobody else's number appears in it
+    if (lay.world > 1 && (!a.hist || !a.hits || !a.own_hits || !a.cnt)) throw std::invalid_argument("notify: several ranks need the scratch");
     if (a.T < 0 || a.T > lay.max_tokens) throw std::invalid_argument("token count exceeds num_max_tokens_per_rank");
     if (a.K != lay.topk) throw std::invalid_argument("top-k width differs from the buffer's num_topk");
     if (a.E < a.ctx.world || a.E > kMaxExperts || a.E % a.ctx.world) throw std::invalid_argument("num_experts must be a multiple of the world size and at most 1024");

@@ -20,7 +20,7 @@ struct NotifyArgs {
   int alignment;               // every local expert's row block starts at a multiple of this
   int meta_stride;             // ints per stage_meta record: 2 + max(2, min(K, E / world))
   int seq;                     // the host's number of this call, which it waits for in the mailbox (0: it does not)
-  // scratch owned by the buffer
+  // scratch owned by the buffer (several ranks only)
   int* hist;                   // [P][NT][E]
   int* hits;                   // [P][NT]
   int* own_hits;               // [NT][P]

@@ -6,7 +6,7 @@
 // latency-critical step), or a plain C/C++ caller that has no tensor framework whose allocator
 // could own the scratch.  For them the routing-layout kernel (ep_notify, single rank) is offered
 // with all of its scratch memory inside the library: a file-scope device array of
-// DEEPEP_NOALLOC_SCRATCH_BYTES (1 MiB) that every GPU which loads this library holds until the
+// DEEPEP_NOALLOC_SCRATCH_BYTES (65 KiB) that every GPU which loads this library holds until the
 // process exits.  The caller passes only inputs and outputs.
 //
 // Limits: one rank, at most DEEPEP_NOALLOC_MAX_TOKENS tokens, top-k <= 16, at most 1024 experts.
@@ -24,7 +24,7 @@ extern "C" {
 #endif
 
 #define DEEPEP_NOALLOC_MAX_TOKENS 4096
-#define DEEPEP_NOALLOC_SCRATCH_BYTES (1 << 20)
+#define DEEPEP_NOALLOC_SCRATCH_BYTES (65 << 10)
 
 // Expanded-layout routing metadata of one rank that owns all `num_experts` experts.
 //   topk_idx      [num_tokens][num_topk] int64 (device), <0 or >= num_experts marks an empty slot

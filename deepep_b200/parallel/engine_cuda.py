@@ -173,13 +173,13 @@ class CudaEngine:
         # opt-in device-side records (the profile instantiation of the dispatch / combine kernels): one record per block
         self._device_profile = False
         self._prof: dict = {}
-        self._scratch = []
-        for _ in range(self.n):
-            self._scratch.append(dict(
+        self._scratch = [{} for _ in range(self.n)]
+        for scratch in self._scratch if self.world > 1 else ():      # a single rank's routing pass keeps its counts on the chip
+            scratch.update(
                 hist=torch.empty((self.world * nt * self.C.max_experts,), dtype=torch.int32, device=device),
                 hits=torch.empty((self.world * nt,), dtype=torch.int32, device=device),
                 own_hits=torch.empty((nt * self.world,), dtype=torch.int32, device=device),
-                cnt=torch.empty((self.world * self.C.max_experts,), dtype=torch.int32, device=device)))
+                cnt=torch.empty((self.world * self.C.max_experts,), dtype=torch.int32, device=device))
 
     # ------------------------------------------------------------------ helpers
     def _stream(self, stream=None) -> int:
@@ -369,8 +369,8 @@ class CudaEngine:
             v1 = at if rank_matrix else lambda name: None       # (cleared by the launcher, on its stream, where that is needed)
             sc = self._scratch[i]
             args.append(dict(topk_idx=idx.data_ptr(), topk_w=_ptr(topk_w[i]), T=T, E=num_experts, K=K, expand=int(expand),
-                             alignment=alignment, meta_stride=stride, hist=sc["hist"].data_ptr(), hits=sc["hits"].data_ptr(),
-                             own_hits=sc["own_hits"].data_ptr(), cnt=sc["cnt"].data_ptr(), send_slot=at("send_slot"),
+                             alignment=alignment, meta_stride=stride, hist=_ptr(sc.get("hist")), hits=_ptr(sc.get("hits")),
+                             own_hits=_ptr(sc.get("own_hits")), cnt=_ptr(sc.get("cnt")), send_slot=at("send_slot"),
                              slot_row=at("slot_row"), stage_meta=at("stage_meta"), chunk_start=at("chunk_start"),
                              rank_tokens=at("rank_tokens"), rank_rows=at("rank_rows"), expert_counts=at("expert_counts"),
                              expert_offsets=at("expert_offsets"), recv_row_src=at("recv_row_src"),

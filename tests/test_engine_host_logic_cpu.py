@@ -158,3 +158,18 @@ def test_argument_keys_agree_between_python_and_the_bindings():
                                ("op_ll_combine", "ll_bindings.cpp", "ll_combine")):
         native, python = cpp_keys(path, func), py_keys(method)
         assert python and native == python, (func, sorted(python - native), sorted(native - python))
+
+
+@pytest.mark.parametrize("world", [1, 2])
+def test_scratch_of_the_routing_pass(monkeypatch, world):
+    """Several ranks' counts pass through memory that the engine owns; a single rank's stay on the chip, and nothing is allocated."""
+    monkeypatch.setattr(EC, "require_native", lambda name: types.SimpleNamespace(chunk_tokens=64, max_experts=1024))
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda device: types.SimpleNamespace(multi_processor_count=148))
+    eng = EC.CudaEngine([None], types.SimpleNamespace(world=world, max_tokens=100, partial_tokens=100, topk=2, hidden=64), torch.device("cpu"))
+    shapes = {name: tuple(t.shape) for name, t in eng._scratch[0].items()}
+    assert shapes == ({} if world == 1 else dict(hist=(4 * 1024,), hits=(4,), own_hits=(4,), cnt=(2 * 1024,)))
+    calls = []
+    eng.C.notify = lambda lay, sessions, args, *rest: calls.append(args[0])
+    eng._stream = lambda stream=None: 0
+    eng.notify([torch.zeros((100, 2), dtype=torch.int64)], [None], 4, cpu_sync=False)
+    assert all((calls[0][name] is None) == (world == 1) for name in ("hist", "hits", "own_hits", "cnt"))
