@@ -8,8 +8,7 @@
 //
 // The copies are bound by the bytes that they write or read, and blocks that the hardware deals out as they finish move them faster
 // than persistent ones (2048 rows of 4096 bf16, top-6 of 64: expand 51 us as one cooperative kernel of 296 blocks with grid barriers
-// between its passes, 6 us of plan and 18 of copies here;
-// aggregate 47 us in 296 blocks that hold sixteen rows at a time, 25 here).
+// between its passes, 6 us of plan and 18 of copies here; aggregate 47 us in 296 blocks that hold sixteen rows at a time, 25 here).
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 

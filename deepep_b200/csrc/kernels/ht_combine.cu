@@ -424,11 +424,11 @@ __global__ void __launch_bounds__(kCombineThreads, 1) ep_combine_local_kernel(co
 // 4096 rows of 7168, top-8 97 / 89 / 94, 8192 of 4096, top-6 114 / 80 / 93, 1531 of 4096, top-6 28 / 20 / 22, 4096 of 4096,
 // top-2 37 / 24 / 36, top-16 123 / 99 / -.  With a single row per token U = 4, B = 1: rank layout, 2048 of 4096, 13.5 / 11.1 as
 // U = 1, B = 3 and 8.7; 4096 of 4096, top-1 30 / 20.5 and 17.2.
-constexpr int kLocalCombineThreads = 256;
-
 //
 // kWeighted (the training layer): every row is multiplied by its weight on the way, the weight and the product rounded to bf16, as if
 // a pass over the rows had done it before; that pass alone reads and writes every row once more.
+constexpr int kLocalCombineThreads = 256;
+
 template <int U, int B, bool kWeighted>
 __global__ void __launch_bounds__(kLocalCombineThreads) ep_combine_items_kernel(const __grid_constant__ CombineParams p) {
   const CombineArgs& a = p.r[0];

@@ -106,8 +106,8 @@ __global__ void __launch_bounds__(kSwigluThreads) row_scale_kernel(const __grid_
 }
 
 // One block per token: the token's gradient is read once and stays in registers, kReturnRows of its rows are in flight at a time.
-// Bound by memory (rows read once, their gradients written once).  49152 rows
-// of 4096, six per token: 140 us in a training step; as a dispatch of the gradient, a product with two outputs and a sum 480 us there.
+// Bound by memory (rows read once, their gradients written once).  49152 rows of 4096, six per token: 140 us in a training step; as a
+// dispatch of the gradient, a product with two outputs and a sum 480 us there.
 constexpr int kReturnRows = 3;
 constexpr int kReturnThreads = 256;
 
