@@ -15,6 +15,7 @@
 #include "kernels/ll_api.h"
 #include "kernels/mega_api.h"
 #include "kernels/ws_layout.h"
+#include "rows.h"
 #include "runtime/fake_cuda.h"
 #include "runtime/session.h"
 
@@ -100,6 +101,7 @@ void op_dispatch(const WsLayout& lay, const std::vector<py::object>& sessions, c
     if (!a.pad_counts != !a.pad_offsets || (a.pad_offsets && a.E < a.ctx.world)) throw std::invalid_argument("dispatch: padding needs the expert counts, offsets and E");
     a.recv_x = ptr<void>(d, "recv_x"); a.recv_sf = ptr<float>(d, "recv_sf");
     a.prof = ptr<unsigned long long>(d, "prof");
+    require_rows(a.T, {a.x}, "dispatch"); require_rows(a.recv_rows, {a.recv_x}, "dispatch");
     // (a rank without tokens, or without received rows, passes empty tensors whose address is null)
     if (!a.send_slot || !a.stage_meta || !a.rank_tokens || !a.rank_rows || (!a.x && a.T > 0))
       throw std::invalid_argument("dispatch: a required pointer is missing");
@@ -140,6 +142,7 @@ void op_combine(const WsLayout& lay, const std::vector<py::object>& sessions, co
     a.prof = ptr<unsigned long long>(d, "prof");
     if (!a.stage_meta || !a.rank_rows || !a.rank_tokens || !a.send_slot || ((!a.topk_idx || !a.out) && a.T > 0))
       throw std::invalid_argument("combine: a required pointer is missing");
+    require_rows(a.x_rows, {a.x}, "combine"); require_rows(a.T, {a.bias0, a.bias1, a.out}, "combine");
     if (p.whole_gpu && lay.world == 1 && a.expand && !a.slot_row && a.T > 0) throw std::invalid_argument("combine: slot_row is missing");
     if (a.row_w && !(p.whole_gpu && lay.world == 1 && n == 1 && a.expand && local_direct && !profile))
       throw std::invalid_argument("combine: rows are weighed by a single rank's kernel only");

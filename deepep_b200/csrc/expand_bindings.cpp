@@ -8,6 +8,7 @@
 
 #include "kernels/expand_api.h"
 #include "kernels/swiglu_api.h"
+#include "rows.h"
 
 namespace py = pybind11;
 using namespace dep;
@@ -94,6 +95,7 @@ void bind_expand(py::module_& m) {
       if ((int)caps.size() != p.L) throw std::invalid_argument("expand needs a capacity per expert");
       for (int e = 0; e < p.L; ++e) p.caps[e] = caps[e].cast<int>();
     }
+    require_rows(p.R, {p.x}, "expand"); require_rows(p.N, {p.out}, "expand");
     if ((p.x_sf == nullptr) != (p.out_sf == nullptr)) throw std::invalid_argument("scales need an input and an output");
     check_launch(launch_expand(p, blocks, reinterpret_cast<cudaStream_t>(stream)), "expand launch");
   });
@@ -107,6 +109,7 @@ void bind_expand(py::module_& m) {
     if (p.H <= 0 || p.H % 8) throw std::invalid_argument("hidden must be a positive multiple of 8");
     if (p.R > 0 && (!p.mapping || !p.out || (p.N > 0 && !p.x))) throw std::invalid_argument("missing tensor");
     if (p.R == 0) return;
+    require_rows(p.N, {p.x}, "aggregate"); require_rows(p.R, {p.out}, "aggregate");
     check_launch(launch_aggregate(p, reinterpret_cast<cudaStream_t>(stream)), "aggregate launch");
   });
 }

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "kernels/gmm_api.h"
+#include "rows.h"
 #include "runtime/session.h"
 
 namespace py = pybind11;
@@ -45,6 +46,8 @@ bool fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session
   if ((gather ? a.rows_in : a.out_rows_cap) > max_rows) throw std::invalid_argument("more rows than the group was sized for");
   if (!a.counts || (a.out_rows_cap > 0 && !a.out) || !a.tile_info || !a.num_tiles || (a.rows_in > 0 && !a.x) || (gather && !a.pulled))
     throw std::invalid_argument("missing tensor");
+  require_rows(a.rows_in, {a.x}, "grouped GEMM"); require_rows(a.out_rows_cap, {a.out}, "grouped GEMM");
+  if (gather) require_rows(a.gathered_cap, {a.gathered}, "grouped GEMM");
   // The single-rank kernel reads x and the weights while it writes the output and the gathered rows, so these must be
   // disjoint from them; the general kernels write only after they have copied what an overlap would destroy.
   const long long L = a.E / a.ctx.world;
@@ -60,8 +63,7 @@ bool fill(GmmArgs& a, const WsLayout& lay, const py::dict& d, py::object session
   const bool local = a.ctx.world == 1 && !overlap(a.out, out_bytes, a.x, x_bytes) && !overlap(a.out, out_bytes, weight, w_bytes) &&
                      !overlap(a.gathered, g_bytes, a.x, x_bytes) && !overlap(a.gathered, g_bytes, weight, w_bytes) &&
                      !overlap(a.gathered, g_bytes, a.out, out_bytes) &&
-                     !overlap(a.counts, c_bytes, a.out, out_bytes) && !overlap(a.counts, c_bytes, a.gathered, g_bytes) &&
-                     ((uintptr_t)a.x | (uintptr_t)a.out | (keep ? (uintptr_t)a.gathered : 0)) % 16 == 0;
+                     !overlap(a.counts, c_bytes, a.out, out_bytes) && !overlap(a.counts, c_bytes, a.gathered, g_bytes);
   const char* err = nullptr;
   const void* a_base = gather && !local ? (const void*)a.gathered : (const void*)a.x;
   const long long a_rows = gather && !local ? (a.gathered ? a.gathered_cap : 0) : a.rows_in;

@@ -7,6 +7,7 @@
 #include <string>
 
 #include "kernels/ll_api.h"
+#include "rows.h"
 #include "runtime/session.h"
 
 namespace py = pybind11;
@@ -52,6 +53,7 @@ void op_ll_dispatch(const WsLayout& lay, const std::vector<py::object>& sessions
     a.mailbox = geti(d, "use_mailbox", 0) ? s.mailbox_device() : nullptr;
     a.capacity = d["capacity"].cast<long long>();
     if (!a.local_row && a.T > 0) throw std::invalid_argument("low-latency dispatch: local_row is missing");
+    require_rows(a.T, {a.x}, "low-latency dispatch"); require_rows(a.capacity, {a.recv_x}, "low-latency dispatch");
     if (a.T < 0 || a.T > lay.max_tokens) throw std::invalid_argument("token count exceeds num_max_tokens_per_rank");
     if (a.E < a.ctx.world || a.E > kMaxExperts || a.E % a.ctx.world) throw std::invalid_argument("num_experts must be a multiple of the world size and at most 1024");
     if (a.mode != 0 && lay.hidden % 128) throw std::invalid_argument("fp8 dispatch needs hidden % 128 == 0");
@@ -76,6 +78,7 @@ void op_ll_combine(const WsLayout& lay, const std::vector<py::object>& sessions,
     a.topk_w = ptr<const float>(d, "topk_w"); a.T = geti(d, "T"); a.E = geti(d, "E"); a.x_rows = geti(d, "x_rows");
     a.out = ptr<__nv_bfloat16>(d, "out"); a.local_row = ptr<const int>(d, "local_row");
     if (!a.local_row && a.T > 0) throw std::invalid_argument("low-latency combine: local_row is missing");
+    require_rows(a.x_rows, {a.x}, "low-latency combine"); require_rows(a.T, {a.out}, "low-latency combine");
   }
   check(launch_ll_combine(p, n, blocks, reinterpret_cast<cudaStream_t>(stream)), "ep_combine_ll launch");
 }

@@ -8,6 +8,7 @@
 #include <string>
 
 #include "kernels/mega_api.h"
+#include "rows.h"
 #include "runtime/session.h"
 
 namespace py = pybind11;
@@ -96,6 +97,7 @@ void fill_route(MegaRouteArgs& a, const py::dict& d, py::object session) {
   if (a.S < 0 || a.K + a.S > kMaxTopk || a.E / a.ctx.world + a.S > kMaxExperts)
     throw std::invalid_argument("top-k plus shared experts must not exceed 16, local plus shared experts 1024");
   if (a.H % 128 || a.E % a.ctx.world || a.E > kMaxExperts) throw std::invalid_argument("hidden % 128 == 0 and experts % world == 0 are required");
+  require_rows(a.T, {a.x_bf16}, "mega_moe");
 }
 
 void fill_finish(MegaFinishArgs& a, const py::dict& d, py::object session) {
@@ -107,6 +109,7 @@ void fill_finish(MegaFinishArgs& a, const py::dict& d, py::object session) {
   a.timer = ptr<unsigned long long>(d, "timer");
   a.expert_rows = ptr<const int>(d, "expert_rows"); a.stats = ptr<int>(d, "stats"); a.stats_set = geti(d, "stats_set", 0);
   if (a.stats && !a.expert_rows) throw std::invalid_argument("statistics need the row counts");
+  require_rows(a.T, {a.y}, "mega_moe");
 }
 
 // One persistent launch for the whole layer: args[i] = {"route": {...}, "gemm1": {...}, "gemm2": {...}, "finish": {...}, "ready": ptr}

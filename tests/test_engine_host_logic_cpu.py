@@ -98,6 +98,72 @@ def test_a_handle_watches_the_tables_that_kernels_read_again():
                 handle._check_unchanged()
 
 
+def test_rows_off_their_boundary_are_refused(monkeypatch):
+    """The kernels read and write rows in pieces of 16 bytes: a tensor that starts between two of them (a slice of a longer one) is
+    refused by every launch, before anything is queued.  Sessions on host-memory doubles of the CUDA entry points."""
+    from deepep_b200.models.mega_moe import MegaEngine, MegaWeights
+    from deepep_b200.ops import ep_gmm_fused as G, load_native
+
+    C = load_native(build_if_missing=True)
+    C.testing_install_fake_cuda(True)
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda device: types.SimpleNamespace(multi_processor_count=148))
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: types.SimpleNamespace(cuda_stream=0, synchronize=lambda: None))
+    cpu, T, H, K, E = torch.device("cpu"), 4, 128, 2, 4
+    rows = lambda n, shift=1, dtype=torch.bfloat16, width=H: torch.zeros((n * width + 8,), dtype=dtype)[shift:shift + n * width].view(n, width)
+    assert rows(T).is_contiguous() and rows(T).data_ptr() % 16 and rows(T, 0).data_ptr() % 16 == 0
+    sessions = []
+
+    def session(layout):
+        sessions.append(C.Session(0, 1, layout.total, 5.0, "ipc"))
+        sessions[-1].attach_peers([sessions[-1].workspace])
+        return [sessions[-1]]
+
+    try:
+        layout = C.make_layout(1, T, H, K, C.ll_region_bytes(1, T, K, H), 0, 0)
+        eng = EC.CudaEngine(session(layout), layout, cpu)
+        idx, w = torch.zeros((T, K), dtype=torch.int64), torch.ones((T, K))
+        ints, views = EC._slab_layout(T, 1, K, T, 4, 1, E, T * K, 0)
+        slab = torch.zeros((ints,), dtype=torch.int32)
+        plan = EC.RoutingPlan(num_tokens=T, num_experts=E, num_topk=K, expand=True, alignment=1, meta_stride=4, num_rows=T * K,
+                              num_staged_rows=T, expert_counts_list=[T * K, 0, 0, 0], topk_idx=idx, recv_w=None, recv_idx=None, slab=slab,
+                              slab_ptr=slab.data_ptr(), views=views)
+        low = EC.RoutingPlan(num_tokens=T, num_experts=E, num_topk=K, expand=True, alignment=1, meta_stride=0, num_rows=T, num_staged_rows=0,
+                             expert_counts_list=None, topk_idx=idx, recv_w=None, recv_idx=None, topk_w=w, local_row_ptr=slab.data_ptr())
+        low.recv_row_src = low.num_rows_dev = slab
+        calls = [lambda: eng.dispatch([rows(T)], [plan], 0), lambda: eng.dispatch([(rows(T, 1, torch.float8_e4m3fn), torch.ones((T, 1)))], [plan], 1),
+                 lambda: eng.combine([rows(T * K)], [plan], [None]),
+                 lambda: eng.combine([rows(T * K, 0)], [plan], [None], bias=[(rows(T, 0), rows(T))]),
+                 lambda: eng.ll_dispatch([rows(T)], [idx], [w], E, 0, cpu_sync=False), lambda: eng.ll_combine([rows(T)], [low])]
+        glayout = C.make_mega_layout(1, 1, H, 1, G.GmmEngine.region_bytes(C, 8, H, H))
+        gmm = G.GmmEngine(session(glayout), glayout, cpu, 8, H, H)
+        weight, counts = torch.zeros((2, H, H), dtype=torch.bfloat16), torch.tensor([2, 2], dtype=torch.int32)
+        calls += [lambda: gmm.a2av_gmm([rows(T)], [weight], [counts], [rows(T, 0)], num_experts=2),
+                  lambda: gmm.a2av_gmm([rows(T, 0)], [weight], [counts], [rows(T, 0)], [rows(T)], num_experts=2),
+                  lambda: gmm.gmm_a2av([rows(T, 0)], [weight], [counts], [rows(T)], num_experts=2)]
+        mlayout = C.make_mega_layout(1, T, 256, K, MegaEngine.mega_bytes(C, T, 256, K))
+        mega = MegaEngine(session(mlayout), mlayout, cpu, E, 128)
+        one = [MegaWeights(torch.zeros((64, 64), dtype=torch.uint8), torch.zeros((512,), dtype=torch.uint8), E, 256, 256)]
+        wide = lambda shift: rows(T, shift, width=256)
+        stream = types.SimpleNamespace(cuda_stream=0)
+        calls += [lambda: mega.forward([wide(1)], [T], one, one, stream), lambda: mega.forward([wide(0)], [T], one, one, stream, x_bf16=[wide(1)])]
+        table = dict(mapping=slab.data_ptr(), rows=T, topk=K, expanded_rows=T)
+        fixed = dict(table, out_sf=None, out_w=None, x_sf=None, topk_idx=None, topk_w=None, expert_offsets=slab.data_ptr(),
+                     actual_counts=slab.data_ptr(), tile_counts=None, err=None, caps=None, experts=E, row_bytes=2 * H, num_sf=0, cached=1)
+        good, bad = rows(T, 0), rows(T)
+        for x, out in ((bad, good), (good, bad)):
+            calls += [lambda x=x, out=out: C.expand(dict(fixed, x=x.data_ptr(), out=out.data_ptr()), 1, 0),
+                      lambda x=x, out=out: C.aggregate(dict(table, x=x.data_ptr(), out=out.data_ptr(), row_w=None, values=None, out_values=None,
+                                                            hidden=H, is_half=0), 0)]
+        for call in calls:
+            with pytest.raises(ValueError, match="16-byte boundary"):
+                call()
+    finally:
+        for s in sessions:
+            s.close()
+        C.testing_restore_cuda()
+        C.testing_clear()
+
+
 def test_status_block_becomes_a_readable_error():
     class Session:
         def __init__(self, **status):
