@@ -579,6 +579,8 @@ class ElasticBuffer:
         for b in biases:
             if b is not None and (tuple(b.shape) != (handle._tokens, self.hidden) or b.dtype != torch.bfloat16):
                 raise ValueError("bias must be bf16 [tokens, hidden]")
+        if any(t is not None and t.is_cuda != self.on_cuda for t in (x, topk_weights, *biases)):
+            raise ValueError("x, topk_weights and bias must live on the buffer's device")
         self._preflight("combine", (self.hidden, plan.expand, topk_weights is not None, bias is not None,
                                     handle.is_low_latency))
         for name, v in (("combine_num_sms", combine_num_sms), ("reduce_num_sms", reduce_num_sms)):
@@ -591,6 +593,10 @@ class ElasticBuffer:
             split = None                      # one kernel role per SM only exists on the high-throughput CUDA path
         comm = self._enter(previous_event, previous_event_before_epilogue)
         allocate_on_comm_stream = self._allocates_on_comm(allocate_on_comm_stream, previous_event, previous_event_before_epilogue)
+        given = [topk_weights, *biases]           # the kernels read them row behind row
+        if any(t is not None and not t.is_contiguous() for t in given):
+            with self._on(comm):
+                topk_weights, *biases = [None if t is None else t.contiguous() for t in given]
         with self._on(comm if allocate_on_comm_stream else None):
             if handle.is_low_latency:
                 if topk_weights is not None or bias is not None:
@@ -601,7 +607,7 @@ class ElasticBuffer:
                                                  blocks=num_sms or self.num_sms, stream=comm,
                                                  **({"split": split} if split is not None else {}),
                                                  **({"row_weights": _row_weights} if _row_weights is not None else {}))[0]
-        event = self._leave(comm, async_with_compute_stream, [out, out_w, x, topk_weights, _row_weights] + [b for b in biases if b is not None],
+        event = self._leave(comm, async_with_compute_stream, [out, out_w, x, _row_weights, topk_weights, *biases, *given],
                             handle, allocate_on_comm_stream)
         return out, out_w, event
 

@@ -107,6 +107,33 @@ def test_high_throughput_calls(buf, expand, alignment):
     _check(buf, event)
 
 
+def test_combine_operands_that_are_not_rows_behind_rows(buf, monkeypatch):
+    """A bias that is one row for all tokens, or strided, and strided weights are copied, on the communication stream: what the kernel
+    gets lies row behind row, and the event holds it and what it was copied from."""
+    x, idx, w = _inputs()
+    rx, _, rw, handle, event = buf.dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E, do_expand=True, do_cpu_sync=False,
+                                            num_max_tokens_per_rank=512, async_with_compute_stream=True)
+    _check(buf, event)
+    where = []
+    monkeypatch.setattr(buf, "_on", lambda comm: (where.append(comm), contextlib.nullcontext())[1])
+    seen = []
+    launch = buf.engine.combine
+    monkeypatch.setattr(buf.engine, "combine", lambda xs, plans, ws, bias=None, **k: (seen.append((ws[0], *bias[0])), launch(xs, plans, ws, bias=bias, **k))[1])
+    one, wide = torch.randn(H).bfloat16(), torch.randn(T, 2 * H).bfloat16()
+    for weights, bias in ((rw, (one.expand(T, H), None)), (rw, (wide[:, ::2], x)), (torch.stack([rw, rw], 1)[:, 0], (x, one.expand(T, H)))):
+        event = buf.combine(rx, handle, topk_weights=weights, bias=bias, async_with_compute_stream=True)[2]
+        for got, want in zip(seen.pop(), (weights, *bias)):
+            assert (got is None) == (want is None)
+            assert got is None or got.is_contiguous() and torch.equal(got.nan_to_num(), want.nan_to_num()) and (got is want) == want.is_contiguous()
+        held = [t for t in event._retained_objects if isinstance(t, torch.Tensor)]
+        assert all(any(t is h for h in held) for t in (weights, *bias) if t is not None) and where[0] is buf.runtime.stream
+        _check(buf, event)
+        where.clear()
+    with pytest.raises(ValueError, match="buffer's device"):
+        monkeypatch.setattr(buf, "on_cuda", True)
+        buf.combine(rx, handle)
+
+
 def test_v1_rank_matrix(buf):
     """The per-rank counts of the V1 handle are added up on the communication stream: kept alive by the event, and not cleared by
     torch on the current stream, which nothing would order before the additions (the launcher clears them)."""

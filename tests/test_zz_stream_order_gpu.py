@@ -74,6 +74,25 @@ def test_v1_token_in_rank_of_an_asynchronous_call(worst):
     buf.destroy()
 
 
+@pytest.mark.parametrize("T", [1, 77])
+def test_combine_operands_that_are_not_rows_behind_rows(T):
+    """One row as the bias of all tokens, a strided bias and strided weights give the bits of their contiguous copies."""
+    import deepep_b200 as deep_ep
+
+    dev, H, E, K = torch.device("cuda"), 256, 8, 3
+    g = torch.Generator().manual_seed(T)
+    x, one, wide = (torch.randn(s, generator=g).bfloat16().to(dev) for s in ((T, H), (H,), (T, 2 * H)))
+    idx, w = make_routes("random", T, E, K, 1, 4).to(dev), make_weights(T, K, 5).to(dev)
+    buf = deep_ep.ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K, explicitly_destroy=True)
+    rx, _, rw, handle, _ = buf.dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E, do_expand=True)
+    strided = torch.stack([rw, -rw], 1)[:, 0]
+    for bias in ((one.expand(T, H), wide[:, ::2]), (wide[:, 1::2], one.expand(T, H))):
+        got = buf.combine(rx, handle, topk_weights=strided, bias=bias)
+        want = buf.combine(rx, handle, topk_weights=rw, bias=tuple(b.contiguous() for b in bias))
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and torch.equal(got[1], w)
+    buf.destroy()
+
+
 def test_two_live_buffers_in_one_process():
     """A prefill buffer and a decode buffer alive at the same time, their calls interleaved (each has its own workspace,
     control block and communication stream); a handle of one is refused by the other.  Parity: the reference's
