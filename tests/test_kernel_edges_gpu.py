@@ -147,7 +147,8 @@ def test_v1_tables_of_several_ranks():
         assert torch.equal(plan.recv_src_idx[:plan.num_rows].cpu().long(), sources)
 
 
-@pytest.mark.parametrize("tokens,experts,topk,world", [(0, 8, 2, 2), (1, 1024, 16, 8), (40000, 24, 5, 1), (16385, 1000, 8, 4)])
+@pytest.mark.parametrize("tokens,experts,topk,world", [(0, 8, 2, 2), (1, 1024, 16, 8), (40000, 24, 5, 1), (16385, 1000, 8, 4), (0, 1024, 16, 8),
+                                                       (1, 512, 16, 8), (511, 64, 6, 1), (2048, 512, 3, 2), (2049, 512, 3, 2), (2048, 513, 8, 1)])
 def test_v1_layout(tokens, experts, topk, world):
     from deepep_b200.ops import load_native
 
