@@ -575,12 +575,14 @@ class ElasticBuffer:
             want = (plan.num_rows,) if plan.expand else (plan.num_rows, self.num_topk)
             if tuple(topk_weights.shape) != want or topk_weights.dtype != torch.float32:
                 raise ValueError(f"topk_weights must be fp32 of shape {want}")
+        if x.is_cuda != self.on_cuda or (topk_weights is not None and topk_weights.is_cuda != self.on_cuda):
+            raise ValueError("x, topk_weights and bias must live on the buffer's device")
         biases = bias if isinstance(bias, (tuple, list)) else (bias, None)
         for b in biases:
             if b is not None and (tuple(b.shape) != (handle._tokens, self.hidden) or b.dtype != torch.bfloat16):
                 raise ValueError("bias must be bf16 [tokens, hidden]")
-        if any(t is not None and t.is_cuda != self.on_cuda for t in (x, topk_weights, *biases)):
-            raise ValueError("x, topk_weights and bias must live on the buffer's device")
+            if b is not None and b.is_cuda != self.on_cuda:
+                raise ValueError("x, topk_weights and bias must live on the buffer's device")
         self._preflight("combine", (self.hidden, plan.expand, topk_weights is not None, bias is not None,
                                     handle.is_low_latency))
         for name, v in (("combine_num_sms", combine_num_sms), ("reduce_num_sms", reduce_num_sms)):
@@ -593,9 +595,11 @@ class ElasticBuffer:
             split = None                      # one kernel role per SM only exists on the high-throughput CUDA path
         comm = self._enter(previous_event, previous_event_before_epilogue)
         allocate_on_comm_stream = self._allocates_on_comm(allocate_on_comm_stream, previous_event, previous_event_before_epilogue)
-        given = [topk_weights, *biases]           # the kernels read them row behind row
-        if any(t is not None and not t.is_contiguous() for t in given):
-            with self._on(comm):
+        given = ()
+        if ((topk_weights is not None and not topk_weights.is_contiguous())
+                or (bias is not None and not all(b is None or b.is_contiguous() for b in biases))):
+            given = (topk_weights, *biases)
+            with self._on(comm):               # the kernels read them row behind row
                 topk_weights, *biases = [None if t is None else t.contiguous() for t in given]
         with self._on(comm if allocate_on_comm_stream else None):
             if handle.is_low_latency:

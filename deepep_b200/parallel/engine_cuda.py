@@ -47,7 +47,7 @@ class CommunicationError(RuntimeError):
 
 class _View:
     """A tensor of a plan that lies in its ``slab``, made when somebody asks for it; the kernels get its address (``_address``).
-    One that no kernel reads again (not ``watched``) counts its changes by itself: they are the owner's business."""
+    Changes of one that no kernel reads again (not ``watched``) are not counted with the others': they are the owner's business."""
 
     def __init__(self, name: str, watched: bool):
         self.name, self.watched = name, watched
@@ -58,8 +58,9 @@ class _View:
         if plan.slab is None:
             return None
         begin, shape = plan.views[self.name]
-        slab = plan.slab if self.watched else plan.slab.data
-        made = slab.as_strided(shape, (shape[1], 1) if len(shape) == 2 else (1,), begin)
+        if plan.unwatched is None and not self.watched:
+            plan.unwatched = plan.slab.data
+        made = (plan.slab if self.watched else plan.unwatched).as_strided(shape, (shape[1], 1) if len(shape) == 2 else (1,), begin)
         plan.__dict__[self.name] = made
         return made
 
@@ -98,6 +99,7 @@ class RoutingPlan:
     token_in_rank: Optional[torch.Tensor] = None      # V1 handle: [T, P], when the caller did not bring it
     slab: Optional[torch.Tensor] = None
     slab_ptr: int = 0
+    unwatched: Optional[torch.Tensor] = None          # the slab under a version counter of its own
     views: Optional[dict] = None        # name -> (first int, shape)
 
     def tensors(self):
